@@ -2,8 +2,9 @@
 // inverse, plus the padded expert-sorted row layout the grouped GEMMs consume.
 //
 // Replaces get_token_indices (reference: src/moe_explore/expert_permute.py:19-41), which runs
-// torch.argsort + torch.histc + torch.cumsum as three or more launches.  Here it is a
-// three-kernel counting sort (the number of distinct keys, E, is small):
+// torch.argsort + torch.histc + torch.cumsum as three or more launches.  Here it is a counting sort (the number of
+// distinct keys, E, is small): one launch of one cluster (route_cluster_kernel) up to kClusterRows rows, and for
+// more rows the chip-wide three-kernel form:
 //   1. chunk_histogram : each warp owns a contiguous chunk of kChunk flat positions and counts
 //                        its ids per expert in shared memory (warp-aggregated via match.any);
 //   2. scan_offsets    : turns the [chunks, E] histogram into per-(chunk, expert) exclusive
@@ -14,8 +15,10 @@
 //                        match.any + popc (which preserves flat-position order) and writes
 //                        perm / row_src / dst_row.
 // All arithmetic is integer; results are bit-exact with torch.sort(stable=True).
-// HBM traffic: 2 x 8R bytes read (ids, twice) + 8R (perm) + 4R (dst_row) + 4RP (row_src) written.
+// HBM traffic: 8R bytes read (ids; twice in the chip-wide form) + 8R (perm) + 4R (dst_row) + 4RP (row_src) written.
 #include "common.cuh"
+
+#include <atomic>
 
 namespace moe {
 
@@ -234,6 +237,246 @@ place_rows_kernel(const int64_t* __restrict__ ids, int64_t R, int E, const int32
   }
 }
 
+// ----------------------------------------------------------------------------------
+// One launch for everything (the usual case): a single cluster of up to 16 CTAs.
+//
+// The work is latency, not bytes (28 bytes per row): histogram, prefix sums and placement used to be a memset and
+// three or four launches, in which one warp walked 1024 positions through 32 dependent match.any / shared-memory
+// steps (27-50 us per layer pass at 4 ... 65536 rows).  Here every lane keeps at most kHeld ids and their ranks in
+// registers, the per-warp counts are scanned in shared memory, the per-CTA counts cross the cluster through
+// distributed shared memory, and the same threads then place their rows: ids are read once, nothing is staged in
+// global memory and there is one launch.  B200, E = 64, us per call in a captured graph, before -> now:
+// 4 rows 24.0 -> 6.1, 8008 rows 31.9 -> 7.2, 65536 rows 35.2 -> 13.3, 131072 rows 34.4 -> 20.8.  From there on the
+// scattered stores of 16 SMs are the limit (the time doubles with the rows) while the chip-wide kernels above stay
+// almost flat (524288 rows: 38.8), hence the line at kClusterRows, which is also what kHeld ids per lane hold.
+// ----------------------------------------------------------------------------------
+constexpr int kRouteThreads = 1024;
+constexpr int kRouteWarps = kRouteThreads / 32;
+constexpr int kMaxCluster = 16;
+constexpr int kHeld = 8;                                                     // ids per lane kept in registers
+constexpr int64_t kClusterRows = int64_t(kMaxCluster) * kRouteThreads * kHeld;  // 131072
+
+struct RouteOut {
+  int32_t* group_indices;
+  int64_t* perm;
+  int32_t* pad_offsets;
+  int32_t* row_src;
+  int32_t* dst_row;
+  int32_t* mtile_expert;
+  int32_t* tile_pairs;
+  int32_t* num_mtiles;
+  int32_t mtiles_bound;
+  int32_t padded_bound;
+};
+
+__device__ __forceinline__ int32_t ld_cluster(const int32_t* p, uint32_t rank) {
+  int32_t v;
+  asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(mapa_shared(smem_u32(p), rank)) : "memory");
+  return v;
+}
+
+__global__ void __launch_bounds__(kRouteThreads)
+route_cluster_kernel(const int64_t* __restrict__ ids, int64_t R, int E, int held, RouteOut out, int32_t* status) {
+  extern __shared__ int32_t route_smem[];
+  int32_t* const warp_cnt = route_smem;                  // [kRouteWarps][E]: counts, then offsets of the warp in the CTA
+  int32_t* const cta_cnt = warp_cnt + kRouteWarps * E;   // [E] rows of this CTA (read by the whole cluster)
+  int32_t* const sh_group = cta_cnt + E;                 // [E]   first sorted position of this CTA's rows of expert e
+  int32_t* const sh_place = sh_group + E;                // [E]   first padded row of this CTA's rows
+  int32_t* const sh_pad = sh_place + E;                  // [E+1] padded row offsets
+  int32_t* const sh_pair = sh_pad + E + 1;               // [E+1] pair prefix
+  int32_t* const sh_end = sh_pair + E + 1;               // [E]   one past the last routed row of expert e (padded rows)
+  __shared__ int32_t sums[3][32];
+  __shared__ int32_t kept;  // rows with a valid id
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int rank = static_cast<int>(cluster_ctarank());
+  const int ctas = gridDim.x;
+  for (int i = tid; i < kRouteWarps * E; i += kRouteThreads) warp_cnt[i] = 0;
+  __syncthreads();
+
+  // 1. count, and rank every id inside its warp's run of 32 * held positions (lanes are in position order: stable)
+  const int64_t begin = (static_cast<int64_t>(rank) * kRouteWarps + warp) * 32 * held + lane;
+  int32_t* const cnt = warp_cnt + warp * E;
+  int key[kHeld];
+  int32_t pos[kHeld];
+  bool bad = false;
+#pragma unroll
+  for (int g = 0; g < kHeld; ++g) {
+    const int64_t j = begin + 32 * g;
+    const bool in = g < held && j < R;
+    const int64_t raw = in ? ids[j] : -1;
+    const bool ok = raw >= 0 && raw < E;
+    bad |= in && !ok;
+    key[g] = ok ? static_cast<int>(raw) : -1 - lane;
+  }
+#pragma unroll
+  for (int g = 0; g < kHeld; ++g) {
+    pos[g] = 0;
+    if (g >= held) break;
+    const unsigned peers = match_key(key[g]);
+    const unsigned before = peers & ((1u << lane) - 1);
+    if (key[g] >= 0) pos[g] = cnt[key[g]] + __popc(before);
+    __syncwarp();
+    if (key[g] >= 0 && before == 0) cnt[key[g]] += __popc(peers);
+    __syncwarp();
+  }
+  if (bad && status != nullptr) atomicCAS(status, 0, DS_BAD_EXPERT_ID);
+  __syncthreads();
+
+  // 2. offsets of the warps inside the CTA (one thread per expert), then of the CTAs inside the cluster
+  const int e = tid;
+  if (e < E) {
+    int32_t run = 0;
+#pragma unroll 8
+    for (int w = 0; w < kRouteWarps; ++w) {
+      const int32_t c = warp_cnt[w * E + e];
+      warp_cnt[w * E + e] = run;
+      run += c;
+    }
+    cta_cnt[e] = run;
+  }
+  cluster_sync_all();
+  int32_t total = 0, before = 0;
+  if (e < E) {
+    for (int c = 0; c < ctas; ++c) {
+      const int32_t v = ld_cluster(cta_cnt + e, static_cast<uint32_t>(c));
+      before += c < rank ? v : 0;
+      total += v;
+    }
+  }
+  // no CTA may exit while another still reads its counts: arrive here, wait at the end
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+
+  // 3. prefix sums over the experts (every CTA for itself): rows, padded rows, row-tile pairs
+  const int32_t padded = (total + MOE_TILE_M - 1) / MOE_TILE_M * MOE_TILE_M;
+  const int32_t pairs = (padded / MOE_TILE_M + 1) / 2;
+  int32_t in_g = total, in_p = padded, in_q = pairs;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const int32_t a = __shfl_up_sync(0xFFFFFFFFu, in_g, off);
+    const int32_t b = __shfl_up_sync(0xFFFFFFFFu, in_p, off);
+    const int32_t c = __shfl_up_sync(0xFFFFFFFFu, in_q, off);
+    if (lane >= off) { in_g += a; in_p += b; in_q += c; }
+  }
+  if (lane == 31) { sums[0][warp] = in_g; sums[1][warp] = in_p; sums[2][warp] = in_q; }
+  __syncthreads();
+  if (warp < 3) {
+    int32_t v = sums[warp][lane];
+    const int32_t own = v;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int32_t a = __shfl_up_sync(0xFFFFFFFFu, v, off);
+      if (lane >= off) v += a;
+    }
+    sums[warp][lane] = v - own;
+  }
+  __syncthreads();
+  if (e < E) {
+    const int32_t g1 = in_g + sums[0][warp], p1 = in_p + sums[1][warp], q1 = in_q + sums[2][warp];
+    sh_group[e] = g1 - total + before;
+    sh_place[e] = p1 - padded + before;
+    sh_pad[e] = p1 - padded;
+    sh_pair[e] = q1 - pairs;
+    sh_end[e] = p1 - padded + total;
+    if (e == E - 1) {
+      sh_pad[E] = p1;
+      sh_pair[E] = q1;
+      kept = g1;
+    }
+    if (rank == 0) {
+      out.group_indices[e + 1] = g1;
+      out.pad_offsets[e + 1] = p1;
+      if (e == 0) { out.group_indices[0] = 0; out.pad_offsets[0] = 0; }
+      if (out.tile_pairs != nullptr) {
+        out.tile_pairs[out.mtiles_bound + e] = q1 - pairs;
+        if (e == E - 1) out.tile_pairs[out.mtiles_bound + E] = q1;
+      }
+      if (out.num_mtiles != nullptr && e == E - 1) {
+        out.num_mtiles[0] = p1 / MOE_TILE_M;
+        out.num_mtiles[1] = q1;
+        out.num_mtiles[2] = out.mtiles_bound;
+        out.num_mtiles[3] = 0;
+      }
+    }
+  }
+  __syncthreads();
+
+  // 4. place this CTA's rows
+#pragma unroll
+  for (int g = 0; g < kHeld; ++g) {
+    const int64_t j = begin + 32 * g;
+    if (g >= held || j >= R) break;
+    if (key[g] >= 0) {
+      const int32_t r = cnt[key[g]] + pos[g];
+      if (out.perm != nullptr) out.perm[sh_group[key[g]] + r] = j;
+      const int32_t p = sh_place[key[g]] + r;
+      if (out.row_src != nullptr) out.row_src[p] = static_cast<int32_t>(j);
+      if (out.dst_row != nullptr) out.dst_row[j] = p;
+    } else if (out.dst_row != nullptr) {
+      out.dst_row[j] = -1;  // id out of range: the row is in no expert's segment; consumers skip negative rows
+    }
+  }
+
+  // 5. what no row wrote: padding rows, the tail of the row map, dropped positions, the tile maps
+  const int gw = rank * kRouteWarps + warp, gws = ctas * kRouteWarps;
+  const int gt = rank * kRouteThreads + tid, gts = ctas * kRouteThreads;
+  if (out.row_src != nullptr) {
+    for (int x = gw; x < E; x += gws)
+      for (int32_t p = sh_end[x] + lane; p < sh_pad[x + 1]; p += 32) out.row_src[p] = -1;
+    for (int32_t p = sh_pad[E] + gt; p < out.padded_bound; p += gts) out.row_src[p] = -1;
+  }
+  if (out.perm != nullptr)
+    for (int64_t r = kept + gt; r < R; r += gts) out.perm[r] = -1;
+  if (out.mtile_expert != nullptr) {
+    const int tiles = sh_pad[E] / MOE_TILE_M;
+    for (int m = gt; m < tiles; m += gts) {
+      int lo = 0, hi = E;  // the expert whose padded rows hold tile m: last one that starts at or before it
+      while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (sh_pad[mid] <= m * MOE_TILE_M) lo = mid; else hi = mid;
+      }
+      out.mtile_expert[m] = lo;
+      const int in_expert = m - sh_pad[lo] / MOE_TILE_M;
+      if (out.tile_pairs != nullptr && (in_expert & 1) == 0)
+        out.tile_pairs[sh_pair[lo] + in_expert / 2] =
+            static_cast<int32_t>(static_cast<uint32_t>(m) | (static_cast<uint32_t>(lo) << 20) |
+                                 ((m + 1) * MOE_TILE_M < sh_pad[lo + 1] ? 0x80000000u : 0u));
+    }
+  }
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+static int route_cluster(const int64_t* ids, int64_t R, int E, const RouteOut& out, int32_t* status, cudaStream_t s) {
+  // as many CTAs as there are 1024-row shares (the scattered stores of the placement are what one SM is slow at)
+  int ctas = 1;
+  while (ctas < kMaxCluster && static_cast<int64_t>(ctas) * kRouteThreads < R) ctas *= 2;
+  const int64_t share = static_cast<int64_t>(ctas) * kRouteThreads;
+  const int held = static_cast<int>((R + share - 1) / share);
+  const size_t smem = (static_cast<size_t>(kRouteWarps) * E + 6 * static_cast<size_t>(E) + 2) * sizeof(int32_t);
+  static std::atomic<bool> ready[64];
+  int dev = 0;
+  MOE_CUDA(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 64 || !ready[dev].load(std::memory_order_acquire)) {
+    MOE_CUDA(cudaFuncSetAttribute(route_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (kRouteWarps + 6) * kMaxExperts * 4 + 8));
+    MOE_CUDA(cudaFuncSetAttribute(route_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    if (dev >= 0 && dev < 64) ready[dev].store(true, std::memory_order_release);
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(ctas), 1, 1);
+  cfg.blockDim = dim3(kRouteThreads, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = static_cast<unsigned>(ctas);
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  MOE_CUDA(cudaLaunchKernelEx(&cfg, route_cluster_kernel, ids, R, E, held, out, status));
+  return MOE_OK;
+}
+
 // Layout from an existing exclusive prefix (rows already grouped): one CTA, thread per expert for
 // the padded prefix, then all threads fill the row maps.
 __global__ void __launch_bounds__(kMaxExperts)
@@ -341,6 +584,12 @@ extern "C" int moe_routing_metadata(const int64_t* expert_idx, int64_t num_rows,
                 "moe_routing_metadata: workspace of %zu bytes is smaller than the %zu required", workspace_bytes,
                 moe_routing_workspace_bytes(num_rows, num_experts));
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (num_rows <= kClusterRows) {
+    const RouteOut out{group_indices, perm, pad_offsets, row_src, dst_row, mtile_expert, tile_pairs, num_mtiles,
+                       static_cast<int32_t>(moe_mtiles_bound(num_rows, num_experts)),
+                       static_cast<int32_t>(moe_padded_rows_bound(num_rows, num_experts))};
+    return route_cluster(expert_idx, num_rows, num_experts, out, status, s);
+  }
   int32_t* chunk_hist = static_cast<int32_t*>(workspace);
   const int64_t chunks = num_chunks(num_rows);
   int32_t* chunk_off = chunk_hist + (chunks > 0 ? chunks : 1) * num_experts;

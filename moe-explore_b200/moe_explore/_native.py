@@ -20,6 +20,7 @@ MOE_DTYPE_BF16 = 0
 MOE_DTYPE_F16 = 1
 ACT_CODES = {None: 0, "none": 0, "silu": 1, "gelu": 2, "swiglu": 3, "geglu": 4, "approx_gelu": 5}
 TILE_M = 128
+ROUTE_ONE_LAUNCH_ROWS = 131072   # csrc/routing.cu: up to here the routing metadata is one launch
 # codes a kernel may leave in a status word (include/moe_sm100.h, moe_check_status)
 STATUS_WAVE_FALLBACK = 4
 STATUS_BAD_LAYOUT = 5
@@ -219,7 +220,7 @@ def routing_metadata(expert_idx, num_experts, group_indices, perm, pad_offsets, 
                                      _ptr(workspace),
                                      workspace.numel() * workspace.element_size(), _stream())
     _check("moe_routing_metadata", rc)
-    _count(3 if expert_idx.numel() > 0 else 1)
+    _count(1 if expert_idx.numel() <= ROUTE_ONE_LAUNCH_ROWS else 3)
 
 
 def routing_metadata_static(expert_idx, num_experts, group_indices, perm, pad_offsets, row_src, dst_row, mtile_expert,
@@ -232,7 +233,7 @@ def routing_metadata_static(expert_idx, num_experts, group_indices, perm, pad_of
                                             _ptr(mtile_expert), _ptr(tile_pairs), _ptr(num_mtiles), _ptr(status),
                                             _stream())
     _check("moe_routing_metadata_static", rc)
-    _count(3 if expert_idx.numel() > 0 else 1)
+    _count(1 if expert_idx.numel() <= ROUTE_ONE_LAUNCH_ROWS else 3)
 
 
 def routing_workspace_bytes(num_rows: int, num_experts: int) -> int:
