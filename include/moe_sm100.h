@@ -177,6 +177,11 @@ int moe_dispatch_rows(const void* src, const int32_t* dst_row, const int32_t* ro
                       const int32_t* num_mtiles, void* dst, int64_t num_tokens, int topk,
                       int64_t padded_rows, int cols, int dtype, void* stream);
 
+/* The same without the padding rows, which keep whatever dst held: for passes in which no contraction runs over the rows
+ * (a forward pass without gradients: rows do not mix, and nobody reads the padding rows of its results). */
+int moe_dispatch_rows_only(const void* src, const int32_t* dst_row, void* dst, int64_t num_tokens,
+                           int topk, int cols, int dtype, void* stream);
+
 /* Expert-parallel dispatch as a pull: dst[p, :] = scale[p] * peer_bases[src_rank[p]][src_row[p], :]
  * for padded rows p < 128*num_mtiles, zeros where src_rank[p] < 0.  peer_bases is a DEVICE array with
  * one base pointer per rank of the node (peer-mapped buffers of [*, cols] rows, e.g. symmetric memory);
@@ -214,6 +219,11 @@ int moe_zero_padding_rows(const int32_t* row_src, const int32_t* num_mtiles, voi
 int moe_unpad_rows(const void* src, const int32_t* dst_row, void* out, int64_t num_rows,
                    int cols, int dtype, void* stream);
 
+/* out[r, :] = src[index[r] / div, :] with int64 indices (the permutation moe_routing_metadata writes), zeros where
+ * index[r] < 0. */
+int moe_index_rows(const void* src, const int64_t* index, void* out, int64_t num_rows, int div,
+                   int cols, int dtype, void* stream);
+
 /* out[t, :] = sum_s scale(t,s) * ys[dst_row[t*topk+s], :], fp32 accumulation, one rounding.
  * scores: [T, topk] in `dtype`, or NULL for scale 1 (used for dX). */
 int moe_combine_topk(const void* ys, const void* scores, const int32_t* dst_row, void* out,
@@ -227,6 +237,13 @@ int moe_combine_bwd(const void* dout, const void* scores, const void* ys,
                     const int32_t* row_src, const int32_t* num_mtiles, void* gs, void* dscores,
                     int64_t num_tokens, int topk, int64_t padded_rows, int cols, int dtype,
                     void* stream);
+
+/* The same result walked in token order (p = dst_row[j]), which reads every dout row once; dscores of a dropped slot
+ * (dst_row[j] < 0) is 0, so dscores [T, topk] is written completely. */
+int moe_combine_bwd_tokens(const void* dout, const void* scores, const void* ys,
+                           const int32_t* dst_row, const int32_t* row_src, const int32_t* num_mtiles,
+                           void* gs, void* dscores, int64_t num_tokens, int topk, int cols, int dtype,
+                           void* stream);
 
 /* ---------------------------------------------------------------------------------
  * (b),(c),(d) Grouped GEMMs on tcgen05 tensor cores (TMA operand tiles, TMEM accumulators,

@@ -11,19 +11,57 @@ namespace moe {
 
 constexpr int kRowThreads = 256;
 
-// dst[p, :] = src[row_src[p] / div, :], zeros for padding rows.  One CTA per padded row.
+// How the threads of a CTA are spread over rows: TPR consecutive threads move one row and 256 / TPR rows are under way in a
+// CTA, so narrow rows do not leave lanes idle.  Every thread has four independent 16-byte loads in flight before its
+// first store: with one load per thread (one CTA per row) these kernels were bound by the latency of index -> load ->
+// store.  B200, 65536 rows of 4 KB, one load -> four: gather 71.7 -> 61.5 us, dispatch 70.6 -> 65.6; 14 KB rows 286 -> 262,
+// 238 -> 231.
+constexpr int kRowLoads = 4;
+
+// dst[r, :] = src[index[r] / div, :], zeros where index[r] < 0.  `num_mtiles` (nullable): only the first
+// 128 * num_mtiles[0] rows are in use.
+template <typename Index, int TPR>
 __global__ void __launch_bounds__(kRowThreads)
-gather_rows_kernel(const uint4* __restrict__ src, const int32_t* __restrict__ row_src,
-                   const int32_t* __restrict__ num_mtiles, uint4* __restrict__ dst, int vec_per_row, int div) {
-  const int64_t rows_in_use = static_cast<int64_t>(*num_mtiles) * MOE_TILE_M;
-  for (int64_t p = blockIdx.x; p < rows_in_use; p += gridDim.x) {
-    const int32_t j = row_src[p];
-    uint4* d = dst + p * vec_per_row;
-    if (j < 0) {
-      for (int v = threadIdx.x; v < vec_per_row; v += kRowThreads) d[v] = make_uint4(0, 0, 0, 0);
-    } else {
-      const uint4* s = src + static_cast<int64_t>(j / div) * vec_per_row;
-      for (int v = threadIdx.x; v < vec_per_row; v += kRowThreads) d[v] = s[v];
+copy_rows_kernel(const uint4* __restrict__ src, const Index* __restrict__ index, const int32_t* __restrict__ num_mtiles,
+                 uint4* __restrict__ dst, int64_t rows, int vec_per_row, int div) {
+  constexpr int kRows = kRowThreads / TPR;
+  if (num_mtiles != nullptr) {
+    const int64_t in_use = static_cast<int64_t>(*num_mtiles) * MOE_TILE_M;
+    rows = in_use < rows ? in_use : rows;
+  }
+  const int lane = threadIdx.x % TPR;
+  for (int64_t r = static_cast<int64_t>(blockIdx.x) * kRows + threadIdx.x / TPR; r < rows;
+       r += static_cast<int64_t>(gridDim.x) * kRows) {
+    const int32_t j = static_cast<int32_t>(index[r]);
+    const uint4* s = src + static_cast<int64_t>(j / div) * vec_per_row;
+    uint4* d = dst + r * vec_per_row;
+    for (int v0 = lane; v0 < vec_per_row; v0 += TPR * kRowLoads) {
+      uint4 u[kRowLoads];
+#pragma unroll
+      for (int i = 0; i < kRowLoads; ++i) {
+        const int v = v0 + i * TPR;
+        u[i] = (j >= 0 && v < vec_per_row) ? s[v] : make_uint4(0, 0, 0, 0);
+      }
+#pragma unroll
+      for (int i = 0; i < kRowLoads; ++i)
+        if (v0 + i * TPR < vec_per_row) d[v0 + i * TPR] = u[i];
+    }
+  }
+}
+
+// Zeroes the padding rows (row_src < 0) among the rows in use: a warp looks at 32 rows at a time (one load and a ballot;
+// a load per row made this the longest part of a dispatch) and clears the ones it finds.
+__device__ __forceinline__ void zero_padding(const int32_t* __restrict__ row_src, const int32_t* __restrict__ num_mtiles,
+                                             uint4* __restrict__ dst, int vec_per_row, int warp, int warps) {
+  const int64_t rows_in_use = static_cast<int64_t>(*num_mtiles) * MOE_TILE_M;  // a multiple of 32
+  const int lane = threadIdx.x & 31;
+  for (int64_t p0 = static_cast<int64_t>(warp) * 32; p0 < rows_in_use; p0 += static_cast<int64_t>(warps) * 32) {
+    unsigned pads = __ballot_sync(0xFFFFFFFFu, row_src[p0 + lane] < 0);
+    while (pads != 0) {
+      const int b = __ffs(pads) - 1;
+      pads &= pads - 1;
+      uint4* d = dst + (p0 + b) * vec_per_row;
+      for (int v = lane; v < vec_per_row; v += 32) d[v] = make_uint4(0, 0, 0, 0);
     }
   }
 }
@@ -32,32 +70,35 @@ gather_rows_kernel(const uint4* __restrict__ src, const int32_t* __restrict__ ro
 // Every token row is read from HBM once and written topk times (the row-major gather re-reads it topk
 // times, and the tokens of an expert are scattered over the whole input).  The second part of the grid
 // zeroes the padding rows.
+template <int TPR>
 __global__ void __launch_bounds__(kRowThreads)
 dispatch_rows_kernel(const uint4* __restrict__ src, const int32_t* __restrict__ dst_row,
                      const int32_t* __restrict__ row_src, const int32_t* __restrict__ num_mtiles,
                      uint4* __restrict__ dst, int64_t num_tokens, int topk, int vec_per_row, int token_blocks) {
-  if (static_cast<int>(blockIdx.x) < token_blocks) {
-    for (int64_t t = blockIdx.x; t < num_tokens; t += token_blocks) {
-      const uint4* s = src + t * vec_per_row;
-      const int32_t* rows = dst_row + t * topk;
-      for (int v = threadIdx.x; v < vec_per_row; v += kRowThreads) {
-        const uint4 u = s[v];
-        for (int k = 0; k < topk; ++k) {
-          const int32_t p = rows[k];  // negative: the routing metadata dropped this (token, slot)
-          if (p >= 0) dst[static_cast<int64_t>(p) * vec_per_row + v] = u;
-        }
+  constexpr int kRows = kRowThreads / TPR;
+  if (static_cast<int>(blockIdx.x) >= token_blocks) {
+    zero_padding(row_src, num_mtiles, dst, vec_per_row, (blockIdx.x - token_blocks) * (kRowThreads / 32) + (threadIdx.x >> 5),
+                 (gridDim.x - token_blocks) * (kRowThreads / 32));
+    return;
+  }
+  const int lane = threadIdx.x % TPR;
+  for (int64_t t = static_cast<int64_t>(blockIdx.x) * kRows + threadIdx.x / TPR; t < num_tokens;
+       t += static_cast<int64_t>(token_blocks) * kRows) {
+    const uint4* s = src + t * vec_per_row;
+    const int32_t* rows = dst_row + t * topk;
+    for (int v0 = lane; v0 < vec_per_row; v0 += TPR * kRowLoads) {
+      uint4 u[kRowLoads];
+#pragma unroll
+      for (int i = 0; i < kRowLoads; ++i)
+        u[i] = v0 + i * TPR < vec_per_row ? s[v0 + i * TPR] : make_uint4(0, 0, 0, 0);
+      for (int k = 0; k < topk; ++k) {
+        const int32_t p = rows[k];  // negative: the routing metadata dropped this (token, slot)
+        if (p < 0) continue;
+        uint4* d = dst + static_cast<int64_t>(p) * vec_per_row;
+#pragma unroll
+        for (int i = 0; i < kRowLoads; ++i)
+          if (v0 + i * TPR < vec_per_row) d[v0 + i * TPR] = u[i];
       }
-    }
-  } else {
-    // padding rows: one warp per row, only rows whose row_src is negative
-    const int64_t rows_in_use = static_cast<int64_t>(*num_mtiles) * MOE_TILE_M;
-    const int warps = (gridDim.x - token_blocks) * (kRowThreads / 32);
-    const int warp = (blockIdx.x - token_blocks) * (kRowThreads / 32) + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    for (int64_t p = warp; p < rows_in_use; p += warps) {
-      if (row_src[p] >= 0) continue;
-      uint4* d = dst + p * vec_per_row;
-      for (int v = lane; v < vec_per_row; v += 32) d[v] = make_uint4(0, 0, 0, 0);
     }
   }
 }
@@ -258,22 +299,6 @@ pull_rows_bulk_kernel(const uint4* const* __restrict__ bases, const int32_t* __r
   if (lane == 0) bulk_wait_all();
 }
 
-// out[j, :] = src[dst_row[j], :]
-__global__ void __launch_bounds__(kRowThreads)
-unpad_rows_kernel(const uint4* __restrict__ src, const int32_t* __restrict__ dst_row, uint4* __restrict__ out,
-                  int64_t num_rows, int vec_per_row) {
-  for (int64_t j = blockIdx.x; j < num_rows; j += gridDim.x) {
-    const int32_t p = dst_row[j];
-    uint4* d = out + j * vec_per_row;
-    if (p < 0) {  // no source row (dropped by the routing metadata): zeros
-      for (int v = threadIdx.x; v < vec_per_row; v += kRowThreads) d[v] = make_uint4(0, 0, 0, 0);
-      continue;
-    }
-    const uint4* s = src + static_cast<int64_t>(p) * vec_per_row;
-    for (int v = threadIdx.x; v < vec_per_row; v += kRowThreads) d[v] = s[v];
-  }
-}
-
 template <typename T>
 __device__ __forceinline__ void fma8(float (&acc)[8], const uint4& u, float scale) {
   const uint32_t w[4] = {u.x, u.y, u.z, u.w};
@@ -286,20 +311,31 @@ __device__ __forceinline__ void fma8(float (&acc)[8], const uint4& u, float scal
 }
 
 // out[t, :] = sum_s scale(t, s) * ys[dst_row[t*topk + s], :]
-template <typename T>
+// HBM-bound (each slot's row read once, one row written).  The loads of up to SLOTS slots are issued together -- a loop over
+// the slots keeps one in flight per thread -- and added in slot order.  B200, 8 slots, 8192 tokens: 14 KB rows
+// 221 -> 172 us (4.8 -> 6.1 TB/s), 4 KB rows 72 -> 61; 1001 tokens 18.5 -> 14.4; 4 slots, 16384 tokens of 4 KB 77 -> 65.
+template <typename T, int TPR, int SLOTS>
 __global__ void __launch_bounds__(kRowThreads)
 combine_topk_kernel(const uint4* __restrict__ ys, const T* __restrict__ scores, const int32_t* __restrict__ dst_row,
                     uint4* __restrict__ out, int64_t num_tokens, int topk, int vec_per_row) {
-  for (int64_t t = blockIdx.x; t < num_tokens; t += gridDim.x) {
-    for (int v = threadIdx.x; v < vec_per_row; v += kRowThreads) {
+  constexpr int kRows = kRowThreads / TPR;
+  const int lane = threadIdx.x % TPR;
+  for (int64_t t = static_cast<int64_t>(blockIdx.x) * kRows + threadIdx.x / TPR; t < num_tokens;
+       t += static_cast<int64_t>(gridDim.x) * kRows) {
+    for (int v = lane; v < vec_per_row; v += TPR) {
       float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-      for (int s = 0; s < topk; ++s) {
-        const int64_t j = t * topk + s;
-        const int32_t p = dst_row[j];
-        if (p < 0) continue;  // slot dropped by the routing metadata: contributes nothing
-        const float scale = scores != nullptr ? Elem<T>::to_float(scores[j]) : 1.0f;
-        const uint4 u = ys[static_cast<int64_t>(p) * vec_per_row + v];
-        fma8<T>(acc, u, scale);
+      for (int s0 = 0; s0 < topk; s0 += SLOTS) {
+        uint4 u[SLOTS];
+        float scale[SLOTS];
+#pragma unroll
+        for (int i = 0; i < SLOTS; ++i) {
+          const int64_t j = t * topk + s0 + i;
+          const int32_t p = s0 + i < topk ? dst_row[j] : -1;  // negative: slot dropped by the routing metadata
+          scale[i] = p < 0 ? 0.0f : (scores != nullptr ? Elem<T>::to_float(scores[j]) : 1.0f);
+          u[i] = p < 0 ? make_uint4(0, 0, 0, 0) : ys[static_cast<int64_t>(p) * vec_per_row + v];
+        }
+#pragma unroll
+        for (int i = 0; i < SLOTS; ++i) fma8<T>(acc, u[i], scale[i]);
       }
       uint4 r;
       r.x = Elem<T>::pack2(acc[0], acc[1]);
@@ -308,6 +344,65 @@ combine_topk_kernel(const uint4* __restrict__ ys, const T* __restrict__ scores, 
       r.w = Elem<T>::pack2(acc[6], acc[7]);
       out[t * vec_per_row + v] = r;
     }
+  }
+}
+
+// One warp's share of the backward fold: gs row = scale * dout row (unless gs is null), and the dot product of the dout and
+// ys rows (complete in every lane).
+template <typename T>
+__device__ __forceinline__ float combine_bwd_row(const uint4* __restrict__ d, const uint4* __restrict__ y, uint4* __restrict__ g,
+                                                 float scale, int vec_per_row, int lane) {
+  float dot = 0.0f;
+  for (int v = lane; v < vec_per_row; v += 32) {
+    const uint4 du = d[v];
+    const uint4 yu = y[v];
+    const uint32_t dw[4] = {du.x, du.y, du.z, du.w};
+    const uint32_t yw[4] = {yu.x, yu.y, yu.z, yu.w};
+    uint32_t ow[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 df = Elem<T>::unpack2(dw[i]);
+      const float2 yf = Elem<T>::unpack2(yw[i]);
+      dot = fmaf(df.x, yf.x, dot);
+      dot = fmaf(df.y, yf.y, dot);
+      ow[i] = Elem<T>::pack2(scale * df.x, scale * df.y);
+    }
+    if (g != nullptr) g[v] = make_uint4(ow[0], ow[1], ow[2], ow[3]);
+  }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) dot += __shfl_xor_sync(0xFFFFFFFFu, dot, off);
+  return dot;
+}
+
+// The backward fold in token order: a warp per (token, slot) j, p = dst_row[j]:
+//   gs[p, :] = scores[j] * dout[j / topk, :];  dscores[j] = dot(dout[j / topk, :], ys[p, :]), 0 for a dropped slot (p < 0).
+// The warps of a CTA take consecutive j, so a dout row is fetched once and its other slots find it in L1; walking the
+// padded rows instead (combine_bwd_kernel) fetches it topk times, from all over the tensor.  The second part of the
+// grid zeroes the padding rows of gs.  B200: 16384 tokens x 4 slots of 4 KB 127 -> 107 us, 8192 x 8 of 14 KB 430 -> 339,
+// 128 x 8 of 4 KB 16.4 -> 12.5.
+template <typename T>
+__global__ void __launch_bounds__(kRowThreads)
+combine_bwd_tokens_kernel(const uint4* __restrict__ dout, const T* __restrict__ scores, const uint4* __restrict__ ys,
+                          const int32_t* __restrict__ dst_row, const int32_t* __restrict__ row_src,
+                          const int32_t* __restrict__ num_mtiles, uint4* __restrict__ gs, T* __restrict__ dscores,
+                          int64_t num_slots, int topk, int vec_per_row, int slot_blocks) {
+  constexpr int kWarps = kRowThreads / 32;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (static_cast<int>(blockIdx.x) >= slot_blocks) {
+    zero_padding(row_src, num_mtiles, gs, vec_per_row, (blockIdx.x - slot_blocks) * kWarps + warp,
+                 (gridDim.x - slot_blocks) * kWarps);
+    return;
+  }
+  for (int64_t j = static_cast<int64_t>(blockIdx.x) * kWarps + warp; j < num_slots;
+       j += static_cast<int64_t>(slot_blocks) * kWarps) {
+    const int32_t p = dst_row[j];
+    float dot = 0.0f;
+    if (p >= 0) {
+      const int64_t row = static_cast<int64_t>(p) * vec_per_row;
+      dot = combine_bwd_row<T>(dout + (j / topk) * vec_per_row, ys + row, gs + row, Elem<T>::to_float(scores[j]), vec_per_row,
+                               lane);
+    }
+    if (lane == 0) dscores[j] = Elem<T>::from_float(dot);
   }
 }
 
@@ -330,28 +425,8 @@ combine_bwd_kernel(const uint4* __restrict__ dout, const T* __restrict__ scores,
         for (int v = lane; v < vec_per_row; v += 32) g[v] = make_uint4(0, 0, 0, 0);
       continue;
     }
-    const float scale = Elem<T>::to_float(scores[j]);
-    const uint4* d = dout + static_cast<int64_t>(j / topk) * vec_per_row;
-    const uint4* y = ys + p * vec_per_row;
-    float dot = 0.0f;
-    for (int v = lane; v < vec_per_row; v += 32) {
-      const uint4 du = d[v];
-      const uint4 yu = y[v];
-      const uint32_t dw[4] = {du.x, du.y, du.z, du.w};
-      const uint32_t yw[4] = {yu.x, yu.y, yu.z, yu.w};
-      uint32_t ow[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float2 df = Elem<T>::unpack2(dw[i]);
-        const float2 yf = Elem<T>::unpack2(yw[i]);
-        dot = fmaf(df.x, yf.x, dot);
-        dot = fmaf(df.y, yf.y, dot);
-        ow[i] = Elem<T>::pack2(scale * df.x, scale * df.y);
-      }
-      if (g != nullptr) g[v] = make_uint4(ow[0], ow[1], ow[2], ow[3]);
-    }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) dot += __shfl_xor_sync(0xFFFFFFFFu, dot, off);
+    const float dot = combine_bwd_row<T>(dout + static_cast<int64_t>(j / topk) * vec_per_row, ys + p * vec_per_row, g,
+                                         Elem<T>::to_float(scores[j]), vec_per_row, lane);
     if (lane == 0) dscores[j] = Elem<T>::from_float(dot);
   }
 }
@@ -371,19 +446,71 @@ __global__ void store_words_to_host_kernel(const unsigned long long* __restrict_
 __global__ void __launch_bounds__(kRowThreads)
 zero_padding_rows_kernel(const int32_t* __restrict__ row_src, const int32_t* __restrict__ num_mtiles, uint4* __restrict__ dst,
                          int vec_per_row) {
-  const int64_t rows_in_use = static_cast<int64_t>(*num_mtiles) * MOE_TILE_M;
-  const int warps = gridDim.x * (kRowThreads / 32);
-  const int lane = threadIdx.x & 31;
-  for (int64_t p = blockIdx.x * (kRowThreads / 32) + (threadIdx.x >> 5); p < rows_in_use; p += warps) {
-    if (row_src[p] >= 0) continue;
-    uint4* d = dst + p * vec_per_row;
-    for (int v = lane; v < vec_per_row; v += 32) d[v] = make_uint4(0, 0, 0, 0);
-  }
+  zero_padding(row_src, num_mtiles, dst, vec_per_row, blockIdx.x * (kRowThreads / 32) + (threadIdx.x >> 5),
+               gridDim.x * (kRowThreads / 32));
 }
 
 static int row_grid(int64_t rows) {
   const int64_t cap = static_cast<int64_t>(sm_count()) * 16;
   return static_cast<int>(rows < cap ? (rows > 0 ? rows : 1) : cap);
+}
+
+// Threads per row of the kernels above.  Copies: 64 (four loads each cover 4 KB; wider splits leave lanes idle at the end
+// of a row, narrower ones measured 5-10 % slower at 14 KB rows), 32 for rows of at most 1 KB.  The fold has one column
+// vector per thread and its loads spread over the slots: 128 keep enough loads in flight when there are few tokens (128
+// tokens x 8 slots: 10.2 us against 12.3 with 64), narrow rows take fewer.
+static int copy_threads_per_row(int vec_per_row) { return vec_per_row <= 64 ? 32 : 64; }
+static int fold_threads_per_row(int vec_per_row) { return vec_per_row <= 32 ? 32 : (vec_per_row <= 64 ? 64 : 128); }
+
+template <typename Index>
+static void launch_copy_rows(const void* src, const Index* index, const int32_t* num_mtiles, void* dst, int64_t rows,
+                             int vec_per_row, int div, cudaStream_t s) {
+  const int tpr = copy_threads_per_row(vec_per_row);
+  // one CTA per group of rows (no cap): 61.5 us against 67.6 with 16 CTAs per SM looping (65536 rows of 4 KB)
+  const int64_t groups = (rows + kRowThreads / tpr - 1) / (kRowThreads / tpr);
+  const int grid = static_cast<int>(groups < (1 << 30) ? (groups > 0 ? groups : 1) : (1 << 30));
+  const uint4* in = static_cast<const uint4*>(src);
+  uint4* out = static_cast<uint4*>(dst);
+  if (tpr == 32) copy_rows_kernel<Index, 32><<<grid, kRowThreads, 0, s>>>(in, index, num_mtiles, out, rows, vec_per_row, div);
+  else copy_rows_kernel<Index, 64><<<grid, kRowThreads, 0, s>>>(in, index, num_mtiles, out, rows, vec_per_row, div);
+}
+
+// row_src == nullptr: the padding rows are left as they are.
+static void launch_dispatch(const void* src, const int32_t* dst_row, const int32_t* row_src, const int32_t* num_mtiles, void* dst,
+                            int64_t num_tokens, int topk, int vec_per_row, cudaStream_t s) {
+  const int tpr = copy_threads_per_row(vec_per_row);
+  const int64_t groups = (num_tokens + kRowThreads / tpr - 1) / (kRowThreads / tpr);
+  const int token_blocks = static_cast<int>(groups < (1 << 30) ? groups : (1 << 30));
+  const int blocks = token_blocks + (row_src != nullptr ? sm_count() : 0);
+  const uint4* in = static_cast<const uint4*>(src);
+  uint4* out = static_cast<uint4*>(dst);
+  if (tpr == 32) dispatch_rows_kernel<32><<<blocks, kRowThreads, 0, s>>>(in, dst_row, row_src, num_mtiles, out, num_tokens, topk, vec_per_row, token_blocks);
+  else dispatch_rows_kernel<64><<<blocks, kRowThreads, 0, s>>>(in, dst_row, row_src, num_mtiles, out, num_tokens, topk, vec_per_row, token_blocks);
+}
+
+// The slots whose loads are issued together: the smallest power of two that covers topk, at most 8 (a wider one wastes
+// predicated loads: 2 slots with 8, 59 us; with 2 or 4, 47).
+template <typename T, int TPR>
+static void launch_combine_slots(const uint4* ys, const T* scores, const int32_t* dst_row, uint4* out, int64_t num_tokens,
+                                 int topk, int vec_per_row, cudaStream_t s) {
+  const int grid = row_grid((num_tokens + kRowThreads / TPR - 1) / (kRowThreads / TPR));
+  if (topk == 1) combine_topk_kernel<T, TPR, 1><<<grid, kRowThreads, 0, s>>>(ys, scores, dst_row, out, num_tokens, topk, vec_per_row);
+  else if (topk == 2) combine_topk_kernel<T, TPR, 2><<<grid, kRowThreads, 0, s>>>(ys, scores, dst_row, out, num_tokens, topk, vec_per_row);
+  else if (topk <= 4) combine_topk_kernel<T, TPR, 4><<<grid, kRowThreads, 0, s>>>(ys, scores, dst_row, out, num_tokens, topk, vec_per_row);
+  else combine_topk_kernel<T, TPR, 8><<<grid, kRowThreads, 0, s>>>(ys, scores, dst_row, out, num_tokens, topk, vec_per_row);
+}
+
+template <typename T>
+static void launch_combine(const void* ys, const void* scores, const int32_t* dst_row, void* out, int64_t num_tokens, int topk,
+                           int vec_per_row, cudaStream_t s) {
+  const uint4* in = static_cast<const uint4*>(ys);
+  const T* sc = static_cast<const T*>(scores);
+  uint4* o = static_cast<uint4*>(out);
+  switch (fold_threads_per_row(vec_per_row)) {
+    case 32: return launch_combine_slots<T, 32>(in, sc, dst_row, o, num_tokens, topk, vec_per_row, s);
+    case 64: return launch_combine_slots<T, 64>(in, sc, dst_row, o, num_tokens, topk, vec_per_row, s);
+    default: return launch_combine_slots<T, 128>(in, sc, dst_row, o, num_tokens, topk, vec_per_row, s);
+  }
 }
 
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
@@ -446,8 +573,7 @@ extern "C" int moe_gather_rows(const void* src, int64_t src_rows, const int32_t*
   MOE_CHECK_ARG(aligned16(src) && aligned16(dst), "moe_gather_rows: pointers must be 16-byte aligned");
   MOE_CHECK_ARG(src_rows >= 0 && padded_rows > 0 && div > 0, "moe_gather_rows: bad sizes");
   MOE_ROW_COMMON_CHECKS("moe_gather_rows", cols, dtype);
-  gather_rows_kernel<<<row_grid(padded_rows), kRowThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const uint4*>(src), row_src, num_mtiles, static_cast<uint4*>(dst), cols / 8, div);
+  launch_copy_rows(src, row_src, num_mtiles, dst, padded_rows, cols / 8, div, static_cast<cudaStream_t>(stream));
   MOE_CUDA(cudaGetLastError());
   return MOE_OK;
 }
@@ -459,11 +585,19 @@ extern "C" int moe_dispatch_rows(const void* src, const int32_t* dst_row, const 
   MOE_CHECK_ARG(src && dst_row && row_src && num_mtiles && dst, "moe_dispatch_rows: null pointer argument");
   MOE_CHECK_ARG(aligned16(src) && aligned16(dst), "moe_dispatch_rows: pointers must be 16-byte aligned");
   MOE_ROW_COMMON_CHECKS("moe_dispatch_rows", cols, dtype);
-  const int token_blocks = row_grid(num_tokens);
-  const int pad_blocks = sm_count();
-  dispatch_rows_kernel<<<token_blocks + pad_blocks, kRowThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const uint4*>(src), dst_row, row_src, num_mtiles, static_cast<uint4*>(dst), num_tokens, topk, cols / 8,
-      token_blocks);
+  launch_dispatch(src, dst_row, row_src, num_mtiles, dst, num_tokens, topk, cols / 8, static_cast<cudaStream_t>(stream));
+  MOE_CUDA(cudaGetLastError());
+  return MOE_OK;
+}
+
+extern "C" int moe_dispatch_rows_only(const void* src, const int32_t* dst_row, void* dst, int64_t num_tokens, int topk,
+                                      int cols, int dtype, void* stream) {
+  MOE_CHECK_ARG(num_tokens >= 0 && topk > 0, "moe_dispatch_rows_only: bad sizes");
+  MOE_CHECK_ARG(src && dst_row && dst, "moe_dispatch_rows_only: null pointer argument");
+  MOE_CHECK_ARG(aligned16(src) && aligned16(dst), "moe_dispatch_rows_only: pointers must be 16-byte aligned");
+  MOE_ROW_COMMON_CHECKS("moe_dispatch_rows_only", cols, dtype);
+  if (num_tokens == 0) return MOE_OK;
+  launch_dispatch(src, dst_row, nullptr, nullptr, dst, num_tokens, topk, cols / 8, static_cast<cudaStream_t>(stream));
   MOE_CUDA(cudaGetLastError());
   return MOE_OK;
 }
@@ -549,8 +683,19 @@ extern "C" int moe_unpad_rows(const void* src, const int32_t* dst_row, void* out
   MOE_CHECK_ARG(src && dst_row && out, "moe_unpad_rows: null pointer argument");
   MOE_CHECK_ARG(aligned16(src) && aligned16(out), "moe_unpad_rows: pointers must be 16-byte aligned");
   MOE_ROW_COMMON_CHECKS("moe_unpad_rows", cols, dtype);
-  unpad_rows_kernel<<<row_grid(num_rows), kRowThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const uint4*>(src), dst_row, static_cast<uint4*>(out), num_rows, cols / 8);
+  launch_copy_rows(src, dst_row, nullptr, out, num_rows, cols / 8, 1, static_cast<cudaStream_t>(stream));
+  MOE_CUDA(cudaGetLastError());
+  return MOE_OK;
+}
+
+extern "C" int moe_index_rows(const void* src, const int64_t* index, void* out, int64_t num_rows, int div, int cols, int dtype,
+                              void* stream) {
+  MOE_CHECK_ARG(num_rows >= 0 && div > 0, "moe_index_rows: bad sizes");
+  if (num_rows == 0) return MOE_OK;
+  MOE_CHECK_ARG(src && index && out, "moe_index_rows: null pointer argument");
+  MOE_CHECK_ARG(aligned16(src) && aligned16(out), "moe_index_rows: pointers must be 16-byte aligned");
+  MOE_ROW_COMMON_CHECKS("moe_index_rows", cols, dtype);
+  launch_copy_rows(src, index, nullptr, out, num_rows, cols / 8, div, static_cast<cudaStream_t>(stream));
   MOE_CUDA(cudaGetLastError());
   return MOE_OK;
 }
@@ -563,15 +708,32 @@ extern "C" int moe_combine_topk(const void* ys, const void* scores, const int32_
   MOE_CHECK_ARG(aligned16(ys) && aligned16(out), "moe_combine_topk: pointers must be 16-byte aligned");
   MOE_ROW_COMMON_CHECKS("moe_combine_topk", cols, dtype);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const int grid = row_grid(num_tokens);
+  if (dtype == MOE_DTYPE_BF16) launch_combine<__nv_bfloat16>(ys, scores, dst_row, out, num_tokens, topk, cols / 8, s);
+  else launch_combine<__half>(ys, scores, dst_row, out, num_tokens, topk, cols / 8, s);
+  MOE_CUDA(cudaGetLastError());
+  return MOE_OK;
+}
+
+extern "C" int moe_combine_bwd_tokens(const void* dout, const void* scores, const void* ys, const int32_t* dst_row,
+                                      const int32_t* row_src, const int32_t* num_mtiles, void* gs, void* dscores,
+                                      int64_t num_tokens, int topk, int cols, int dtype, void* stream) {
+  MOE_CHECK_ARG(dout && scores && ys && dst_row && row_src && num_mtiles && gs && dscores,
+                "moe_combine_bwd_tokens: null pointer argument");
+  MOE_CHECK_ARG(aligned16(dout) && aligned16(ys) && aligned16(gs), "moe_combine_bwd_tokens: pointers must be 16-byte aligned");
+  MOE_CHECK_ARG(num_tokens >= 0 && topk > 0, "moe_combine_bwd_tokens: bad sizes");
+  MOE_ROW_COMMON_CHECKS("moe_combine_bwd_tokens", cols, dtype);
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const int64_t slots = num_tokens * topk;
+  const int slot_blocks = row_grid((slots + kRowThreads / 32 - 1) / (kRowThreads / 32));
+  const int blocks = slot_blocks + sm_count();
   if (dtype == MOE_DTYPE_BF16) {
-    combine_topk_kernel<__nv_bfloat16><<<grid, kRowThreads, 0, s>>>(
-        static_cast<const uint4*>(ys), static_cast<const __nv_bfloat16*>(scores), dst_row, static_cast<uint4*>(out),
-        num_tokens, topk, cols / 8);
+    combine_bwd_tokens_kernel<__nv_bfloat16><<<blocks, kRowThreads, 0, s>>>(
+        static_cast<const uint4*>(dout), static_cast<const __nv_bfloat16*>(scores), static_cast<const uint4*>(ys), dst_row,
+        row_src, num_mtiles, static_cast<uint4*>(gs), static_cast<__nv_bfloat16*>(dscores), slots, topk, cols / 8, slot_blocks);
   } else {
-    combine_topk_kernel<__half><<<grid, kRowThreads, 0, s>>>(static_cast<const uint4*>(ys),
-                                                             static_cast<const __half*>(scores), dst_row,
-                                                             static_cast<uint4*>(out), num_tokens, topk, cols / 8);
+    combine_bwd_tokens_kernel<__half><<<blocks, kRowThreads, 0, s>>>(
+        static_cast<const uint4*>(dout), static_cast<const __half*>(scores), static_cast<const uint4*>(ys), dst_row, row_src,
+        num_mtiles, static_cast<uint4*>(gs), static_cast<__half*>(dscores), slots, topk, cols / 8, slot_blocks);
   }
   MOE_CUDA(cudaGetLastError());
   return MOE_OK;

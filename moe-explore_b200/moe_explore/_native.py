@@ -59,9 +59,12 @@ SIGNATURES = {
     "moe_gather_rows_peer": (c_int, [c_void_p] * 6 + [c_int, c_int, c_int, c_int, c_int, c_void_p, c_int64, c_int, c_int,
                                      c_int, c_int, c_void_p, c_void_p]),
     "moe_unpad_rows": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int, c_void_p]),
+    "moe_index_rows": (c_int, [c_void_p] * 3 + [c_int64, c_int, c_int, c_int, c_void_p]),
     "moe_combine_topk": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int, c_int, c_void_p]),
     "moe_combine_bwd": (c_int, [c_void_p] * 7 + [c_int64, c_int, c_int64, c_int, c_int, c_void_p]),
     "moe_dispatch_rows": (c_int, [c_void_p] * 5 + [c_int64, c_int, c_int64, c_int, c_int, c_void_p]),
+    "moe_dispatch_rows_only": (c_int, [c_void_p] * 3 + [c_int64, c_int, c_int, c_int, c_void_p]),
+    "moe_combine_bwd_tokens": (c_int, [c_void_p] * 8 + [c_int64, c_int, c_int, c_int, c_void_p]),
     "moe_mgrouped_gemm": (c_int, [c_void_p] * 7 + [c_int64, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, _OPT,
                                   c_void_p, c_void_p]),
     "moe_mgrouped_gemm_gather": (c_int, [c_void_p, c_int64, c_void_p, c_int] + [c_void_p] * 6 +
@@ -367,6 +370,17 @@ def unpad_rows(src, dst_row, out):
     _count(1)
 
 
+def index_rows(src, index, out, div=1):
+    """out[r] = src[index[r] // div] for int64 indices, zeros where index[r] < 0."""
+    require_cuda(src, index, out)
+    assert index.dtype is torch.int64
+    with timed("rows:gather"):
+        rc = load().moe_index_rows(_ptr(src), _ptr(index), _ptr(out), out.size(0), div, out.size(1), dtype_code(src.dtype),
+                                   _stream())
+    _check("moe_index_rows", rc)
+    _count(1)
+
+
 def combine_topk(ys, scores, dst_row, out, topk):
     require_cuda(ys, out)
     with timed("rows:combine"):
@@ -383,6 +397,27 @@ def dispatch_rows(src, dst_row, row_src, num_mtiles, dst, topk):
         rc = load().moe_dispatch_rows(_ptr(src), _ptr(dst_row), _ptr(row_src), _ptr(num_mtiles), _ptr(dst), src.size(0),
                                       topk, dst.size(0), src.size(1), dtype_code(src.dtype), _stream())
     _check("moe_dispatch_rows", rc)
+    _count(1)
+
+
+def dispatch_rows_only(src, dst_row, dst, topk):
+    """dst[dst_row[t*topk+s]] = src[t]; the padding rows of dst are left as they are."""
+    require_cuda(src, dst)
+    with timed("rows:gather"):
+        rc = load().moe_dispatch_rows_only(_ptr(src), _ptr(dst_row), _ptr(dst), src.size(0), topk, src.size(1),
+                                           dtype_code(src.dtype), _stream())
+    _check("moe_dispatch_rows_only", rc)
+    _count(1)
+
+
+def combine_bwd_tokens(dout, scores, ys, dst_row, row_src, num_mtiles, gs, dscores, topk):
+    """``combine_bwd`` in token order; writes every element of ``dscores`` (0 for dropped slots)."""
+    require_cuda(dout, ys, dscores)
+    with timed("rows:combine_bwd"):
+        rc = load().moe_combine_bwd_tokens(_ptr(dout), _ptr(scores), _ptr(ys), _ptr(dst_row), _ptr(row_src),
+                                           _ptr(num_mtiles), _ptr(gs), _ptr(dscores), dout.size(0), topk, dout.size(1),
+                                           dtype_code(dout.dtype), _stream())
+    _check("moe_combine_bwd_tokens", rc)
     _count(1)
 
 

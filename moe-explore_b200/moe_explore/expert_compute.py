@@ -81,8 +81,8 @@ class ExpertCompute(torch.autograd.Function):
         new = lambda *shape: torch.empty(*shape, dtype=grad_out.dtype, device=grad_out.device)
 
         gs = new(rp, d)
-        d_scores = torch.zeros(T, plan.topk, dtype=grad_out.dtype, device=grad_out.device)  # dropped slots keep 0
-        _native.combine_bwd(grad_out, scores, ys, plan.row_src, plan.num_mtiles, gs, d_scores, plan.topk)
+        d_scores = new(T, plan.topk)
+        _native.combine_bwd_tokens(grad_out, scores, ys, plan.dst_row, plan.row_src, plan.num_mtiles, gs, d_scores, plan.topk)
         d_pre = new(rp, weight1.size(2))
         if act is None:     # linear "activation": d_pre = gs @ W2^T
             _native.mgrouped_gemm(gs, weight2, d_pre, None, plan.mtile_expert, plan.tile_pairs, plan.num_mtiles, True, None,

@@ -1,0 +1,84 @@
+"""Row kernels at the edges of their thread splits: row widths around 32 / 64 / 128 sixteen-byte pieces, slot counts around the
+powers of two their loads are grouped by, one to a few hundred tokens, dropped slots."""
+import pytest
+import torch
+
+from moe_explore.expert_permute import expert_input_permute, expert_output_permute
+from moe_explore.routing_plan import build_routing_plan
+
+pytestmark = pytest.mark.gpu
+
+WIDTHS = [8, 256, 264, 512, 520, 1024, 1032, 2056, 7168]
+
+
+def _case(T, k, cols, E=7, dtype=torch.bfloat16):
+    g = torch.Generator(device="cuda").manual_seed(T * 1000 + k * 100 + cols)
+    idx = torch.stack([torch.randperm(max(E, k), generator=g, device="cuda")[:k] for _ in range(T)])
+    if T > 2:
+        idx[T // 2, 0] = 10_000   # out of range: dropped by the routing metadata
+    plan = build_routing_plan(idx, max(E, k), k)
+    plan.status.zero_()
+    mk = lambda *s: torch.randn(*s, generator=g, device="cuda").to(dtype)
+    return plan, mk(T, cols), mk(T, k), mk(plan.padded_rows, cols)
+
+
+@pytest.mark.parametrize("cols", WIDTHS)
+@pytest.mark.parametrize("T,k", [(1, 1), (3, 2), (33, 3), (130, 4), (7, 5), (129, 8), (5, 9)])
+def test_rows_against_torch(T, k, cols, native):
+    plan, x, scores, ys = _case(T, k, cols)
+    dst = plan.dst_row.long()
+    live = dst >= 0
+    rows = int(plan.num_mtiles[0]) * 128
+    # dispatch: copies, so exact; padding rows zero, or untouched
+    expect = torch.zeros(plan.padded_rows, cols, dtype=x.dtype, device="cuda")
+    expect[dst[live]] = x.repeat_interleave(k, 0)[live]
+    xs = torch.full_like(expect, 7.0)
+    native.dispatch_rows(x, plan.dst_row, plan.row_src, plan.num_mtiles, xs, k)
+    assert torch.equal(xs[:rows], expect[:rows]) and bool((xs[rows:] == 7).all())
+    only = torch.full_like(expect, 7.0)
+    native.dispatch_rows_only(x, plan.dst_row, only, k)
+    pads = plan.row_src[:rows] < 0
+    assert torch.equal(only[:rows][~pads], expect[:rows][~pads]) and bool((only[:rows][pads] == 7).all())
+    # gathers
+    again = torch.full_like(expect, 7.0)
+    native.gather_rows(x, plan.row_src, plan.num_mtiles, again, k)
+    assert torch.equal(again[:rows], expect[:rows]) and bool((again[rows:] == 7).all())
+    out = torch.empty(T * k, cols, dtype=x.dtype, device="cuda")
+    native.unpad_rows(ys, plan.dst_row, out)
+    assert torch.equal(out, torch.where(live[:, None], ys[dst.clamp_min(0)], torch.zeros_like(out)))
+    native.index_rows(x, plan.perm, out, div=k)
+    assert torch.equal(out, torch.where(plan.perm[:, None] >= 0, x[plan.perm.clamp_min(0) // k], torch.zeros_like(out)))
+    # folds: fp32 sums of exact products, one rounding (half a unit in the last place of 8 bits; sums differ in order by
+    # k * 2^-24 of the sum of magnitudes)
+    picked = torch.where(live[:, None], ys[dst.clamp_min(0)], torch.zeros_like(out)).float().view(T, k, cols)
+    for s in (scores, None):
+        terms = picked if s is None else picked * s.float()[..., None]
+        fold = torch.empty(T, cols, dtype=x.dtype, device="cuda")
+        native.combine_topk(ys, s, plan.dst_row, fold, k)
+        bound = terms.sum(1).abs() * 2.0 ** -8 + k * 2.0 ** -23 * terms.abs().sum(1)
+        assert bool(((fold.float() - terms.sum(1)).abs() <= bound).all())
+    # backward fold: the token-order kernel is the padded-order kernel bit for bit, and zero where a slot was dropped
+    gs, gs2 = torch.full_like(ys, 7.0), torch.full_like(ys, 7.0)
+    ds, ds2 = torch.full_like(scores, 7.0), torch.zeros_like(scores)
+    native.combine_bwd_tokens(x, scores, ys, plan.dst_row, plan.row_src, plan.num_mtiles, gs, ds, k)
+    native.combine_bwd(x, scores, ys, plan.row_src, plan.num_mtiles, gs2, ds2, k)
+    assert torch.equal(gs, gs2) and torch.equal(ds, ds2)
+
+
+@pytest.mark.parametrize("T,k,cols", [(1, 1, 8), (65, 3, 520), (700, 8, 2048)])
+def test_permute_round_trip_with_and_without_a_score_gradient(T, k, cols, native):
+    g = torch.Generator(device="cuda").manual_seed(T)
+    x = torch.randn(T, cols, generator=g, device="cuda").bfloat16()
+    idx = torch.stack([torch.randperm(16, generator=g, device="cuda")[:k] for _ in range(T)])
+    scores = torch.rand(T, k, generator=g, device="cuda").bfloat16()
+    grouped = expert_input_permute(x, idx, 16, k)
+    order = torch.sort(idx.reshape(-1), stable=True).indices
+    assert torch.equal(grouped.indices, order) and torch.equal(grouped.tokens, x[order // k])
+    out = expert_output_permute(grouped, scores, k, x.shape)
+    leaf = scores.clone().requires_grad_()
+    out_grad = expert_output_permute(grouped, leaf, k, x.shape)   # through the un-permuted copy
+    assert torch.equal(out, out_grad) and not out.requires_grad
+    out_grad.backward(x)
+    ref = (x.float()[:, None, :] * x.float()[:, None, :].expand(T, k, cols)).sum(-1)
+    # fp32 sum of `cols` products, rounded once to bf16
+    assert bool(((leaf.grad.float() - ref).abs() <= ref.abs() * 2.0 ** -8 + cols * 2.0 ** -23 * ref.abs()).all())
