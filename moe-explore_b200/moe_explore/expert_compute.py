@@ -42,14 +42,17 @@ class ExpertCompute(torch.autograd.Function):
         hidden = new(rp, inter)
         # the un-activated product, needed by the backward pass (not kept for inference or without an activation)
         keep = act is not None and needs_grad
-        pre_act = new(rp, n1) if (is_glu(act) or keep) else None
+        pre_act = new(rp, n1) if keep else None
         if gather_in_gemm:
             xs = None
             _native.mgrouped_gemm_gather(x, plan.row_src, plan.topk, weight1, hidden, pre_act, plan.mtile_expert,
                                          plan.tile_pairs, plan.num_mtiles, rp, act, plan.status, rows=plan.num_rows)
         else:
             xs = new(rp, d)
-            _native.dispatch_rows(x, plan.dst_row, plan.row_src, plan.num_mtiles, xs, plan.topk)
+            if needs_grad:
+                _native.dispatch_rows(x, plan.dst_row, plan.row_src, plan.num_mtiles, xs, plan.topk)
+            else:   # rows do not mix in a forward pass, and only a weight gradient would contract over the padding rows
+                _native.dispatch_rows_only(x, plan.dst_row, xs, plan.topk)
             _native.mgrouped_gemm(xs, weight1, hidden, pre_act, plan.mtile_expert, plan.tile_pairs, plan.num_mtiles, False,
                                   act, plan.status, rows=plan.num_rows)
         if fused_combine and not needs_grad:
