@@ -400,7 +400,16 @@ template <> __device__ __forceinline__ void red_add_v8<__half>(void* ptr, const 
 }
 
 // Activation math (fp32).
-__device__ __forceinline__ float sigmoidf_fast(float x) { return 1.0f / (1.0f + __expf(-x)); }
+// 1 / y for y >= 1: the hardware's approximation and one Newton step, without the range checks and the slow-path branch of a
+// division.  The branch kept the compiler from interleaving the elements of an epilogue row, which with two warps per
+// scheduler is the whole speed of the gated epilogues.  y is capped below infinity (1 / inf would turn into inf * 0).
+__device__ __forceinline__ float reciprocal_ge1(float y) {
+  y = fminf(y, 3.0e38f);
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(y));
+  return fmaf(r, fmaf(-y, r, 1.0f), r);
+}
+__device__ __forceinline__ float sigmoidf_fast(float x) { return reciprocal_ge1(1.0f + __expf(-x)); }
 __device__ __forceinline__ float silu_f(float x) { return x * sigmoidf_fast(x); }
 __device__ __forceinline__ float gelu_f(float x) { return 0.5f * x * (1.0f + erff(x * 0.70710678118654752f)); }
 // tanh form: 0.5 x (1 + tanh(sqrt(2/pi) (x + 0.044715 x^3)))

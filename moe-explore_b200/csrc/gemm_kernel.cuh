@@ -171,9 +171,9 @@ __device__ __forceinline__ constexpr uint32_t make_idesc() {
 }
 
 // Shared-memory plan: [operand stages][epilogue staging][barriers].  The staging area holds, per epilogue warp,
-// swizzled 32-row x 128-byte tiles: one for the plain-store and GLU epilogues, two for the dGLU epilogue (the
-// saved product of the next chunk lands in one while the other is computed on and stored from), which costs the
-// dGLU kernels one operand stage.
+// swizzled 32-row x 128-byte tiles: one for the plain-store and GLU epilogues, two for the dGLU and the ungated AUX
+// epilogues (the saved product of the next chunk lands in one while the other is computed on and stored from; or the
+// un-activated and the activated product are stored side by side), which costs those kernels one operand stage.
 template <int BN, int CTAS, int EPI>
 struct SmemPlan {
   static constexpr int kABytes = BM * BK * 2;
@@ -181,7 +181,7 @@ struct SmemPlan {
   static constexpr int kBBytes = kBCols * BK * 2;
   static constexpr int kStageBytes = kABytes + kBBytes;
   static constexpr int kStagingTile = 32 * 128;
-  static constexpr int kTilesPerWarp = EPI == EPI_DGLU ? 2 : 1;
+  static constexpr int kTilesPerWarp = (EPI == EPI_DGLU || EPI == EPI_ACT_AUX) ? 2 : 1;
   static constexpr int kStagingBytes = kEpilogueWarps * kTilesPerWarp * kStagingTile;
   static constexpr int kBarrierBytes = 512;
   static constexpr int kBudget = 232448 - 1024 - kBarrierBytes - kStagingBytes;  // 227 KB minus alignment slack
@@ -359,11 +359,70 @@ __device__ __forceinline__ uint4 pack8(const float* v) {
   return r;
 }
 
-__device__ __forceinline__ float act_plain(float x, int act) {
-  return act == MOE_ACT_SILU ? silu_f(x) : (act == MOE_ACT_GELU ? gelu_f(x) : gelu_tanh_f(x));
+// Element-wise activation of a register row, and its derivative as a factor.  The choice is made once per row: inside the
+// element loop its branches kept the elements from being interleaved.
+__device__ __forceinline__ void apply_act(float (&v)[32], int act) {
+  if (act == MOE_ACT_SILU) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = silu_f(v[i]);
+  } else if (act == MOE_ACT_GELU) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = gelu_f(v[i]);
+  } else if (act != MOE_ACT_NONE) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = gelu_tanh_f(v[i]);
+  }
 }
-__device__ __forceinline__ float dact_plain(float x, int act) {
-  return act == MOE_ACT_SILU ? dsilu_f(x) : (act == MOE_ACT_GELU ? dgelu_f(x) : dgelu_tanh_f(x));
+template <typename T>
+__device__ __forceinline__ void mul_dact(float (&v)[32], const uint4 (&pre)[4], int act) {
+  float x[32];
+#pragma unroll
+  for (int qq = 0; qq < 4; ++qq) {
+    const uint32_t w[4] = {pre[qq].x, pre[qq].y, pre[qq].z, pre[qq].w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 f = Elem<T>::unpack2(w[i]);
+      x[qq * 8 + 2 * i] = f.x;
+      x[qq * 8 + 2 * i + 1] = f.y;
+    }
+  }
+  if (act == MOE_ACT_SILU) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] *= dsilu_f(x[i]);
+  } else if (act == MOE_ACT_GELU) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] *= dgelu_f(x[i]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] *= dgelu_tanh_f(x[i]);
+  }
+}
+
+// Gated backward of one register row: da = gradient of the activated value, h = the saved (gate, up) pairs, replaced by
+// (d_gate, d_up).
+template <typename T, bool GEGLU>
+__device__ __forceinline__ void dglu_row(const float (&da)[32], uint4 (&h)[8]) {
+#pragma unroll
+  for (int qq = 0; qq < 8; ++qq) {  // 8 elements = 4 (gate, up) pairs per 16 bytes
+    const uint32_t hw[4] = {h[qq].x, h[qq].y, h[qq].z, h[qq].w};
+    float o[8];
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+      const float2 gu = Elem<T>::unpack2(hw[p]);
+      float act_g, dact_g;
+      if (GEGLU) {
+        act_g = gelu_f(gu.x);
+        dact_g = dgelu_f(gu.x);
+      } else {
+        const float sg = sigmoidf_fast(gu.x);
+        act_g = gu.x * sg;
+        dact_g = sg * (1.0f + gu.x * (1.0f - sg));
+      }
+      o[2 * p] = da[qq * 4 + p] * gu.y * dact_g;
+      o[2 * p + 1] = da[qq * 4 + p] * act_g;
+    }
+    h[qq] = pack8<T>(o);
+  }
 }
 
 // Source rows of four consecutive padded rows, as the gather4 copy wants them: row_src / div, or `oob` (a row
@@ -379,7 +438,8 @@ __device__ __forceinline__ int4 gather_rows4(const int32_t* row_src, int first, 
 }
 
 // tmap_a / tmap_b: the operands.  tmap_c / tmap_d (EPI_DGLU): the saved product and the output, both
-// [rows, 2N] with a {64 columns, 32 rows} box.  tmap_d (EPI_ACT with out_tma): the output, [rows, N] or
+// [rows, 2N] with a {64 columns, 32 rows} box; EPI_ACT_AUX: the un-activated product (saved or read) and the output, both
+// [rows, N], same box.  tmap_d (EPI_ACT with out_tma): the output, [rows, N] or
 // [E, M, N], same box.
 template <typename T, int BN, bool A_K, bool B_K, int EPI, bool KG, int CTAS, bool GATHER>
 __global__ void __launch_bounds__(kThreads, 1)
@@ -430,8 +490,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     mbar_fence_init();
     tma_prefetch_desc(&tmap_a);
     tma_prefetch_desc(&tmap_b);
-    if (EPI == EPI_DGLU) tma_prefetch_desc(&tmap_c);
-    if (EPI == EPI_DGLU || (EPI == EPI_ACT && args.out_tma)) tma_prefetch_desc(&tmap_d);
+    if (EPI == EPI_DGLU || EPI == EPI_ACT_AUX) tma_prefetch_desc(&tmap_c);
+    if (EPI == EPI_DGLU || EPI == EPI_ACT_AUX || (EPI == EPI_ACT && args.out_tma)) tma_prefetch_desc(&tmap_d);
   }
   if (warp == 1) {
     if (kPair) {
@@ -691,7 +751,6 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     uint32_t acc_phase = 0;
     T* out = reinterpret_cast<T*>(args.out);
     T* aux_out = reinterpret_cast<T*>(args.aux_out);
-    const T* aux_in = reinterpret_cast<const T*>(args.aux_in);
     const int N = args.n_dim;
     const uint32_t tempty_leader = kPair ? mapa_shared(tempty_bar, 0) : tempty_bar;
     // this warp's staging tile(s): 32 rows x 128 bytes, 16-byte pieces XOR-swizzled by (row % 8), i.e. the layout
@@ -741,7 +800,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         }
       }
       const long long warp_row0 = static_cast<long long>(c.m0) + quad * 32;
-      if (EPI == EPI_DGLU) {
+      const bool side_input = EPI == EPI_DGLU || (EPI == EPI_ACT_AUX && args.aux_in != nullptr);
+      if (side_input) {
         // The saved product does not depend on the accumulator: request the first chunk's tile before waiting
         // for the MMAs.  The buffer it lands in was last read by the store issued two chunks ago.
         const int col0 = c.n0 + chunk_begin * 32;
@@ -749,7 +809,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
           bulk_wait_read_all();
           const uint32_t bar = my_epi_bar + 8 * (q & 1);
           mbar_arrive_expect_tx(bar, Plan::kStagingTile);
-          tma_load_2d_plain(stage_base + (q & 1) * Plan::kStagingTile, &tmap_c, 2 * col0, static_cast<int>(warp_row0), bar);
+          tma_load_2d_plain(stage_base + (q & 1) * Plan::kStagingTile, &tmap_c, EPI == EPI_DGLU ? 2 * col0 : col0,
+                            static_cast<int>(warp_row0), bar);
         }
         __syncwarp();
       }
@@ -758,105 +819,158 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         tc_fence_after();
       }
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + acc * BN;
-      if (EPI == EPI_ACT || EPI == EPI_ACT_AUX) {
+      if (EPI == EPI_ACT) {
         // Plain store (optionally with an activation, optionally into another GPU's buffer, optionally scaled and
         // added into token-order rows): two 32-column chunks at a time go through the swizzled shared-memory tile so
         // that every store instruction of the warp writes four 128-byte row segments instead of 32 scattered
         // 16-byte pieces.
-        // EPI_ACT_AUX with aux_out: pass 0 stores the un-activated product there, pass 1 the activated one
-        // into out.  EPI_ACT_AUX with aux_in: one pass, accumulator * act'(saved product).
         const unsigned long long my_base = reinterpret_cast<unsigned long long>(row_out + out_row * N);
-        const bool two_outputs = EPI == EPI_ACT_AUX && aux_out != nullptr;
-        const unsigned long long my_aux = two_outputs ? reinterpret_cast<unsigned long long>(aux_out + out_row * N) : 0ull;
-        const int first_pass = two_outputs ? 0 : 1;
-        const bool accumulate = EPI == EPI_ACT && !KG && args.combine_row_src != nullptr;
+        const bool accumulate = !KG && args.combine_row_src != nullptr;
         // Without a row map the 32-row x 64-column piece this warp has staged leaves as ONE bulk tensor store (the copy
         // engine clips it at the edges of the matrix) instead of eight 16-byte stores per lane; the staging tile is
         // written again only after that store has read it.
-        const bool tma_out = EPI == EPI_ACT && args.out_tma != 0;
+        const bool tma_out = args.out_tma != 0;
         const bool tile_stored = KG ? (c.m0 + quad * 32 < args.m_dim) : c.active;
 #pragma unroll 1
         for (int chunk = chunk_begin; chunk < chunk_begin + kChunksPerWarp; chunk += 2) {
+#pragma unroll
+          for (int hc = 0; hc < 2; ++hc) {
+            float v[32];
+            if (have_acc) {
+              uint32_t raw[32];
+              tmem_ld_32x32(taddr + (chunk + hc) * 32, raw);
+              tmem_ld_wait();
+#pragma unroll
+              for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(raw[i]);
+            } else {
+#pragma unroll
+              for (int i = 0; i < 32; ++i) v[i] = 0.0f;
+            }
+            apply_act(v, args.act);
+            if (accumulate) {
+#pragma unroll
+              for (int i = 0; i < 32; ++i) v[i] *= row_scale;
+            }
+            if (tma_out && hc == 0) {
+              if (lane == 0) bulk_wait_read_all();  // the previous round's store has read the staging tile
+              __syncwarp();
+            }
+#pragma unroll
+            for (int qq = 0; qq < 4; ++qq) {
+              const uint4 u = pack8<T>(v + qq * 8);
+              const uint32_t addr = stage_base + lane * 128 + (((hc * 4 + qq) ^ (lane & 7)) << 4);
+              asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(u.x), "r"(u.y), "r"(u.z), "r"(u.w)
+                           : "memory");
+            }
+          }
+          const int col_pair0 = c.n0 + chunk * 32;  // first of the 64 columns staged
+          if (tma_out) {
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0 && tile_stored && col_pair0 < N) {
+              if (KG) tma_store_3d(&tmap_d, col_pair0, c.m0 + quad * 32, c.expert, stage_base);
+              else tma_store_2d(&tmap_d, col_pair0, static_cast<int>(warp_row0), stage_base);
+              bulk_commit();
+            }
+            continue;
+          }
+          __syncwarp();
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const int r = j * 4 + co_row;  // row of the warp's 32 this lane writes in this step
+            const unsigned long long base = __shfl_sync(0xFFFFFFFFu, my_base, r);
+            const int ok = __shfl_sync(0xFFFFFFFFu, row_ok ? 1 : 0, r);
+            uint4 u;
+            const uint32_t addr = stage_base + r * 128 + ((co_ck ^ (r & 7)) << 4);
+            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(u.x), "=r"(u.y), "=r"(u.z), "=r"(u.w) : "r"(addr));
+            const int col = col_pair0 + co_ck * 8;
+            if (ok && col < N) {
+              if (accumulate) red_add_v8<T>(reinterpret_cast<T*>(base) + col, u);
+              else *reinterpret_cast<uint4*>(reinterpret_cast<T*>(base) + col) = u;
+            }
+          }
+          __syncwarp();
+        }
+      } else if (EPI == EPI_ACT_AUX) {
+        // Ungated experts in training, 64 columns per round, moved by tensor copies of the warp's 32-row tiles:
+        // with aux_out the un-activated and the activated product leave from one tile each; with aux_in the saved
+        // product comes in one round ahead (as in the dGLU epilogue) and the row is replaced in place.  The accumulator is
+        // read once.
+        bool failed = false;
 #pragma unroll 1
-          for (int pass = first_pass; pass < 2; ++pass) {
-#pragma unroll
-            for (int hc = 0; hc < 2; ++hc) {
-              float v[32];
-              if (have_acc) {
-                uint32_t raw[32];
-                tmem_ld_32x32(taddr + (chunk + hc) * 32, raw);
-                tmem_ld_wait();
-#pragma unroll
-                for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(raw[i]);
-              } else {
-#pragma unroll
-                for (int i = 0; i < 32; ++i) v[i] = 0.0f;
+        for (int chunk = chunk_begin; chunk < chunk_begin + kChunksPerWarp; chunk += 2) {
+          const int col0 = c.n0 + chunk * 32;
+          const bool live = c.active && col0 < N;  // uniform over the warp
+          const uint32_t buf = side_input ? stage_base + (q & 1) * Plan::kStagingTile : stage_base;
+          if (side_input) {
+            if (live) {
+              const int ncol0 = col0 + 64;
+              if (chunk + 2 < chunk_begin + kChunksPerWarp && ncol0 < N && lane == 0) {
+                bulk_wait_read_all();
+                const uint32_t nbar = my_epi_bar + 8 * ((q + 1) & 1);
+                mbar_arrive_expect_tx(nbar, Plan::kStagingTile);
+                tma_load_2d_plain(stage_base + ((q + 1) & 1) * Plan::kStagingTile, &tmap_c, ncol0,
+                                  static_cast<int>(warp_row0), nbar);
               }
-              if (EPI == EPI_ACT_AUX && aux_in != nullptr) {
-                const int col = c.n0 + (chunk + hc) * 32;
-                const T* src = aux_in + out_row * N + col;
-#pragma unroll
-                for (int qq = 0; qq < 4; ++qq) {
-                  const uint4 h = (row_ok && col + qq * 8 < N) ? __ldg(reinterpret_cast<const uint4*>(src + qq * 8))
-                                                               : make_uint4(0, 0, 0, 0);
-                  const uint32_t hw[4] = {h.x, h.y, h.z, h.w};
-#pragma unroll
-                  for (int p2 = 0; p2 < 4; ++p2) {
-                    const float2 pre = Elem<T>::unpack2(hw[p2]);
-                    v[qq * 8 + 2 * p2] *= dact_plain(pre.x, args.act);
-                    v[qq * 8 + 2 * p2 + 1] *= dact_plain(pre.y, args.act);
-                  }
-                }
-              } else if (pass == 1 && args.act != MOE_ACT_NONE) {
-#pragma unroll
-                for (int i = 0; i < 32; ++i) v[i] = act_plain(v[i], args.act);
+              __syncwarp();
+              if (!__all_sync(0xFFFFFFFFu, mbar_wait(my_epi_bar + 8 * (q & 1), (q >> 1) & 1, wctx, DS_TIMEOUT_EPILOGUE))) {
+                failed = true;
+                break;
               }
-              if (accumulate) {
+            }
+          } else if (lane == 0) {
+            bulk_wait_read_all();  // the previous round's stores have read both tiles
+          }
+          __syncwarp();
+#pragma unroll 1
+          for (int hc = 0; hc < 2; ++hc) {
+            uint32_t raw[32];
+            tmem_ld_32x32(taddr + (chunk + hc) * 32, raw);
+            tmem_ld_wait();
+            float v[32];
 #pragma unroll
-                for (int i = 0; i < 32; ++i) v[i] *= row_scale;
-              }
-              if (tma_out && hc == 0) {
-                if (lane == 0) bulk_wait_read_all();  // the previous round's store has read the staging tile
-                __syncwarp();
-              }
+            for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(raw[i]);
+            if (!live) continue;
+            const uint32_t row_addr = buf + lane * 128;
+            if (side_input) {
+              uint4 pre[4];
+#pragma unroll
+              for (int qq = 0; qq < 4; ++qq)
+                asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                             : "=r"(pre[qq].x), "=r"(pre[qq].y), "=r"(pre[qq].z), "=r"(pre[qq].w)
+                             : "r"(row_addr + (((hc * 4 + qq) ^ (lane & 7)) << 4)));
+              mul_dact<T>(v, pre, args.act);
+            } else {
 #pragma unroll
               for (int qq = 0; qq < 4; ++qq) {
                 const uint4 u = pack8<T>(v + qq * 8);
-                const uint32_t addr = stage_base + lane * 128 + (((hc * 4 + qq) ^ (lane & 7)) << 4);
-                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(u.x), "r"(u.y), "r"(u.z), "r"(u.w)
+                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(row_addr + Plan::kStagingTile +
+                                                                             (((hc * 4 + qq) ^ (lane & 7)) << 4)),
+                             "r"(u.x), "r"(u.y), "r"(u.z), "r"(u.w)
                              : "memory");
               }
+              apply_act(v, args.act);
             }
-            const int col_pair0 = c.n0 + chunk * 32;  // first of the 64 columns staged
-            if (tma_out) {
-              fence_proxy_async_smem();
-              __syncwarp();
-              if (lane == 0 && tile_stored && col_pair0 < N) {
-                if (KG) tma_store_3d(&tmap_d, col_pair0, c.m0 + quad * 32, c.expert, stage_base);
-                else tma_store_2d(&tmap_d, col_pair0, static_cast<int>(warp_row0), stage_base);
-                bulk_commit();
-              }
-              continue;
-            }
-            __syncwarp();
-            const unsigned long long pass_base = pass == 0 ? my_aux : my_base;
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              const int r = j * 4 + co_row;  // row of the warp's 32 this lane writes in this step
-              const unsigned long long base = __shfl_sync(0xFFFFFFFFu, pass_base, r);
-              const int ok = __shfl_sync(0xFFFFFFFFu, row_ok ? 1 : 0, r);
-              uint4 u;
-              const uint32_t addr = stage_base + r * 128 + ((co_ck ^ (r & 7)) << 4);
-              asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(u.x), "=r"(u.y), "=r"(u.z), "=r"(u.w) : "r"(addr));
-              const int col = col_pair0 + co_ck * 8;
-              if (ok && col < N) {
-                if (accumulate) red_add_v8<T>(reinterpret_cast<T*>(base) + col, u);
-                else *reinterpret_cast<uint4*>(reinterpret_cast<T*>(base) + col) = u;
-              }
+            for (int qq = 0; qq < 4; ++qq) {
+              const uint4 u = pack8<T>(v + qq * 8);
+              asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(row_addr + (((hc * 4 + qq) ^ (lane & 7)) << 4)),
+                           "r"(u.x), "r"(u.y), "r"(u.z), "r"(u.w)
+                           : "memory");
             }
-            __syncwarp();
-          }  // pass
+          }
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (live) {
+            if (lane == 0) {
+              tma_store_2d(&tmap_d, col0, static_cast<int>(warp_row0), buf);
+              if (!side_input) tma_store_2d(&tmap_c, col0, static_cast<int>(warp_row0), buf + Plan::kStagingTile);
+              bulk_commit();
+            }
+            if (side_input) ++q;
+          }
         }
+        if (failed) break;
       } else if (EPI == EPI_GLU) {
         // Two 32-column chunks per round.  The un-activated product (128 bytes per row) and the activated
         // half (64 bytes per row) each go through the warp's swizzled shared-memory tile, so that every store
@@ -991,29 +1105,13 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
           }
           if (live) {
             // v = d(activated)[row, col0..col0+32); pre-activation (gate, up) pairs at columns 2*col
+            if (args.act == MOE_ACT_GEGLU) dglu_row<T, true>(v, h_cur);
+            else dglu_row<T, false>(v, h_cur);
 #pragma unroll
-            for (int qq = 0; qq < 8; ++qq) {  // 8 pre-activation elements = 4 (gate, up) pairs per 16 bytes
-              const uint32_t hw[4] = {h_cur[qq].x, h_cur[qq].y, h_cur[qq].z, h_cur[qq].w};
-              float o[8];
-#pragma unroll
-              for (int p = 0; p < 4; ++p) {
-                const float2 gu = Elem<T>::unpack2(hw[p]);
-                const float da = v[qq * 4 + p];
-                float act_g, dact_g;
-                if (args.act == MOE_ACT_GEGLU) {
-                  act_g = gelu_f(gu.x);
-                  dact_g = dgelu_f(gu.x);
-                } else {
-                  const float sg = sigmoidf_fast(gu.x);
-                  act_g = gu.x * sg;
-                  dact_g = sg * (1.0f + gu.x * (1.0f - sg));
-                }
-                o[2 * p] = da * gu.y * dact_g;
-                o[2 * p + 1] = da * act_g;
-              }
-              const uint4 u = pack8<T>(o);
+            for (int qq = 0; qq < 8; ++qq) {
               const uint32_t addr = buf + lane * 128 + ((qq ^ (lane & 7)) << 4);
-              asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(u.x), "r"(u.y), "r"(u.z), "r"(u.w)
+              asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(h_cur[qq].x), "r"(h_cur[qq].y),
+                           "r"(h_cur[qq].z), "r"(h_cur[qq].w)
                            : "memory");
             }
             fence_proxy_async_smem();
@@ -1038,7 +1136,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         if (++acc == 2) { acc = 0; acc_phase ^= 1; }
       }
     }
-    if ((EPI == EPI_DGLU || EPI == EPI_ACT) && lane == 0) bulk_wait_all();  // this warp's bulk stores are complete
+    if ((EPI == EPI_DGLU || EPI == EPI_ACT || EPI == EPI_ACT_AUX) && lane == 0) bulk_wait_all();  // this warp's bulk stores are complete
   }
 
   tc_fence_before();

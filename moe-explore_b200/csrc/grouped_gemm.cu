@@ -235,11 +235,20 @@ static int mgrouped_dispatch(const void* a, const void* w, int64_t a_rows, int K
     return gather ? launch<T, BN, true, false, EPI_GLU, false, CTAS, true>(ta, tb, ta, ta, args, lp)
                   : launch<T, BN, true, false, EPI_GLU, false, CTAS, false>(ta, tb, ta, ta, args, lp);
   } else if (epi == EPI_ACT_AUX) {
+    // the un-activated product (written in the forward pass, read in the backward pass) and the result: tensor copies of
+    // 32-row x 64-column boxes
+    CUtensorMap tc, td;
+    const uint64_t dims[2] = {(uint64_t)N, (uint64_t)(args.mtiles_bound) * BM};
+    const uint32_t box[2] = {64, 32};
+    int rc = make_tmap(&tc, dtype, args.aux_in != nullptr ? args.aux_in : args.aux_out, 2, dims, box);
+    if (rc != MOE_OK) return rc;
+    rc = make_tmap(&td, dtype, args.out, 2, dims, box);
+    if (rc != MOE_OK) return rc;
     if (gather)
-      return w_transposed ? launch<T, BN, true, true, EPI_ACT_AUX, false, CTAS, true>(ta, tb, ta, ta, args, lp)
-                          : launch<T, BN, true, false, EPI_ACT_AUX, false, CTAS, true>(ta, tb, ta, ta, args, lp);
-    return w_transposed ? launch<T, BN, true, true, EPI_ACT_AUX, false, CTAS, false>(ta, tb, ta, ta, args, lp)
-                        : launch<T, BN, true, false, EPI_ACT_AUX, false, CTAS, false>(ta, tb, ta, ta, args, lp);
+      return w_transposed ? launch<T, BN, true, true, EPI_ACT_AUX, false, CTAS, true>(ta, tb, tc, td, args, lp)
+                          : launch<T, BN, true, false, EPI_ACT_AUX, false, CTAS, true>(ta, tb, tc, td, args, lp);
+    return w_transposed ? launch<T, BN, true, true, EPI_ACT_AUX, false, CTAS, false>(ta, tb, tc, td, args, lp)
+                        : launch<T, BN, true, false, EPI_ACT_AUX, false, CTAS, false>(ta, tb, tc, td, args, lp);
   }
   // EPI_DGLU (always with the transposed weight: dAct = g @ W2^T): the saved product and the result are moved by
   // tensor copies of 32-row x 64-column boxes
@@ -308,8 +317,8 @@ static int mgrouped_common(const char* name, const void* a, const void* w, void*
   args.a_div = x.gather_div;
   args.a_rows = static_cast<int32_t>(x.gather_rows);
   args.b_blocked = (!w_transposed && N % 64 == 0 && o.separate_copies == 0) ? 1 : 0;
-  // plain stores in the padded layout leave through bulk tensor stores (64-column boxes: N a multiple of 64)
-  args.out_tma = (epi == EPI_ACT && x.push_row == nullptr && x.combine_row_src == nullptr && out != nullptr && N % 64 == 0 &&
+  // plain stores in the padded layout leave through bulk tensor stores (the copy engine clips the 64-column boxes at N)
+  args.out_tma = (epi == EPI_ACT && x.push_row == nullptr && x.combine_row_src == nullptr && out != nullptr &&
                   o.lane_stores == 0) ? 1 : 0;
   args.out = out;
   args.aux_out = x.aux_out;
@@ -422,7 +431,7 @@ static int kgrouped_common(const char* name, const void* a, int64_t gather_rows,
   args.a_rows = static_cast<int32_t>(gather_rows);
   args.a_blocked = (gather_row_src == nullptr && M % 64 == 0 && o.separate_copies == 0) ? 1 : 0;
   args.b_blocked = (N % 64 == 0 && o.separate_copies == 0) ? 1 : 0;
-  args.out_tma = (N % 64 == 0 && o.lane_stores == 0) ? 1 : 0;
+  args.out_tma = o.lane_stores == 0 ? 1 : 0;
   args.out = dw;
   args.act = MOE_ACT_NONE;
   args.group_m = o.group_m > 0 ? o.group_m : kDefaultGroupM;
