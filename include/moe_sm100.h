@@ -398,6 +398,53 @@ int moe_kgrouped_gemm_gather(const void* src, int64_t src_rows, const int32_t* r
                              int64_t padded_rows, int M, int N, int num_experts, int dtype,
                              const moe_gemm_options* options, int32_t* status, void* stream);
 
+/* ---------------------------------------------------------------------------------
+ * The expert part of a layer pass in one call: the launches below in their order, on `stream`, nothing else (the same
+ * results as the entry points they stand for).  `steps` selects which: MOE_FWD_ALL / MOE_BWD_ALL, or single steps for a
+ * caller that wants to time or interleave them.  All buffers are the caller's; those of steps not asked for may be NULL.
+ *   gather         token rows are gathered by the gate/up GEMM's loads (x is read again for d_w1); xs is then unused
+ *   fused_combine  the down GEMM adds the scaled rows into out (zeroed first); ys and the fold are then unused
+ *   keep           a backward pass will follow: padding rows of xs are zeroed, pre_act (unless act is none) is written
+ *   workspace      for MOE_FWD_ROUTE of more than 131072 rows, moe_routing_workspace_bytes(num_tokens * topk, num_experts)
+ *                  bytes
+ * w1 [E, d, inter or 2*inter], w2 [E, inter, d]; xs, ys, gs, dxs [padded_rows, d]; pre_act, d_pre like w1's width; hidden
+ * [padded_rows, inter]; out, dx, grad_out, x [num_tokens, d]; scores, d_scores [num_tokens, topk].
+ * --------------------------------------------------------------------------------- */
+typedef struct moe_expert_pass {
+  int64_t num_tokens;
+  int64_t padded_rows;
+  int32_t d, inter, num_experts, topk, act, dtype;
+  int32_t gather, fused_combine, keep;
+  const int64_t* expert_idx; /* [num_tokens, topk] */
+  const void *x, *scores, *w1, *w2;
+  int32_t *group_indices, *pad_offsets, *row_src, *dst_row, *mtile_expert, *tile_pairs, *num_mtiles, *status;
+  void* workspace;
+  size_t workspace_bytes;
+  void *xs, *pre_act, *hidden, *ys, *out;
+  const void* grad_out;
+  void *gs, *d_scores, *d_pre, *dxs, *dx, *d_w1, *d_w2;
+} moe_expert_pass;
+
+/* sizeof(moe_expert_pass), for bindings that declare the struct themselves. */
+size_t moe_expert_pass_size(void);
+
+#define MOE_FWD_ROUTE 1
+#define MOE_FWD_DISPATCH 2
+#define MOE_FWD_UP 4
+#define MOE_FWD_DOWN 8
+#define MOE_FWD_FOLD 16
+#define MOE_FWD_ALL 31
+int moe_expert_forward(const moe_expert_pass* pass, int steps, void* stream);
+
+#define MOE_BWD_FOLD 1    /* gs, d_scores */
+#define MOE_BWD_DOWN 2    /* d_pre */
+#define MOE_BWD_UP 4      /* dxs */
+#define MOE_BWD_FOLD_DX 8 /* dx */
+#define MOE_BWD_DW1 16
+#define MOE_BWD_DW2 32
+#define MOE_BWD_ALL 63
+int moe_expert_backward(const moe_expert_pass* pass, int steps, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -11,7 +11,7 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "libmoe_sm100.so")
-SOURCES = ["api.cu", "routing.cu", "rows.cu", "router.cu", "grouped_gemm.cu", "no_alloc.cu"] + \
+SOURCES = ["api.cu", "routing.cu", "rows.cu", "router.cu", "grouped_gemm.cu", "layer.cu", "no_alloc.cu"] + \
           [f"gemm_inst_{t}_{c}{g}.cu" for t in ("bf16", "f16") for c in ("pair", "single") for g in ("", "_gather")]
 HEADERS = [os.path.join(CSRC, "common.cuh"), os.path.join(CSRC, "gemm_kernel.cuh"),
            os.path.join(os.path.dirname(HERE), "include", "moe_sm100.h")]

@@ -40,6 +40,12 @@ int cuda_fail(cudaError_t e, const char* what);
 
 int sm_count();  // SM count of the current device (cached per device)
 
+// moe_routing_metadata; `workspace_always` false: a workspace is asked for only where the kernels use one (csrc/routing.cu).
+int routing_metadata(const int64_t* expert_idx, int64_t num_rows, int num_experts, int32_t* group_indices, int64_t* perm,
+                     int32_t* pad_offsets, int32_t* row_src, int32_t* dst_row, int32_t* mtile_expert, int32_t* tile_pairs,
+                     int32_t* num_mtiles, int32_t* status, void* workspace, size_t workspace_bytes,
+                     bool workspace_always, void* stream);
+
 // Status codes written by kernels into the caller's device status word.
 enum DeviceStatus : int {
   DS_OK = 0,

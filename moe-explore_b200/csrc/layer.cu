@@ -1,0 +1,96 @@
+// The expert part of a layer pass in one host call: the launches of moe_expert_forward / moe_expert_backward are the ones a caller
+// could make one by one through the entry points below; issuing them from native code is what a pass over a few tokens
+// is bound by (from Python, each call costs 5-12 us of argument handling against 2-3 us for the launch itself).
+#include "common.cuh"
+
+namespace moe {
+
+static bool glu(int act) { return act == MOE_ACT_SWIGLU || act == MOE_ACT_GEGLU; }
+
+#define MOE_STEP(call)              \
+  do {                              \
+    const int rc__ = (call);        \
+    if (rc__ != MOE_OK) return rc__; \
+  } while (0)
+
+}  // namespace moe
+
+using namespace moe;
+
+extern "C" size_t moe_expert_pass_size(void) { return sizeof(moe_expert_pass); }
+
+extern "C" int moe_expert_forward(const moe_expert_pass* p, int steps, void* stream) {
+  MOE_CHECK_ARG(p != nullptr, "moe_expert_forward: null pointer argument");
+  const int up_cols = glu(p->act) ? 2 * p->inter : p->inter;
+  const int64_t rows = p->num_tokens * p->topk;
+  if (steps & MOE_FWD_ROUTE)
+    MOE_STEP(routing_metadata(p->expert_idx, rows, p->num_experts, p->group_indices, nullptr, p->pad_offsets, p->row_src,
+                              p->dst_row, p->mtile_expert, p->tile_pairs, p->num_mtiles, p->status, p->workspace,
+                              p->workspace_bytes, false, stream));
+  if ((steps & MOE_FWD_DISPATCH) && !p->gather) {
+    // rows do not mix in a forward pass, and only a weight gradient contracts over the padding rows
+    if (p->keep)
+      MOE_STEP(moe_dispatch_rows(p->x, p->dst_row, p->row_src, p->num_mtiles, p->xs, p->num_tokens, p->topk, p->padded_rows, p->d,
+                                 p->dtype, stream));
+    else
+      MOE_STEP(moe_dispatch_rows_only(p->x, p->dst_row, p->xs, p->num_tokens, p->topk, p->d, p->dtype, stream));
+  }
+  if (steps & MOE_FWD_UP) {
+    if (p->gather)
+      MOE_STEP(moe_mgrouped_gemm_gather(p->x, p->num_tokens, p->row_src, p->topk, p->w1, p->hidden, p->pre_act, p->mtile_expert,
+                                        p->tile_pairs, p->num_mtiles, p->padded_rows, p->d, up_cols, p->num_experts, p->act,
+                                        p->dtype, nullptr, p->status, stream));
+    else
+      MOE_STEP(moe_mgrouped_gemm(p->xs, p->w1, p->hidden, p->pre_act, p->mtile_expert, p->tile_pairs, p->num_mtiles,
+                                 p->padded_rows, p->d, up_cols, p->num_experts, 0, p->act, p->dtype, 0, 1, nullptr, p->status,
+                                 stream));
+  }
+  if (steps & MOE_FWD_DOWN) {
+    if (p->fused_combine) {
+      MOE_CUDA(cudaMemsetAsync(p->out, 0, static_cast<size_t>(p->num_tokens) * p->d * 2, static_cast<cudaStream_t>(stream)));
+      MOE_STEP(moe_mgrouped_gemm_combine(p->hidden, p->w2, p->out, p->row_src, p->scores, p->topk, p->mtile_expert, p->tile_pairs,
+                                         p->num_mtiles, p->padded_rows, p->inter, p->d, p->num_experts, 0, p->dtype, nullptr,
+                                         p->status, stream));
+    } else {
+      MOE_STEP(moe_mgrouped_gemm(p->hidden, p->w2, p->ys, nullptr, p->mtile_expert, p->tile_pairs, p->num_mtiles, p->padded_rows,
+                                 p->inter, p->d, p->num_experts, 0, MOE_ACT_NONE, p->dtype, 0, 1, nullptr, p->status, stream));
+    }
+  }
+  if ((steps & MOE_FWD_FOLD) && !p->fused_combine)
+    MOE_STEP(moe_combine_topk(p->ys, p->scores, p->dst_row, p->out, p->num_tokens, p->topk, p->d, p->dtype, stream));
+  return MOE_OK;
+}
+
+extern "C" int moe_expert_backward(const moe_expert_pass* p, int steps, void* stream) {
+  MOE_CHECK_ARG(p != nullptr, "moe_expert_backward: null pointer argument");
+  const int up_cols = glu(p->act) ? 2 * p->inter : p->inter;
+  if (steps & MOE_BWD_FOLD)
+    MOE_STEP(moe_combine_bwd_tokens(p->grad_out, p->scores, p->ys, p->dst_row, p->row_src, p->num_mtiles, p->gs, p->d_scores,
+                                    p->num_tokens, p->topk, p->d, p->dtype, stream));
+  if (steps & MOE_BWD_DOWN) {
+    if (p->act == MOE_ACT_NONE)  // linear "activation": d_pre = gs @ W2^T
+      MOE_STEP(moe_mgrouped_gemm(p->gs, p->w2, p->d_pre, nullptr, p->mtile_expert, p->tile_pairs, p->num_mtiles, p->padded_rows,
+                                 p->d, p->inter, p->num_experts, 1, MOE_ACT_NONE, p->dtype, 0, 1, nullptr, p->status, stream));
+    else
+      MOE_STEP(moe_mgrouped_gemm_dglu(p->gs, p->w2, p->pre_act, p->d_pre, p->mtile_expert, p->tile_pairs, p->num_mtiles,
+                                      p->padded_rows, p->d, p->inter, p->num_experts, p->act, p->dtype, 0, 1, nullptr, p->status,
+                                      stream));
+  }
+  if (steps & MOE_BWD_UP)
+    MOE_STEP(moe_mgrouped_gemm(p->d_pre, p->w1, p->dxs, nullptr, p->mtile_expert, p->tile_pairs, p->num_mtiles, p->padded_rows,
+                               up_cols, p->d, p->num_experts, 1, MOE_ACT_NONE, p->dtype, 0, 1, nullptr, p->status, stream));
+  if (steps & MOE_BWD_FOLD_DX)
+    MOE_STEP(moe_combine_topk(p->dxs, nullptr, p->dst_row, p->dx, p->num_tokens, p->topk, p->d, p->dtype, stream));
+  if (steps & MOE_BWD_DW1) {
+    if (p->gather)  // x is the layer input in token order: its rows are gathered by the loads again
+      MOE_STEP(moe_kgrouped_gemm_gather(p->x, p->num_tokens, p->row_src, p->topk, p->d_pre, p->d_w1, p->pad_offsets,
+                                        p->padded_rows, p->d, up_cols, p->num_experts, p->dtype, nullptr, p->status, stream));
+    else
+      MOE_STEP(moe_kgrouped_gemm(p->xs, p->d_pre, p->d_w1, p->pad_offsets, p->padded_rows, p->d, up_cols, p->num_experts, p->dtype,
+                                 nullptr, p->status, stream));
+  }
+  if (steps & MOE_BWD_DW2)
+    MOE_STEP(moe_kgrouped_gemm(p->hidden, p->gs, p->d_w2, p->pad_offsets, p->padded_rows, p->inter, p->d, p->num_experts, p->dtype,
+                               nullptr, p->status, stream));
+  return MOE_OK;
+}

@@ -95,7 +95,7 @@ __device__ __forceinline__ void write_tile_maps(int e, int32_t row_begin, int32_
   }
 }
 
-// Many chunks: one CTA per expert turns its column of the [chunks, E] histogram into exclusive offsets (every
+// One CTA per expert turns its column of the [chunks, E] histogram into exclusive offsets (every
 // thread owns a contiguous run of chunks; block-wide scan of the run sums) and leaves the expert's row count in
 // group_indices[e + 1] for the single-CTA pass below.
 constexpr int kScanThreads = 256;
@@ -132,13 +132,11 @@ scan_chunks_kernel(const int32_t* __restrict__ chunk_hist, int32_t* __restrict__
   if (tid == 0) group_indices[e + 1] = total;
 }
 
-// One CTA, one thread per expert (E <= 1024).  `counts_ready`: the per-expert row counts are already in
-// group_indices[1..E] (scan_chunks_kernel ran); otherwise this kernel scans the chunk axis itself (few chunks).
+// One CTA, one thread per expert (E <= 1024); the per-expert row counts are in group_indices[1..E] (scan_chunks_kernel).
 // num_mtiles receives {tiles in use, tile pairs in use, mtiles_bound, 0}; perm entries past the rows that were
 // kept (ids out of range are dropped) are set to -1.
 __global__ void __launch_bounds__(kMaxExperts)
-scan_offsets_kernel(const int32_t* __restrict__ chunk_hist, int32_t* __restrict__ chunk_off, int64_t nchunks, int E,
-                    int counts_ready, int32_t* __restrict__ group_indices,
+scan_offsets_kernel(int E, int32_t* __restrict__ group_indices,
                     int32_t* __restrict__ pad_offsets, int32_t* __restrict__ mtile_expert,
                     int32_t* __restrict__ tile_pairs, int32_t* __restrict__ num_mtiles, int mtiles_bound,
                     int64_t* __restrict__ perm, int64_t R) {
@@ -146,25 +144,7 @@ scan_offsets_kernel(const int32_t* __restrict__ chunk_hist, int32_t* __restrict_
   __shared__ int32_t sh_b[kMaxExperts];
   __shared__ int32_t sh_c[kMaxExperts];
   const int e = threadIdx.x;
-  int32_t total = 0;
-  if (e < E) {
-    if (counts_ready) {
-      total = group_indices[e + 1];
-    } else {
-      // exclusive scan down the chunk axis for this expert
-      constexpr int kBatch = 16;  // loads in flight per thread
-      for (int64_t c0 = 0; c0 < nchunks; c0 += kBatch) {
-        int32_t v[kBatch];
-#pragma unroll
-        for (int i = 0; i < kBatch; ++i) v[i] = (c0 + i < nchunks) ? chunk_hist[(c0 + i) * E + e] : 0;
-#pragma unroll
-        for (int i = 0; i < kBatch; ++i) {
-          if (c0 + i < nchunks) chunk_off[(c0 + i) * E + e] = total;
-          total += v[i];
-        }
-      }
-    }
-  }
+  const int32_t total = e < E ? group_indices[e + 1] : 0;
   const int32_t padded = (total + MOE_TILE_M - 1) / MOE_TILE_M * MOE_TILE_M;
   const int32_t pairs = (padded / MOE_TILE_M + 1) / 2;  // row tiles of one expert, two at a time
   sh_a[e] = e < E ? total : 0;
@@ -563,11 +543,12 @@ extern "C" size_t moe_routing_workspace_bytes(int64_t num_rows, int num_experts)
   return 2 * static_cast<size_t>(chunks) * num_experts * sizeof(int32_t);  // chunk histogram + chunk offsets
 }
 
-extern "C" int moe_routing_metadata(const int64_t* expert_idx, int64_t num_rows, int num_experts,
-                                    int32_t* group_indices, int64_t* perm, int32_t* pad_offsets, int32_t* row_src,
-                                    int32_t* dst_row, int32_t* mtile_expert, int32_t* tile_pairs,
-                                    int32_t* num_mtiles, int32_t* status, void* workspace, size_t workspace_bytes,
-                                    void* stream) {
+namespace moe {
+
+int routing_metadata(const int64_t* expert_idx, int64_t num_rows, int num_experts, int32_t* group_indices, int64_t* perm,
+                     int32_t* pad_offsets, int32_t* row_src, int32_t* dst_row, int32_t* mtile_expert, int32_t* tile_pairs,
+                     int32_t* num_mtiles, int32_t* status, void* workspace, size_t workspace_bytes,
+                     bool workspace_always, void* stream) {
   MOE_CHECK_ARG(num_rows >= 0, "moe_routing_metadata: num_rows=%lld is negative", (long long)num_rows);
   MOE_CHECK_ARG(num_experts > 0, "moe_routing_metadata: num_experts=%d must be positive", num_experts);
   if (num_experts > kMaxExperts) {
@@ -580,7 +561,8 @@ extern "C" int moe_routing_metadata(const int64_t* expert_idx, int64_t num_rows,
   MOE_CHECK_ARG(num_rows == 0 || expert_idx != nullptr, "moe_routing_metadata: expert_idx is null");
   MOE_CHECK_ARG((mtile_expert == nullptr) == (num_mtiles == nullptr) && (tile_pairs == nullptr || mtile_expert != nullptr),
                 "moe_routing_metadata: mtile_expert, tile_pairs and num_mtiles go together");
-  MOE_CHECK_ARG(workspace != nullptr && workspace_bytes >= moe_routing_workspace_bytes(num_rows, num_experts),
+  MOE_CHECK_ARG((!workspace_always && num_rows <= kClusterRows) ||
+                    (workspace != nullptr && workspace_bytes >= moe_routing_workspace_bytes(num_rows, num_experts)),
                 "moe_routing_metadata: workspace of %zu bytes is smaller than the %zu required", workspace_bytes,
                 moe_routing_workspace_bytes(num_rows, num_experts));
   cudaStream_t s = static_cast<cudaStream_t>(stream);
@@ -592,34 +574,36 @@ extern "C" int moe_routing_metadata(const int64_t* expert_idx, int64_t num_rows,
   }
   int32_t* chunk_hist = static_cast<int32_t*>(workspace);
   const int64_t chunks = num_chunks(num_rows);
-  int32_t* chunk_off = chunk_hist + (chunks > 0 ? chunks : 1) * num_experts;
+  int32_t* chunk_off = chunk_hist + chunks * num_experts;
   const int blocks = static_cast<int>((chunks + kWarpsPerBlock - 1) / kWarpsPerBlock);
   const size_t sh = static_cast<size_t>(kWarpsPerBlock) * num_experts * sizeof(int32_t);
   if (row_src != nullptr) {
     MOE_CUDA(cudaMemsetAsync(row_src, 0xFF, moe_padded_rows_bound(num_rows, num_experts) * sizeof(int32_t), s));
   }
-  if (chunks == 0) {
-    MOE_CUDA(cudaMemsetAsync(chunk_hist, 0, num_experts * sizeof(int32_t), s));
-  } else {
-    chunk_histogram_kernel<<<blocks, kWarpsPerBlock * 32, sh, s>>>(expert_idx, num_rows, num_experts, chunk_hist, status);
-    MOE_CUDA(cudaGetLastError());
-  }
-  // many chunks: scan the chunk axis with one CTA per expert first (a single CTA walking 512 chunks took 53 us)
-  const int split_scan = chunks > 64 ? 1 : 0;
-  if (split_scan) {
-    scan_chunks_kernel<<<num_experts, kScanThreads, 0, s>>>(chunk_hist, chunk_off, chunks, num_experts, group_indices);
-    MOE_CUDA(cudaGetLastError());
-  }
-  scan_offsets_kernel<<<1, kMaxExperts, 0, s>>>(chunk_hist, chunk_off, chunks, num_experts, split_scan, group_indices,
-                                               pad_offsets, mtile_expert, tile_pairs, num_mtiles,
+  chunk_histogram_kernel<<<blocks, kWarpsPerBlock * 32, sh, s>>>(expert_idx, num_rows, num_experts, chunk_hist, status);
+  MOE_CUDA(cudaGetLastError());
+  scan_chunks_kernel<<<num_experts, kScanThreads, 0, s>>>(chunk_hist, chunk_off, chunks, num_experts, group_indices);
+  MOE_CUDA(cudaGetLastError());
+  scan_offsets_kernel<<<1, kMaxExperts, 0, s>>>(num_experts, group_indices, pad_offsets, mtile_expert, tile_pairs, num_mtiles,
                                                static_cast<int>(moe_mtiles_bound(num_rows, num_experts)), perm, num_rows);
   MOE_CUDA(cudaGetLastError());
-  if (chunks > 0 && (perm || row_src || dst_row)) {
+  if (perm || row_src || dst_row) {
     place_rows_kernel<<<blocks, kWarpsPerBlock * 32, sh, s>>>(expert_idx, num_rows, num_experts, chunk_off,
                                                              group_indices, pad_offsets, perm, row_src, dst_row);
     MOE_CUDA(cudaGetLastError());
   }
   return MOE_OK;
+}
+
+}  // namespace moe
+
+extern "C" int moe_routing_metadata(const int64_t* expert_idx, int64_t num_rows, int num_experts,
+                                    int32_t* group_indices, int64_t* perm, int32_t* pad_offsets, int32_t* row_src,
+                                    int32_t* dst_row, int32_t* mtile_expert, int32_t* tile_pairs,
+                                    int32_t* num_mtiles, int32_t* status, void* workspace, size_t workspace_bytes,
+                                    void* stream) {
+  return routing_metadata(expert_idx, num_rows, num_experts, group_indices, perm, pad_offsets, row_src, dst_row, mtile_expert,
+                          tile_pairs, num_mtiles, status, workspace, workspace_bytes, true, stream);
 }
 
 extern "C" int moe_layout_from_groups(const int32_t* group_indices, int64_t num_rows, int num_experts,

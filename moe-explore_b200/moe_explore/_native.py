@@ -35,6 +35,17 @@ class GemmOptions(ctypes.Structure):
                 ("wave_counter", c_void_p)]
 
 
+class ExpertPass(ctypes.Structure):
+    """``moe_expert_pass``: sizes and buffers of one forward or backward pass over the experts."""
+    _fields_ = [(f, c_int64) for f in ("num_tokens", "padded_rows")] + \
+               [(f, c_int32) for f in ("d", "inter", "num_experts", "topk", "act", "dtype", "gather", "fused_combine", "keep")] + \
+               [(f, c_void_p) for f in ("expert_idx", "x", "scores", "w1", "w2", "group_indices", "pad_offsets", "row_src",
+                                        "dst_row", "mtile_expert", "tile_pairs", "num_mtiles", "status", "workspace")] + \
+               [("workspace_bytes", c_size_t)] + \
+               [(f, c_void_p) for f in ("xs", "pre_act", "hidden", "ys", "out", "grad_out", "gs", "d_scores", "d_pre", "dxs", "dx",
+                                        "d_w1", "d_w2")]
+
+
 # name -> (restype, argtypes); the single source for both binding and the symbol-export test
 _OPT = POINTER(GemmOptions)
 SIGNATURES = {
@@ -63,6 +74,9 @@ SIGNATURES = {
     "moe_combine_topk": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int, c_int, c_void_p]),
     "moe_combine_bwd": (c_int, [c_void_p] * 7 + [c_int64, c_int, c_int64, c_int, c_int, c_void_p]),
     "moe_dispatch_rows": (c_int, [c_void_p] * 5 + [c_int64, c_int, c_int64, c_int, c_int, c_void_p]),
+    "moe_expert_pass_size": (c_size_t, []),
+    "moe_expert_forward": (c_int, [POINTER(ExpertPass), c_int, c_void_p]),
+    "moe_expert_backward": (c_int, [POINTER(ExpertPass), c_int, c_void_p]),
     "moe_dispatch_rows_only": (c_int, [c_void_p] * 3 + [c_int64, c_int, c_int, c_int, c_void_p]),
     "moe_combine_bwd_tokens": (c_int, [c_void_p] * 8 + [c_int64, c_int, c_int, c_int, c_void_p]),
     "moe_mgrouped_gemm": (c_int, [c_void_p] * 7 + [c_int64, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, _OPT,
@@ -137,6 +151,8 @@ def load() -> ctypes.CDLL:
             fn.argtypes = argtypes
         if lib.moe_gemm_options_size() != ctypes.sizeof(GemmOptions):
             raise ImportError(f"{LIB_PATH} was built with another layout of moe_gemm_options: rebuild it")
+        if lib.moe_expert_pass_size() != ctypes.sizeof(ExpertPass):
+            raise ImportError(f"{LIB_PATH} was built with another layout of moe_expert_pass: rebuild it")
         _lib = lib
     return _lib
 
@@ -151,7 +167,8 @@ def _ptr(t):
 
 
 def _stream():
-    return torch.cuda.current_stream().cuda_stream
+    # what torch.cuda.current_stream().cuda_stream reads, without building a Stream object (2 us a call)
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def dtype_code(dtype: torch.dtype) -> int:
@@ -212,6 +229,28 @@ def gemm_options(max_ctas: int = 0, wave_sync: int = 0, wave_workers: int = 0, g
 
 def _opt(options):
     return None if options is None else ctypes.byref(options)
+
+
+FWD_ROUTE, FWD_DISPATCH, FWD_UP, FWD_DOWN, FWD_FOLD = 1, 2, 4, 8, 16
+BWD_FOLD, BWD_DOWN, BWD_UP, BWD_FOLD_DX, BWD_DW1, BWD_DW2 = 1, 2, 4, 8, 16, 32
+
+
+def expert_pass(backward: bool, p: ExpertPass, steps, rows: int) -> None:
+    """The launches of one pass over the experts on the current stream; ``steps`` = [(step, name, launches)].  One call
+    into the library, or, with a ``TRACER``, one per step, so that each is counted and can be timed by itself."""
+    lib = load()
+    name = "moe_expert_backward" if backward else "moe_expert_forward"
+    fn = lib.moe_expert_backward if backward else lib.moe_expert_forward
+    if TRACER is None:
+        mask = 0
+        for step, _, _ in steps:
+            mask |= step
+        _check(name, fn(ctypes.byref(p), mask, _stream()))
+        return
+    for step, key, launches in steps:
+        with timed(key, None if key.startswith("ro") else rows):
+            _check(name, fn(ctypes.byref(p), step, _stream()))
+        _count(launches)
 
 
 def routing_metadata(expert_idx, num_experts, group_indices, perm, pad_offsets, row_src, dst_row, mtile_expert,

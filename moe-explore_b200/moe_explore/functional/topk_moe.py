@@ -10,11 +10,10 @@ from __future__ import annotations
 
 import torch
 
-from moe_explore.expert_compute import expert_compute
+from moe_explore.expert_compute import routed_expert_compute
 from moe_explore.functional.activation import activation
 from moe_explore.params import MLPParams, MOEParams, TopkRouterParams
 from moe_explore.router import fused_topk_router, router
-from moe_explore.routing_plan import build_routing_plan
 
 
 def _shared_expert(input: torch.Tensor, shared) -> torch.Tensor:
@@ -30,8 +29,7 @@ def _shared_expert(input: torch.Tensor, shared) -> torch.Tensor:
         T = input.size(0)
         indices = torch.arange(num_shared, device=input.device, dtype=torch.int64).repeat(T, 1)
         ones = torch.ones(T, num_shared, dtype=input.dtype, device=input.device)
-        plan = build_routing_plan(indices, num_shared, num_shared, want_perm=False)
-        return expert_compute(input, ones, up, down, plan, shared.activation)
+        return routed_expert_compute(input, ones, up, down, indices, num_shared, num_shared, shared.activation)
     h = input @ up
     h = activation(h, shared.activation)
     h = h @ down
@@ -48,9 +46,8 @@ def topk_moe_forward(input: torch.Tensor, params: MOEParams, autotune_mode=None,
         scores, indices = fused_topk_router(input, params.router_params)
     else:
         scores, indices = router(input, params.router_params)
-    plan = build_routing_plan(indices, params.num_experts, params.topk, want_perm=False)
-    out = expert_compute(input, scores, ep.weight1, ep.weight2, plan, ep.activation, gather_in_gemm=gather_in_gemm,
-                         fused_combine=fused_combine)
+    out = routed_expert_compute(input, scores, ep.weight1, ep.weight2, indices, params.num_experts, params.topk, ep.activation,
+                                gather_in_gemm=gather_in_gemm, fused_combine=fused_combine)
     shared = getattr(params, "shared_expert_params", None)
     if shared is not None:
         out = out + _shared_expert(input, shared)

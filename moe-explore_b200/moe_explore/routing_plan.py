@@ -14,6 +14,7 @@ of a step after which it raised.
 """
 from __future__ import annotations
 
+import functools
 import warnings
 from dataclasses import dataclass
 from typing import Dict, Optional
@@ -27,6 +28,11 @@ _DEVICE_STATUS: Dict[int, torch.Tensor] = {}
 
 def device_status(device=None) -> torch.Tensor:
     """The int32 [1] status word of ``device`` (created zeroed on first use)."""
+    if type(device) is int:   # a device index
+        word = _DEVICE_STATUS.get(device)
+        if word is not None:
+            return word
+        device = torch.device("cuda", device)
     dev = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
     index = dev.index if dev.index is not None else torch.cuda.current_device()
     word = _DEVICE_STATUS.get(index)
@@ -80,6 +86,21 @@ class RoutingPlan:
     def check(self) -> None:
         """Synchronise and raise if any kernel reported a problem through this plan's status word."""
         _report(_native.read_status(self.status, reset=True))
+
+
+@functools.lru_cache(maxsize=256)
+def packed_layout(num_rows: int, num_experts: int):
+    """(padded rows, byte offsets of the seven index arrays in the order of ``moe_expert_pass``, int32 words of the whole):
+    the arrays of a plan in ONE allocation, each 16-byte aligned.  A function of the sizes alone."""
+    rp = _native.padded_rows_bound(num_rows, num_experts)
+    tiles = rp // _native.TILE_M
+    # group_indices, pad_offsets, row_src, dst_row, mtile_expert, tile_pairs, num_mtiles
+    sizes = (num_experts + 1, num_experts + 1, rp, num_rows, tiles, tiles + num_experts + 1, 4)
+    offsets, words = [], 0
+    for n in sizes:
+        offsets.append(4 * words)
+        words += (n + 3) // 4 * 4
+    return rp, tuple(offsets), words
 
 
 def _alloc(num_rows: int, num_experts: int, device, want_perm: bool):
