@@ -25,6 +25,11 @@ int cuda_fail(cudaError_t e, const char* what) {
   return MOE_ERR_CUDA;
 }
 
+bool& chained_launches() {
+  static thread_local bool on = false;
+  return on;
+}
+
 int sm_count() {
   static int cached[64];
   int dev = 0;

@@ -40,6 +40,27 @@ int cuda_fail(cudaError_t e, const char* what);
 
 int sm_count();  // SM count of the current device (cached per device)
 
+// Chained launches.  Inside one library call that launches several kernels in a row on one stream, the kernels after the
+// first are launched with programmatic stream serialization: their launch and prologue (barriers, TMEM, descriptors)
+// overlap the tail of the kernel before, and grid_wait() holds them back until that kernel has completed and its writes are
+// visible.  Every kernel that can be launched so calls grid_wait() before its first access to global memory, so the
+// order of the stream holds for all earlier kernels too.  Thread-local and set only for the duration of such a call.
+bool& chained_launches();
+
+template <typename... Params, typename... Args>
+inline cudaError_t launch_kernel(void (*kernel)(Params...), int grid, int block, cudaStream_t stream, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(grid), 1, 1);
+  cfg.blockDim = dim3(static_cast<unsigned>(block), 1, 1);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = chained_launches() ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
 // moe_routing_metadata; `workspace_always` false: a workspace is asked for only where the kernels use one (csrc/routing.cu).
 int routing_metadata(const int64_t* expert_idx, int64_t num_rows, int num_experts, int32_t* group_indices, int64_t* perm,
                      int32_t* pad_offsets, int32_t* row_src, int32_t* dst_row, int32_t* mtile_expert, int32_t* tile_pairs,
@@ -98,6 +119,10 @@ template <> struct Elem<__half> {
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
+
+// See chained_launches(): waits for the kernels this one was chained to / lets the next chained kernel start its prologue.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");

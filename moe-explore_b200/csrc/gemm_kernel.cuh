@@ -502,6 +502,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       tmem_relinquish();
     }
   }
+  grid_wait();  // nothing above reads or writes global memory
   tc_fence_before();
   __syncthreads();
   if (kPair) cluster_sync_all();  // the peer's barriers must be initialised before anything arrives on them
@@ -659,6 +660,9 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
           if (++stage == kStages) { stage = 0; phase ^= 1; }
         }
       }
+      // all operand loads are issued: the next chained kernel may come up beside the last tile's contraction and epilogue (from
+      // the start of this kernel on, its waiting CTAs cost more than they hid)
+      grid_release();
       if (!KG && args.wave_counter != nullptr && rank == 0 && lane == 0) {
         // workers without an item in the remaining waves still count, so that the others do not wait for them
         // (arrivals for waves up to `wave` were made inside the items that preceded them)
@@ -1155,6 +1159,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
 // ----------------------------------------------------------------------------------
 struct LaunchParams {
   int max_ctas;  // 0 = one CTA per SM
+  bool chained;  // launched with programmatic stream serialization (chained_launches)
   cudaStream_t stream;
 };
 
@@ -1177,13 +1182,16 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, 
   cfg.blockDim = dim3(kThreads, 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = lp.stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = CTAS;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
+  constexpr int kClusterAttrs = CTAS > 1 ? 1 : 0;
+  attr[kClusterAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[kClusterAttrs].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = CTAS > 1 ? 1 : 0;
+  cfg.numAttrs = kClusterAttrs;
   int grid = (dev >= 0 && dev < 64) ? grid_for_device[dev].load(std::memory_order_acquire) : 0;
   if (grid == 0) {
     // First launch of this variant on this device (two threads racing here compute the same value twice).
@@ -1209,6 +1217,7 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, 
   }
   if (args.wave_workers <= 0) args.wave_workers = grid / CTAS;
   cfg.gridDim = dim3(static_cast<unsigned>(grid), 1, 1);
+  cfg.numAttrs = kClusterAttrs + (lp.chained ? 1 : 0);
   MOE_CUDA(cudaLaunchKernelEx(&cfg, kernel, ta, tb, tc, td, args));
   return MOE_OK;
 }

@@ -336,6 +336,7 @@ static int mgrouped_common(const char* name, const void* a, const void* w, void*
   LaunchParams lp;
   lp.stream = static_cast<cudaStream_t>(stream);
   lp.max_ctas = o.max_ctas > 0 ? o.max_ctas : 0;
+  lp.chained = chained_launches();
   {
     // The wave barrier cuts the DRAM reads of every M-grouped GEMM to about the algorithmic bytes (gate/up at
     // the Mixtral shape: 6.4 -> 2.1 GB), but only long contractions get faster (K = 14336: -1.2 %, K = 28672:
@@ -351,6 +352,7 @@ static int mgrouped_common(const char* name, const void* a, const void* w, void*
         if (rc != MOE_OK) return rc;
       }
       MOE_CUDA(cudaMemsetAsync(args.wave_counter, 0, sizeof(uint32_t), lp.stream));
+      lp.chained = false;  // the memset stands between this kernel and the one before
     }
   }
   const int bn = pick_bn(N);
@@ -440,6 +442,7 @@ static int kgrouped_common(const char* name, const void* a, int64_t gather_rows,
   LaunchParams lp;
   lp.stream = static_cast<cudaStream_t>(stream);
   lp.max_ctas = o.max_ctas > 0 ? o.max_ctas : 0;
+  lp.chained = chained_launches();
   const int bn = pick_bn(N);
   // CTA pairs unless the contraction is at most one 64-row step per expert on average (measured at 64 rows per
   // expert, DeepSeek-V3 shape: weight1 gradient 4.00 -> 3.48 ms; at 128 rows per expert pairs are 9 % faster)

@@ -7,10 +7,19 @@ namespace moe {
 
 static bool glu(int act) { return act == MOE_ACT_SWIGLU || act == MOE_ACT_GEGLU; }
 
+// The kernels of one call are chained (common.cuh): all but the first.  B200, tail of one kernel to work of the next: see the
+// figures at moe_expert_forward.
+class Chain {
+ public:
+  Chain() { chained_launches() = false; }
+  ~Chain() { chained_launches() = false; }
+};
+
 #define MOE_STEP(call)              \
   do {                              \
     const int rc__ = (call);        \
     if (rc__ != MOE_OK) return rc__; \
+    chained_launches() = true;      \
   } while (0)
 
 }  // namespace moe
@@ -23,6 +32,7 @@ extern "C" int moe_expert_forward(const moe_expert_pass* p, int steps, void* str
   MOE_CHECK_ARG(p != nullptr, "moe_expert_forward: null pointer argument");
   const int up_cols = glu(p->act) ? 2 * p->inter : p->inter;
   const int64_t rows = p->num_tokens * p->topk;
+  const Chain chain;
   if (steps & MOE_FWD_ROUTE)
     MOE_STEP(routing_metadata(p->expert_idx, rows, p->num_experts, p->group_indices, nullptr, p->pad_offsets, p->row_src,
                               p->dst_row, p->mtile_expert, p->tile_pairs, p->num_mtiles, p->status, p->workspace,
@@ -48,6 +58,7 @@ extern "C" int moe_expert_forward(const moe_expert_pass* p, int steps, void* str
   if (steps & MOE_FWD_DOWN) {
     if (p->fused_combine) {
       MOE_CUDA(cudaMemsetAsync(p->out, 0, static_cast<size_t>(p->num_tokens) * p->d * 2, static_cast<cudaStream_t>(stream)));
+      chained_launches() = false;  // the memset stands between
       MOE_STEP(moe_mgrouped_gemm_combine(p->hidden, p->w2, p->out, p->row_src, p->scores, p->topk, p->mtile_expert, p->tile_pairs,
                                          p->num_mtiles, p->padded_rows, p->inter, p->d, p->num_experts, 0, p->dtype, nullptr,
                                          p->status, stream));
@@ -64,6 +75,7 @@ extern "C" int moe_expert_forward(const moe_expert_pass* p, int steps, void* str
 extern "C" int moe_expert_backward(const moe_expert_pass* p, int steps, void* stream) {
   MOE_CHECK_ARG(p != nullptr, "moe_expert_backward: null pointer argument");
   const int up_cols = glu(p->act) ? 2 * p->inter : p->inter;
+  const Chain chain;
   if (steps & MOE_BWD_FOLD)
     MOE_STEP(moe_combine_bwd_tokens(p->grad_out, p->scores, p->ys, p->dst_row, p->row_src, p->num_mtiles, p->gs, p->d_scores,
                                     p->num_tokens, p->topk, p->d, p->dtype, stream));

@@ -270,6 +270,7 @@ route_cluster_kernel(const int64_t* __restrict__ ids, int64_t R, int E, int held
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int rank = static_cast<int>(cluster_ctarank());
   const int ctas = gridDim.x;
+  grid_release();
   for (int i = tid; i < kRouteWarps * E; i += kRouteThreads) warp_cnt[i] = 0;
   __syncthreads();
 

@@ -75,6 +75,8 @@ __global__ void __launch_bounds__(kRowThreads)
 dispatch_rows_kernel(const uint4* __restrict__ src, const int32_t* __restrict__ dst_row,
                      const int32_t* __restrict__ row_src, const int32_t* __restrict__ num_mtiles,
                      uint4* __restrict__ dst, int64_t num_tokens, int topk, int vec_per_row, int token_blocks) {
+  grid_release();
+  grid_wait();
   constexpr int kRows = kRowThreads / TPR;
   if (static_cast<int>(blockIdx.x) >= token_blocks) {
     zero_padding(row_src, num_mtiles, dst, vec_per_row, (blockIdx.x - token_blocks) * (kRowThreads / 32) + (threadIdx.x >> 5),
@@ -318,6 +320,8 @@ template <typename T, int TPR, int SLOTS>
 __global__ void __launch_bounds__(kRowThreads)
 combine_topk_kernel(const uint4* __restrict__ ys, const T* __restrict__ scores, const int32_t* __restrict__ dst_row,
                     uint4* __restrict__ out, int64_t num_tokens, int topk, int vec_per_row) {
+  grid_release();
+  grid_wait();
   constexpr int kRows = kRowThreads / TPR;
   const int lane = threadIdx.x % TPR;
   for (int64_t t = static_cast<int64_t>(blockIdx.x) * kRows + threadIdx.x / TPR; t < num_tokens;
@@ -386,6 +390,8 @@ combine_bwd_tokens_kernel(const uint4* __restrict__ dout, const T* __restrict__ 
                           const int32_t* __restrict__ dst_row, const int32_t* __restrict__ row_src,
                           const int32_t* __restrict__ num_mtiles, uint4* __restrict__ gs, T* __restrict__ dscores,
                           int64_t num_slots, int topk, int vec_per_row, int slot_blocks) {
+  grid_release();
+  grid_wait();
   constexpr int kWarps = kRowThreads / 32;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (static_cast<int>(blockIdx.x) >= slot_blocks) {
@@ -484,8 +490,8 @@ static void launch_dispatch(const void* src, const int32_t* dst_row, const int32
   const int blocks = token_blocks + (row_src != nullptr ? sm_count() : 0);
   const uint4* in = static_cast<const uint4*>(src);
   uint4* out = static_cast<uint4*>(dst);
-  if (tpr == 32) dispatch_rows_kernel<32><<<blocks, kRowThreads, 0, s>>>(in, dst_row, row_src, num_mtiles, out, num_tokens, topk, vec_per_row, token_blocks);
-  else dispatch_rows_kernel<64><<<blocks, kRowThreads, 0, s>>>(in, dst_row, row_src, num_mtiles, out, num_tokens, topk, vec_per_row, token_blocks);
+  if (tpr == 32) launch_kernel(dispatch_rows_kernel<32>, blocks, kRowThreads, s, in, dst_row, row_src, num_mtiles, out, num_tokens, topk, vec_per_row, token_blocks);
+  else launch_kernel(dispatch_rows_kernel<64>, blocks, kRowThreads, s, in, dst_row, row_src, num_mtiles, out, num_tokens, topk, vec_per_row, token_blocks);
 }
 
 // The slots whose loads are issued together: the smallest power of two that covers topk, at most 8 (a wider one wastes
@@ -494,10 +500,10 @@ template <typename T, int TPR>
 static void launch_combine_slots(const uint4* ys, const T* scores, const int32_t* dst_row, uint4* out, int64_t num_tokens,
                                  int topk, int vec_per_row, cudaStream_t s) {
   const int grid = row_grid((num_tokens + kRowThreads / TPR - 1) / (kRowThreads / TPR));
-  if (topk == 1) combine_topk_kernel<T, TPR, 1><<<grid, kRowThreads, 0, s>>>(ys, scores, dst_row, out, num_tokens, topk, vec_per_row);
-  else if (topk == 2) combine_topk_kernel<T, TPR, 2><<<grid, kRowThreads, 0, s>>>(ys, scores, dst_row, out, num_tokens, topk, vec_per_row);
-  else if (topk <= 4) combine_topk_kernel<T, TPR, 4><<<grid, kRowThreads, 0, s>>>(ys, scores, dst_row, out, num_tokens, topk, vec_per_row);
-  else combine_topk_kernel<T, TPR, 8><<<grid, kRowThreads, 0, s>>>(ys, scores, dst_row, out, num_tokens, topk, vec_per_row);
+  if (topk == 1) launch_kernel(combine_topk_kernel<T, TPR, 1>, grid, kRowThreads, s, ys, scores, dst_row, out, num_tokens, topk, vec_per_row);
+  else if (topk == 2) launch_kernel(combine_topk_kernel<T, TPR, 2>, grid, kRowThreads, s, ys, scores, dst_row, out, num_tokens, topk, vec_per_row);
+  else if (topk <= 4) launch_kernel(combine_topk_kernel<T, TPR, 4>, grid, kRowThreads, s, ys, scores, dst_row, out, num_tokens, topk, vec_per_row);
+  else launch_kernel(combine_topk_kernel<T, TPR, 8>, grid, kRowThreads, s, ys, scores, dst_row, out, num_tokens, topk, vec_per_row);
 }
 
 template <typename T>
@@ -727,12 +733,12 @@ extern "C" int moe_combine_bwd_tokens(const void* dout, const void* scores, cons
   const int slot_blocks = row_grid((slots + kRowThreads / 32 - 1) / (kRowThreads / 32));
   const int blocks = slot_blocks + sm_count();
   if (dtype == MOE_DTYPE_BF16) {
-    combine_bwd_tokens_kernel<__nv_bfloat16><<<blocks, kRowThreads, 0, s>>>(
-        static_cast<const uint4*>(dout), static_cast<const __nv_bfloat16*>(scores), static_cast<const uint4*>(ys), dst_row,
+    launch_kernel(
+        combine_bwd_tokens_kernel<__nv_bfloat16>, blocks, kRowThreads, s, static_cast<const uint4*>(dout), static_cast<const __nv_bfloat16*>(scores), static_cast<const uint4*>(ys), dst_row,
         row_src, num_mtiles, static_cast<uint4*>(gs), static_cast<__nv_bfloat16*>(dscores), slots, topk, cols / 8, slot_blocks);
   } else {
-    combine_bwd_tokens_kernel<__half><<<blocks, kRowThreads, 0, s>>>(
-        static_cast<const uint4*>(dout), static_cast<const __half*>(scores), static_cast<const uint4*>(ys), dst_row, row_src,
+    launch_kernel(
+        combine_bwd_tokens_kernel<__half>, blocks, kRowThreads, s, static_cast<const uint4*>(dout), static_cast<const __half*>(scores), static_cast<const uint4*>(ys), dst_row, row_src,
         num_mtiles, static_cast<uint4*>(gs), static_cast<__half*>(dscores), slots, topk, cols / 8, slot_blocks);
   }
   MOE_CUDA(cudaGetLastError());
