@@ -67,6 +67,42 @@ int routing_metadata(const int64_t* expert_idx, int64_t num_rows, int num_expert
                      int32_t* num_mtiles, int32_t* status, void* workspace, size_t workspace_bytes,
                      bool workspace_always, void* stream);
 
+// The rows that exist in the padded layout (both null: all of them): see GemmArgs::group_indices.
+struct RowCounts {
+  const int32_t* pad_offsets = nullptr;
+  const int32_t* group_indices = nullptr;
+};
+
+// The entry points of the same names, told which rows exist.
+int mgrouped_gemm(const void* a, const void* w, void* out, void* pre_act, const int32_t* mtile_expert, const int32_t*
+                  tile_pairs, const int32_t* num_mtiles, int64_t padded_rows, int K, int N, int num_experts, int
+                  w_transposed, int act, int dtype, int chunk_index, int chunk_count, const moe_gemm_options* options,
+                  int32_t* status, void* stream, const RowCounts& counts);
+int mgrouped_gemm_gather(const void* src, int64_t src_rows, const int32_t* row_src, int div, const void* w, void* out,
+                         void* pre_act, const int32_t* mtile_expert, const int32_t* tile_pairs, const int32_t* num_mtiles,
+                         int64_t padded_rows, int K, int N, int num_experts, int act, int dtype, const moe_gemm_options*
+                         options, int32_t* status, void* stream, const RowCounts& counts);
+int mgrouped_gemm_combine(const void* a, const void* w, void* out, const int32_t* row_src, const void* scores, int topk,
+                          const int32_t* mtile_expert, const int32_t* tile_pairs, const int32_t* num_mtiles, int64_t
+                          padded_rows, int K, int N, int num_experts, int w_transposed, int dtype, const moe_gemm_options*
+                          options, int32_t* status, void* stream, const RowCounts& counts);
+int mgrouped_gemm_dglu(const void* g, const void* w, const void* pre_act, void* d_pre, const int32_t* mtile_expert, const
+                       int32_t* tile_pairs, const int32_t* num_mtiles, int64_t padded_rows, int K, int N, int num_experts,
+                       int act, int dtype, int chunk_index, int chunk_count, const moe_gemm_options* options, int32_t*
+                       status, void* stream, const RowCounts& counts);
+int kgrouped_gemm(const void* a, const void* b, void* dw, const int32_t* pad_offsets, int64_t padded_rows, int M, int N,
+                  int num_experts, int dtype, const moe_gemm_options* options, int32_t* status, void* stream, const
+                  RowCounts& counts);
+int kgrouped_gemm_gather(const void* src, int64_t src_rows, const int32_t* row_src, int div, const void* b, void* dw,
+                         const int32_t* pad_offsets, int64_t padded_rows, int M, int N, int num_experts, int dtype, const
+                         moe_gemm_options* options, int32_t* status, void* stream, const RowCounts& counts);
+
+int dispatch_rows(const void* src, const int32_t* dst_row, const int32_t* row_src, const int32_t* num_mtiles, void* dst,
+                  int64_t num_tokens, int topk, int64_t padded_rows, int cols, int dtype, void* stream, bool live_blocks_only);
+int combine_bwd_tokens(const void* dout, const void* scores, const void* ys, const int32_t* dst_row, const int32_t* row_src,
+                       const int32_t* num_mtiles, void* gs, void* dscores, int64_t num_tokens, int topk, int cols, int dtype,
+                       void* stream, bool live_blocks_only);
+
 // Status codes written by kernels into the caller's device status word.
 enum DeviceStatus : int {
   DS_OK = 0,

@@ -73,7 +73,11 @@ struct GemmArgs {
   const int32_t* tile_pairs;    // M-grouped, CTA pairs: first tile | expert << 20 | (pair has a second tile) << 31
   const int32_t* pair_prefix;   // M-grouped: exclusive prefix of the per-expert pair counts [E+1]
   const int32_t* num_mtiles;    // M-grouped: device int32[4] = {tiles in use, tile pairs in use, tile bound, 0}
-  const int32_t* pad_offsets;   // K-grouped: padded row offsets [E+1]
+  const int32_t* pad_offsets;   // K-grouped, and with group_indices: padded row offsets [E+1]
+  // Optional prefix of the routed rows per expert [E+1].  With it, only the 64-row blocks of an expert's padded range that
+  // hold a routed row exist: M-grouped kernels store nothing into the others (and the one-CTA kernels do not load them),
+  // K-grouped kernels contract over the others' rows not at all.
+  const int32_t* group_indices;
   int32_t mtiles_bound;         // M-grouped: padded_rows / 128 as the caller sees it (checked against num_mtiles[2])
   int32_t num_experts;
   int32_t m_dim;  // K-grouped: rows of each output matrix
@@ -129,7 +133,15 @@ struct TileCoord {
   int k_row0;   // K-grouped: first padded row of the contraction
   int kiters;   // number of BK-deep stages to contract
   bool active;  // false for the second CTA of a pair whose expert has an odd number of row tiles
+  int live;     // M-grouped: rows of the tile that exist (64 or 128, see GemmArgs::group_indices)
 };
+
+// Rows of expert e that exist, in whole 64-row blocks, at most its padded range (whatever the prefix says).
+__device__ __forceinline__ int live_rows(const GemmArgs& args, int e, int padded) {
+  if (args.group_indices == nullptr) return padded;
+  const int rows = (__ldg(args.group_indices + e + 1) - __ldg(args.group_indices + e) + 63) & ~63;
+  return rows < padded ? (rows > 0 ? rows : 0) : padded;
+}
 
 // ----------------------------------------------------------------------------------
 // Shared-memory matrix descriptors (64-bit) for tcgen05.mma.
@@ -294,7 +306,8 @@ __device__ __forceinline__ TileCoord decode_tile(int t, int mt, int nt, const Wi
     c.m0 = (m_idx * CTAS + rank) * BM;
     c.expert = expert;
     c.k_row0 = __ldg(args.pad_offsets + expert);
-    c.kiters = (__ldg(args.pad_offsets + expert + 1) - c.k_row0) / BK;  // padded ranges are multiples of 128
+    c.kiters = live_rows(args, expert, __ldg(args.pad_offsets + expert + 1) - c.k_row0) / BK;  // multiples of 64
+    c.live = BM;
   } else {
     int tile = m_idx;
     if (CTAS == 2) {
@@ -309,6 +322,12 @@ __device__ __forceinline__ TileCoord decode_tile(int t, int mt, int nt, const Wi
       c.expert = __ldg(args.mtile_expert + tile);
     }
     c.m0 = tile * BM;
+    c.live = BM;
+    if (args.group_indices != nullptr) {
+      const int base = __ldg(args.pad_offsets + c.expert);
+      const int left = live_rows(args, c.expert, 1 << 30) - (c.m0 - base);
+      c.live = left < BM ? (left > 64 ? left : 64) : BM;
+    }
     c.k_row0 = 0;
     c.kiters = (args.k_dim + BK - 1) / BK;
   }
@@ -577,9 +596,12 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
           const bool remote = kPair && rank != 0;
           const uint32_t fb = remote ? mapa_shared(full_bar + 8 * stage, 0) : full_bar + 8 * stage;
           const bool leader_lane = elect_one();
+          // one-CTA kernels (few rows per expert) fetch the A tile in halves and leave out a half without routed rows
+          constexpr bool kHalves = !KG && !kPair && !GATHER;
+          const bool both = !kHalves || c.live > 64;
           if (leader_lane) {
             if (remote) mbar_arrive_expect_tx_cluster(fb, Plan::kStageBytes);
-            else mbar_arrive_expect_tx(fb, Plan::kStageBytes);
+            else mbar_arrive_expect_tx(fb, both ? Plan::kStageBytes : Plan::kStageBytes - Plan::kABytes / 2);
           }
           if (gather) {
             // all 32 lanes: 4 rows x 128 bytes each = the whole 128 x 64 (or 64 x 128) A tile of the stage
@@ -644,6 +666,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
               }
             } else {
               if (!gather) tma_load_2d(sa, &tmap_a, kb * BK, c.m0, fb, pol);
+              if (kHalves && both) tma_load_2d(sa + Plan::kABytes / 2, &tmap_a, kb * BK, c.m0 + 64, fb, pol);
               if (B_K) {
                 tma_load_3d(sb, &tmap_b, kb * BK, c.n0 + bcol, c.expert, fb, pol);
               } else if (args.b_blocked) {
@@ -770,7 +793,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       if (t + num_units < ntiles) c_next = decode_tile<KG, CTAS>(t + num_units, mt, nt, win, args, BN, rank);
       const bool have_acc = c.kiters != 0;
       const int row = c.m0 + row_in_tile;
-      bool row_ok = c.active;
+      const bool quad_live = KG || (c.active && quad * 32 < c.live);  // this warp's 32 rows exist
+      bool row_ok = quad_live;
       long long out_row;  // row index into the output matrix
       T* row_out = out;  // base of the matrix this lane's row is stored into
       float row_scale = 1.0f;
@@ -809,7 +833,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         // The saved product does not depend on the accumulator: request the first chunk's tile before waiting
         // for the MMAs.  The buffer it lands in was last read by the store issued two chunks ago.
         const int col0 = c.n0 + chunk_begin * 32;
-        if (c.active && col0 < N && lane == 0) {
+        if (quad_live && col0 < N && lane == 0) {
           bulk_wait_read_all();
           const uint32_t bar = my_epi_bar + 8 * (q & 1);
           mbar_arrive_expect_tx(bar, Plan::kStagingTile);
@@ -823,7 +847,9 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         tc_fence_after();
       }
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + acc * BN;
-      if (EPI == EPI_ACT) {
+      if (!quad_live) {
+        // nothing to store
+      } else if (EPI == EPI_ACT) {
         // Plain store (optionally with an activation, optionally into another GPU's buffer, optionally scaled and
         // added into token-order rows): two 32-column chunks at a time go through the swizzled shared-memory tile so
         // that every store instruction of the warp writes four 128-byte row segments instead of 32 scattered
@@ -834,7 +860,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         // engine clips it at the edges of the matrix) instead of eight 16-byte stores per lane; the staging tile is
         // written again only after that store has read it.
         const bool tma_out = args.out_tma != 0;
-        const bool tile_stored = KG ? (c.m0 + quad * 32 < args.m_dim) : c.active;
+        const bool tile_stored = !KG || c.m0 + quad * 32 < args.m_dim;
 #pragma unroll 1
         for (int chunk = chunk_begin; chunk < chunk_begin + kChunksPerWarp; chunk += 2) {
 #pragma unroll
@@ -904,7 +930,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
 #pragma unroll 1
         for (int chunk = chunk_begin; chunk < chunk_begin + kChunksPerWarp; chunk += 2) {
           const int col0 = c.n0 + chunk * 32;
-          const bool live = c.active && col0 < N;  // uniform over the warp
+          const bool live = col0 < N;  // uniform over the warp
           const uint32_t buf = side_input ? stage_base + (q & 1) * Plan::kStagingTile : stage_base;
           if (side_input) {
             if (live) {
@@ -1069,7 +1095,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
 #pragma unroll 1
         for (int chunk = chunk_begin; chunk < chunk_begin + kChunksPerWarp; ++chunk) {
           const int col0 = c.n0 + chunk * 32;
-          const bool live = c.active && col0 < N;  // uniform over the warp
+          const bool live = col0 < N;  // uniform over the warp
           const uint32_t buf = stage_base + (q & 1) * Plan::kStagingTile;
           uint4 h_cur[8];
           if (live) {

@@ -191,6 +191,7 @@ struct MExtras {
   int combine_topk = 1;
   int chunk_index = 0;
   int chunk_count = 1;
+  RowCounts counts;
 };
 
 template <typename T, int BN, int CTAS>
@@ -200,7 +201,7 @@ static int mgrouped_dispatch(const void* a, const void* w, int64_t a_rows, int K
   const bool gather = args.a_row_src != nullptr;  // selects the kernel variant whose operand loads gather rows
   {
     const uint64_t dims[2] = {(uint64_t)K, (uint64_t)a_rows};
-    const uint32_t box[2] = {BK, args.a_row_src != nullptr ? 1u : (uint32_t)BM};
+    const uint32_t box[2] = {BK, args.a_row_src != nullptr ? 1u : (uint32_t)(CTAS == 1 ? BM / 2 : BM)};
     int rc = make_tmap(&ta, dtype, a, 2, dims, box);
     if (rc != MOE_OK) return rc;
   }
@@ -309,6 +310,8 @@ static int mgrouped_common(const char* name, const void* a, const void* w, void*
     args.align_experts = tile_pairs == nullptr ? 0 : (o.align_experts != 0 ? (o.align_experts > 0 ? 1 : 0)
                                                                           : (mean_rows >= 6 * 2 * BM ? 1 : 0));
   }
+  args.pad_offsets = x.counts.pad_offsets;
+  args.group_indices = x.counts.pad_offsets != nullptr ? x.counts.group_indices : nullptr;
   args.num_mtiles = num_mtiles;
   args.num_experts = E;
   args.n_dim = N;
@@ -409,7 +412,7 @@ static int kgrouped_dispatch(const void* a, const void* b, int64_t a_rows, int64
 static int kgrouped_common(const char* name, const void* a, int64_t gather_rows, const int32_t* gather_row_src,
                            int gather_div, const void* b, void* dw, const int32_t* pad_offsets, int64_t padded_rows, int M,
                            int N, int num_experts, int dtype, const moe_gemm_options* options, int32_t* status,
-                           void* stream) {
+                           void* stream, const int32_t* group_indices) {
   MOE_CHECK_ARG(a && b && dw && pad_offsets, "%s: null pointer argument", name);
   MOE_CHECK_ARG(aligned16(a) && aligned16(b) && aligned16(dw), "%s: pointers must be 16-byte aligned", name);
   MOE_CHECK_ARG(padded_rows > 0 && padded_rows % BM == 0, "%s: padded_rows=%lld must be a positive multiple of %d", name,
@@ -425,6 +428,7 @@ static int kgrouped_common(const char* name, const void* a, int64_t gather_rows,
   const moe_gemm_options o = resolve(options);
   GemmArgs args{};
   args.pad_offsets = pad_offsets;
+  args.group_indices = group_indices;
   args.num_experts = num_experts;
   args.m_dim = M;
   args.n_dim = N;
@@ -461,19 +465,17 @@ static int kgrouped_common(const char* name, const void* a, int64_t gather_rows,
 
 static bool act_is_glu(int act) { return act == MOE_ACT_SWIGLU || act == MOE_ACT_GEGLU; }
 
-}  // namespace moe
 
-using namespace moe;
-
-extern "C" int moe_mgrouped_gemm(const void* a, const void* w, void* out, void* pre_act, const int32_t* mtile_expert,
-                                 const int32_t* tile_pairs, const int32_t* num_mtiles, int64_t padded_rows, int K,
-                                 int N, int num_experts, int w_transposed, int act, int dtype, int chunk_index,
-                                 int chunk_count, const moe_gemm_options* options, int32_t* status, void* stream) {
+int mgrouped_gemm(const void* a, const void* w, void* out, void* pre_act, const int32_t* mtile_expert, const int32_t*
+                  tile_pairs, const int32_t* num_mtiles, int64_t padded_rows, int K, int N, int num_experts, int
+                  w_transposed, int act, int dtype, int chunk_index, int chunk_count, const moe_gemm_options* options,
+                  int32_t* status, void* stream, const RowCounts& counts) {
   MOE_CHECK_ARG(act >= MOE_ACT_NONE && act <= MOE_ACT_GELU_TANH, "moe_mgrouped_gemm: unknown activation %d", act);
   const bool glu = act_is_glu(act);
   MOE_CHECK_ARG(!(glu && w_transposed), "moe_mgrouped_gemm: gated activations need w as [E, K, N]");
   if (!glu && (act == MOE_ACT_NONE || pre_act == nullptr)) pre_act = nullptr;  // nothing to save without an activation
   MExtras x;
+  x.counts = counts;
   x.aux_out = pre_act;
   x.chunk_index = chunk_index;
   x.chunk_count = chunk_count;
@@ -482,16 +484,16 @@ extern "C" int moe_mgrouped_gemm(const void* a, const void* w, void* out, void* 
                          num_experts, w_transposed, epi, act, dtype, options, status, stream);
 }
 
-extern "C" int moe_mgrouped_gemm_gather(const void* src, int64_t src_rows, const int32_t* row_src, int div, const void* w,
-                                        void* out, void* pre_act, const int32_t* mtile_expert, const int32_t* tile_pairs,
-                                        const int32_t* num_mtiles, int64_t padded_rows, int K, int N, int num_experts,
-                                        int act, int dtype, const moe_gemm_options* options, int32_t* status,
-                                        void* stream) {
+int mgrouped_gemm_gather(const void* src, int64_t src_rows, const int32_t* row_src, int div, const void* w, void* out,
+                         void* pre_act, const int32_t* mtile_expert, const int32_t* tile_pairs, const int32_t* num_mtiles,
+                         int64_t padded_rows, int K, int N, int num_experts, int act, int dtype, const moe_gemm_options*
+                         options, int32_t* status, void* stream, const RowCounts& counts) {
   MOE_CHECK_ARG(act >= MOE_ACT_NONE && act <= MOE_ACT_GELU_TANH, "moe_mgrouped_gemm_gather: unknown activation %d", act);
   MOE_CHECK_ARG(row_src != nullptr, "moe_mgrouped_gemm_gather: row_src is null");
   const bool glu = act_is_glu(act);
   if (!glu && (act == MOE_ACT_NONE || pre_act == nullptr)) pre_act = nullptr;
   MExtras x;
+  x.counts = counts;
   x.aux_out = pre_act;
   x.gather_row_src = row_src;
   x.gather_div = div;
@@ -501,13 +503,13 @@ extern "C" int moe_mgrouped_gemm_gather(const void* src, int64_t src_rows, const
                          N, num_experts, 0, epi, act, dtype, options, status, stream);
 }
 
-extern "C" int moe_mgrouped_gemm_combine(const void* a, const void* w, void* out, const int32_t* row_src,
-                                         const void* scores, int topk, const int32_t* mtile_expert,
-                                         const int32_t* tile_pairs, const int32_t* num_mtiles, int64_t padded_rows, int K,
-                                         int N, int num_experts, int w_transposed, int dtype,
-                                         const moe_gemm_options* options, int32_t* status, void* stream) {
+int mgrouped_gemm_combine(const void* a, const void* w, void* out, const int32_t* row_src, const void* scores, int topk,
+                          const int32_t* mtile_expert, const int32_t* tile_pairs, const int32_t* num_mtiles, int64_t
+                          padded_rows, int K, int N, int num_experts, int w_transposed, int dtype, const moe_gemm_options*
+                          options, int32_t* status, void* stream, const RowCounts& counts) {
   MOE_CHECK_ARG(row_src != nullptr && out != nullptr, "moe_mgrouped_gemm_combine: null pointer argument");
   MExtras x;
+  x.counts = counts;
   x.combine_row_src = row_src;
   x.combine_scores = scores;
   x.combine_topk = topk;
@@ -515,20 +517,86 @@ extern "C" int moe_mgrouped_gemm_combine(const void* a, const void* w, void* out
                          N, num_experts, w_transposed, EPI_ACT, MOE_ACT_NONE, dtype, options, status, stream);
 }
 
-extern "C" int moe_mgrouped_gemm_dglu(const void* g, const void* w, const void* pre_act, void* d_pre,
-                                      const int32_t* mtile_expert, const int32_t* tile_pairs,
-                                      const int32_t* num_mtiles, int64_t padded_rows, int K, int N, int num_experts,
-                                      int act, int dtype, int chunk_index, int chunk_count,
-                                      const moe_gemm_options* options, int32_t* status, void* stream) {
+int mgrouped_gemm_dglu(const void* g, const void* w, const void* pre_act, void* d_pre, const int32_t* mtile_expert, const
+                       int32_t* tile_pairs, const int32_t* num_mtiles, int64_t padded_rows, int K, int N, int num_experts,
+                       int act, int dtype, int chunk_index, int chunk_count, const moe_gemm_options* options, int32_t*
+                       status, void* stream, const RowCounts& counts) {
   MOE_CHECK_ARG(act >= MOE_ACT_SILU && act <= MOE_ACT_GELU_TANH, "moe_mgrouped_gemm_dglu: activation %d has no derivative here",
                 act);
   MOE_CHECK_ARG(pre_act != nullptr, "moe_mgrouped_gemm_dglu: pre_act is null");
   MExtras x;
+  x.counts = counts;
   x.aux_in = pre_act;
   x.chunk_index = chunk_index;
   x.chunk_count = chunk_count;
   return mgrouped_common("moe_mgrouped_gemm_dglu", g, w, d_pre, x, mtile_expert, tile_pairs, num_mtiles, padded_rows, K, N,
                          num_experts, 1, act_is_glu(act) ? EPI_DGLU : EPI_ACT_AUX, act, dtype, options, status, stream);
+}
+
+int kgrouped_gemm(const void* a, const void* b, void* dw, const int32_t* pad_offsets, int64_t padded_rows, int M, int N,
+                  int num_experts, int dtype, const moe_gemm_options* options, int32_t* status, void* stream, const
+                  RowCounts& counts) {
+  return kgrouped_common("moe_kgrouped_gemm", a, 0, nullptr, 1, b, dw, pad_offsets, padded_rows, M, N, num_experts, dtype,
+                         options, status, stream, counts.group_indices);
+}
+
+int kgrouped_gemm_gather(const void* src, int64_t src_rows, const int32_t* row_src, int div, const void* b, void* dw,
+                         const int32_t* pad_offsets, int64_t padded_rows, int M, int N, int num_experts, int dtype, const
+                         moe_gemm_options* options, int32_t* status, void* stream, const RowCounts& counts) {
+  MOE_CHECK_ARG(row_src != nullptr, "moe_kgrouped_gemm_gather: row_src is null");
+  return kgrouped_common("moe_kgrouped_gemm_gather", src, src_rows, row_src, div, b, dw, pad_offsets, padded_rows, M, N,
+                         num_experts, dtype, options, status, stream, counts.group_indices);
+}
+
+}  // namespace moe
+
+using namespace moe;
+
+extern "C" int moe_mgrouped_gemm(const void* a, const void* w, void* out, void* pre_act, const int32_t* mtile_expert,
+                                 const int32_t* tile_pairs, const int32_t* num_mtiles, int64_t padded_rows, int K, int N,
+                                 int num_experts, int w_transposed, int act, int dtype, int chunk_index, int chunk_count,
+                                 const moe_gemm_options* options, int32_t* status, void* stream) {
+  return mgrouped_gemm(a, w, out, pre_act, mtile_expert, tile_pairs, num_mtiles, padded_rows, K, N, num_experts,
+                       w_transposed, act, dtype, chunk_index, chunk_count, options, status, stream, RowCounts{});
+}
+
+extern "C" int moe_mgrouped_gemm_gather(const void* src, int64_t src_rows, const int32_t* row_src, int div, const void* w,
+                                        void* out, void* pre_act, const int32_t* mtile_expert, const int32_t* tile_pairs,
+                                        const int32_t* num_mtiles, int64_t padded_rows, int K, int N, int num_experts, int
+                                        act, int dtype, const moe_gemm_options* options, int32_t* status, void* stream) {
+  return mgrouped_gemm_gather(src, src_rows, row_src, div, w, out, pre_act, mtile_expert, tile_pairs, num_mtiles,
+                              padded_rows, K, N, num_experts, act, dtype, options, status, stream, RowCounts{});
+}
+
+extern "C" int moe_mgrouped_gemm_combine(const void* a, const void* w, void* out, const int32_t* row_src, const void*
+                                         scores, int topk, const int32_t* mtile_expert, const int32_t* tile_pairs, const
+                                         int32_t* num_mtiles, int64_t padded_rows, int K, int N, int num_experts, int
+                                         w_transposed, int dtype, const moe_gemm_options* options, int32_t* status, void*
+                                         stream) {
+  return mgrouped_gemm_combine(a, w, out, row_src, scores, topk, mtile_expert, tile_pairs, num_mtiles, padded_rows, K, N,
+                               num_experts, w_transposed, dtype, options, status, stream, RowCounts{});
+}
+
+extern "C" int moe_mgrouped_gemm_dglu(const void* g, const void* w, const void* pre_act, void* d_pre, const int32_t*
+                                      mtile_expert, const int32_t* tile_pairs, const int32_t* num_mtiles, int64_t
+                                      padded_rows, int K, int N, int num_experts, int act, int dtype, int chunk_index, int
+                                      chunk_count, const moe_gemm_options* options, int32_t* status, void* stream) {
+  return mgrouped_gemm_dglu(g, w, pre_act, d_pre, mtile_expert, tile_pairs, num_mtiles, padded_rows, K, N, num_experts,
+                            act, dtype, chunk_index, chunk_count, options, status, stream, RowCounts{});
+}
+
+extern "C" int moe_kgrouped_gemm(const void* a, const void* b, void* dw, const int32_t* pad_offsets, int64_t padded_rows,
+                                 int M, int N, int num_experts, int dtype, const moe_gemm_options* options, int32_t*
+                                 status, void* stream) {
+  return kgrouped_gemm(a, b, dw, pad_offsets, padded_rows, M, N, num_experts, dtype, options, status, stream, RowCounts{});
+}
+
+extern "C" int moe_kgrouped_gemm_gather(const void* src, int64_t src_rows, const int32_t* row_src, int div, const void* b,
+                                        void* dw, const int32_t* pad_offsets, int64_t padded_rows, int M, int N, int
+                                        num_experts, int dtype, const moe_gemm_options* options, int32_t* status, void*
+                                        stream) {
+  return kgrouped_gemm_gather(src, src_rows, row_src, div, b, dw, pad_offsets, padded_rows, M, N, num_experts, dtype,
+                              options, status, stream, RowCounts{});
 }
 
 extern "C" int moe_mgrouped_gemm_push(const void* a, const void* w, void* const* peer_bases, const int32_t* dest_rank,
@@ -564,20 +632,4 @@ extern "C" int moe_mgrouped_gemm_scatter(const void* a, int64_t a_rows, const in
   }
   return mgrouped_common("moe_mgrouped_gemm_scatter", a, w, out, x, mtile_expert, tile_pairs, num_mtiles, padded_rows, K,
                          N, num_experts, w_transposed, EPI_ACT, act, dtype, options, status, stream);
-}
-
-extern "C" int moe_kgrouped_gemm(const void* a, const void* b, void* dw, const int32_t* pad_offsets,
-                                 int64_t padded_rows, int M, int N, int num_experts, int dtype,
-                                 const moe_gemm_options* options, int32_t* status, void* stream) {
-  return kgrouped_common("moe_kgrouped_gemm", a, 0, nullptr, 1, b, dw, pad_offsets, padded_rows, M, N, num_experts, dtype,
-                         options, status, stream);
-}
-
-extern "C" int moe_kgrouped_gemm_gather(const void* src, int64_t src_rows, const int32_t* row_src, int div, const void* b,
-                                        void* dw, const int32_t* pad_offsets, int64_t padded_rows, int M, int N,
-                                        int num_experts, int dtype, const moe_gemm_options* options, int32_t* status,
-                                        void* stream) {
-  MOE_CHECK_ARG(row_src != nullptr, "moe_kgrouped_gemm_gather: row_src is null");
-  return kgrouped_common("moe_kgrouped_gemm_gather", src, src_rows, row_src, div, b, dw, pad_offsets, padded_rows, M, N,
-                         num_experts, dtype, options, status, stream);
 }

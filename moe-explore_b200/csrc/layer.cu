@@ -33,6 +33,7 @@ extern "C" int moe_expert_forward(const moe_expert_pass* p, int steps, void* str
   const int up_cols = glu(p->act) ? 2 * p->inter : p->inter;
   const int64_t rows = p->num_tokens * p->topk;
   const Chain chain;
+  const RowCounts counts{p->pad_offsets, p->group_indices};
   if (steps & MOE_FWD_ROUTE)
     MOE_STEP(routing_metadata(p->expert_idx, rows, p->num_experts, p->group_indices, nullptr, p->pad_offsets, p->row_src,
                               p->dst_row, p->mtile_expert, p->tile_pairs, p->num_mtiles, p->status, p->workspace,
@@ -40,31 +41,31 @@ extern "C" int moe_expert_forward(const moe_expert_pass* p, int steps, void* str
   if ((steps & MOE_FWD_DISPATCH) && !p->gather) {
     // rows do not mix in a forward pass, and only a weight gradient contracts over the padding rows
     if (p->keep)
-      MOE_STEP(moe_dispatch_rows(p->x, p->dst_row, p->row_src, p->num_mtiles, p->xs, p->num_tokens, p->topk, p->padded_rows, p->d,
-                                 p->dtype, stream));
+      MOE_STEP(dispatch_rows(p->x, p->dst_row, p->row_src, p->num_mtiles, p->xs, p->num_tokens, p->topk, p->padded_rows, p->d,
+                                 p->dtype, stream, true));
     else
       MOE_STEP(moe_dispatch_rows_only(p->x, p->dst_row, p->xs, p->num_tokens, p->topk, p->d, p->dtype, stream));
   }
   if (steps & MOE_FWD_UP) {
     if (p->gather)
-      MOE_STEP(moe_mgrouped_gemm_gather(p->x, p->num_tokens, p->row_src, p->topk, p->w1, p->hidden, p->pre_act, p->mtile_expert,
+      MOE_STEP(mgrouped_gemm_gather(p->x, p->num_tokens, p->row_src, p->topk, p->w1, p->hidden, p->pre_act, p->mtile_expert,
                                         p->tile_pairs, p->num_mtiles, p->padded_rows, p->d, up_cols, p->num_experts, p->act,
-                                        p->dtype, nullptr, p->status, stream));
+                                        p->dtype, nullptr, p->status, stream, counts));
     else
-      MOE_STEP(moe_mgrouped_gemm(p->xs, p->w1, p->hidden, p->pre_act, p->mtile_expert, p->tile_pairs, p->num_mtiles,
+      MOE_STEP(mgrouped_gemm(p->xs, p->w1, p->hidden, p->pre_act, p->mtile_expert, p->tile_pairs, p->num_mtiles,
                                  p->padded_rows, p->d, up_cols, p->num_experts, 0, p->act, p->dtype, 0, 1, nullptr, p->status,
-                                 stream));
+                                 stream, counts));
   }
   if (steps & MOE_FWD_DOWN) {
     if (p->fused_combine) {
       MOE_CUDA(cudaMemsetAsync(p->out, 0, static_cast<size_t>(p->num_tokens) * p->d * 2, static_cast<cudaStream_t>(stream)));
       chained_launches() = false;  // the memset stands between
-      MOE_STEP(moe_mgrouped_gemm_combine(p->hidden, p->w2, p->out, p->row_src, p->scores, p->topk, p->mtile_expert, p->tile_pairs,
+      MOE_STEP(mgrouped_gemm_combine(p->hidden, p->w2, p->out, p->row_src, p->scores, p->topk, p->mtile_expert, p->tile_pairs,
                                          p->num_mtiles, p->padded_rows, p->inter, p->d, p->num_experts, 0, p->dtype, nullptr,
-                                         p->status, stream));
+                                         p->status, stream, counts));
     } else {
-      MOE_STEP(moe_mgrouped_gemm(p->hidden, p->w2, p->ys, nullptr, p->mtile_expert, p->tile_pairs, p->num_mtiles, p->padded_rows,
-                                 p->inter, p->d, p->num_experts, 0, MOE_ACT_NONE, p->dtype, 0, 1, nullptr, p->status, stream));
+      MOE_STEP(mgrouped_gemm(p->hidden, p->w2, p->ys, nullptr, p->mtile_expert, p->tile_pairs, p->num_mtiles, p->padded_rows,
+                                 p->inter, p->d, p->num_experts, 0, MOE_ACT_NONE, p->dtype, 0, 1, nullptr, p->status, stream, counts));
     }
   }
   if ((steps & MOE_FWD_FOLD) && !p->fused_combine)
@@ -76,33 +77,34 @@ extern "C" int moe_expert_backward(const moe_expert_pass* p, int steps, void* st
   MOE_CHECK_ARG(p != nullptr, "moe_expert_backward: null pointer argument");
   const int up_cols = glu(p->act) ? 2 * p->inter : p->inter;
   const Chain chain;
+  const RowCounts counts{p->pad_offsets, p->group_indices};
   if (steps & MOE_BWD_FOLD)
-    MOE_STEP(moe_combine_bwd_tokens(p->grad_out, p->scores, p->ys, p->dst_row, p->row_src, p->num_mtiles, p->gs, p->d_scores,
-                                    p->num_tokens, p->topk, p->d, p->dtype, stream));
+    MOE_STEP(combine_bwd_tokens(p->grad_out, p->scores, p->ys, p->dst_row, p->row_src, p->num_mtiles, p->gs, p->d_scores,
+                                    p->num_tokens, p->topk, p->d, p->dtype, stream, true));
   if (steps & MOE_BWD_DOWN) {
     if (p->act == MOE_ACT_NONE)  // linear "activation": d_pre = gs @ W2^T
-      MOE_STEP(moe_mgrouped_gemm(p->gs, p->w2, p->d_pre, nullptr, p->mtile_expert, p->tile_pairs, p->num_mtiles, p->padded_rows,
-                                 p->d, p->inter, p->num_experts, 1, MOE_ACT_NONE, p->dtype, 0, 1, nullptr, p->status, stream));
+      MOE_STEP(mgrouped_gemm(p->gs, p->w2, p->d_pre, nullptr, p->mtile_expert, p->tile_pairs, p->num_mtiles, p->padded_rows,
+                                 p->d, p->inter, p->num_experts, 1, MOE_ACT_NONE, p->dtype, 0, 1, nullptr, p->status, stream, counts));
     else
-      MOE_STEP(moe_mgrouped_gemm_dglu(p->gs, p->w2, p->pre_act, p->d_pre, p->mtile_expert, p->tile_pairs, p->num_mtiles,
+      MOE_STEP(mgrouped_gemm_dglu(p->gs, p->w2, p->pre_act, p->d_pre, p->mtile_expert, p->tile_pairs, p->num_mtiles,
                                       p->padded_rows, p->d, p->inter, p->num_experts, p->act, p->dtype, 0, 1, nullptr, p->status,
-                                      stream));
+                                      stream, counts));
   }
   if (steps & MOE_BWD_UP)
-    MOE_STEP(moe_mgrouped_gemm(p->d_pre, p->w1, p->dxs, nullptr, p->mtile_expert, p->tile_pairs, p->num_mtiles, p->padded_rows,
-                               up_cols, p->d, p->num_experts, 1, MOE_ACT_NONE, p->dtype, 0, 1, nullptr, p->status, stream));
+    MOE_STEP(mgrouped_gemm(p->d_pre, p->w1, p->dxs, nullptr, p->mtile_expert, p->tile_pairs, p->num_mtiles, p->padded_rows,
+                               up_cols, p->d, p->num_experts, 1, MOE_ACT_NONE, p->dtype, 0, 1, nullptr, p->status, stream, counts));
   if (steps & MOE_BWD_FOLD_DX)
     MOE_STEP(moe_combine_topk(p->dxs, nullptr, p->dst_row, p->dx, p->num_tokens, p->topk, p->d, p->dtype, stream));
   if (steps & MOE_BWD_DW1) {
     if (p->gather)  // x is the layer input in token order: its rows are gathered by the loads again
-      MOE_STEP(moe_kgrouped_gemm_gather(p->x, p->num_tokens, p->row_src, p->topk, p->d_pre, p->d_w1, p->pad_offsets,
-                                        p->padded_rows, p->d, up_cols, p->num_experts, p->dtype, nullptr, p->status, stream));
+      MOE_STEP(kgrouped_gemm_gather(p->x, p->num_tokens, p->row_src, p->topk, p->d_pre, p->d_w1, p->pad_offsets,
+                                        p->padded_rows, p->d, up_cols, p->num_experts, p->dtype, nullptr, p->status, stream, counts));
     else
-      MOE_STEP(moe_kgrouped_gemm(p->xs, p->d_pre, p->d_w1, p->pad_offsets, p->padded_rows, p->d, up_cols, p->num_experts, p->dtype,
-                                 nullptr, p->status, stream));
+      MOE_STEP(kgrouped_gemm(p->xs, p->d_pre, p->d_w1, p->pad_offsets, p->padded_rows, p->d, up_cols, p->num_experts, p->dtype,
+                                 nullptr, p->status, stream, counts));
   }
   if (steps & MOE_BWD_DW2)
-    MOE_STEP(moe_kgrouped_gemm(p->hidden, p->gs, p->d_w2, p->pad_offsets, p->padded_rows, p->inter, p->d, p->num_experts, p->dtype,
-                               nullptr, p->status, stream));
+    MOE_STEP(kgrouped_gemm(p->hidden, p->gs, p->d_w2, p->pad_offsets, p->padded_rows, p->inter, p->d, p->num_experts, p->dtype,
+                               nullptr, p->status, stream, counts));
   return MOE_OK;
 }

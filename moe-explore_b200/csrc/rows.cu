@@ -49,16 +49,21 @@ copy_rows_kernel(const uint4* __restrict__ src, const Index* __restrict__ index,
   }
 }
 
-// Zeroes the padding rows (row_src < 0) among the rows in use: a warp looks at 32 rows at a time (one load and a ballot;
-// a load per row made this the longest part of a dispatch) and clears the ones it finds.
+// Zeroes the padding rows (row_src < 0) among the rows in use: a warp looks at 64 rows at a time (two loads and ballots;
+// a load per row made this the longest part of a dispatch) and clears the ones it finds.  `live_blocks_only`: 64-row blocks
+// without a routed row are left alone.
 __device__ __forceinline__ void zero_padding(const int32_t* __restrict__ row_src, const int32_t* __restrict__ num_mtiles,
-                                             uint4* __restrict__ dst, int vec_per_row, int warp, int warps) {
-  const int64_t rows_in_use = static_cast<int64_t>(*num_mtiles) * MOE_TILE_M;  // a multiple of 32
+                                             uint4* __restrict__ dst, int vec_per_row, int warp, int warps,
+                                             bool live_blocks_only) {
+  const int64_t rows_in_use = static_cast<int64_t>(*num_mtiles) * MOE_TILE_M;  // a multiple of 64
   const int lane = threadIdx.x & 31;
-  for (int64_t p0 = static_cast<int64_t>(warp) * 32; p0 < rows_in_use; p0 += static_cast<int64_t>(warps) * 32) {
-    unsigned pads = __ballot_sync(0xFFFFFFFFu, row_src[p0 + lane] < 0);
+  for (int64_t p0 = static_cast<int64_t>(warp) * 64; p0 < rows_in_use; p0 += static_cast<int64_t>(warps) * 64) {
+    const unsigned lo = __ballot_sync(0xFFFFFFFFu, row_src[p0 + lane] < 0);
+    const unsigned hi = __ballot_sync(0xFFFFFFFFu, row_src[p0 + 32 + lane] < 0);
+    unsigned long long pads = (static_cast<unsigned long long>(hi) << 32) | lo;
+    if (live_blocks_only && pads == ~0ull) continue;
     while (pads != 0) {
-      const int b = __ffs(pads) - 1;
+      const int b = __ffsll(static_cast<long long>(pads)) - 1;
       pads &= pads - 1;
       uint4* d = dst + (p0 + b) * vec_per_row;
       for (int v = lane; v < vec_per_row; v += 32) d[v] = make_uint4(0, 0, 0, 0);
@@ -74,13 +79,14 @@ template <int TPR>
 __global__ void __launch_bounds__(kRowThreads)
 dispatch_rows_kernel(const uint4* __restrict__ src, const int32_t* __restrict__ dst_row,
                      const int32_t* __restrict__ row_src, const int32_t* __restrict__ num_mtiles,
-                     uint4* __restrict__ dst, int64_t num_tokens, int topk, int vec_per_row, int token_blocks) {
+                     uint4* __restrict__ dst, int64_t num_tokens, int topk, int vec_per_row, int token_blocks,
+                     bool live_blocks_only) {
   grid_release();
   grid_wait();
   constexpr int kRows = kRowThreads / TPR;
   if (static_cast<int>(blockIdx.x) >= token_blocks) {
     zero_padding(row_src, num_mtiles, dst, vec_per_row, (blockIdx.x - token_blocks) * (kRowThreads / 32) + (threadIdx.x >> 5),
-                 (gridDim.x - token_blocks) * (kRowThreads / 32));
+                 (gridDim.x - token_blocks) * (kRowThreads / 32), live_blocks_only);
     return;
   }
   const int lane = threadIdx.x % TPR;
@@ -389,14 +395,14 @@ __global__ void __launch_bounds__(kRowThreads)
 combine_bwd_tokens_kernel(const uint4* __restrict__ dout, const T* __restrict__ scores, const uint4* __restrict__ ys,
                           const int32_t* __restrict__ dst_row, const int32_t* __restrict__ row_src,
                           const int32_t* __restrict__ num_mtiles, uint4* __restrict__ gs, T* __restrict__ dscores,
-                          int64_t num_slots, int topk, int vec_per_row, int slot_blocks) {
+                          int64_t num_slots, int topk, int vec_per_row, int slot_blocks, bool live_blocks_only) {
   grid_release();
   grid_wait();
   constexpr int kWarps = kRowThreads / 32;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (static_cast<int>(blockIdx.x) >= slot_blocks) {
     zero_padding(row_src, num_mtiles, gs, vec_per_row, (blockIdx.x - slot_blocks) * kWarps + warp,
-                 (gridDim.x - slot_blocks) * kWarps);
+                 (gridDim.x - slot_blocks) * kWarps, live_blocks_only);
     return;
   }
   for (int64_t j = static_cast<int64_t>(blockIdx.x) * kWarps + warp; j < num_slots;
@@ -453,7 +459,7 @@ __global__ void __launch_bounds__(kRowThreads)
 zero_padding_rows_kernel(const int32_t* __restrict__ row_src, const int32_t* __restrict__ num_mtiles, uint4* __restrict__ dst,
                          int vec_per_row) {
   zero_padding(row_src, num_mtiles, dst, vec_per_row, blockIdx.x * (kRowThreads / 32) + (threadIdx.x >> 5),
-               gridDim.x * (kRowThreads / 32));
+               gridDim.x * (kRowThreads / 32), false);
 }
 
 static int row_grid(int64_t rows) {
@@ -483,15 +489,15 @@ static void launch_copy_rows(const void* src, const Index* index, const int32_t*
 
 // row_src == nullptr: the padding rows are left as they are.
 static void launch_dispatch(const void* src, const int32_t* dst_row, const int32_t* row_src, const int32_t* num_mtiles, void* dst,
-                            int64_t num_tokens, int topk, int vec_per_row, cudaStream_t s) {
+                            int64_t num_tokens, int topk, int vec_per_row, cudaStream_t s, bool live_blocks_only = false) {
   const int tpr = copy_threads_per_row(vec_per_row);
   const int64_t groups = (num_tokens + kRowThreads / tpr - 1) / (kRowThreads / tpr);
   const int token_blocks = static_cast<int>(groups < (1 << 30) ? groups : (1 << 30));
   const int blocks = token_blocks + (row_src != nullptr ? sm_count() : 0);
   const uint4* in = static_cast<const uint4*>(src);
   uint4* out = static_cast<uint4*>(dst);
-  if (tpr == 32) launch_kernel(dispatch_rows_kernel<32>, blocks, kRowThreads, s, in, dst_row, row_src, num_mtiles, out, num_tokens, topk, vec_per_row, token_blocks);
-  else launch_kernel(dispatch_rows_kernel<64>, blocks, kRowThreads, s, in, dst_row, row_src, num_mtiles, out, num_tokens, topk, vec_per_row, token_blocks);
+  if (tpr == 32) launch_kernel(dispatch_rows_kernel<32>, blocks, kRowThreads, s, in, dst_row, row_src, num_mtiles, out, num_tokens, topk, vec_per_row, token_blocks, live_blocks_only);
+  else launch_kernel(dispatch_rows_kernel<64>, blocks, kRowThreads, s, in, dst_row, row_src, num_mtiles, out, num_tokens, topk, vec_per_row, token_blocks, live_blocks_only);
 }
 
 // The slots whose loads are issued together: the smallest power of two that covers topk, at most 8 (a wider one wastes
@@ -584,16 +590,24 @@ extern "C" int moe_gather_rows(const void* src, int64_t src_rows, const int32_t*
   return MOE_OK;
 }
 
-extern "C" int moe_dispatch_rows(const void* src, const int32_t* dst_row, const int32_t* row_src,
-                                 const int32_t* num_mtiles, void* dst, int64_t num_tokens, int topk,
-                                 int64_t padded_rows, int cols, int dtype, void* stream) {
+namespace moe {
+int dispatch_rows(const void* src, const int32_t* dst_row, const int32_t* row_src, const int32_t* num_mtiles, void* dst,
+                  int64_t num_tokens, int topk, int64_t padded_rows, int cols, int dtype, void* stream, bool
+                  live_blocks_only) {
   MOE_CHECK_ARG(num_tokens >= 0 && topk > 0 && padded_rows > 0, "moe_dispatch_rows: bad sizes");
   MOE_CHECK_ARG(src && dst_row && row_src && num_mtiles && dst, "moe_dispatch_rows: null pointer argument");
   MOE_CHECK_ARG(aligned16(src) && aligned16(dst), "moe_dispatch_rows: pointers must be 16-byte aligned");
   MOE_ROW_COMMON_CHECKS("moe_dispatch_rows", cols, dtype);
-  launch_dispatch(src, dst_row, row_src, num_mtiles, dst, num_tokens, topk, cols / 8, static_cast<cudaStream_t>(stream));
+  launch_dispatch(src, dst_row, row_src, num_mtiles, dst, num_tokens, topk, cols / 8, static_cast<cudaStream_t>(stream), live_blocks_only);
   MOE_CUDA(cudaGetLastError());
   return MOE_OK;
+}
+}  // namespace moe
+
+extern "C" int moe_dispatch_rows(const void* src, const int32_t* dst_row, const int32_t* row_src, const int32_t*
+                                 num_mtiles, void* dst, int64_t num_tokens, int topk, int64_t padded_rows, int cols, int
+                                 dtype, void* stream) {
+  return dispatch_rows(src, dst_row, row_src, num_mtiles, dst, num_tokens, topk, padded_rows, cols, dtype, stream, false);
 }
 
 extern "C" int moe_dispatch_rows_only(const void* src, const int32_t* dst_row, void* dst, int64_t num_tokens, int topk,
@@ -720,9 +734,10 @@ extern "C" int moe_combine_topk(const void* ys, const void* scores, const int32_
   return MOE_OK;
 }
 
-extern "C" int moe_combine_bwd_tokens(const void* dout, const void* scores, const void* ys, const int32_t* dst_row,
-                                      const int32_t* row_src, const int32_t* num_mtiles, void* gs, void* dscores,
-                                      int64_t num_tokens, int topk, int cols, int dtype, void* stream) {
+namespace moe {
+int combine_bwd_tokens(const void* dout, const void* scores, const void* ys, const int32_t* dst_row, const int32_t*
+                       row_src, const int32_t* num_mtiles, void* gs, void* dscores, int64_t num_tokens, int topk, int
+                       cols, int dtype, void* stream, bool live_blocks_only) {
   MOE_CHECK_ARG(dout && scores && ys && dst_row && row_src && num_mtiles && gs && dscores,
                 "moe_combine_bwd_tokens: null pointer argument");
   MOE_CHECK_ARG(aligned16(dout) && aligned16(ys) && aligned16(gs), "moe_combine_bwd_tokens: pointers must be 16-byte aligned");
@@ -735,14 +750,22 @@ extern "C" int moe_combine_bwd_tokens(const void* dout, const void* scores, cons
   if (dtype == MOE_DTYPE_BF16) {
     launch_kernel(
         combine_bwd_tokens_kernel<__nv_bfloat16>, blocks, kRowThreads, s, static_cast<const uint4*>(dout), static_cast<const __nv_bfloat16*>(scores), static_cast<const uint4*>(ys), dst_row,
-        row_src, num_mtiles, static_cast<uint4*>(gs), static_cast<__nv_bfloat16*>(dscores), slots, topk, cols / 8, slot_blocks);
+        row_src, num_mtiles, static_cast<uint4*>(gs), static_cast<__nv_bfloat16*>(dscores), slots, topk, cols / 8, slot_blocks, live_blocks_only);
   } else {
     launch_kernel(
         combine_bwd_tokens_kernel<__half>, blocks, kRowThreads, s, static_cast<const uint4*>(dout), static_cast<const __half*>(scores), static_cast<const uint4*>(ys), dst_row, row_src,
-        num_mtiles, static_cast<uint4*>(gs), static_cast<__half*>(dscores), slots, topk, cols / 8, slot_blocks);
+        num_mtiles, static_cast<uint4*>(gs), static_cast<__half*>(dscores), slots, topk, cols / 8, slot_blocks, live_blocks_only);
   }
   MOE_CUDA(cudaGetLastError());
   return MOE_OK;
+}
+}  // namespace moe
+
+extern "C" int moe_combine_bwd_tokens(const void* dout, const void* scores, const void* ys, const int32_t* dst_row, const
+                                      int32_t* row_src, const int32_t* num_mtiles, void* gs, void* dscores, int64_t
+                                      num_tokens, int topk, int cols, int dtype, void* stream) {
+  return combine_bwd_tokens(dout, scores, ys, dst_row, row_src, num_mtiles, gs, dscores, num_tokens, topk, cols, dtype,
+                            stream, false);
 }
 
 extern "C" int moe_combine_bwd(const void* dout, const void* scores, const void* ys, const int32_t* row_src,

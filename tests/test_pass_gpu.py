@@ -1,0 +1,64 @@
+"""A pass over the experts where whole 64-row blocks of the padded layout hold no routed row: those blocks are neither written nor
+read, so whatever the allocator hands out there (here: NaN) must not reach a result."""
+import pytest
+import torch
+
+from moe_explore.expert_compute import expert_compute, routed_expert_compute
+from moe_explore.routing_plan import build_routing_plan
+from oracle import moe_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _poison(mb=512):
+    blocks = [torch.full((n << 18,), float("nan"), device="cuda") for n in (1, 1, 2, 4, 8, 16, 32, mb // 4)]
+    del blocks
+
+
+def _relerr(a, b):
+    return float((a.float() - b.float()).abs().max() / b.float().abs().max().clamp_min(1e-30))
+
+
+@pytest.mark.parametrize("act", ["swiglu", "gelu"])
+@pytest.mark.parametrize("rows", [
+    (1, 63, 64, 65, 127, 128, 129, 0, 2),       # one-CTA kernels: at most one row tile per expert on average
+    (33, 0, 0, 1),                              # empty experts, weight gradients over one 64-row step
+    (193, 255, 256, 257, 320, 0, 449, 129),     # CTA pairs with a half-empty second tile
+])
+def test_blocks_without_rows_do_not_leak(rows, act, native):
+    d, inter, E = 136, 200, len(rows)
+    ids = torch.repeat_interleave(torch.arange(E), torch.tensor(rows))
+    g = torch.Generator().manual_seed(len(ids))
+    ids = ids[torch.randperm(len(ids), generator=g)].view(-1, 1).cuda()
+    T = ids.size(0)
+    gen = torch.Generator(device="cuda").manual_seed(T)
+    mk = lambda *s, std=1.0: (torch.randn(*s, generator=gen, device="cuda") * std).bfloat16()
+    up = 2 * inter if act == "swiglu" else inter
+    leaves = [mk(T, d), torch.rand(T, 1, generator=gen, device="cuda").bfloat16(), mk(E, d, up, std=0.1), mk(E, inter, d, std=0.1)]
+    grad = mk(T, d)
+
+    def run(how):
+        p = [t.clone().requires_grad_() for t in leaves]
+        _poison()
+        out = how(p)
+        _poison()
+        return [out.detach()] + list(torch.autograd.grad(out, p, grad))
+
+    routed = run(lambda p: routed_expert_compute(*p, ids, E, 1, act))
+    planned = run(lambda p: expert_compute(*p, build_routing_plan(ids, E, 1), act))
+    gathered = run(lambda p: routed_expert_compute(*p, ids, E, 1, act, gather_in_gemm=True))
+    f = [t.float().requires_grad_() for t in leaves]
+    ref = O.expert_compute(f[0], f[1], ids, f[2], f[3], act)
+    expect = [ref.detach()] + list(torch.autograd.grad(ref, f, grad.float()))
+    for a, b, c, e in zip(routed, planned, gathered, expect):
+        assert torch.equal(a, b) and torch.equal(a, c)
+        assert _relerr(a, e) <= 2e-2     # bf16 storage of every intermediate row, as in the layer tests
+    for e, n in enumerate(rows):
+        if n == 0:
+            assert not routed[3][e].any() and not routed[4][e].any()
+    with torch.no_grad():
+        _poison()
+        assert torch.equal(routed_expert_compute(*leaves, ids, E, 1, act), routed[0])
+        _poison()
+        assert _relerr(routed_expert_compute(*leaves, ids, E, 1, act, fused_combine=True), expect[0]) <= 2e-2
+    assert native.read_status(build_routing_plan(ids, E, 1).status) == 0
