@@ -445,6 +445,32 @@ int moe_expert_forward(const moe_expert_pass* pass, int steps, void* stream);
 #define MOE_BWD_ALL 63
 int moe_expert_backward(const moe_expert_pass* pass, int steps, void* stream);
 
+/* The functional grouped GEMM in one call, rows grouped by `group_indices` [num_experts + 1]:
+ *   out[o(r)] = act(a[i(r)] @ w[expert of r]) for sorted rows r < num_rows, w [num_experts, k_dim, n_dim];
+ *   i(r) = perm[r] / topk with gather, else r;  o(r) = perm[r] with scatter, else r.
+ * MOE_ROWS_LAYOUT writes the maps, MOE_ROWS_GATHER copies gathered rows into `padded` [moe_padded_rows_bound, k_dim] (unused
+ * without gather), MOE_ROWS_GEMM contracts; rows that are in expert order already are read where they are.
+ * The maps are the caller's buffers: pad_offsets [num_experts + 1], in_rows and out_rows [moe_padded_rows_bound],
+ * mtile_expert, tile_pairs and num_mtiles as in moe_routing_metadata.  Negative entries of perm: a zero input row / not stored. */
+typedef struct moe_rows_pass {
+  int64_t num_rows, a_rows;
+  int32_t num_experts, k_dim, n_dim, topk, act, dtype, gather, scatter;
+  const void *a, *w;
+  void* out;
+  const int32_t* group_indices;
+  const int64_t* perm;
+  int32_t *pad_offsets, *in_rows, *out_rows, *mtile_expert, *tile_pairs, *num_mtiles, *status;
+  void* padded;
+} moe_rows_pass;
+
+size_t moe_rows_pass_size(void);
+
+#define MOE_ROWS_LAYOUT 1
+#define MOE_ROWS_GATHER 2
+#define MOE_ROWS_GEMM 4
+#define MOE_ROWS_ALL 7
+int moe_rows_gemm(const moe_rows_pass* pass, int steps, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

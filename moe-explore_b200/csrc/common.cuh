@@ -47,6 +47,22 @@ int sm_count();  // SM count of the current device (cached per device)
 // order of the stream holds for all earlier kernels too.  Thread-local and set only for the duration of such a call.
 bool& chained_launches();
 
+class Chain {
+ public:
+  Chain() { chained_launches() = false; }
+  ~Chain() { chained_launches() = false; }
+};
+
+#define MOE_STEP(call)                  \
+  do {                                  \
+    const int rc__ = (call);            \
+    if (rc__ != MOE_OK) return rc__;    \
+    ::moe::chained_launches() = true;   \
+  } while (0)
+
+// In a row map for moe_gather_rows: leave the row of dst as it is.
+constexpr int32_t kSkipRow = -2;
+
 template <typename... Params, typename... Args>
 inline cudaError_t launch_kernel(void (*kernel)(Params...), int grid, int block, cudaStream_t stream, Args... args) {
   cudaLaunchConfig_t cfg = {};
@@ -97,6 +113,12 @@ int kgrouped_gemm_gather(const void* src, int64_t src_rows, const int32_t* row_s
                          const int32_t* pad_offsets, int64_t padded_rows, int M, int N, int num_experts, int dtype, const
                          moe_gemm_options* options, int32_t* status, void* stream, const RowCounts& counts);
 
+// Grouped GEMM whose row p goes to out_rows[p] (negative: nowhere), gated activations included; compact_rows >= 0: `a` holds
+// that many rows in expert order without padding.
+int mgrouped_gemm_rows(const void* a, int64_t compact_rows, const void* w, void* out, const int32_t* out_rows,
+                       const int32_t* mtile_expert, const int32_t* tile_pairs, const int32_t* num_mtiles, int64_t padded_rows,
+                       int K, int N, int num_experts, int act, int dtype, int32_t* status, void* stream,
+                       const RowCounts& counts);
 int dispatch_rows(const void* src, const int32_t* dst_row, const int32_t* row_src, const int32_t* num_mtiles, void* dst,
                   int64_t num_tokens, int topk, int64_t padded_rows, int cols, int dtype, void* stream, bool live_blocks_only);
 int combine_bwd_tokens(const void* dout, const void* scores, const void* ys, const int32_t* dst_row, const int32_t* row_src,

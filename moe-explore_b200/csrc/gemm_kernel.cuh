@@ -78,6 +78,7 @@ struct GemmArgs {
   // hold a routed row exist: M-grouped kernels store nothing into the others (and the one-CTA kernels do not load them),
   // K-grouped kernels contract over the others' rows not at all.
   const int32_t* group_indices;
+  int32_t a_compact;            // M-grouped, with group_indices: A holds the routed rows without padding, expert by expert
   int32_t mtiles_bound;         // M-grouped: padded_rows / 128 as the caller sees it (checked against num_mtiles[2])
   int32_t num_experts;
   int32_t m_dim;  // K-grouped: rows of each output matrix
@@ -98,7 +99,7 @@ struct GemmArgs {
   void* out;           // EPI_ACT: [rows, N]; EPI_GLU: [rows, N/2]; EPI_DGLU: [rows, 2N]
   void* aux_out;       // EPI_GLU, EPI_ACT_AUX: un-activated product [rows, N] or null
   const void* aux_in;  // EPI_DGLU: saved un-activated product [rows, 2N]; EPI_ACT_AUX: the same, [rows, N], or null
-  // EPI_ACT, M-grouped only: when push_row != null, accumulator row p is stored at row push_row[p] (skipped when
+  // EPI_ACT (EPI_GLU without push_bases), M-grouped only: when push_row != null, accumulator row p is stored at row push_row[p] (skipped when
   // negative) instead of row p -- of `out`, or, when push_bases != null, of the [*, N] matrix based at
   // push_bases[push_rank[p]] (another GPU's buffer, peer-mapped; rows with push_rank[p] < 0 are not stored).
   void* const* push_bases;
@@ -133,6 +134,8 @@ struct TileCoord {
   int k_row0;   // K-grouped: first padded row of the contraction
   int kiters;   // number of BK-deep stages to contract
   bool active;  // false for the second CTA of a pair whose expert has an odd number of row tiles
+  int a_row;    // M-grouped: row of A the tile begins at (m0, or its unpadded counterpart; the rows after the expert's last
+                // one are then the next expert's, and nothing is stored for them)
   int live;     // M-grouped: rows of the tile that exist (64 or 128, see GemmArgs::group_indices)
 };
 
@@ -308,6 +311,7 @@ __device__ __forceinline__ TileCoord decode_tile(int t, int mt, int nt, const Wi
     c.k_row0 = __ldg(args.pad_offsets + expert);
     c.kiters = live_rows(args, expert, __ldg(args.pad_offsets + expert + 1) - c.k_row0) / BK;  // multiples of 64
     c.live = BM;
+    c.a_row = 0;
   } else {
     int tile = m_idx;
     if (CTAS == 2) {
@@ -322,11 +326,13 @@ __device__ __forceinline__ TileCoord decode_tile(int t, int mt, int nt, const Wi
       c.expert = __ldg(args.mtile_expert + tile);
     }
     c.m0 = tile * BM;
+    c.a_row = c.m0;
     c.live = BM;
     if (args.group_indices != nullptr) {
       const int base = __ldg(args.pad_offsets + c.expert);
       const int left = live_rows(args, c.expert, 1 << 30) - (c.m0 - base);
       c.live = left < BM ? (left > 64 ? left : 64) : BM;
+      if (args.a_compact) c.a_row = c.m0 - base + __ldg(args.group_indices + c.expert);
     }
     c.k_row0 = 0;
     c.kiters = (args.k_dim + BK - 1) / BK;
@@ -635,7 +641,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                   tma_load_2d_pair(sb + j * (BK * 128), &tmap_b, c.n0 + bcol + 64 * j, krow, fb, pol);
               }
             } else {
-              if (!gather) tma_load_2d_pair(sa, &tmap_a, kb * BK, c.m0, fb, pol);
+              if (!gather) tma_load_2d_pair(sa, &tmap_a, kb * BK, c.a_row, fb, pol);
               if (B_K) {
                 tma_load_3d_pair(sb, &tmap_b, kb * BK, c.n0 + bcol, c.expert, fb, pol);
               } else if (args.b_blocked) {
@@ -665,8 +671,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                   tma_load_2d(sb + j * (BK * 128), &tmap_b, c.n0 + bcol + 64 * j, krow, fb, pol);
               }
             } else {
-              if (!gather) tma_load_2d(sa, &tmap_a, kb * BK, c.m0, fb, pol);
-              if (kHalves && both) tma_load_2d(sa + Plan::kABytes / 2, &tmap_a, kb * BK, c.m0 + 64, fb, pol);
+              if (!gather) tma_load_2d(sa, &tmap_a, kb * BK, c.a_row, fb, pol);
+              if (kHalves && both) tma_load_2d(sa + Plan::kABytes / 2, &tmap_a, kb * BK, c.a_row + 64, fb, pol);
               if (B_K) {
                 tma_load_3d(sb, &tmap_b, kb * BK, c.n0 + bcol, c.expert, fb, pol);
               } else if (args.b_blocked) {
@@ -803,7 +809,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         out_row = static_cast<long long>(c.expert) * args.m_dim + row;
       } else {
         out_row = row;
-        if (EPI == EPI_ACT && args.push_row != nullptr) {
+        if ((EPI == EPI_ACT || EPI == EPI_GLU) && args.push_row != nullptr) {
           int32_t r = -1;
           if (row_ok) {
             if (args.push_bases != nullptr) {
@@ -1005,8 +1011,9 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         // Two 32-column chunks per round.  The un-activated product (128 bytes per row) and the activated
         // half (64 bytes per row) each go through the warp's swizzled shared-memory tile, so that every store
         // instruction writes whole row segments (4 rows x 128 bytes, then 8 rows x 64 bytes) instead of 32
-        // scattered 16-byte pieces.  Rows are valid or not per CTA here (no per-row mask).
+        // scattered 16-byte pieces.
         const int half_n = N >> 1;
+        const int glu_row = row_ok ? static_cast<int>(out_row) : -1;
 #pragma unroll 1
         for (int chunk = chunk_begin; chunk < chunk_begin + kChunksPerWarp; chunk += 2) {
           uint4 act_pk[4];  // this lane's 32 activated values of the round
@@ -1046,7 +1053,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
           }
           if (aux_out != nullptr) {
             __syncwarp();
-            const bool ok = row_ok && col0 + co_ck * 8 < N;
+            const bool ok = col0 + co_ck * 8 < N;  // all 32 rows exist (aux_out does not go with a row map)
             T* dst = aux_out + (warp_row0 + co_row) * N + col0 + co_ck * 8;
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
@@ -1073,16 +1080,17 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
             const int hr = lane >> 2;  // row within a group of eight
             const int hk = lane & 3;   // 16-byte piece of the row's 64 bytes
             const int hcol = (col0 >> 1) + hk * 8;
-            const bool ok = row_ok && hcol < half_n;
-            T* dst = out + (warp_row0 + hr) * half_n + hcol;
+            const bool ok = hcol < half_n;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
               const int r = j * 8 + hr;
+              // row of the output, negative: not stored (each lane holds its own row's; without a row map they are consecutive)
+              const int dst_row = __shfl_sync(0xFFFFFFFFu, glu_row, r);
               const int slot = (hk | ((r & 1) << 2)) ^ ((r >> 1) & 3);
               uint4 u;
               const uint32_t addr = stage_base + r * 128 + (slot << 4);
               asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(u.x), "=r"(u.y), "=r"(u.z), "=r"(u.w) : "r"(addr));
-              if (ok) *reinterpret_cast<uint4*>(dst + static_cast<long long>(j) * 8 * half_n) = u;
+              if (ok && dst_row >= 0) *reinterpret_cast<uint4*>(out + static_cast<long long>(dst_row) * half_n + hcol) = u;
             }
           }
           __syncwarp();

@@ -192,6 +192,7 @@ struct MExtras {
   int chunk_index = 0;
   int chunk_count = 1;
   RowCounts counts;
+  int64_t compact_rows = -1;  // >= 0: A has this many rows, without padding (counts given)
 };
 
 template <typename T, int BN, int CTAS>
@@ -312,6 +313,7 @@ static int mgrouped_common(const char* name, const void* a, const void* w, void*
   }
   args.pad_offsets = x.counts.pad_offsets;
   args.group_indices = x.counts.pad_offsets != nullptr ? x.counts.group_indices : nullptr;
+  args.a_compact = x.compact_rows >= 0 ? 1 : 0;
   args.num_mtiles = num_mtiles;
   args.num_experts = E;
   args.n_dim = N;
@@ -365,7 +367,7 @@ static int mgrouped_common(const char* name, const void* a, const void* w, void*
   // OLMoE shape: -6..12 %; at 128 rows per expert 0..5 %).
   const long long mean_rows_per_expert = (padded_rows - static_cast<long long>(E) * (BM - 1)) / E;
   const bool pairs = tile_pairs != nullptr && (o.single_cta == 0 ? mean_rows_per_expert > BM : o.single_cta < 0);
-  const int64_t a_rows = x.gather_row_src != nullptr ? x.gather_rows : padded_rows;
+  const int64_t a_rows = x.gather_row_src != nullptr ? x.gather_rows : (x.compact_rows >= 0 ? x.compact_rows : padded_rows);
 #define MOE_MG(TYPE)                                                                                              \
   (pairs ? (bn == 256 ? mgrouped_dispatch<TYPE, 256, 2>(a, w, a_rows, K, N, E, w_transposed, epi, args, dtype, lp) \
                       : mgrouped_dispatch<TYPE, 128, 2>(a, w, a_rows, K, N, E, w_transposed, epi, args, dtype, lp)) \
@@ -546,6 +548,18 @@ int kgrouped_gemm_gather(const void* src, int64_t src_rows, const int32_t* row_s
   MOE_CHECK_ARG(row_src != nullptr, "moe_kgrouped_gemm_gather: row_src is null");
   return kgrouped_common("moe_kgrouped_gemm_gather", src, src_rows, row_src, div, b, dw, pad_offsets, padded_rows, M, N,
                          num_experts, dtype, options, status, stream, counts.group_indices);
+}
+
+int mgrouped_gemm_rows(const void* a, int64_t compact_rows, const void* w, void* out, const int32_t* out_rows,
+                       const int32_t* mtile_expert, const int32_t* tile_pairs, const int32_t* num_mtiles, int64_t padded_rows,
+                       int K, int N, int num_experts, int act, int dtype, int32_t* status, void* stream,
+                       const RowCounts& counts) {
+  MExtras x;
+  x.counts = counts;
+  x.compact_rows = compact_rows;
+  x.push_row = out_rows;
+  return mgrouped_common("moe_rows_gemm", a, w, out, x, mtile_expert, tile_pairs, num_mtiles, padded_rows, K, N, num_experts, 0,
+                         act_is_glu(act) ? EPI_GLU : EPI_ACT, act, dtype, nullptr, status, stream);
 }
 
 }  // namespace moe

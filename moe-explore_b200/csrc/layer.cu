@@ -7,21 +7,6 @@ namespace moe {
 
 static bool glu(int act) { return act == MOE_ACT_SWIGLU || act == MOE_ACT_GEGLU; }
 
-// The kernels of one call are chained (common.cuh): all but the first.  B200, tail of one kernel to work of the next: see the
-// figures at moe_expert_forward.
-class Chain {
- public:
-  Chain() { chained_launches() = false; }
-  ~Chain() { chained_launches() = false; }
-};
-
-#define MOE_STEP(call)              \
-  do {                              \
-    const int rc__ = (call);        \
-    if (rc__ != MOE_OK) return rc__; \
-    chained_launches() = true;      \
-  } while (0)
-
 }  // namespace moe
 
 using namespace moe;

@@ -458,68 +458,132 @@ static int route_cluster(const int64_t* ids, int64_t R, int E, const RouteOut& o
   return MOE_OK;
 }
 
-// Layout from an existing exclusive prefix (rows already grouped): one CTA, thread per expert for
-// the padded prefix, then all threads fill the row maps.
+// Layout from an existing exclusive prefix (rows already grouped), in one launch: every CTA computes the padded prefix for
+// itself (E values) and fills its share of the maps.  It replaces a memset, a one-CTA scan and a row kernel, and in the
+// functional grouped GEMM six index operations besides (16 launches of 2-4 us each for 4111 tokens x 8 slots, two calls).
+// `perm` (nullable): flat position of sorted row r.  Maps of padded row p that holds sorted row r, all nullable:
+//   row_src r | in_rows perm[r] (r without perm) | out_rows perm[r] if scatter, else r;  padding rows: -1, -2 (skip), -1
+struct GroupsOut {
+  int32_t* pad_offsets;
+  int32_t* row_src;
+  int32_t* dst_row;
+  int32_t* mtile_expert;
+  int32_t* tile_pairs;
+  int32_t* num_mtiles;
+  int32_t* in_rows;
+  int32_t* out_rows;
+  int32_t mtiles_bound;
+};
+
 __global__ void __launch_bounds__(kMaxExperts)
-layout_from_groups_kernel(const int32_t* __restrict__ group_indices, int64_t R, int E, int32_t* __restrict__ pad_offsets,
-                          int32_t* __restrict__ mtile_expert, int32_t* __restrict__ tile_pairs,
-                          int32_t* __restrict__ num_mtiles, int mtiles_bound, int32_t* status) {
-  __shared__ int32_t sh_b[kMaxExperts];
-  __shared__ int32_t sh_c[kMaxExperts];
-  const int e = threadIdx.x;
-  int32_t padded = 0;
+layout_from_groups_kernel(const int32_t* __restrict__ group_indices, int64_t R, int E, const int64_t* __restrict__ perm,
+                          int scatter, GroupsOut out, int32_t* status) {
+  __shared__ int32_t sh_lo[kMaxExperts], sh_cnt[kMaxExperts], sh_pad[kMaxExperts + 1], sh_pair[kMaxExperts + 1];
+  __shared__ int32_t sums[2][32];
+  const int e = threadIdx.x, lane = e & 31, warp = e >> 5;
+  grid_release();
+  int32_t cnt = 0, lo = 0;
   if (e < E) {
     // a prefix that is not monotone, does not start at 0 or does not end at R describes no layout: such experts
     // get no rows here and the status word says so
-    const int32_t lo = group_indices[e], hi = group_indices[e + 1];
+    lo = group_indices[e];
+    const int32_t hi = group_indices[e + 1];
     const bool bad = hi < lo || lo < 0 || hi > R || (e == 0 && lo != 0) || (e == E - 1 && hi != R);
-    if (bad && status != nullptr) atomicCAS(status, 0, DS_BAD_LAYOUT);
-    const int32_t cnt = bad ? 0 : hi - lo;
-    padded = (cnt + MOE_TILE_M - 1) / MOE_TILE_M * MOE_TILE_M;
+    if (bad && blockIdx.x == 0 && status != nullptr) atomicCAS(status, 0, DS_BAD_LAYOUT);
+    cnt = bad ? 0 : hi - lo;
   }
+  const int32_t padded = (cnt + MOE_TILE_M - 1) / MOE_TILE_M * MOE_TILE_M;
   const int32_t pairs = (padded / MOE_TILE_M + 1) / 2;
-  sh_b[e] = padded;
-  sh_c[e] = pairs;
-  __syncthreads();
-  for (int off = 1; off < kMaxExperts; off <<= 1) {
-    int32_t b = 0, c = 0;
-    if (e >= off) { b = sh_b[e - off]; c = sh_c[e - off]; }
-    __syncthreads();
-    sh_b[e] += b;
-    sh_c[e] += c;
-    __syncthreads();
+  int32_t in_p = padded, in_q = pairs;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const int32_t a = __shfl_up_sync(0xFFFFFFFFu, in_p, off);
+    const int32_t b = __shfl_up_sync(0xFFFFFFFFu, in_q, off);
+    if (lane >= off) { in_p += a; in_q += b; }
   }
+  if (lane == 31) { sums[0][warp] = in_p; sums[1][warp] = in_q; }
+  __syncthreads();
+  if (warp < 2) {
+    int32_t v = sums[warp][lane];
+    const int32_t own = v;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int32_t a = __shfl_up_sync(0xFFFFFFFFu, v, off);
+      if (lane >= off) v += a;
+    }
+    sums[warp][lane] = v - own;
+  }
+  __syncthreads();
+  const int32_t p1 = in_p + sums[0][warp], q1 = in_q + sums[1][warp];
   if (e < E) {
-    pad_offsets[e + 1] = sh_b[e];
-    if (e == 0) pad_offsets[0] = 0;
-    int32_t* pair_prefix = tile_pairs != nullptr ? tile_pairs + mtiles_bound : nullptr;
-    if (mtile_expert != nullptr) write_tile_maps(e, sh_b[e] - padded, padded, sh_c[e] - pairs, mtile_expert, tile_pairs, pair_prefix);
-    if (num_mtiles != nullptr && e == E - 1) {
-      num_mtiles[0] = sh_b[e] / MOE_TILE_M;
-      num_mtiles[1] = sh_c[e];
-      num_mtiles[2] = mtiles_bound;
-      num_mtiles[3] = 0;
-      if (pair_prefix != nullptr) pair_prefix[E] = sh_c[e];
+    sh_lo[e] = lo;
+    sh_cnt[e] = cnt;
+    sh_pad[e] = p1 - padded;
+    sh_pair[e] = q1 - pairs;
+    if (e == E - 1) { sh_pad[E] = p1; sh_pair[E] = q1; }
+    if (blockIdx.x == 0) {
+      out.pad_offsets[e + 1] = p1;
+      if (e == 0) out.pad_offsets[0] = 0;
+      if (out.tile_pairs != nullptr) {
+        out.tile_pairs[out.mtiles_bound + e] = q1 - pairs;
+        if (e == E - 1) out.tile_pairs[out.mtiles_bound + E] = q1;
+      }
+      if (out.num_mtiles != nullptr && e == E - 1) {
+        out.num_mtiles[0] = p1 / MOE_TILE_M;
+        out.num_mtiles[1] = q1;
+        out.num_mtiles[2] = out.mtiles_bound;
+        out.num_mtiles[3] = 0;
+      }
     }
   }
-}
-
-__global__ void layout_rows_kernel(const int32_t* __restrict__ group_indices, const int32_t* __restrict__ pad_offsets,
-                                   int64_t R, int E, int32_t* __restrict__ row_src, int32_t* __restrict__ dst_row) {
-  const int64_t j = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (j >= R) return;
-  // binary search: largest e with group_indices[e] <= j
-  int lo = 0, hi = E;
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (group_indices[mid] <= j) lo = mid; else hi = mid;
+  __syncthreads();
+  const int tid = blockIdx.x * kMaxExperts + e, threads = gridDim.x * kMaxExperts;
+  // last expert whose padded rows begin at or before p (empty experts begin where the next one does)
+  const auto owner = [&](int32_t p) {
+    int a = 0, b = E;
+    while (b - a > 1) {
+      const int mid = (a + b) >> 1;
+      if (sh_pad[mid] <= p) a = mid; else b = mid;
+    }
+    return a;
+  };
+  if (out.row_src != nullptr || out.in_rows != nullptr || out.out_rows != nullptr) {
+    const int32_t bound = out.mtiles_bound * MOE_TILE_M;
+    for (int32_t p = tid; p < bound; p += threads) {
+      const int x = owner(p);
+      const int32_t in_seg = p - sh_pad[x];
+      const bool ok = p < sh_pad[E] && in_seg < sh_cnt[x];
+      const int32_t r = sh_lo[x] + in_seg;
+      const int32_t f = ok ? (perm != nullptr ? static_cast<int32_t>(perm[r]) : r) : -1;
+      if (out.row_src != nullptr) out.row_src[p] = ok ? r : -1;
+      if (out.in_rows != nullptr) out.in_rows[p] = ok ? f : kSkipRow;
+      if (out.out_rows != nullptr) out.out_rows[p] = ok ? (scatter ? f : r) : -1;
+    }
   }
-  // rows of a segment the layout kernel refused (bad prefix) have no padded row
-  const int64_t in_seg = j - group_indices[lo];
-  const bool ok = in_seg >= 0 && in_seg < pad_offsets[lo + 1] - pad_offsets[lo] && j < group_indices[lo + 1];
-  const int32_t p = ok ? pad_offsets[lo] + static_cast<int32_t>(in_seg) : -1;
-  if (ok && row_src != nullptr) row_src[p] = static_cast<int32_t>(j);
-  if (dst_row != nullptr) dst_row[j] = p;
+  if (out.dst_row != nullptr) {
+    for (int64_t j = tid; j < R; j += threads) {
+      int a = 0, b = E;  // largest e with group_indices[e] <= j
+      while (b - a > 1) {
+        const int mid = (a + b) >> 1;
+        if (sh_lo[mid] <= j) a = mid; else b = mid;
+      }
+      // rows of a segment that was refused (bad prefix) have no padded row
+      const int64_t in_seg = j - sh_lo[a];
+      out.dst_row[j] = in_seg >= 0 && in_seg < sh_cnt[a] ? sh_pad[a] + static_cast<int32_t>(in_seg) : -1;
+    }
+  }
+  if (out.mtile_expert != nullptr) {
+    const int tiles = sh_pad[E] / MOE_TILE_M;
+    for (int m = tid; m < tiles; m += threads) {
+      const int x = owner(m * MOE_TILE_M);
+      out.mtile_expert[m] = x;
+      const int in_expert = m - sh_pad[x] / MOE_TILE_M;
+      if (out.tile_pairs != nullptr && (in_expert & 1) == 0)
+        out.tile_pairs[sh_pair[x] + in_expert / 2] =
+            static_cast<int32_t>(static_cast<uint32_t>(m) | (static_cast<uint32_t>(x) << 20) |
+                                 ((m + 1) * MOE_TILE_M < sh_pad[x + 1] ? 0x80000000u : 0u));
+    }
+  }
 }
 
 }  // namespace moe
@@ -607,6 +671,16 @@ extern "C" int moe_routing_metadata(const int64_t* expert_idx, int64_t num_rows,
                           tile_pairs, num_mtiles, status, workspace, workspace_bytes, true, stream);
 }
 
+static int layout_from_groups(const int32_t* group_indices, int64_t num_rows, int num_experts, const int64_t* perm, int scatter,
+                              const GroupsOut& out, int32_t* status, cudaStream_t s) {
+  // a CTA per 2048 padded rows: enough of them to spread the maps, few enough that the repeated prefix stays free
+  const int64_t ctas = (static_cast<int64_t>(out.mtiles_bound) * MOE_TILE_M + 2047) / 2048;
+  const int grid = static_cast<int>(ctas < sm_count() ? ctas : sm_count());
+  layout_from_groups_kernel<<<grid, kMaxExperts, 0, s>>>(group_indices, num_rows, num_experts, perm, scatter, out, status);
+  MOE_CUDA(cudaGetLastError());
+  return MOE_OK;
+}
+
 extern "C" int moe_layout_from_groups(const int32_t* group_indices, int64_t num_rows, int num_experts,
                                       int32_t* pad_offsets, int32_t* row_src, int32_t* dst_row, int32_t* mtile_expert,
                                       int32_t* tile_pairs, int32_t* num_mtiles, int32_t* status, void* stream) {
@@ -621,19 +695,44 @@ extern "C" int moe_layout_from_groups(const int32_t* group_indices, int64_t num_
   }
   MOE_CHECK_ARG((mtile_expert == nullptr) == (num_mtiles == nullptr) && (tile_pairs == nullptr || mtile_expert != nullptr),
                 "moe_layout_from_groups: mtile_expert, tile_pairs and num_mtiles go together");
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (row_src != nullptr) {
-    MOE_CUDA(cudaMemsetAsync(row_src, 0xFF, moe_padded_rows_bound(num_rows, num_experts) * sizeof(int32_t), s));
+  return layout_from_groups(group_indices, num_rows, num_experts, nullptr, 0,
+                            GroupsOut{pad_offsets, row_src, dst_row, mtile_expert, tile_pairs, num_mtiles, nullptr, nullptr,
+                                      static_cast<int32_t>(moe_mtiles_bound(num_rows, num_experts))},
+                            status, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" size_t moe_rows_pass_size(void) { return sizeof(moe_rows_pass); }
+
+extern "C" int moe_rows_gemm(const moe_rows_pass* p, int steps, void* stream) {
+  MOE_CHECK_ARG(p != nullptr, "moe_rows_gemm: null pointer argument");
+  MOE_CHECK_ARG(p->group_indices && p->pad_offsets && p->out_rows && p->mtile_expert && p->tile_pairs && p->num_mtiles && p->a &&
+                    (!p->gather || (p->in_rows && p->padded)) && ((!p->gather && !p->scatter) || p->perm),
+                "moe_rows_gemm: null pointer argument");
+  MOE_CHECK_ARG(p->num_rows > 0 && p->num_experts > 0 && p->a_rows >= 0 && p->topk > 0, "moe_rows_gemm: bad sizes");
+  MOE_CHECK_ARG(p->act >= MOE_ACT_NONE && p->act <= MOE_ACT_GELU_TANH, "moe_rows_gemm: unknown activation %d", p->act);
+  const int64_t mtiles = moe_mtiles_bound(p->num_rows, p->num_experts);
+  MOE_CHECK_ARG(mtiles < (1ll << 20), "moe_rows_gemm: num_rows=%lld needs more than 2^20 row tiles", (long long)p->num_rows);
+  if (p->num_experts > kMaxExperts) {
+    set_error("moe_rows_gemm: num_experts=%d exceeds the supported maximum %d", p->num_experts, kMaxExperts);
+    return MOE_ERR_UNSUPPORTED;
   }
-  layout_from_groups_kernel<<<1, kMaxExperts, 0, s>>>(group_indices, num_rows, num_experts, pad_offsets, mtile_expert,
-                                                     tile_pairs, num_mtiles,
-                                                     static_cast<int>(moe_mtiles_bound(num_rows, num_experts)), status);
-  MOE_CUDA(cudaGetLastError());
-  if (num_rows > 0 && (row_src || dst_row)) {
-    const int threads = 256;
-    const int blocks = static_cast<int>((num_rows + threads - 1) / threads);
-    layout_rows_kernel<<<blocks, threads, 0, s>>>(group_indices, pad_offsets, num_rows, num_experts, row_src, dst_row);
-    MOE_CUDA(cudaGetLastError());
+  const Chain chain;
+  const int64_t padded_rows = mtiles * MOE_TILE_M;
+  if (steps & MOE_ROWS_LAYOUT)
+    MOE_STEP(layout_from_groups(p->group_indices, p->num_rows, p->num_experts, p->gather || p->scatter ? p->perm : nullptr,
+                                p->scatter,
+                                GroupsOut{p->pad_offsets, nullptr, nullptr, p->mtile_expert, p->tile_pairs, p->num_mtiles,
+                                          p->gather ? p->in_rows : nullptr, p->out_rows, static_cast<int32_t>(mtiles)},
+                                p->status, static_cast<cudaStream_t>(stream)));
+  if ((steps & MOE_ROWS_GATHER) && p->gather)
+    MOE_STEP(moe_gather_rows(p->a, p->a_rows, p->in_rows, p->num_mtiles, p->padded, padded_rows, p->k_dim, p->topk, p->dtype,
+                             stream));
+  if (steps & MOE_ROWS_GEMM) {
+    const RowCounts counts{p->pad_offsets, p->group_indices};
+    // rows that are in expert order already are read where they are; gathered ones from their padded copy
+    MOE_STEP(mgrouped_gemm_rows(p->gather ? p->padded : p->a, p->gather ? -1 : p->a_rows, p->w, p->out, p->out_rows,
+                                p->mtile_expert, p->tile_pairs, p->num_mtiles, padded_rows, p->k_dim, p->n_dim, p->num_experts,
+                                p->act, p->dtype, p->status, stream, counts));
   }
   return MOE_OK;
 }

@@ -18,13 +18,15 @@ constexpr int kRowThreads = 256;
 // 238 -> 231.
 constexpr int kRowLoads = 4;
 
-// dst[r, :] = src[index[r] / div, :], zeros where index[r] < 0.  `num_mtiles` (nullable): only the first
+// dst[r, :] = src[index[r] / div, :], zeros where index[r] < 0 (kSkipRow: untouched).  `num_mtiles` (nullable): only the first
 // 128 * num_mtiles[0] rows are in use.
 template <typename Index, int TPR>
 __global__ void __launch_bounds__(kRowThreads)
 copy_rows_kernel(const uint4* __restrict__ src, const Index* __restrict__ index, const int32_t* __restrict__ num_mtiles,
                  uint4* __restrict__ dst, int64_t rows, int vec_per_row, int div) {
   constexpr int kRows = kRowThreads / TPR;
+  grid_release();
+  grid_wait();
   if (num_mtiles != nullptr) {
     const int64_t in_use = static_cast<int64_t>(*num_mtiles) * MOE_TILE_M;
     rows = in_use < rows ? in_use : rows;
@@ -33,6 +35,7 @@ copy_rows_kernel(const uint4* __restrict__ src, const Index* __restrict__ index,
   for (int64_t r = static_cast<int64_t>(blockIdx.x) * kRows + threadIdx.x / TPR; r < rows;
        r += static_cast<int64_t>(gridDim.x) * kRows) {
     const int32_t j = static_cast<int32_t>(index[r]);
+    if (j == kSkipRow) continue;
     const uint4* s = src + static_cast<int64_t>(j / div) * vec_per_row;
     uint4* d = dst + r * vec_per_row;
     for (int v0 = lane; v0 < vec_per_row; v0 += TPR * kRowLoads) {
@@ -483,8 +486,8 @@ static void launch_copy_rows(const void* src, const Index* index, const int32_t*
   const int grid = static_cast<int>(groups < (1 << 30) ? (groups > 0 ? groups : 1) : (1 << 30));
   const uint4* in = static_cast<const uint4*>(src);
   uint4* out = static_cast<uint4*>(dst);
-  if (tpr == 32) copy_rows_kernel<Index, 32><<<grid, kRowThreads, 0, s>>>(in, index, num_mtiles, out, rows, vec_per_row, div);
-  else copy_rows_kernel<Index, 64><<<grid, kRowThreads, 0, s>>>(in, index, num_mtiles, out, rows, vec_per_row, div);
+  if (tpr == 32) launch_kernel(copy_rows_kernel<Index, 32>, grid, kRowThreads, s, in, index, num_mtiles, out, rows, vec_per_row, div);
+  else launch_kernel(copy_rows_kernel<Index, 64>, grid, kRowThreads, s, in, index, num_mtiles, out, rows, vec_per_row, div);
 }
 
 // row_src == nullptr: the padding rows are left as they are.

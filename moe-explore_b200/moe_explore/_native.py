@@ -46,6 +46,14 @@ class ExpertPass(ctypes.Structure):
                                         "d_w1", "d_w2")]
 
 
+class RowsPass(ctypes.Structure):
+    """``moe_rows_pass``: sizes and buffers of one functional grouped GEMM."""
+    _fields_ = [(f, c_int64) for f in ("num_rows", "a_rows")] + \
+               [(f, c_int32) for f in ("num_experts", "k_dim", "n_dim", "topk", "act", "dtype", "gather", "scatter")] + \
+               [(f, c_void_p) for f in ("a", "w", "out", "group_indices", "perm", "pad_offsets", "in_rows", "out_rows",
+                                        "mtile_expert", "tile_pairs", "num_mtiles", "status", "padded")]
+
+
 # name -> (restype, argtypes); the single source for both binding and the symbol-export test
 _OPT = POINTER(GemmOptions)
 SIGNATURES = {
@@ -77,6 +85,8 @@ SIGNATURES = {
     "moe_expert_pass_size": (c_size_t, []),
     "moe_expert_forward": (c_int, [POINTER(ExpertPass), c_int, c_void_p]),
     "moe_expert_backward": (c_int, [POINTER(ExpertPass), c_int, c_void_p]),
+    "moe_rows_pass_size": (c_size_t, []),
+    "moe_rows_gemm": (c_int, [POINTER(RowsPass), c_int, c_void_p]),
     "moe_dispatch_rows_only": (c_int, [c_void_p] * 3 + [c_int64, c_int, c_int, c_int, c_void_p]),
     "moe_combine_bwd_tokens": (c_int, [c_void_p] * 8 + [c_int64, c_int, c_int, c_int, c_void_p]),
     "moe_mgrouped_gemm": (c_int, [c_void_p] * 7 + [c_int64, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, _OPT,
@@ -153,6 +163,8 @@ def load() -> ctypes.CDLL:
             raise ImportError(f"{LIB_PATH} was built with another layout of moe_gemm_options: rebuild it")
         if lib.moe_expert_pass_size() != ctypes.sizeof(ExpertPass):
             raise ImportError(f"{LIB_PATH} was built with another layout of moe_expert_pass: rebuild it")
+        if lib.moe_rows_pass_size() != ctypes.sizeof(RowsPass):
+            raise ImportError(f"{LIB_PATH} was built with another layout of moe_rows_pass: rebuild it")
         _lib = lib
     return _lib
 
@@ -231,16 +243,16 @@ def _opt(options):
     return None if options is None else ctypes.byref(options)
 
 
+ROWS_LAYOUT, ROWS_GATHER, ROWS_GEMM = 1, 2, 4
 FWD_ROUTE, FWD_DISPATCH, FWD_UP, FWD_DOWN, FWD_FOLD = 1, 2, 4, 8, 16
 BWD_FOLD, BWD_DOWN, BWD_UP, BWD_FOLD_DX, BWD_DW1, BWD_DW2 = 1, 2, 4, 8, 16, 32
 
 
-def expert_pass(backward: bool, p: ExpertPass, steps, rows: int) -> None:
-    """The launches of one pass over the experts on the current stream; ``steps`` = [(step, name, launches)].  One call
-    into the library, or, with a ``TRACER``, one per step, so that each is counted and can be timed by itself."""
-    lib = load()
-    name = "moe_expert_backward" if backward else "moe_expert_forward"
-    fn = lib.moe_expert_backward if backward else lib.moe_expert_forward
+def run_pass(name: str, p, steps, rows: int) -> None:
+    """The launches of the pass ``p`` (an ``ExpertPass`` or ``RowsPass``) on the current stream; ``steps`` = [(step, name,
+    launches)].  One call into the library, or, with a ``TRACER``, one per step, so that each is counted and can be timed by
+    itself."""
+    fn = getattr(load(), name)
     if TRACER is None:
         mask = 0
         for step, _, _ in steps:
@@ -289,7 +301,7 @@ def layout_from_groups(group_indices, num_rows, num_experts, pad_offsets, row_sr
                                        _ptr(dst_row), _ptr(mtile_expert), _ptr(tile_pairs), _ptr(num_mtiles),
                                        _ptr(status), _stream())
     _check("moe_layout_from_groups", rc)
-    _count(2 if num_rows > 0 else 1)
+    _count(1)
 
 
 def router_topk(logits, topk: int, softmax_before_topk: bool, normalize: bool, want_counts: bool = False):

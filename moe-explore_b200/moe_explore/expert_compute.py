@@ -93,7 +93,7 @@ class ExpertCompute(torch.autograd.Function):
         else:
             steps.append((_native.FWD_DOWN, "mgrouped_gemm:combine", 1))
         ptr = _native._ptr
-        _native.expert_pass(False, _native.ExpertPass(
+        _native.run_pass("moe_expert_forward", _native.ExpertPass(
             T, rp, d, inter, E, topk, act_code, code, gather_in_gemm, not fold, needs_grad, ids, x.data_ptr(), scores.data_ptr(),
             weight1.data_ptr(), weight2.data_ptr(), *plan_ptrs, ptr(workspace),
             0 if workspace is None else workspace.numel(), ptr(xs), ptr(pre_act), hidden.data_ptr(), ptr(ys), out.data_ptr()),
@@ -122,7 +122,7 @@ class ExpertCompute(torch.autograd.Function):
         else:
             plan_ptrs = _packed_pointers(words, packed_layout(rows, E)[1], device_status(words.get_device()))
         ptr = _native._ptr
-        _native.expert_pass(True, _native.ExpertPass(
+        _native.run_pass("moe_expert_backward", _native.ExpertPass(
             T, rp, d, inter, E, topk, _native.ACT_CODES[act], _native.dtype_code(grad_out.dtype), ctx.gathered, False, True, None,
             xs.data_ptr(), scores.data_ptr(), weight1.data_ptr(), weight2.data_ptr(), *plan_ptrs, None, 0, xs.data_ptr(),
             ptr(pre_act), hidden.data_ptr(), ys.data_ptr(), None, grad_out.data_ptr(), gs.data_ptr(), d_scores.data_ptr(),

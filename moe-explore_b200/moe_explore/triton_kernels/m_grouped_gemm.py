@@ -8,6 +8,7 @@ the contraction runs on the library's tcgen05 kernel over the padded expert-sort
 """
 from __future__ import annotations
 
+import functools
 from dataclasses import dataclass
 from typing import Optional
 
@@ -15,7 +16,7 @@ import torch
 
 from moe_explore import _native
 from moe_explore.functional.activation import is_glu
-from moe_explore.routing_plan import plan_from_groups
+from moe_explore.routing_plan import device_status
 
 
 @dataclass
@@ -37,8 +38,9 @@ class MGroupedGEMMParams:
 def m_grouped_gemm(token: torch.Tensor, params: MGroupedGEMMParams, autotune_mode=None) -> torch.Tensor:
     """Rows [g[e], g[e+1]) of the (optionally gathered) input times ``weight[e]``, optional activation epilogue,
     optional scatter of the output rows.  As in the reference kernel the scatter happens inside the GEMM's epilogue
-    (m_grouped_gemm.py:168-172): no un-scattered copy of the output exists.  The input rows are copied into
-    128-row-aligned expert segments first (one HBM-bound pass) so that the GEMM loads whole tiles."""
+    (m_grouped_gemm.py:168-172): no un-scattered copy of the output exists.  Gathered input rows are copied into
+    128-row-aligned expert segments first (one HBM-bound pass) so that the GEMM loads whole tiles; rows that are in expert
+    order already are read where they are."""
     assert token.dim() == 2
     assert params.weight.dim() == 3
     assert token.size(1) == params.weight.size(1)
@@ -55,34 +57,41 @@ def m_grouped_gemm(token: torch.Tensor, params: MGroupedGEMMParams, autotune_mod
     if rows == 0:
         return out
 
-    plan = plan_from_groups(params.group_indices.to(torch.int32), rows)
+    assert params.group_indices.dim() == 1 and params.group_indices.numel() == num_experts + 1
+    groups = params.group_indices.to(torch.int32).contiguous()
     token = token.contiguous()
     weight = params.weight.contiguous()
-    # padded row p holds sorted position r = row_src[p]; with gather or scatter its flat (token, slot) position is
-    # perm[r]: the input row is token[perm[r] // topk], the output row perm[r]
-    flat_of_row = None
+    perm = None
     if params.gather or params.scatter:
-        perm32 = params.permute_indices.to(torch.int32)
-        flat_of_row = torch.where(plan.row_src >= 0, perm32[plan.row_src.clamp_min(0).long()], plan.row_src)
-    in_rows = flat_of_row if params.gather else plan.row_src     # input row of padded row p (before // div)
-    in_div = params.topk if params.gather else 1
-    out_rows = flat_of_row if params.scatter else plan.row_src   # output row of padded row p
-    # input rows into the padded layout with one copy kernel (the gather could ride on the GEMM's operand loads --
-    # mgrouped_gemm_gather -- but four-row gather copies are several times slower than 128-row tile copies)
-    a = torch.empty(plan.padded_rows, k_dim, dtype=token.dtype, device=token.device)
-    _native.gather_rows(token, in_rows, plan.num_mtiles, a, in_div)
-    if not is_glu(act):
-        # element-wise epilogue: the rows are scattered to their final place by the stores of the GEMM itself
-        _native.mgrouped_gemm_scatter(a, weight, out, out_rows, plan.mtile_expert, plan.tile_pairs, plan.num_mtiles,
-                                      plan.padded_rows, False, act, status=plan.status)
-        return out
-    # gated epilogue (two input columns per output column): output in the padded layout, then one un-pad pass
-    y = torch.empty(plan.padded_rows, out_cols, dtype=token.dtype, device=token.device)
-    _native.mgrouped_gemm(a, weight, y, None, plan.mtile_expert, plan.tile_pairs, plan.num_mtiles, False, act, plan.status)
-    if params.scatter:
-        src_of_out = torch.empty(rows, dtype=torch.int32, device=token.device)
-        src_of_out[params.permute_indices] = plan.dst_row   # out[perm[r]] = y[dst_row[r]]
-        _native.unpad_rows(y, src_of_out, out)
-    else:
-        _native.unpad_rows(y, plan.dst_row, out)
+        _native.require_cuda(params.permute_indices)
+        perm = params.permute_indices.to(torch.int64).contiguous()
+        assert perm.numel() >= rows, "permute_indices is shorter than the routed rows"
+    rp, offsets, words = _maps_layout(rows, num_experts)
+    maps = torch.empty(words, dtype=torch.int32, device=token.device)
+    base = maps.data_ptr()
+    padded = torch.empty(rp, k_dim, dtype=token.dtype, device=token.device) if params.gather else None
+    ptr = _native._ptr
+    steps = [(_native.ROWS_LAYOUT, "routing", 1)]
+    if params.gather:
+        # (the gather could ride on the GEMM's operand loads -- mgrouped_gemm_gather -- but four-row gather copies are several
+        # times slower than 128-row tile copies)
+        steps.append((_native.ROWS_GATHER, "rows:gather", 1))
+    steps.append((_native.ROWS_GEMM, "mgrouped_gemm:scatter", 1))
+    _native.run_pass("moe_rows_gemm", _native.RowsPass(
+        rows, token.size(0), num_experts, k_dim, n_dim, params.topk if params.gather else 1, _native.ACT_CODES[act],
+        _native.dtype_code(token.dtype), bool(params.gather), bool(params.scatter), token.data_ptr(), weight.data_ptr(),
+        out.data_ptr(), groups.data_ptr(), ptr(perm), *[base + o for o in offsets],
+        device_status(token.get_device()).data_ptr(), ptr(padded)), steps, rows)
     return out
+
+
+@functools.lru_cache(maxsize=256)
+def _maps_layout(rows: int, num_experts: int):
+    """(padded rows, byte offsets of pad_offsets, in_rows, out_rows, mtile_expert, tile_pairs, num_mtiles, int32 words)."""
+    rp = _native.padded_rows_bound(rows, num_experts)
+    tiles = rp // _native.TILE_M
+    offsets, words = [], 0
+    for n in (num_experts + 1, rp, rp, tiles, tiles + num_experts + 1, 4):
+        offsets.append(4 * words)
+        words += (n + 3) // 4 * 4
+    return rp, tuple(offsets), words

@@ -62,3 +62,38 @@ def test_blocks_without_rows_do_not_leak(rows, act, native):
         _poison()
         assert _relerr(routed_expert_compute(*leaves, ids, E, 1, act, fused_combine=True), expect[0]) <= 2e-2
     assert native.read_status(build_routing_plan(ids, E, 1).status) == 0
+
+
+@pytest.mark.parametrize("act", [None, "silu", "swiglu"])
+@pytest.mark.parametrize("gather,scatter", [(False, False), (True, False), (False, True), (True, True)])
+@pytest.mark.parametrize("rows", [(1, 63, 64, 65, 127, 128, 129, 0, 3), (0, 520, 1, 255, 0, 384), (2049,)])
+def test_functional_gemm_against_its_steps(rows, gather, scatter, act, native):
+    """Rows read without padding, rows gathered, rows stored through the map (gated ones too): bit for bit what copying into the
+    padded layout, contracting there and copying back gives."""
+    from moe_explore.routing_plan import plan_from_groups
+    from moe_explore.triton_kernels.m_grouped_gemm import MGroupedGEMMParams, m_grouped_gemm
+
+    E, K, N, topk, R = len(rows), 136, 208, 1 if gather and scatter else 3, sum(rows)
+    if R % topk:
+        topk = 1
+    g = torch.Generator(device="cuda").manual_seed(R)
+    groups = torch.tensor([0] + list(rows), dtype=torch.int32).cumsum(0).to(torch.int32).cuda()
+    perm = torch.randperm(R, generator=g, device="cuda")
+    w = (torch.randn(E, K, N, generator=g, device="cuda") * 0.1).bfloat16()
+    x = torch.randn(R // topk if gather else R, K, generator=g, device="cuda").bfloat16()
+    tokens = R // topk if (gather or scatter) else R
+    out = m_grouped_gemm(x, MGroupedGEMMParams(w, groups, perm, gather, scatter, tokens, topk, activation=act))
+
+    plan = plan_from_groups(groups, R)
+    pos = plan.row_src.long()
+    src = torch.where(pos >= 0, perm[pos.clamp_min(0)] // topk if gather else pos, -1).int()
+    a = torch.empty(plan.padded_rows, K, dtype=x.dtype, device="cuda")
+    native.gather_rows(x, src, plan.num_mtiles, a, 1)
+    cols = N // 2 if act == "swiglu" else N
+    y = torch.empty(plan.padded_rows, cols, dtype=x.dtype, device="cuda")
+    native.mgrouped_gemm(a, w, y, None, plan.mtile_expert, plan.tile_pairs, plan.num_mtiles, False, act, plan.status)
+    ref = torch.empty(R, cols, dtype=x.dtype, device="cuda")
+    native.unpad_rows(y, plan.dst_row, ref)
+    if scatter:
+        ref = torch.empty_like(ref).index_copy_(0, perm, ref)
+    assert torch.equal(out, ref)
