@@ -365,8 +365,13 @@ static int mgrouped_common(const char* name, const void* a, const void* w, void*
   // a work item streams half as many weight columns per tensor-core cycle as two independent CTAs do (measured at
   // 64 rows per expert, DeepSeek-V3 shape: gate/up 4.10 -> 2.69 ms, down 2.01 -> 1.38; at 16 rows per expert,
   // OLMoE shape: -6..12 %; at 128 rows per expert 0..5 %).
+  // Epilogues that move only the result (plain stores, gated without the saved product) leave the one-CTA kernels ahead up
+  // to 192 rows per expert, where a pair's second CTA is idle for a third of the pairs (188 rows, 128 experts, K 2048:
+  // gate/up 232 -> 218 us, down 180 -> 166; at 256 rows 185 -> 188 and 121 -> 119; with side tiles 239 -> 248 at 188).
+  const bool light = epi == EPI_ACT || (epi == EPI_GLU && x.aux_out == nullptr);
   const long long mean_rows_per_expert = (padded_rows - static_cast<long long>(E) * (BM - 1)) / E;
-  const bool pairs = tile_pairs != nullptr && (o.single_cta == 0 ? mean_rows_per_expert > BM : o.single_cta < 0);
+  const bool pairs = tile_pairs != nullptr &&
+                     (o.single_cta == 0 ? mean_rows_per_expert > (light ? BM + BM / 2 : BM) : o.single_cta < 0);
   const int64_t a_rows = x.gather_row_src != nullptr ? x.gather_rows : (x.compact_rows >= 0 ? x.compact_rows : padded_rows);
 #define MOE_MG(TYPE)                                                                                              \
   (pairs ? (bn == 256 ? mgrouped_dispatch<TYPE, 256, 2>(a, w, a_rows, K, N, E, w_transposed, epi, args, dtype, lp) \
