@@ -189,6 +189,11 @@ __device__ __forceinline__ constexpr uint32_t make_idesc() {
 // swizzled 32-row x 128-byte tiles: one for the plain-store and GLU epilogues, two for the dGLU and the ungated AUX
 // epilogues (the saved product of the next chunk lands in one while the other is computed on and stored from; or the
 // un-activated and the activated product are stored side by side), which costs those kernels one operand stage.
+// One-CTA kernels have 48 KB stages and stream weights past few rows, so what they keep in flight is their speed: the dGLU
+// epilogue takes one staging tile there (its copies in and out then alternate, hidden by the next item) and keeps a
+// fourth stage: 1001 tokens x 8 slots, 64 experts, K 2048 95 -> 90 us, 64 tokens on 8 wide experts 224 -> 211.  (A second
+// tile and three stages for their weight-gradient kernels: 113 -> 122 us at two steps per item, 0.6 % of a pass at one; not
+// taken.)
 template <int BN, int CTAS, int EPI>
 struct SmemPlan {
   static constexpr int kABytes = BM * BK * 2;
@@ -196,7 +201,7 @@ struct SmemPlan {
   static constexpr int kBBytes = kBCols * BK * 2;
   static constexpr int kStageBytes = kABytes + kBBytes;
   static constexpr int kStagingTile = 32 * 128;
-  static constexpr int kTilesPerWarp = (EPI == EPI_DGLU || EPI == EPI_ACT_AUX) ? 2 : 1;
+  static constexpr int kTilesPerWarp = ((EPI == EPI_DGLU && CTAS == 2) || EPI == EPI_ACT_AUX) ? 2 : 1;
   static constexpr int kStagingBytes = kEpilogueWarps * kTilesPerWarp * kStagingTile;
   static constexpr int kBarrierBytes = 512;
   static constexpr int kBudget = 232448 - 1024 - kBarrierBytes - kStagingBytes;  // 227 KB minus alignment slack
@@ -790,7 +795,10 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     // the 128-byte-swizzle tensor copies read and write
     const uint32_t stage_base = staging_addr + (warp - 2) * (Plan::kTilesPerWarp * Plan::kStagingTile);
     const uint32_t my_epi_bar = epi_bar + (warp - 2) * 16;
-    uint32_t q = 0;  // dGLU: running count of side-input tiles this warp has received (buffer = q & 1)
+    // running count of side-input tiles this warp has received; two staging tiles are used in turn
+    uint32_t q = 0;
+    const auto side_buf = [](uint32_t n) { return Plan::kTilesPerWarp == 2 ? (n & 1) : 0u; };
+    const auto side_parity = [](uint32_t n) { return Plan::kTilesPerWarp == 2 ? (n >> 1) & 1 : n & 1; };
     const int co_row = lane >> 3;  // coalesced access: row within a group of four
     const int co_ck = lane & 7;    // and 16-byte piece of the row's 128 bytes
     TileCoord c_next = decode_tile<KG, CTAS>(unit < ntiles ? unit : 0, mt, nt, win, args, BN, rank);
@@ -841,9 +849,9 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         const int col0 = c.n0 + chunk_begin * 32;
         if (quad_live && col0 < N && lane == 0) {
           bulk_wait_read_all();
-          const uint32_t bar = my_epi_bar + 8 * (q & 1);
+          const uint32_t bar = my_epi_bar + 8 * side_buf(q);
           mbar_arrive_expect_tx(bar, Plan::kStagingTile);
-          tma_load_2d_plain(stage_base + (q & 1) * Plan::kStagingTile, &tmap_c, EPI == EPI_DGLU ? 2 * col0 : col0,
+          tma_load_2d_plain(stage_base + side_buf(q) * Plan::kStagingTile, &tmap_c, EPI == EPI_DGLU ? 2 * col0 : col0,
                             static_cast<int>(warp_row0), bar);
         }
         __syncwarp();
@@ -1104,11 +1112,11 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         for (int chunk = chunk_begin; chunk < chunk_begin + kChunksPerWarp; ++chunk) {
           const int col0 = c.n0 + chunk * 32;
           const bool live = col0 < N;  // uniform over the warp
-          const uint32_t buf = stage_base + (q & 1) * Plan::kStagingTile;
+          const uint32_t buf = stage_base + side_buf(q) * Plan::kStagingTile;
           uint4 h_cur[8];
           if (live) {
             const int ncol0 = col0 + 32;
-            if (chunk + 1 < chunk_begin + kChunksPerWarp && ncol0 < N && lane == 0) {
+            if (Plan::kTilesPerWarp == 2 && chunk + 1 < chunk_begin + kChunksPerWarp && ncol0 < N && lane == 0) {
               // next chunk's tile into the other buffer, once the store that last read it is done with it
               bulk_wait_read_all();
               const uint32_t nbar = my_epi_bar + 8 * ((q + 1) & 1);
@@ -1117,7 +1125,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                                 static_cast<int>(warp_row0), nbar);
             }
             __syncwarp();
-            if (!__all_sync(0xFFFFFFFFu, mbar_wait(my_epi_bar + 8 * (q & 1), (q >> 1) & 1, wctx, DS_TIMEOUT_EPILOGUE))) {
+            if (!__all_sync(0xFFFFFFFFu, mbar_wait(my_epi_bar + 8 * side_buf(q), side_parity(q), wctx, DS_TIMEOUT_EPILOGUE))) {
               failed = true;
               break;
             }
@@ -1157,6 +1165,12 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
             if (lane == 0) {
               tma_store_2d(&tmap_d, 2 * col0, static_cast<int>(warp_row0), buf);
               bulk_commit();
+              if (Plan::kTilesPerWarp == 1 && chunk + 1 < chunk_begin + kChunksPerWarp && col0 + 32 < N) {
+                // the only tile: the next chunk comes in when this one has been read
+                bulk_wait_read_all();
+                mbar_arrive_expect_tx(my_epi_bar, Plan::kStagingTile);
+                tma_load_2d_plain(buf, &tmap_c, 2 * (col0 + 32), static_cast<int>(warp_row0), my_epi_bar);
+              }
             }
             ++q;
           }
