@@ -269,8 +269,7 @@ int moe_combine_bwd_tokens(const void* dout, const void* scores, const void* ys,
  *                 of one copy over a blocked view of the matrix (which needs the column count to be a multiple
  *                 of 64 and is otherwise the default): for comparison measurements
  *   lane_stores   1 = output tiles in the padded layout are written with 16-byte stores by the lanes instead of bulk
- *                 tensor stores from the staging tile (the default when the column count is a multiple of 64): for
- *                 comparison measurements
+ *                 tensor stores from the staging tile (the default): for comparison measurements
  *   expert_begin, expert_end  M-grouped kernels: when end > begin, process exactly the experts [begin, end) (needs
  *                 tile_pairs); overrides chunk_index / chunk_count.  Lets a caller cut the expert list into slices
  *                 of unequal size, e.g. by row counts
@@ -405,8 +404,17 @@ int moe_kgrouped_gemm_gather(const void* src, int64_t src_rows, const int32_t* r
  *   gather         token rows are gathered by the gate/up GEMM's loads (x is read again for d_w1); xs is then unused
  *   fused_combine  the down GEMM adds the scaled rows into out (zeroed first); ys and the fold are then unused
  *   keep           a backward pass will follow: padding rows of xs are zeroed, pre_act (unless act is none) is written
+ *   identity       num_experts = topk = 1 and every score is 1: group_indices holds {0, num_tokens} (read, not written); x,
+ *                  grad_out, out and dx stand in the place of xs, gs, ys and dxs, and MOE_FWD_DISPATCH / FOLD and MOE_BWD_FOLD /
+ *                  FOLD_DX / ROUTER do not apply
  *   workspace      for MOE_FWD_ROUTE of more than 131072 rows, moe_routing_workspace_bytes(num_tokens * topk, num_experts)
  *                  bytes
+ *   addend         NULL, or a [num_tokens, d] tensor that the fold adds (not with fused_combine)
+ *   dl             NULL, or the router's backward is part of the pass: scores are the softmax of the selected `logits`
+ *                  [num_tokens, num_experts] = x @ router_w [d, num_experts], renormalised or not (all in `dtype`).  MOE_BWD_ROUTER
+ *                  (after MOE_BWD_FOLD) writes the gradient of the selected logits to dl [num_tokens, topk] (fp32) and that of
+ *                  all logits to dlogits [num_tokens, num_experts rounded up to 8] (zeros past the experts), and the transpose
+ *                  of router_w to router_t; MOE_BWD_FOLD_DX then adds the router's share to dx
  * w1 [E, d, inter or 2*inter], w2 [E, inter, d]; xs, ys, gs, dxs [padded_rows, d]; pre_act, d_pre like w1's width; hidden
  * [padded_rows, inter]; out, dx, grad_out, x [num_tokens, d]; scores, d_scores [num_tokens, topk].
  * --------------------------------------------------------------------------------- */
@@ -414,7 +422,7 @@ typedef struct moe_expert_pass {
   int64_t num_tokens;
   int64_t padded_rows;
   int32_t d, inter, num_experts, topk, act, dtype;
-  int32_t gather, fused_combine, keep;
+  int32_t gather, fused_combine, keep, identity;
   const int64_t* expert_idx; /* [num_tokens, topk] */
   const void *x, *scores, *w1, *w2;
   int32_t *group_indices, *pad_offsets, *row_src, *dst_row, *mtile_expert, *tile_pairs, *num_mtiles, *status;
@@ -423,6 +431,10 @@ typedef struct moe_expert_pass {
   void *xs, *pre_act, *hidden, *ys, *out;
   const void* grad_out;
   void *gs, *d_scores, *d_pre, *dxs, *dx, *d_w1, *d_w2;
+  const void* addend;
+  const void *logits, *router_w;
+  float* dl;
+  void *dlogits, *router_t;
 } moe_expert_pass;
 
 /* sizeof(moe_expert_pass), for bindings that declare the struct themselves. */
@@ -442,7 +454,8 @@ int moe_expert_forward(const moe_expert_pass* pass, int steps, void* stream);
 #define MOE_BWD_FOLD_DX 8 /* dx */
 #define MOE_BWD_DW1 16
 #define MOE_BWD_DW2 32
-#define MOE_BWD_ALL 63
+#define MOE_BWD_ROUTER 64 /* dl, dlogits, router_t */
+#define MOE_BWD_ALL 127
 int moe_expert_backward(const moe_expert_pass* pass, int steps, void* stream);
 
 /* The functional grouped GEMM in one call, rows grouped by `group_indices` [num_experts + 1]:

@@ -87,6 +87,12 @@ int routing_metadata(const int64_t* expert_idx, int64_t num_rows, int num_expert
 struct RowCounts {
   const int32_t* pad_offsets = nullptr;
   const int32_t* group_indices = nullptr;
+  // Operands and results that are not in the padded layout but hold their rows without padding, expert by expert: their row
+  // counts (-1: padded).  With one expert that is a plain matrix; the copy engine fills loads past its end with zeros and
+  // drops stores there.
+  int64_t a_rows = -1;
+  int64_t b_rows = -1;    // K-grouped
+  int64_t out_rows = -1;  // M-grouped plain stores, one expert
 };
 
 // The entry points of the same names, told which rows exist.
@@ -121,6 +127,14 @@ int mgrouped_gemm_rows(const void* a, int64_t compact_rows, const void* w, void*
                        const RowCounts& counts);
 int dispatch_rows(const void* src, const int32_t* dst_row, const int32_t* row_src, const int32_t* num_mtiles, void* dst,
                   int64_t num_tokens, int topk, int64_t padded_rows, int cols, int dtype, void* stream, bool live_blocks_only);
+// moe_combine_topk with further summands, all nullable (FoldExtra in csrc/rows.cu).
+int combine_topk(const void* ys, const void* scores, const int32_t* dst_row, void* out, int64_t num_tokens, int topk, int cols,
+                 int dtype, const void* addend, const float* dlogits, const int64_t* experts, const void* router_t,
+                 void* stream);
+// Backward of "softmax over the selected logits" (csrc/router.cu).
+int router_backward(const void* logits, const int64_t* experts, const void* d_scores, const void* router_w, float* dl,
+                    void* dlogits, void* router_t, int64_t num_tokens, int num_experts, int topk, int cols, int dtype,
+                    void* stream);
 int combine_bwd_tokens(const void* dout, const void* scores, const void* ys, const int32_t* dst_row, const int32_t* row_src,
                        const int32_t* num_mtiles, void* gs, void* dscores, int64_t num_tokens, int topk, int cols, int dtype,
                        void* stream, bool live_blocks_only);

@@ -192,11 +192,10 @@ struct MExtras {
   int chunk_index = 0;
   int chunk_count = 1;
   RowCounts counts;
-  int64_t compact_rows = -1;  // >= 0: A has this many rows, without padding (counts given)
 };
 
 template <typename T, int BN, int CTAS>
-static int mgrouped_dispatch(const void* a, const void* w, int64_t a_rows, int K, int N, int E, int w_transposed, int epi,
+static int mgrouped_dispatch(const void* a, const void* w, int64_t a_rows, int64_t out_rows, int K, int N, int E, int w_transposed, int epi,
                              const GemmArgs& args, int dtype, const LaunchParams& lp) {
   CUtensorMap ta, tb;
   const bool gather = args.a_row_src != nullptr;  // selects the kernel variant whose operand loads gather rows
@@ -223,7 +222,7 @@ static int mgrouped_dispatch(const void* a, const void* w, int64_t a_rows, int K
   if (epi == EPI_ACT) {
     CUtensorMap td = ta;
     if (args.out_tma) {
-      const uint64_t dims[2] = {(uint64_t)N, (uint64_t)(args.mtiles_bound) * BM};
+      const uint64_t dims[2] = {(uint64_t)N, (uint64_t)out_rows};
       const uint32_t box[2] = {64, 32};
       int rc = make_tmap(&td, dtype, args.out, 2, dims, box);
       if (rc != MOE_OK) return rc;
@@ -256,7 +255,7 @@ static int mgrouped_dispatch(const void* a, const void* w, int64_t a_rows, int K
   // tensor copies of 32-row x 64-column boxes
   CUtensorMap tc, td;
   {
-    const uint64_t dims[2] = {(uint64_t)(2 * N), (uint64_t)a_rows};
+    const uint64_t dims[2] = {(uint64_t)(2 * N), (uint64_t)(args.mtiles_bound) * BM};
     const uint32_t box[2] = {64, 32};
     int rc = make_tmap(&tc, dtype, args.aux_in, 2, dims, box);
     if (rc != MOE_OK) return rc;
@@ -313,7 +312,7 @@ static int mgrouped_common(const char* name, const void* a, const void* w, void*
   }
   args.pad_offsets = x.counts.pad_offsets;
   args.group_indices = x.counts.pad_offsets != nullptr ? x.counts.group_indices : nullptr;
-  args.a_compact = x.compact_rows >= 0 ? 1 : 0;
+  args.a_compact = x.counts.a_rows >= 0 ? 1 : 0;
   args.num_mtiles = num_mtiles;
   args.num_experts = E;
   args.n_dim = N;
@@ -372,19 +371,20 @@ static int mgrouped_common(const char* name, const void* a, const void* w, void*
   const long long mean_rows_per_expert = (padded_rows - static_cast<long long>(E) * (BM - 1)) / E;
   const bool pairs = tile_pairs != nullptr &&
                      (o.single_cta == 0 ? mean_rows_per_expert > (light ? BM + BM / 2 : BM) : o.single_cta < 0);
-  const int64_t a_rows = x.gather_row_src != nullptr ? x.gather_rows : (x.compact_rows >= 0 ? x.compact_rows : padded_rows);
+  const int64_t a_rows = x.gather_row_src != nullptr ? x.gather_rows : (x.counts.a_rows >= 0 ? x.counts.a_rows : padded_rows);
+  const int64_t out_rows = x.counts.out_rows >= 0 ? x.counts.out_rows : padded_rows;
 #define MOE_MG(TYPE)                                                                                              \
-  (pairs ? (bn == 256 ? mgrouped_dispatch<TYPE, 256, 2>(a, w, a_rows, K, N, E, w_transposed, epi, args, dtype, lp) \
-                      : mgrouped_dispatch<TYPE, 128, 2>(a, w, a_rows, K, N, E, w_transposed, epi, args, dtype, lp)) \
-         : (bn == 256 ? mgrouped_dispatch<TYPE, 256, 1>(a, w, a_rows, K, N, E, w_transposed, epi, args, dtype, lp) \
-                      : mgrouped_dispatch<TYPE, 128, 1>(a, w, a_rows, K, N, E, w_transposed, epi, args, dtype, lp)))
+  (pairs ? (bn == 256 ? mgrouped_dispatch<TYPE, 256, 2>(a, w, a_rows, out_rows, K, N, E, w_transposed, epi, args, dtype, lp) \
+                      : mgrouped_dispatch<TYPE, 128, 2>(a, w, a_rows, out_rows, K, N, E, w_transposed, epi, args, dtype, lp)) \
+         : (bn == 256 ? mgrouped_dispatch<TYPE, 256, 1>(a, w, a_rows, out_rows, K, N, E, w_transposed, epi, args, dtype, lp) \
+                      : mgrouped_dispatch<TYPE, 128, 1>(a, w, a_rows, out_rows, K, N, E, w_transposed, epi, args, dtype, lp)))
   if (dtype == MOE_DTYPE_BF16) return MOE_MG(__nv_bfloat16);
   return MOE_MG(__half);
 #undef MOE_MG
 }
 
 template <typename T, int BN, int CTAS>
-static int kgrouped_dispatch(const void* a, const void* b, int64_t a_rows, int64_t padded_rows, int M, int N,
+static int kgrouped_dispatch(const void* a, const void* b, int64_t a_rows, int64_t b_rows, int M, int N,
                              const GemmArgs& args, int dtype, const LaunchParams& lp) {
   CUtensorMap ta, tb;
   if (args.a_blocked) {
@@ -397,10 +397,10 @@ static int kgrouped_dispatch(const void* a, const void* b, int64_t a_rows, int64
     if (rc != MOE_OK) return rc;
   }
   if (args.b_blocked) {
-    int rc = make_tmap_blocked(&tb, dtype, b, (uint64_t)padded_rows, (uint64_t)N, 0, BK, (uint32_t)(BN / CTAS / 64));
+    int rc = make_tmap_blocked(&tb, dtype, b, (uint64_t)b_rows, (uint64_t)N, 0, BK, (uint32_t)(BN / CTAS / 64));
     if (rc != MOE_OK) return rc;
   } else {
-    const uint64_t dims[2] = {(uint64_t)N, (uint64_t)padded_rows};
+    const uint64_t dims[2] = {(uint64_t)N, (uint64_t)b_rows};
     const uint32_t box[2] = {64, BK};
     int rc = make_tmap(&tb, dtype, b, 2, dims, box);
     if (rc != MOE_OK) return rc;
@@ -419,7 +419,7 @@ static int kgrouped_dispatch(const void* a, const void* b, int64_t a_rows, int64
 static int kgrouped_common(const char* name, const void* a, int64_t gather_rows, const int32_t* gather_row_src,
                            int gather_div, const void* b, void* dw, const int32_t* pad_offsets, int64_t padded_rows, int M,
                            int N, int num_experts, int dtype, const moe_gemm_options* options, int32_t* status,
-                           void* stream, const int32_t* group_indices) {
+                           void* stream, const RowCounts& counts) {
   MOE_CHECK_ARG(a && b && dw && pad_offsets, "%s: null pointer argument", name);
   MOE_CHECK_ARG(aligned16(a) && aligned16(b) && aligned16(dw), "%s: pointers must be 16-byte aligned", name);
   MOE_CHECK_ARG(padded_rows > 0 && padded_rows % BM == 0, "%s: padded_rows=%lld must be a positive multiple of %d", name,
@@ -435,7 +435,7 @@ static int kgrouped_common(const char* name, const void* a, int64_t gather_rows,
   const moe_gemm_options o = resolve(options);
   GemmArgs args{};
   args.pad_offsets = pad_offsets;
-  args.group_indices = group_indices;
+  args.group_indices = counts.group_indices;
   args.num_experts = num_experts;
   args.m_dim = M;
   args.n_dim = N;
@@ -459,12 +459,13 @@ static int kgrouped_common(const char* name, const void* a, int64_t gather_rows,
   // expert, DeepSeek-V3 shape: weight1 gradient 4.00 -> 3.48 ms; at 128 rows per expert pairs are 9 % faster)
   const long long mean_rows_per_expert = (padded_rows - static_cast<long long>(num_experts) * (BM - 1)) / num_experts;
   const bool pairs = o.single_cta == 0 ? mean_rows_per_expert > 64 : o.single_cta < 0;
-  const int64_t a_rows = gather_row_src != nullptr ? gather_rows : padded_rows;
+  const int64_t a_rows = gather_row_src != nullptr ? gather_rows : (counts.a_rows >= 0 ? counts.a_rows : padded_rows);
+  const int64_t b_rows = counts.b_rows >= 0 ? counts.b_rows : padded_rows;
 #define MOE_KG(TYPE)                                                                                      \
-  (pairs ? (bn == 256 ? kgrouped_dispatch<TYPE, 256, 2>(a, b, a_rows, padded_rows, M, N, args, dtype, lp)  \
-                      : kgrouped_dispatch<TYPE, 128, 2>(a, b, a_rows, padded_rows, M, N, args, dtype, lp)) \
-         : (bn == 256 ? kgrouped_dispatch<TYPE, 256, 1>(a, b, a_rows, padded_rows, M, N, args, dtype, lp)  \
-                      : kgrouped_dispatch<TYPE, 128, 1>(a, b, a_rows, padded_rows, M, N, args, dtype, lp)))
+  (pairs ? (bn == 256 ? kgrouped_dispatch<TYPE, 256, 2>(a, b, a_rows, b_rows, M, N, args, dtype, lp)  \
+                      : kgrouped_dispatch<TYPE, 128, 2>(a, b, a_rows, b_rows, M, N, args, dtype, lp)) \
+         : (bn == 256 ? kgrouped_dispatch<TYPE, 256, 1>(a, b, a_rows, b_rows, M, N, args, dtype, lp)  \
+                      : kgrouped_dispatch<TYPE, 128, 1>(a, b, a_rows, b_rows, M, N, args, dtype, lp)))
   if (dtype == MOE_DTYPE_BF16) return MOE_KG(__nv_bfloat16);
   return MOE_KG(__half);
 #undef MOE_KG
@@ -544,7 +545,7 @@ int kgrouped_gemm(const void* a, const void* b, void* dw, const int32_t* pad_off
                   int num_experts, int dtype, const moe_gemm_options* options, int32_t* status, void* stream, const
                   RowCounts& counts) {
   return kgrouped_common("moe_kgrouped_gemm", a, 0, nullptr, 1, b, dw, pad_offsets, padded_rows, M, N, num_experts, dtype,
-                         options, status, stream, counts.group_indices);
+                         options, status, stream, counts);
 }
 
 int kgrouped_gemm_gather(const void* src, int64_t src_rows, const int32_t* row_src, int div, const void* b, void* dw,
@@ -552,7 +553,7 @@ int kgrouped_gemm_gather(const void* src, int64_t src_rows, const int32_t* row_s
                          moe_gemm_options* options, int32_t* status, void* stream, const RowCounts& counts) {
   MOE_CHECK_ARG(row_src != nullptr, "moe_kgrouped_gemm_gather: row_src is null");
   return kgrouped_common("moe_kgrouped_gemm_gather", src, src_rows, row_src, div, b, dw, pad_offsets, padded_rows, M, N,
-                         num_experts, dtype, options, status, stream, counts.group_indices);
+                         num_experts, dtype, options, status, stream, counts);
 }
 
 int mgrouped_gemm_rows(const void* a, int64_t compact_rows, const void* w, void* out, const int32_t* out_rows,
@@ -561,7 +562,7 @@ int mgrouped_gemm_rows(const void* a, int64_t compact_rows, const void* w, void*
                        const RowCounts& counts) {
   MExtras x;
   x.counts = counts;
-  x.compact_rows = compact_rows;
+  x.counts.a_rows = compact_rows;
   x.push_row = out_rows;
   return mgrouped_common("moe_rows_gemm", a, w, out, x, mtile_expert, tile_pairs, num_mtiles, padded_rows, K, N, num_experts, 0,
                          act_is_glu(act) ? EPI_GLU : EPI_ACT, act, dtype, nullptr, status, stream);

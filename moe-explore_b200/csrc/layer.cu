@@ -18,6 +18,21 @@ extern "C" int moe_expert_forward(const moe_expert_pass* p, int steps, void* str
   const int up_cols = glu(p->act) ? 2 * p->inter : p->inter;
   const int64_t rows = p->num_tokens * p->topk;
   const Chain chain;
+  if (p->identity) {
+    // One expert, weight one: no row moves and nothing is folded.  The GEMMs read x and write out where they are.
+    RowCounts in{p->pad_offsets, p->group_indices}, out = in;
+    in.a_rows = out.out_rows = p->num_tokens;
+    if (steps & MOE_FWD_ROUTE)
+      MOE_STEP(moe_layout_from_groups(p->group_indices, p->num_tokens, 1, p->pad_offsets, nullptr, nullptr, p->mtile_expert,
+                                      p->tile_pairs, p->num_mtiles, p->status, stream));
+    if (steps & MOE_FWD_UP)
+      MOE_STEP(mgrouped_gemm(p->x, p->w1, p->hidden, p->pre_act, p->mtile_expert, p->tile_pairs, p->num_mtiles, p->padded_rows,
+                             p->d, up_cols, 1, 0, p->act, p->dtype, 0, 1, nullptr, p->status, stream, in));
+    if (steps & MOE_FWD_DOWN)
+      MOE_STEP(mgrouped_gemm(p->hidden, p->w2, p->out, nullptr, p->mtile_expert, p->tile_pairs, p->num_mtiles, p->padded_rows,
+                             p->inter, p->d, 1, 0, MOE_ACT_NONE, p->dtype, 0, 1, nullptr, p->status, stream, out));
+    return MOE_OK;
+  }
   const RowCounts counts{p->pad_offsets, p->group_indices};
   if (steps & MOE_FWD_ROUTE)
     MOE_STEP(routing_metadata(p->expert_idx, rows, p->num_experts, p->group_indices, nullptr, p->pad_offsets, p->row_src,
@@ -54,7 +69,8 @@ extern "C" int moe_expert_forward(const moe_expert_pass* p, int steps, void* str
     }
   }
   if ((steps & MOE_FWD_FOLD) && !p->fused_combine)
-    MOE_STEP(moe_combine_topk(p->ys, p->scores, p->dst_row, p->out, p->num_tokens, p->topk, p->d, p->dtype, stream));
+    MOE_STEP(combine_topk(p->ys, p->scores, p->dst_row, p->out, p->num_tokens, p->topk, p->d, p->dtype, p->addend, nullptr,
+                          nullptr, nullptr, stream));
   return MOE_OK;
 }
 
@@ -62,10 +78,35 @@ extern "C" int moe_expert_backward(const moe_expert_pass* p, int steps, void* st
   MOE_CHECK_ARG(p != nullptr, "moe_expert_backward: null pointer argument");
   const int up_cols = glu(p->act) ? 2 * p->inter : p->inter;
   const Chain chain;
+  if (p->identity) {
+    RowCounts in{p->pad_offsets, p->group_indices}, out = in, right = in;
+    in.a_rows = out.out_rows = right.b_rows = p->num_tokens;
+    if (steps & MOE_BWD_DOWN) {
+      if (p->act == MOE_ACT_NONE)
+        MOE_STEP(mgrouped_gemm(p->grad_out, p->w2, p->d_pre, nullptr, p->mtile_expert, p->tile_pairs, p->num_mtiles,
+                               p->padded_rows, p->d, p->inter, 1, 1, MOE_ACT_NONE, p->dtype, 0, 1, nullptr, p->status, stream, in));
+      else
+        MOE_STEP(mgrouped_gemm_dglu(p->grad_out, p->w2, p->pre_act, p->d_pre, p->mtile_expert, p->tile_pairs, p->num_mtiles,
+                                    p->padded_rows, p->d, p->inter, 1, p->act, p->dtype, 0, 1, nullptr, p->status, stream, in));
+    }
+    if (steps & MOE_BWD_UP)
+      MOE_STEP(mgrouped_gemm(p->d_pre, p->w1, p->dx, nullptr, p->mtile_expert, p->tile_pairs, p->num_mtiles, p->padded_rows,
+                             up_cols, p->d, 1, 1, MOE_ACT_NONE, p->dtype, 0, 1, nullptr, p->status, stream, out));
+    if (steps & MOE_BWD_DW1)
+      MOE_STEP(kgrouped_gemm(p->x, p->d_pre, p->d_w1, p->pad_offsets, p->padded_rows, p->d, up_cols, 1, p->dtype, nullptr,
+                             p->status, stream, in));
+    if (steps & MOE_BWD_DW2)
+      MOE_STEP(kgrouped_gemm(p->hidden, p->grad_out, p->d_w2, p->pad_offsets, p->padded_rows, p->inter, p->d, 1, p->dtype,
+                             nullptr, p->status, stream, right));
+    return MOE_OK;
+  }
   const RowCounts counts{p->pad_offsets, p->group_indices};
   if (steps & MOE_BWD_FOLD)
     MOE_STEP(combine_bwd_tokens(p->grad_out, p->scores, p->ys, p->dst_row, p->row_src, p->num_mtiles, p->gs, p->d_scores,
                                     p->num_tokens, p->topk, p->d, p->dtype, stream, true));
+  if ((steps & MOE_BWD_ROUTER) && p->dl != nullptr)
+    MOE_STEP(router_backward(p->logits, p->expert_idx, p->d_scores, p->router_w, p->dl, p->dlogits, p->router_t, p->num_tokens,
+                             p->num_experts, p->topk, p->d, p->dtype, stream));
   if (steps & MOE_BWD_DOWN) {
     if (p->act == MOE_ACT_NONE)  // linear "activation": d_pre = gs @ W2^T
       MOE_STEP(mgrouped_gemm(p->gs, p->w2, p->d_pre, nullptr, p->mtile_expert, p->tile_pairs, p->num_mtiles, p->padded_rows,
@@ -79,7 +120,8 @@ extern "C" int moe_expert_backward(const moe_expert_pass* p, int steps, void* st
     MOE_STEP(mgrouped_gemm(p->d_pre, p->w1, p->dxs, nullptr, p->mtile_expert, p->tile_pairs, p->num_mtiles, p->padded_rows,
                                up_cols, p->d, p->num_experts, 1, MOE_ACT_NONE, p->dtype, 0, 1, nullptr, p->status, stream, counts));
   if (steps & MOE_BWD_FOLD_DX)
-    MOE_STEP(moe_combine_topk(p->dxs, nullptr, p->dst_row, p->dx, p->num_tokens, p->topk, p->d, p->dtype, stream));
+    MOE_STEP(combine_topk(p->dxs, nullptr, p->dst_row, p->dx, p->num_tokens, p->topk, p->d, p->dtype, nullptr, p->dl,
+                          p->expert_idx, p->router_t, stream));
   if (steps & MOE_BWD_DW1) {
     if (p->gather)  // x is the layer input in token order: its rows are gathered by the loads again
       MOE_STEP(kgrouped_gemm_gather(p->x, p->num_tokens, p->row_src, p->topk, p->d_pre, p->d_w1, p->pad_offsets,

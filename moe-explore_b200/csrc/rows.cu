@@ -325,10 +325,22 @@ __device__ __forceinline__ void fma8(float (&acc)[8], const uint4& u, float scal
 // HBM-bound (each slot's row read once, one row written).  The loads of up to SLOTS slots are issued together -- a loop over
 // the slots keeps one in flight per thread -- and added in slot order.  B200, 8 slots, 8192 tokens: 14 KB rows
 // 221 -> 172 us (4.8 -> 6.1 TB/s), 4 KB rows 72 -> 61; 1001 tokens 18.5 -> 14.4; 4 slots, 16384 tokens of 4 KB 77 -> 65.
-template <typename T, int TPR, int SLOTS>
+// With `extra` the fold takes more summands before its one rounding, instead of passes of their own over [T, cols]:
+//   addend   a [T, cols] tensor (the shared experts' output);
+//   dlogits  [T, topk] fp32 and experts [T, topk]: dlogits(t, s) * router_t[experts(t, s), :], the router's share of the input
+//            gradient (its rows stay in L2).  16384 tokens x 4 slots, 60 experts, 4 KB rows: a 43 us GEMM and a 30 us
+//            addition for 12 us more here.
+struct FoldExtra {
+  const uint4* addend;
+  const float* dlogits;
+  const int64_t* experts;
+  const uint4* router_t;
+};
+
+template <typename T, int TPR, int SLOTS, bool EXTRA>
 __global__ void __launch_bounds__(kRowThreads)
 combine_topk_kernel(const uint4* __restrict__ ys, const T* __restrict__ scores, const int32_t* __restrict__ dst_row,
-                    uint4* __restrict__ out, int64_t num_tokens, int topk, int vec_per_row) {
+                    uint4* __restrict__ out, int64_t num_tokens, int topk, int vec_per_row, FoldExtra extra) {
   grid_release();
   grid_wait();
   constexpr int kRows = kRowThreads / TPR;
@@ -349,7 +361,19 @@ combine_topk_kernel(const uint4* __restrict__ ys, const T* __restrict__ scores, 
         }
 #pragma unroll
         for (int i = 0; i < SLOTS; ++i) fma8<T>(acc, u[i], scale[i]);
+        if (EXTRA && extra.dlogits != nullptr) {
+#pragma unroll
+          for (int i = 0; i < SLOTS; ++i) {
+            const int64_t j = t * topk + s0 + i;
+            const bool in = s0 + i < topk;
+            scale[i] = in ? extra.dlogits[j] : 0.0f;
+            u[i] = in ? extra.router_t[extra.experts[j] * vec_per_row + v] : make_uint4(0, 0, 0, 0);
+          }
+#pragma unroll
+          for (int i = 0; i < SLOTS; ++i) fma8<T>(acc, u[i], scale[i]);
+        }
       }
+      if (EXTRA && extra.addend != nullptr) fma8<T>(acc, extra.addend[t * vec_per_row + v], 1.0f);
       uint4 r;
       r.x = Elem<T>::pack2(acc[0], acc[1]);
       r.y = Elem<T>::pack2(acc[2], acc[3]);
@@ -505,26 +529,29 @@ static void launch_dispatch(const void* src, const int32_t* dst_row, const int32
 
 // The slots whose loads are issued together: the smallest power of two that covers topk, at most 8 (a wider one wastes
 // predicated loads: 2 slots with 8, 59 us; with 2 or 4, 47).
-template <typename T, int TPR>
+template <typename T, int TPR, bool EXTRA>
 static void launch_combine_slots(const uint4* ys, const T* scores, const int32_t* dst_row, uint4* out, int64_t num_tokens,
-                                 int topk, int vec_per_row, cudaStream_t s) {
+                                 int topk, int vec_per_row, const FoldExtra& extra, cudaStream_t s) {
   const int grid = row_grid((num_tokens + kRowThreads / TPR - 1) / (kRowThreads / TPR));
-  if (topk == 1) launch_kernel(combine_topk_kernel<T, TPR, 1>, grid, kRowThreads, s, ys, scores, dst_row, out, num_tokens, topk, vec_per_row);
-  else if (topk == 2) launch_kernel(combine_topk_kernel<T, TPR, 2>, grid, kRowThreads, s, ys, scores, dst_row, out, num_tokens, topk, vec_per_row);
-  else if (topk <= 4) launch_kernel(combine_topk_kernel<T, TPR, 4>, grid, kRowThreads, s, ys, scores, dst_row, out, num_tokens, topk, vec_per_row);
-  else launch_kernel(combine_topk_kernel<T, TPR, 8>, grid, kRowThreads, s, ys, scores, dst_row, out, num_tokens, topk, vec_per_row);
+  const auto go = [&](auto kernel) {
+    launch_kernel(kernel, grid, kRowThreads, s, ys, scores, dst_row, out, num_tokens, topk, vec_per_row, extra);
+  };
+  if (topk == 1) go(combine_topk_kernel<T, TPR, 1, EXTRA>);
+  else if (topk == 2) go(combine_topk_kernel<T, TPR, 2, EXTRA>);
+  else if (topk <= 4) go(combine_topk_kernel<T, TPR, 4, EXTRA>);
+  else go(combine_topk_kernel<T, TPR, 8, EXTRA>);
 }
 
-template <typename T>
+template <typename T, bool EXTRA>
 static void launch_combine(const void* ys, const void* scores, const int32_t* dst_row, void* out, int64_t num_tokens, int topk,
-                           int vec_per_row, cudaStream_t s) {
+                           int vec_per_row, const FoldExtra& extra, cudaStream_t s) {
   const uint4* in = static_cast<const uint4*>(ys);
   const T* sc = static_cast<const T*>(scores);
   uint4* o = static_cast<uint4*>(out);
   switch (fold_threads_per_row(vec_per_row)) {
-    case 32: return launch_combine_slots<T, 32>(in, sc, dst_row, o, num_tokens, topk, vec_per_row, s);
-    case 64: return launch_combine_slots<T, 64>(in, sc, dst_row, o, num_tokens, topk, vec_per_row, s);
-    default: return launch_combine_slots<T, 128>(in, sc, dst_row, o, num_tokens, topk, vec_per_row, s);
+    case 32: return launch_combine_slots<T, 32, EXTRA>(in, sc, dst_row, o, num_tokens, topk, vec_per_row, extra, s);
+    case 64: return launch_combine_slots<T, 64, EXTRA>(in, sc, dst_row, o, num_tokens, topk, vec_per_row, extra, s);
+    default: return launch_combine_slots<T, 128, EXTRA>(in, sc, dst_row, o, num_tokens, topk, vec_per_row, extra, s);
   }
 }
 
@@ -723,18 +750,32 @@ extern "C" int moe_index_rows(const void* src, const int64_t* index, void* out, 
   return MOE_OK;
 }
 
-extern "C" int moe_combine_topk(const void* ys, const void* scores, const int32_t* dst_row, void* out,
-                                int64_t num_tokens, int topk, int cols, int dtype, void* stream) {
+namespace moe {
+int combine_topk(const void* ys, const void* scores, const int32_t* dst_row, void* out, int64_t num_tokens, int topk, int cols,
+                 int dtype, const void* addend, const float* dlogits, const int64_t* experts, const void* router_t,
+                 void* stream) {
   MOE_CHECK_ARG(num_tokens >= 0 && topk > 0, "moe_combine_topk: bad sizes T=%lld topk=%d", (long long)num_tokens, topk);
   if (num_tokens == 0) return MOE_OK;
   MOE_CHECK_ARG(ys && dst_row && out, "moe_combine_topk: null pointer argument");
   MOE_CHECK_ARG(aligned16(ys) && aligned16(out), "moe_combine_topk: pointers must be 16-byte aligned");
   MOE_ROW_COMMON_CHECKS("moe_combine_topk", cols, dtype);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (dtype == MOE_DTYPE_BF16) launch_combine<__nv_bfloat16>(ys, scores, dst_row, out, num_tokens, topk, cols / 8, s);
-  else launch_combine<__half>(ys, scores, dst_row, out, num_tokens, topk, cols / 8, s);
+  const FoldExtra extra{static_cast<const uint4*>(addend), dlogits, experts, static_cast<const uint4*>(router_t)};
+  const bool more = addend != nullptr || dlogits != nullptr;
+  MOE_CHECK_ARG(aligned16(addend) && aligned16(router_t), "moe_combine_topk: pointers must be 16-byte aligned");
+  const bool bf16 = dtype == MOE_DTYPE_BF16;
+  if (bf16 && more) launch_combine<__nv_bfloat16, true>(ys, scores, dst_row, out, num_tokens, topk, cols / 8, extra, s);
+  else if (bf16) launch_combine<__nv_bfloat16, false>(ys, scores, dst_row, out, num_tokens, topk, cols / 8, extra, s);
+  else if (more) launch_combine<__half, true>(ys, scores, dst_row, out, num_tokens, topk, cols / 8, extra, s);
+  else launch_combine<__half, false>(ys, scores, dst_row, out, num_tokens, topk, cols / 8, extra, s);
   MOE_CUDA(cudaGetLastError());
   return MOE_OK;
+}
+}  // namespace moe
+
+extern "C" int moe_combine_topk(const void* ys, const void* scores, const int32_t* dst_row, void* out,
+                                int64_t num_tokens, int topk, int cols, int dtype, void* stream) {
+  return combine_topk(ys, scores, dst_row, out, num_tokens, topk, cols, dtype, nullptr, nullptr, nullptr, nullptr, stream);
 }
 
 namespace moe {

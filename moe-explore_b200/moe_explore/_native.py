@@ -38,12 +38,12 @@ class GemmOptions(ctypes.Structure):
 class ExpertPass(ctypes.Structure):
     """``moe_expert_pass``: sizes and buffers of one forward or backward pass over the experts."""
     _fields_ = [(f, c_int64) for f in ("num_tokens", "padded_rows")] + \
-               [(f, c_int32) for f in ("d", "inter", "num_experts", "topk", "act", "dtype", "gather", "fused_combine", "keep")] + \
+               [(f, c_int32) for f in ("d", "inter", "num_experts", "topk", "act", "dtype", "gather", "fused_combine", "keep", "identity")] + \
                [(f, c_void_p) for f in ("expert_idx", "x", "scores", "w1", "w2", "group_indices", "pad_offsets", "row_src",
                                         "dst_row", "mtile_expert", "tile_pairs", "num_mtiles", "status", "workspace")] + \
                [("workspace_bytes", c_size_t)] + \
                [(f, c_void_p) for f in ("xs", "pre_act", "hidden", "ys", "out", "grad_out", "gs", "d_scores", "d_pre", "dxs", "dx",
-                                        "d_w1", "d_w2")]
+                                        "d_w1", "d_w2", "addend", "logits", "router_w", "dl", "dlogits", "router_t")]
 
 
 class RowsPass(ctypes.Structure):
@@ -245,7 +245,7 @@ def _opt(options):
 
 ROWS_LAYOUT, ROWS_GATHER, ROWS_GEMM = 1, 2, 4
 FWD_ROUTE, FWD_DISPATCH, FWD_UP, FWD_DOWN, FWD_FOLD = 1, 2, 4, 8, 16
-BWD_FOLD, BWD_DOWN, BWD_UP, BWD_FOLD_DX, BWD_DW1, BWD_DW2 = 1, 2, 4, 8, 16, 32
+BWD_FOLD, BWD_DOWN, BWD_UP, BWD_FOLD_DX, BWD_DW1, BWD_DW2, BWD_ROUTER = 1, 2, 4, 8, 16, 32, 64
 
 
 def run_pass(name: str, p, steps, rows: int) -> None:

@@ -17,6 +17,8 @@ import torch
 
 from moe_explore import _native
 from moe_explore.functional.activation import is_glu
+from moe_explore.params import TopkRouterParams
+from moe_explore.router import topk_of_logits
 from moe_explore.routing_plan import RoutingPlan, device_status, packed_layout
 
 
@@ -30,109 +32,227 @@ def _packed_pointers(words: torch.Tensor, offsets, status: torch.Tensor):
     return tuple(base + o for o in offsets) + (status.data_ptr(),)
 
 
+class _Pass:
+    """What the backward pass needs to know about its forward pass besides the saved tensors."""
+    __slots__ = ("sizes", "routing", "act", "gathered")
+
+
+def _forward(x, scores, weight1, weight2, routing, act, gather_in_gemm: bool, fused_combine: bool, needs_grad: bool, addend=None):
+    """-> (out, _Pass, tensors to save)."""
+    _native.require_cuda(x, scores, weight1, weight2)
+    assert x.dim() == 2 and weight1.dim() == 3 and weight2.dim() == 3
+    T, d = x.shape
+    E, d1, n1 = weight1.shape
+    inter = weight2.size(1)
+    assert d1 == d and weight2.size(0) == E and weight2.size(2) == d, "weight shapes do not match the input"
+    assert n1 == (2 * inter if is_glu(act) else inter), "weight1 width does not match weight2 and the activation"
+    planned = isinstance(routing, RoutingPlan)
+    if planned:
+        topk = routing.topk
+        assert routing.num_rows == T * topk and routing.num_experts == E
+    else:
+        indices, num_experts, topk = routing
+        flat = indices.reshape(-1).contiguous()
+        assert flat.numel() == T * topk and num_experts == E
+    x = x.contiguous()
+    scores = scores.to(x.dtype).contiguous()
+    weight1 = weight1.contiguous()
+    weight2 = weight2.contiguous()
+    code = _native.dtype_code(x.dtype)
+    act_code = _native.ACT_CODES[act]
+    rows = T * topk
+    new = lambda *shape: torch.empty(shape, dtype=x.dtype, device=x.device)
+    fold = not fused_combine or needs_grad   # the backward pass needs the per-slot rows for the router-weight gradient
+
+    steps = []
+    words = workspace = None
+    if planned:
+        rp = routing.padded_rows
+        ids = None
+        plan_ptrs = _plan_pointers(routing)
+    else:
+        rp, offsets, num_words = packed_layout(rows, E)
+        words = torch.empty(num_words, dtype=torch.int32, device=x.device)
+        status = device_status(x.get_device())
+        plan_ptrs = _packed_pointers(words, offsets, status)
+        ids = flat.data_ptr()
+        if rows > _native.ROUTE_ONE_LAUNCH_ROWS:
+            workspace = torch.empty(max(_native.routing_workspace_bytes(rows, E), 16), dtype=torch.uint8, device=x.device)
+        steps.append((_native.FWD_ROUTE, "routing", 1 if workspace is None else 3))
+    xs = None if gather_in_gemm else new(rp, d)
+    # the un-activated product, needed by the backward pass (not kept for inference or without an activation)
+    pre_act = new(rp, n1) if (act is not None and needs_grad) else None
+    hidden = new(rp, inter)
+    ys = new(rp, d) if fold else None
+    out = new(T, d)
+    kind = "glu" if is_glu(act) else "plain"
+    if not gather_in_gemm:
+        steps.append((_native.FWD_DISPATCH, "rows:gather", 1))
+    steps.append((_native.FWD_UP, "mgrouped_gemm:" + kind + ("+gather" if gather_in_gemm else ""), 1))
+    if fold:
+        steps.append((_native.FWD_DOWN, "mgrouped_gemm:plain", 1))
+        steps.append((_native.FWD_FOLD, "rows:combine", 1))
+    else:
+        steps.append((_native.FWD_DOWN, "mgrouped_gemm:combine", 1))
+    if addend is not None:
+        assert fold and addend.shape == out.shape and addend.dtype is out.dtype and addend.is_cuda
+        addend = addend.contiguous()
+    ptr = _native._ptr
+    p = _native.ExpertPass(
+        T, rp, d, inter, E, topk, act_code, code, gather_in_gemm, not fold, needs_grad, 0, ids, x.data_ptr(), scores.data_ptr(),
+        weight1.data_ptr(), weight2.data_ptr(), *plan_ptrs, ptr(workspace),
+        0 if workspace is None else workspace.numel(), ptr(xs), ptr(pre_act), hidden.data_ptr(), ptr(ys), out.data_ptr())
+    p.addend = ptr(addend)
+    _native.run_pass("moe_expert_forward", p, steps, rows)
+    if not needs_grad:
+        return out, None, ()
+    info = _Pass()
+    info.sizes = (T, d, inter, E, topk, rp, n1)
+    info.routing = routing if planned else None
+    info.act = act
+    info.gathered = bool(gather_in_gemm)
+    return out, info, (x if gather_in_gemm else xs, pre_act, hidden, ys, scores, weight1, weight2, words)
+
+
+def _backward(info: _Pass, saved, grad_out, router=None):
+    """-> (dx, d_scores, d_w1, d_w2[, dlogits]); ``router`` = (logits, router weight, expert indices) makes the router's tail and
+    its share of dx part of the pass."""
+    xs, pre_act, hidden, ys, scores, weight1, weight2, words = saved
+    T, d, inter, E, topk, rp, n1 = info.sizes
+    act = info.act
+    rows = T * topk
+    grad_out = grad_out.contiguous()
+    new = lambda *shape: torch.empty(shape, dtype=grad_out.dtype, device=grad_out.device)
+
+    gs, d_scores, d_pre, dxs, dx = new(rp, d), new(T, topk), new(rp, n1), new(rp, d), new(T, d)
+    d_w1, d_w2 = torch.empty_like(weight1), torch.empty_like(weight2)
+    if info.routing is not None:
+        plan_ptrs = _plan_pointers(info.routing)
+    else:
+        plan_ptrs = _packed_pointers(words, packed_layout(rows, E)[1], device_status(words.get_device()))
+    ptr = _native._ptr
+    p = _native.ExpertPass(
+        T, rp, d, inter, E, topk, _native.ACT_CODES[act], _native.dtype_code(grad_out.dtype), info.gathered, False, True, 0, None,
+        xs.data_ptr(), scores.data_ptr(), weight1.data_ptr(), weight2.data_ptr(), *plan_ptrs, None, 0, xs.data_ptr(),
+        ptr(pre_act), hidden.data_ptr(), ys.data_ptr(), None, grad_out.data_ptr(), gs.data_ptr(), d_scores.data_ptr(),
+        d_pre.data_ptr(), dxs.data_ptr(), dx.data_ptr(), d_w1.data_ptr(), d_w2.data_ptr())
+    steps = [(_native.BWD_FOLD, "rows:combine_bwd", 1),
+             (_native.BWD_DOWN, "mgrouped_gemm:wt" if act is None else "mgrouped_gemm:dglu", 1),
+             (_native.BWD_UP, "mgrouped_gemm:wt", 1), (_native.BWD_FOLD_DX, "rows:combine", 1),
+             (_native.BWD_DW1, "kgrouped_gemm:dw1" + ("+gather" if info.gathered else ""), 1),
+             (_native.BWD_DW2, "kgrouped_gemm:dw2", 1)]
+    dlogits = None
+    if router is not None:
+        logits, router_weight, indices = router
+        dl = torch.empty(T, topk, dtype=torch.float32, device=grad_out.device)
+        dlogits, router_t = new(T, (E + 7) // 8 * 8), new(E, d)
+        p.logits, p.router_w, p.expert_idx = logits.data_ptr(), router_weight.data_ptr(), indices.data_ptr()
+        p.dl, p.dlogits, p.router_t = dl.data_ptr(), dlogits.data_ptr(), router_t.data_ptr()
+        steps.insert(1, (_native.BWD_ROUTER, "router:bwd", 1))
+    _native.run_pass("moe_expert_backward", p, steps, rows)
+    return dx, d_scores, d_w1, d_w2, dlogits
+
+
 class ExpertCompute(torch.autograd.Function):
     """``routing`` is a ``RoutingPlan``, or (expert indices [T, topk], num_experts, topk) to be routed as part of the pass: its
-    index arrays then live in one allocation and one library call issues every launch."""
+    index arrays then live in one allocation and one library call issues every launch.  ``addend`` [T, d] is added by the
+    fold."""
 
     @staticmethod
-    def forward(ctx, x, scores, weight1, weight2, routing, act: str, gather_in_gemm: bool, fused_combine: bool):
-        _native.require_cuda(x, scores, weight1, weight2)
-        assert x.dim() == 2 and weight1.dim() == 3 and weight2.dim() == 3
-        T, d = x.shape
-        E, d1, n1 = weight1.shape
-        inter = weight2.size(1)
-        assert d1 == d and weight2.size(0) == E and weight2.size(2) == d, "weight shapes do not match the input"
-        assert n1 == (2 * inter if is_glu(act) else inter), "weight1 width does not match weight2 and the activation"
-        planned = isinstance(routing, RoutingPlan)
-        if planned:
-            topk = routing.topk
-            assert routing.num_rows == T * topk and routing.num_experts == E
-        else:
-            indices, num_experts, topk = routing
-            flat = indices.reshape(-1).contiguous()
-            assert flat.numel() == T * topk and num_experts == E
-        x = x.contiguous()
-        scores = scores.to(x.dtype).contiguous()
-        weight1 = weight1.contiguous()
-        weight2 = weight2.contiguous()
-        code = _native.dtype_code(x.dtype)
-        act_code = _native.ACT_CODES[act]
-        rows = T * topk
-        new = lambda *shape: torch.empty(shape, dtype=x.dtype, device=x.device)
+    def forward(ctx, x, scores, weight1, weight2, routing, act: str, gather_in_gemm: bool, fused_combine: bool, addend=None):
         needs_grad = any(ctx.needs_input_grad[:4])
-        fold = not fused_combine or needs_grad   # the backward pass needs the per-slot rows for the router-weight gradient
-
-        steps = []
-        words = workspace = None
-        if planned:
-            rp = routing.padded_rows
-            ids = None
-            plan_ptrs = _plan_pointers(routing)
-        else:
-            rp, offsets, num_words = packed_layout(rows, E)
-            words = torch.empty(num_words, dtype=torch.int32, device=x.device)
-            status = device_status(x.get_device())
-            plan_ptrs = _packed_pointers(words, offsets, status)
-            ids = flat.data_ptr()
-            if rows > _native.ROUTE_ONE_LAUNCH_ROWS:
-                workspace = torch.empty(max(_native.routing_workspace_bytes(rows, E), 16), dtype=torch.uint8, device=x.device)
-            steps.append((_native.FWD_ROUTE, "routing", 1 if workspace is None else 3))
-        xs = None if gather_in_gemm else new(rp, d)
-        # the un-activated product, needed by the backward pass (not kept for inference or without an activation)
-        pre_act = new(rp, n1) if (act is not None and needs_grad) else None
-        hidden = new(rp, inter)
-        ys = new(rp, d) if fold else None
-        out = new(T, d)
-        kind = "glu" if is_glu(act) else "plain"
-        if not gather_in_gemm:
-            steps.append((_native.FWD_DISPATCH, "rows:gather", 1))
-        steps.append((_native.FWD_UP, "mgrouped_gemm:" + kind + ("+gather" if gather_in_gemm else ""), 1))
-        if fold:
-            steps.append((_native.FWD_DOWN, "mgrouped_gemm:plain", 1))
-            steps.append((_native.FWD_FOLD, "rows:combine", 1))
-        else:
-            steps.append((_native.FWD_DOWN, "mgrouped_gemm:combine", 1))
-        ptr = _native._ptr
-        _native.run_pass("moe_expert_forward", _native.ExpertPass(
-            T, rp, d, inter, E, topk, act_code, code, gather_in_gemm, not fold, needs_grad, ids, x.data_ptr(), scores.data_ptr(),
-            weight1.data_ptr(), weight2.data_ptr(), *plan_ptrs, ptr(workspace),
-            0 if workspace is None else workspace.numel(), ptr(xs), ptr(pre_act), hidden.data_ptr(), ptr(ys), out.data_ptr()),
-            steps, rows)
-        if needs_grad:
-            ctx.sizes = (T, d, inter, E, topk, rp, n1)
-            ctx.routing = routing if planned else None
-            ctx.act = act
-            ctx.gathered = bool(gather_in_gemm)
-            ctx.save_for_backward(x if gather_in_gemm else xs, pre_act, hidden, ys, scores, weight1, weight2, words)
+        out, ctx.info, saved = _forward(x, scores, weight1, weight2, routing, act, gather_in_gemm, fused_combine, needs_grad, addend)
+        ctx.save_for_backward(*saved)
         return out
 
     @staticmethod
     def backward(ctx, grad_out):
-        xs, pre_act, hidden, ys, scores, weight1, weight2, words = ctx.saved_tensors
-        T, d, inter, E, topk, rp, n1 = ctx.sizes
-        act = ctx.act
-        rows = T * topk
-        grad_out = grad_out.contiguous()
-        new = lambda *shape: torch.empty(shape, dtype=grad_out.dtype, device=grad_out.device)
+        if ctx.info is None:   # only the addend needed a gradient
+            return (None,) * 8 + (grad_out,)
+        return _backward(ctx.info, ctx.saved_tensors, grad_out)[:4] + (None,) * 4 + (grad_out if ctx.needs_input_grad[8] else None,)
 
-        gs, d_scores, d_pre, dxs, dx = new(rp, d), new(T, topk), new(rp, n1), new(rp, d), new(T, d)
-        d_w1, d_w2 = torch.empty_like(weight1), torch.empty_like(weight2)
-        if ctx.routing is not None:
-            plan_ptrs = _plan_pointers(ctx.routing)
-        else:
-            plan_ptrs = _packed_pointers(words, packed_layout(rows, E)[1], device_status(words.get_device()))
-        ptr = _native._ptr
-        _native.run_pass("moe_expert_backward", _native.ExpertPass(
-            T, rp, d, inter, E, topk, _native.ACT_CODES[act], _native.dtype_code(grad_out.dtype), ctx.gathered, False, True, None,
-            xs.data_ptr(), scores.data_ptr(), weight1.data_ptr(), weight2.data_ptr(), *plan_ptrs, None, 0, xs.data_ptr(),
-            ptr(pre_act), hidden.data_ptr(), ys.data_ptr(), None, grad_out.data_ptr(), gs.data_ptr(), d_scores.data_ptr(),
-            d_pre.data_ptr(), dxs.data_ptr(), dx.data_ptr(), d_w1.data_ptr(), d_w2.data_ptr()),
-            [(_native.BWD_FOLD, "rows:combine_bwd", 1),
-             (_native.BWD_DOWN, "mgrouped_gemm:wt" if act is None else "mgrouped_gemm:dglu", 1),
-             (_native.BWD_UP, "mgrouped_gemm:wt", 1), (_native.BWD_FOLD_DX, "rows:combine", 1),
-             (_native.BWD_DW1, "kgrouped_gemm:dw1" + ("+gather" if ctx.gathered else ""), 1),
-             (_native.BWD_DW2, "kgrouped_gemm:dw2", 1)], rows)
-        return dx, d_scores, d_w1, d_w2, None, None, None, None
+
+class RoutedLayer(torch.autograd.Function):
+    """The layer with a router whose softmax runs over the selected logits: scores and indices by the same torch ops as
+    ``topk_router`` (bit-identical selection), their backward as part of the experts' backward pass.  The gradient of such logits
+    is zero outside the selection, so the router's share of the input gradient is topk scaled rows of the transposed
+    router weight, added by the fold in fp32, instead of a dense GEMM and an addition over [T, d]."""
+
+    @staticmethod
+    def forward(ctx, x, router_weight, weight1, weight2, router_params, num_experts: int, act: str, gather_in_gemm: bool, addend):
+        logits = x @ router_weight
+        scores, indices = topk_of_logits(logits, router_params, x.dtype)
+        indices = indices.contiguous()
+        out, ctx.info, saved = _forward(x, scores, weight1, weight2, (indices, num_experts, router_params.topk), act,
+                                        gather_in_gemm, False, True, addend)
+        ctx.save_for_backward(x, logits, router_weight, indices, *saved)
+        return out
+
+    @staticmethod
+    def backward(ctx, grad_out):
+        x, logits, router_weight, indices, *saved = ctx.saved_tensors
+        dx, _, d_w1, d_w2, dlogits = _backward(ctx.info, saved, grad_out,
+                                               (logits.contiguous(), router_weight.contiguous(), indices))
+        d_router = None
+        if ctx.needs_input_grad[1]:   # dlogits' rows are padded to whole 16 bytes
+            d_router = (x.t() @ dlogits)[:, :router_weight.size(1)].contiguous()
+        return dx, d_router, d_w1, d_w2, None, None, None, None, grad_out if ctx.needs_input_grad[8] else None
+
+
+class DenseExpert(torch.autograd.Function):
+    """act(x @ weight1[0]) @ weight2[0]: one expert that every token goes to with weight one.  No row is moved and nothing is
+    folded; the grouped GEMMs read ``x`` and write the result where they are.  (As a top-1 layer it copied x, its
+    result and both gradients once more: 160 of 18500 us at 8192 tokens of 14 KB.)"""
+
+    @staticmethod
+    def forward(ctx, x, weight1, weight2, act):
+        _native.require_cuda(x, weight1, weight2)
+        T, d = x.shape
+        n1, inter = weight1.size(2), weight2.size(1)
+        assert weight1.size(0) == 1 and weight2.size(0) == 1
+        assert weight1.size(1) == d and weight2.size(2) == d, "weight shapes do not match the input"
+        assert n1 == (2 * inter if is_glu(act) else inter), "weight1 width does not match weight2 and the activation"
+        x, weight1, weight2 = x.contiguous(), weight1.contiguous(), weight2.contiguous()
+        needs_grad = any(ctx.needs_input_grad[:3])
+        rp, offsets, num_words = packed_layout(T, 1)
+        words = torch.empty(num_words, dtype=torch.int32, device=x.device)
+        groups = torch.arange(0, T + 1, T, dtype=torch.int32, device=x.device)   # {0, T}
+        new = lambda *shape: torch.empty(shape, dtype=x.dtype, device=x.device)
+        pre_act = new(rp, n1) if (act is not None and needs_grad) else None
+        hidden, out = new(rp, inter), new(T, d)
+        p = DenseExpert._pass(x, weight1, weight2, act, words, groups, offsets, rp, needs_grad)
+        p.pre_act, p.hidden, p.out = _native._ptr(pre_act), hidden.data_ptr(), out.data_ptr()
+        _native.run_pass("moe_expert_forward", p, [
+            (_native.FWD_ROUTE, "routing", 1), (_native.FWD_UP, "mgrouped_gemm:" + ("glu" if is_glu(act) else "plain"), 1),
+            (_native.FWD_DOWN, "mgrouped_gemm:plain", 1)], T)
+        if needs_grad:
+            ctx.act = act
+            ctx.save_for_backward(x, weight1, weight2, pre_act, hidden, words, groups)
+        return out
+
+    @staticmethod
+    def _pass(x, weight1, weight2, act, words, groups, offsets, rp, keep):
+        group_ptr, *plan_ptrs = _packed_pointers(words, offsets, device_status(x.get_device()))
+        return _native.ExpertPass(
+            x.size(0), rp, x.size(1), weight2.size(1), 1, 1, _native.ACT_CODES[act], _native.dtype_code(x.dtype), 0, 0, keep, 1,
+            None, x.data_ptr(), None, weight1.data_ptr(), weight2.data_ptr(), groups.data_ptr(), *plan_ptrs)
+
+    @staticmethod
+    def backward(ctx, grad_out):
+        x, weight1, weight2, pre_act, hidden, words, groups = ctx.saved_tensors
+        T, d = x.shape
+        rp, offsets, _ = packed_layout(T, 1)
+        grad_out = grad_out.contiguous()
+        d_pre = torch.empty(rp, weight1.size(2), dtype=x.dtype, device=x.device)
+        dx, d_w1, d_w2 = torch.empty_like(x), torch.empty_like(weight1), torch.empty_like(weight2)
+        p = DenseExpert._pass(x, weight1, weight2, ctx.act, words, groups, offsets, rp, True)
+        p.pre_act, p.hidden, p.grad_out = _native._ptr(pre_act), hidden.data_ptr(), grad_out.data_ptr()
+        p.d_pre, p.dx, p.d_w1, p.d_w2 = d_pre.data_ptr(), dx.data_ptr(), d_w1.data_ptr(), d_w2.data_ptr()
+        _native.run_pass("moe_expert_backward", p, [
+            (_native.BWD_DOWN, "mgrouped_gemm:wt" if ctx.act is None else "mgrouped_gemm:dglu", 1),
+            (_native.BWD_UP, "mgrouped_gemm:wt", 1), (_native.BWD_DW1, "kgrouped_gemm:dw1", 1),
+            (_native.BWD_DW2, "kgrouped_gemm:dw2", 1)], T)
+        return dx, d_w1, d_w2, None
 
 
 # Fusing the row gather into the gate/up GEMM's loads saves the copy of T*k rows into the expert-sorted layout
@@ -155,15 +275,45 @@ def expert_compute(x, scores, weight1, weight2, plan: RoutingPlan, act, gather_i
     if gather_in_gemm is None:
         gather_in_gemm = GATHER_IN_GEMM_DEFAULT
     return ExpertCompute.apply(x, scores, weight1, weight2, plan, None if act is None else str(act), bool(gather_in_gemm),
-                               bool(fused_combine))
+                               bool(fused_combine), None)
+
+
+def dense_expert(x, weight1, weight2, act) -> torch.Tensor:
+    """One expert for every token: ``weight1`` [1, d, I or 2I], ``weight2`` [1, I, d]."""
+    return DenseExpert.apply(x, weight1, weight2, None if act is None else str(act))
 
 
 def routed_expert_compute(x, scores, weight1, weight2, indices, num_experts: int, topk: int, act, gather_in_gemm=None,
-                          fused_combine: bool = False) -> torch.Tensor:
-    """``expert_compute`` of a routing decision given as expert indices (int64 [T, topk]) instead of a plan."""
+                          fused_combine: bool = False, addend=None) -> torch.Tensor:
+    """``expert_compute`` of a routing decision given as expert indices (int64 [T, topk]) instead of a plan; ``addend`` (like the
+    output, not with ``fused_combine``) is added to the result."""
     _native.require_cuda(indices)
     assert indices.dtype is torch.int64, "expert indices must be int64 (what torch.topk returns)"
     if gather_in_gemm is None:
         gather_in_gemm = GATHER_IN_GEMM_DEFAULT
     return ExpertCompute.apply(x, scores, weight1, weight2, (indices, num_experts, topk), None if act is None else str(act),
-                               bool(gather_in_gemm), bool(fused_combine))
+                               bool(gather_in_gemm), bool(fused_combine), addend)
+
+
+_PLAIN = (torch.Tensor, torch.nn.Parameter)
+
+
+def router_joins_the_pass(x, router_params, num_experts: int, topk: int) -> bool:
+    """Whether ``routed_layer`` stands for the router as well: plain 16-bit CUDA tensors, softmax over the selected logits, a
+    gradient wanted.  Everything else (softmax over all experts has a dense gradient; autocast, mixed types, tensor
+    subclasses and the fp32 router are torch's business) goes through the router's torch ops."""
+    if type(router_params) is not TopkRouterParams or router_params.softmax_before_topk or not torch.is_grad_enabled():
+        return False
+    w = router_params.router_weight
+    return (type(x) in _PLAIN and type(w) in _PLAIN and (x.requires_grad or w.requires_grad) and x.is_cuda and w.is_cuda
+            and x.dtype in (torch.bfloat16, torch.float16) and w.dtype is x.dtype and x.dim() == 2 and w.dim() == 2
+            and x.size(0) > 0 and w.size(1) == num_experts and router_params.topk == topk
+            and not torch.is_autocast_enabled("cuda"))
+
+
+def routed_layer(x, router_params, weight1, weight2, num_experts: int, act, gather_in_gemm=None, addend=None) -> torch.Tensor:
+    """Router and experts in one differentiable step (see ``router_joins_the_pass``)."""
+    if gather_in_gemm is None:
+        gather_in_gemm = GATHER_IN_GEMM_DEFAULT
+    return RoutedLayer.apply(x, router_params.router_weight, weight1, weight2, router_params, num_experts,
+                             None if act is None else str(act), bool(gather_in_gemm), addend)

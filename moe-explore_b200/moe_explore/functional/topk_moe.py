@@ -10,7 +10,7 @@ from __future__ import annotations
 
 import torch
 
-from moe_explore.expert_compute import routed_expert_compute
+from moe_explore.expert_compute import dense_expert, routed_expert_compute, routed_layer, router_joins_the_pass
 from moe_explore.functional.activation import activation
 from moe_explore.params import MLPParams, MOEParams, TopkRouterParams
 from moe_explore.router import fused_topk_router, router
@@ -27,6 +27,8 @@ def _shared_expert(input: torch.Tensor, shared) -> torch.Tensor:
     if up.dim() == 3:
         num_shared = up.size(0)
         T = input.size(0)
+        if num_shared == 1 and T > 0 and input.dim() == 2 and down.dim() == 3 and down.size(0) == 1:
+            return dense_expert(input, up, down, shared.activation)
         indices = torch.arange(num_shared, device=input.device, dtype=torch.int64).repeat(T, 1)
         ones = torch.ones(T, num_shared, dtype=input.dtype, device=input.device)
         return routed_expert_compute(input, ones, up, down, indices, num_shared, num_shared, shared.activation)
@@ -42,15 +44,23 @@ def topk_moe_forward(input: torch.Tensor, params: MOEParams, autotune_mode=None,
     ``fused_router`` runs the router tail in one kernel with its own declared tie rule (see
     ``moe_explore.router.fused_topk_router``); ``gather_in_gemm`` / ``fused_combine`` as in ``expert_compute``."""
     ep: MLPParams = params.expert_params
-    if fused_router and isinstance(params.router_params, TopkRouterParams):
-        scores, indices = fused_topk_router(input, params.router_params)
-    else:
-        scores, indices = router(input, params.router_params)
-    out = routed_expert_compute(input, scores, ep.weight1, ep.weight2, indices, params.num_experts, params.topk, ep.activation,
-                                gather_in_gemm=gather_in_gemm, fused_combine=fused_combine)
     shared = getattr(params, "shared_expert_params", None)
-    if shared is not None:
-        out = out + _shared_expert(input, shared)
+    shared_out = None if shared is None else _shared_expert(input, shared)
+    # a [T, d] shared branch is added by the fold of the routed experts; the fused fold has no such place, and 2-D shared
+    # weights give a broadcast vector
+    addend = shared_out if shared_out is not None and shared.up_weight.dim() == 3 and not fused_combine else None
+    if not fused_router and router_joins_the_pass(input, params.router_params, params.num_experts, params.topk):
+        out = routed_layer(input, params.router_params, ep.weight1, ep.weight2, params.num_experts, ep.activation,
+                           gather_in_gemm=gather_in_gemm, addend=addend)
+    else:
+        if fused_router and isinstance(params.router_params, TopkRouterParams):
+            scores, indices = fused_topk_router(input, params.router_params)
+        else:
+            scores, indices = router(input, params.router_params)
+        out = routed_expert_compute(input, scores, ep.weight1, ep.weight2, indices, params.num_experts, params.topk,
+                                    ep.activation, gather_in_gemm=gather_in_gemm, fused_combine=fused_combine, addend=addend)
+    if shared_out is not None and addend is None:
+        out = out + shared_out
     return out
 
 

@@ -29,7 +29,11 @@ def router(input: torch.Tensor, params: RouterParams):
 
 def topk_router(input: torch.Tensor, router_params: TopkRouterParams):
     """Linear logits -> (softmax ->) top-k (-> softmax over the k) (-> renormalise) (router.py:17-35)."""
-    logits = input @ router_params.router_weight
+    return topk_of_logits(input @ router_params.router_weight, router_params, input.dtype)
+
+
+def topk_of_logits(logits: torch.Tensor, router_params: TopkRouterParams, dtype: torch.dtype):
+    """Everything of ``topk_router`` after the linear layer."""
     if router_params.softmax_before_topk:
         logits = softmax(logits)
     scores, indices = torch.topk(logits, k=router_params.topk, dim=-1, sorted=False)
@@ -37,7 +41,7 @@ def topk_router(input: torch.Tensor, router_params: TopkRouterParams):
         scores = softmax(scores)
     if router_params.normalize_routing:
         scores = scores / scores.sum(dim=-1, keepdim=True)
-    return scores.to(input.dtype), indices
+    return scores.to(dtype), indices
 
 
 class _FusedTopk(torch.autograd.Function):

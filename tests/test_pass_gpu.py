@@ -97,3 +97,75 @@ def test_functional_gemm_against_its_steps(rows, gather, scatter, act, native):
     if scatter:
         ref = torch.empty_like(ref).index_copy_(0, perm, ref)
     assert torch.equal(out, ref)
+
+
+@pytest.mark.parametrize("normalize", [False, True])
+@pytest.mark.parametrize("E,k,d,dtype", [(8, 1, 64, torch.bfloat16), (60, 4, 264, torch.float16), (64, 8, 520, torch.bfloat16),
+                                         (129, 9, 72, torch.bfloat16), (300, 40, 128, torch.bfloat16)])
+def test_router_inside_the_pass(E, k, d, dtype, normalize, native):
+    """Router and experts in one step against the router's torch ops in front of the experts: the forward bit for bit, the
+    gradients against 32-bit autograd no further off than the composed form (whose input gradient is rounded three times)."""
+    from moe_explore.expert_compute import routed_layer, router_joins_the_pass
+    from moe_explore.params import TopkRouterParams
+    from moe_explore.router import topk_router
+
+    T, inter = 203, 64
+    g = torch.Generator(device="cuda").manual_seed(E + k)
+    mk = lambda *s, std=1.0: (torch.randn(*s, generator=g, device="cuda") * std).to(dtype)
+    leaves = [mk(T, d), mk(d, E, std=0.3), mk(E, d, 2 * inter, std=0.1), mk(E, inter, d, std=0.1)]
+    addend, grad = mk(T, d), mk(T, d)
+
+    def run(fused):
+        x, wr, w1, w2 = p = [t.clone().requires_grad_() for t in leaves]
+        a = addend.clone().requires_grad_()
+        rp = TopkRouterParams(wr, k, False, normalize)
+        if fused:
+            assert router_joins_the_pass(x, rp, E, k) and not router_joins_the_pass(x.detach(), TopkRouterParams(wr.detach(), k, False, normalize), E, k)
+            out = routed_layer(x, rp, w1, w2, E, "swiglu", addend=a)
+        else:
+            scores, idx = topk_router(x, rp)
+            out = routed_expert_compute(x, scores, w1, w2, idx, E, k, "swiglu", addend=a)
+        return [out.detach()] + list(torch.autograd.grad(out, p + [a], grad))
+
+    fused, composed = run(True), run(False)
+    assert torch.equal(fused[0], composed[0]) and torch.equal(fused[5], composed[5])
+    f = [t.float().requires_grad_() for t in leaves]
+    with torch.no_grad():
+        _, idx = topk_router(leaves[0], TopkRouterParams(leaves[1], k, False, normalize))
+    scores = torch.softmax(torch.gather(f[0] @ f[1], -1, idx), -1)
+    ref = O.expert_compute(f[0], scores, idx, f[2], f[3], "swiglu") + addend.float()
+    expect = [ref.detach()] + list(torch.autograd.grad(ref, f, grad.float()))
+    for a, c, e in zip(fused, composed, expect):
+        err = lambda t: float((t.float() - e).norm() / e.norm().clamp_min(1e-20))
+        # 1.25: the roundings of the two forms differ, in 2-norms over thousands of elements by far less
+        assert err(a) <= 1.25 * err(c) + 1e-5
+
+
+@pytest.mark.parametrize("act", [None, "silu", "swiglu"])
+@pytest.mark.parametrize("T", [1, 63, 64, 65, 129, 700])
+def test_one_expert_for_every_token(T, act, native):
+    """The in-place form of one always-selected expert against the same expert as a top-1 layer with unit weights: every
+    element is the same sum of the same products, so bit for bit (the fold of one row with weight one is exact)."""
+    from moe_explore.expert_compute import dense_expert
+
+    d, inter = 136, 200
+    g = torch.Generator(device="cuda").manual_seed(T)
+    mk = lambda *s, std=1.0: (torch.randn(*s, generator=g, device="cuda") * std).bfloat16()
+    leaves = [mk(T, d), mk(1, d, 2 * inter if act == "swiglu" else inter, std=0.1), mk(1, inter, d, std=0.1)]
+    grad = mk(T, d)
+    ids = torch.zeros(T, 1, dtype=torch.int64, device="cuda")
+    ones = torch.ones(T, 1, dtype=torch.bfloat16, device="cuda")
+
+    def run(how):
+        p = [t.clone().requires_grad_() for t in leaves]
+        _poison()
+        out = how(*p)
+        _poison()
+        return [out.detach()] + list(torch.autograd.grad(out, p, grad))
+
+    dense = run(lambda x, w1, w2: dense_expert(x, w1, w2, act))
+    layer = run(lambda x, w1, w2: routed_expert_compute(x, ones, w1, w2, ids, 1, 1, act))
+    for a, b in zip(dense, layer):
+        assert torch.equal(a, b)
+    with torch.no_grad():
+        assert torch.equal(dense_expert(*leaves, act), dense[0])
