@@ -229,6 +229,10 @@ int moe_index_rows(const void* src, const int64_t* index, void* out, int64_t num
 int moe_combine_topk(const void* ys, const void* scores, const int32_t* dst_row, void* out,
                      int64_t num_tokens, int topk, int cols, int dtype, void* stream);
 
+/* The same for rows in (token, slot) order: out[t, :] = sum_s scales(t, s) * rows[t*topk + s, :]. */
+int moe_scale_and_reduce(const void* rows, const void* scales, void* out, int64_t num_tokens, int topk,
+                         int cols, int dtype, void* stream);
+
 /* Backward of the combine: for padded row p holding flat position j = (t, s):
  *   gs[p, :]   = scores[j] * dout[t, :]
  *   dscores[j] = dot(dout[t, :], ys[p, :])      (fp32 accumulation, stored in `dtype`)

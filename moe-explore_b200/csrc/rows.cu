@@ -355,7 +355,8 @@ combine_topk_kernel(const uint4* __restrict__ ys, const T* __restrict__ scores, 
 #pragma unroll
         for (int i = 0; i < SLOTS; ++i) {
           const int64_t j = t * topk + s0 + i;
-          const int32_t p = s0 + i < topk ? dst_row[j] : -1;  // negative: slot dropped by the routing metadata
+          // negative: slot dropped by the routing metadata; no map: the rows are in (token, slot) order
+          const int32_t p = s0 + i < topk ? (dst_row != nullptr ? dst_row[j] : static_cast<int32_t>(j)) : -1;
           scale[i] = p < 0 ? 0.0f : (scores != nullptr ? Elem<T>::to_float(scores[j]) : 1.0f);
           u[i] = p < 0 ? make_uint4(0, 0, 0, 0) : ys[static_cast<int64_t>(p) * vec_per_row + v];
         }
@@ -756,7 +757,7 @@ int combine_topk(const void* ys, const void* scores, const int32_t* dst_row, voi
                  void* stream) {
   MOE_CHECK_ARG(num_tokens >= 0 && topk > 0, "moe_combine_topk: bad sizes T=%lld topk=%d", (long long)num_tokens, topk);
   if (num_tokens == 0) return MOE_OK;
-  MOE_CHECK_ARG(ys && dst_row && out, "moe_combine_topk: null pointer argument");
+  MOE_CHECK_ARG(ys && out, "moe_combine_topk: null pointer argument");
   MOE_CHECK_ARG(aligned16(ys) && aligned16(out), "moe_combine_topk: pointers must be 16-byte aligned");
   MOE_ROW_COMMON_CHECKS("moe_combine_topk", cols, dtype);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
@@ -773,8 +774,16 @@ int combine_topk(const void* ys, const void* scores, const int32_t* dst_row, voi
 }
 }  // namespace moe
 
+extern "C" int moe_scale_and_reduce(const void* rows, const void* scales, void* out, int64_t num_tokens, int topk, int cols,
+                                    int dtype, void* stream) {
+  MOE_CHECK_ARG(num_tokens == 0 || scales != nullptr, "moe_scale_and_reduce: scales is null");
+  MOE_CHECK_ARG(num_tokens * topk < (1ll << 31), "moe_scale_and_reduce: 2^31 rows or more");
+  return combine_topk(rows, scales, nullptr, out, num_tokens, topk, cols, dtype, nullptr, nullptr, nullptr, nullptr, stream);
+}
+
 extern "C" int moe_combine_topk(const void* ys, const void* scores, const int32_t* dst_row, void* out,
                                 int64_t num_tokens, int topk, int cols, int dtype, void* stream) {
+  MOE_CHECK_ARG(num_tokens <= 0 || dst_row != nullptr, "moe_combine_topk: null pointer argument");
   return combine_topk(ys, scores, dst_row, out, num_tokens, topk, cols, dtype, nullptr, nullptr, nullptr, nullptr, stream);
 }
 

@@ -80,6 +80,7 @@ SIGNATURES = {
     "moe_unpad_rows": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int, c_void_p]),
     "moe_index_rows": (c_int, [c_void_p] * 3 + [c_int64, c_int, c_int, c_int, c_void_p]),
     "moe_combine_topk": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int, c_int, c_void_p]),
+    "moe_scale_and_reduce": (c_int, [c_void_p] * 3 + [c_int64, c_int, c_int, c_int, c_void_p]),
     "moe_combine_bwd": (c_int, [c_void_p] * 7 + [c_int64, c_int, c_int64, c_int, c_int, c_void_p]),
     "moe_dispatch_rows": (c_int, [c_void_p] * 5 + [c_int64, c_int, c_int64, c_int, c_int, c_void_p]),
     "moe_expert_pass_size": (c_size_t, []),
@@ -438,6 +439,16 @@ def combine_topk(ys, scores, dst_row, out, topk):
         rc = load().moe_combine_topk(_ptr(ys), _ptr(scores), _ptr(dst_row), _ptr(out), out.size(0), topk, out.size(1),
                                      dtype_code(ys.dtype), _stream())
     _check("moe_combine_topk", rc)
+    _count(1)
+
+
+def scale_and_reduce(rows, scales, out, topk):
+    """out[t] = sum_s scales[t, s] * rows[t*topk+s]."""
+    require_cuda(rows, out)
+    with timed("rows:combine"):
+        rc = load().moe_scale_and_reduce(_ptr(rows), _ptr(scales), _ptr(out), out.size(0), topk, out.size(1),
+                                         dtype_code(rows.dtype), _stream())
+    _check("moe_scale_and_reduce", rc)
     _count(1)
 
 

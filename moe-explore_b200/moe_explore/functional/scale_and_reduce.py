@@ -14,9 +14,8 @@ from moe_explore import _native
 class _ScaleAndReduce(torch.autograd.Function):
     @staticmethod
     def forward(ctx, input, scales, num_tokens, topk):
-        rows = torch.arange(num_tokens * topk, dtype=torch.int32, device=input.device)
         out = torch.empty(num_tokens, input.size(1), dtype=input.dtype, device=input.device)
-        _native.combine_topk(input.contiguous(), scales.contiguous(), rows, out, topk)
+        _native.scale_and_reduce(input.contiguous(), scales.contiguous(), out, topk)
         ctx.save_for_backward(input, scales)
         ctx.topk = topk
         return out
