@@ -177,7 +177,7 @@ namespace moe {
 // one)" in one launch: a warp per token recomputes the probabilities p from the logits and leaves
 //   dl[t, s] = p_s (d_s - sum_j p_j d_j)   in fp32, and the dense row of it in the 16-bit type (what the router-weight
 // gradient contracts with; its rows are padded with zeros to whole 16 bytes, so that the contraction is an aligned one: 60
-// experts, 16384 tokens 53 -> 17 us); the CTAs after those transpose the router weight for the fold of the input gradient.
+// experts, 16384 tokens 53 -> 22 us); the CTAs after those transpose the router weight for the fold of the input gradient.
 // It stands for seven element-wise launches (casts, product, softmax backward, fill, scatter: 25-30 us).
 constexpr int kTransposeTile = 32;
 template <typename T>

@@ -4,12 +4,11 @@
 // Replaces get_token_indices (reference: src/moe_explore/expert_permute.py:19-41), which runs
 // torch.argsort + torch.histc + torch.cumsum as three or more launches.  Here it is a counting sort (the number of
 // distinct keys, E, is small): one launch of one cluster (route_cluster_kernel) up to kClusterRows rows, and for
-// more rows the chip-wide three-kernel form:
+// more rows the chip-wide form:
 //   1. chunk_histogram : each warp owns a contiguous chunk of kChunk flat positions and counts
 //                        its ids per expert in shared memory (warp-aggregated via match.any);
-//   2. scan_offsets    : turns the [chunks, E] histogram into per-(chunk, expert) exclusive
-//                        offsets (one CTA per expert scans down the chunk axis when there are many
-//                        chunks), then one CTA derives the per-expert prefix sums (unpadded and
+//   2. scan_chunks     : a CTA per expert turns its column of the [chunks, E] histogram into exclusive
+//                        offsets; scan_offsets: one CTA derives the per-expert prefix sums (unpadded and
 //                        padded to 128-row tiles) and the tile -> expert map;
 //   3. place_rows      : each warp walks its chunk again in order, ranks equal ids with
 //                        match.any + popc (which preserves flat-position order) and writes
