@@ -559,7 +559,9 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       // Mixtral shape with the branches compiled out), because the loop then no longer is the short elected-lane
       // sequence the operand pipeline needs once per 512 tensor-core cycles.
       constexpr bool gather = GATHER;
-      TileCoord c_next = decode_tile<KG, CTAS>(unit < ntiles ? unit : 0, mt, nt, win, args, BN, rank);
+      // (a worker without an item decodes none: when no row tile is in use the maps hold nothing to decode)
+      TileCoord c_next{};
+      if (unit < ntiles) c_next = decode_tile<KG, CTAS>(unit, mt, nt, win, args, BN, rank);
       // M-grouped gather: lane l owns rows 4l..4l+3 of the tile for all of its stages
       int4 rows_next = make_int4(0, 0, 0, 0);
       if (gather && !KG && unit < ntiles) rows_next = gather_rows4(args.a_row_src, c_next.m0 + 4 * lane, args.a_div, args.a_rows);
@@ -720,7 +722,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       uint32_t acc_phase = 0;
       bool ok = true;
       bool ready = false;  // the stage about to be consumed was already seen full
-      TileCoord c_next = decode_tile<KG, CTAS>(unit < ntiles ? unit : 0, mt, nt, win, args, BN, rank);
+      TileCoord c_next{};
+      if (unit < ntiles) c_next = decode_tile<KG, CTAS>(unit, mt, nt, win, args, BN, rank);
       for (int t = unit; t < ntiles && ok; t += num_units) {
         const TileCoord c = c_next;
         if (t + num_units < ntiles) c_next = decode_tile<KG, CTAS>(t + num_units, mt, nt, win, args, BN, rank);
@@ -801,7 +804,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     const auto side_parity = [](uint32_t n) { return Plan::kTilesPerWarp == 2 ? (n >> 1) & 1 : n & 1; };
     const int co_row = lane >> 3;  // coalesced access: row within a group of four
     const int co_ck = lane & 7;    // and 16-byte piece of the row's 128 bytes
-    TileCoord c_next = decode_tile<KG, CTAS>(unit < ntiles ? unit : 0, mt, nt, win, args, BN, rank);
+    TileCoord c_next{};
+    if (unit < ntiles) c_next = decode_tile<KG, CTAS>(unit, mt, nt, win, args, BN, rank);
     for (int t = unit; t < ntiles; t += num_units) {
       const TileCoord c = c_next;
       if (t + num_units < ntiles) c_next = decode_tile<KG, CTAS>(t + num_units, mt, nt, win, args, BN, rank);

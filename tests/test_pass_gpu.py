@@ -4,7 +4,7 @@ import pytest
 import torch
 
 from moe_explore.expert_compute import expert_compute, routed_expert_compute
-from moe_explore.routing_plan import build_routing_plan
+from moe_explore.routing_plan import build_routing_plan, device_status
 from oracle import moe_oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -169,3 +169,54 @@ def test_one_expert_for_every_token(T, act, native):
         assert torch.equal(a, b)
     with torch.no_grad():
         assert torch.equal(dense_expert(*leaves, act), dense[0])
+
+
+def _poison_maps():
+    """Freed blocks full of indices that are out of every range, for the index arrays of the next calls."""
+    blocks = [torch.full((n << 10,), 0x7FFFFFFF, dtype=torch.int32, device="cuda") for n in (1, 1, 1, 2, 4, 16, 64, 256)]
+    del blocks
+
+
+@pytest.mark.parametrize("T,k,E", [(1, 2, 8), (300, 2, 8), (2048, 2, 4)])   # one-CTA kernels; the last one: CTA pairs
+def test_every_row_dropped(T, k, E, native):
+    """All expert ids out of range: no row tile is in use and no map entry may be used.  Zeros everywhere, status 100."""
+    d, inter = 136, 200
+    g = torch.Generator(device="cuda").manual_seed(T)
+    mk = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    leaves = [mk(T, d), mk(T, k), mk(E, d, 2 * inter), mk(E, inter, d)]
+    ids = torch.full((T, k), E + 5, dtype=torch.int64, device="cuda")
+    ids[0, 0] = -1
+
+    def check(tensors):
+        torch.cuda.synchronize()
+        assert all(not t.any() for t in tensors)
+        assert native.read_status(device_status(), reset=True) == 100
+
+    native.read_status(device_status(), reset=True)
+    for gather in (False, True):
+        p = [t.clone().requires_grad_() for t in leaves]
+        _poison_maps()
+        out = routed_expert_compute(*p, ids, E, k, "swiglu", gather_in_gemm=gather)
+        check([out.detach()] + list(torch.autograd.grad(out, p, mk(T, d))))
+        with torch.no_grad():
+            for fused in (False, True):
+                _poison_maps()
+                check([routed_expert_compute(*leaves, ids, E, k, "swiglu", gather_in_gemm=gather, fused_combine=fused)])
+    _poison_maps()
+    check([expert_compute(*leaves, build_routing_plan(ids, E, k), "swiglu")])
+
+
+@pytest.mark.parametrize("gather,scatter", [(False, False), (True, True)])
+def test_refused_group_with_all_the_rows(gather, scatter, native):
+    """A prefix that ends past the rows: the only group with rows is refused (status 5) and nothing is contracted."""
+    from moe_explore.triton_kernels.m_grouped_gemm import MGroupedGEMMParams, m_grouped_gemm
+
+    R, K, N = 70, 136, 208
+    x = torch.randn(R, K, device="cuda").bfloat16()
+    for groups in ([0, R + 1], [0, 0, R + 200]):
+        w = torch.randn(len(groups) - 1, K, N, device="cuda").bfloat16()
+        _poison_maps()
+        out = m_grouped_gemm(x, MGroupedGEMMParams(w, torch.tensor(groups, dtype=torch.int32, device="cuda"),
+                                                   torch.arange(R, device="cuda"), gather, scatter, R, 1))
+        torch.cuda.synchronize()
+        assert out.shape == (R, N) and native.read_status(device_status(), reset=True) == 5
