@@ -60,7 +60,7 @@ class Chain {
     ::moe::chained_launches() = true;   \
   } while (0)
 
-// In a row map for moe_gather_rows: leave the row of dst as it is.
+// In a row map for gather_rows with skip_marked: leave the row of dst as it is.
 constexpr int32_t kSkipRow = -2;
 
 template <typename... Params, typename... Args>
@@ -125,6 +125,9 @@ int mgrouped_gemm_rows(const void* a, int64_t compact_rows, const void* w, void*
                        const int32_t* mtile_expert, const int32_t* tile_pairs, const int32_t* num_mtiles, int64_t padded_rows,
                        int K, int N, int num_experts, int act, int dtype, int32_t* status, void* stream,
                        const RowCounts& counts);
+// moe_gather_rows; `skip_marked`: row_src comes from the library and its kSkipRow entries are obeyed.
+int gather_rows(const void* src, int64_t src_rows, const int32_t* row_src, const int32_t* num_mtiles, void* dst,
+                int64_t padded_rows, int cols, int div, int dtype, void* stream, bool skip_marked);
 int dispatch_rows(const void* src, const int32_t* dst_row, const int32_t* row_src, const int32_t* num_mtiles, void* dst,
                   int64_t num_tokens, int topk, int64_t padded_rows, int cols, int dtype, void* stream, bool live_blocks_only);
 // moe_combine_topk with further summands, all nullable (FoldExtra in csrc/rows.cu).

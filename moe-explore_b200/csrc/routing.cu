@@ -461,7 +461,7 @@ static int route_cluster(const int64_t* ids, int64_t R, int E, const RouteOut& o
 // itself (E values) and fills its share of the maps.  It replaces a memset, a one-CTA scan and a row kernel, and in the
 // functional grouped GEMM six index operations besides (16 launches of 2-4 us each for 4111 tokens x 8 slots, two calls).
 // `perm` (nullable): flat position of sorted row r.  Maps of padded row p that holds sorted row r, all nullable:
-//   row_src r | in_rows perm[r] (r without perm) | out_rows perm[r] if scatter, else r;  padding rows: -1, -2 (skip), -1
+//   row_src r | in_rows perm[r] (r without perm) | out_rows perm[r] if scatter, else r;  padding rows: -1, kSkipRow, -1
 struct GroupsOut {
   int32_t* pad_offsets;
   int32_t* row_src;
@@ -553,7 +553,11 @@ layout_from_groups_kernel(const int32_t* __restrict__ group_indices, int64_t R, 
       const int32_t in_seg = p - sh_pad[x];
       const bool ok = p < sh_pad[E] && in_seg < sh_cnt[x];
       const int32_t r = sh_lo[x] + in_seg;
-      const int32_t f = ok ? (perm != nullptr ? static_cast<int32_t>(perm[r]) : r) : -1;
+      int32_t f = -1;  // a negative entry of perm: no input row (zeros), no output row, whatever its value
+      if (ok) {
+        const int64_t j = perm != nullptr ? perm[r] : r;
+        if (j >= 0) f = static_cast<int32_t>(j);
+      }
       if (out.row_src != nullptr) out.row_src[p] = ok ? r : -1;
       if (out.in_rows != nullptr) out.in_rows[p] = ok ? f : kSkipRow;
       if (out.out_rows != nullptr) out.out_rows[p] = ok ? (scatter ? f : r) : -1;
@@ -724,8 +728,8 @@ extern "C" int moe_rows_gemm(const moe_rows_pass* p, int steps, void* stream) {
                                           p->gather ? p->in_rows : nullptr, p->out_rows, static_cast<int32_t>(mtiles)},
                                 p->status, static_cast<cudaStream_t>(stream)));
   if ((steps & MOE_ROWS_GATHER) && p->gather)
-    MOE_STEP(moe_gather_rows(p->a, p->a_rows, p->in_rows, p->num_mtiles, p->padded, padded_rows, p->k_dim, p->topk, p->dtype,
-                             stream));
+    MOE_STEP(gather_rows(p->a, p->a_rows, p->in_rows, p->num_mtiles, p->padded, padded_rows, p->k_dim, p->topk, p->dtype, stream,
+                         true));
   if (steps & MOE_ROWS_GEMM) {
     const RowCounts counts{p->pad_offsets, p->group_indices};
     // rows that are in expert order already are read where they are; gathered ones from their padded copy

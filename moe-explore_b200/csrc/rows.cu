@@ -18,9 +18,15 @@ constexpr int kRowThreads = 256;
 // 238 -> 231.
 constexpr int kRowLoads = 4;
 
-// dst[r, :] = src[index[r] / div, :], zeros where index[r] < 0 (kSkipRow: untouched).  `num_mtiles` (nullable): only the first
-// 128 * num_mtiles[0] rows are in use.
-template <typename Index, int TPR>
+// Source row of index j >= 0 (a 64-bit division only for the indices that need one).
+__device__ __forceinline__ int64_t source_row(int32_t j, int div) { return j / div; }
+__device__ __forceinline__ int64_t source_row(int64_t j, int div) {
+  return (j >> 31) == 0 ? static_cast<int32_t>(j) / div : j / div;
+}
+
+// dst[r, :] = src[index[r] / div, :], zeros where index[r] < 0.  `num_mtiles` (nullable): only the first 128 * num_mtiles[0]
+// rows are in use.  SKIP (maps the library itself wrote, never a caller's indices): rows marked kSkipRow stay untouched.
+template <typename Index, int TPR, bool SKIP>
 __global__ void __launch_bounds__(kRowThreads)
 copy_rows_kernel(const uint4* __restrict__ src, const Index* __restrict__ index, const int32_t* __restrict__ num_mtiles,
                  uint4* __restrict__ dst, int64_t rows, int vec_per_row, int div) {
@@ -34,9 +40,9 @@ copy_rows_kernel(const uint4* __restrict__ src, const Index* __restrict__ index,
   const int lane = threadIdx.x % TPR;
   for (int64_t r = static_cast<int64_t>(blockIdx.x) * kRows + threadIdx.x / TPR; r < rows;
        r += static_cast<int64_t>(gridDim.x) * kRows) {
-    const int32_t j = static_cast<int32_t>(index[r]);
-    if (j == kSkipRow) continue;
-    const uint4* s = src + static_cast<int64_t>(j / div) * vec_per_row;
+    const Index j = index[r];
+    if (SKIP && j == kSkipRow) continue;
+    const uint4* s = src + (j >= 0 ? source_row(j, div) : 0) * vec_per_row;
     uint4* d = dst + r * vec_per_row;
     for (int v0 = lane; v0 < vec_per_row; v0 += TPR * kRowLoads) {
       uint4 u[kRowLoads];
@@ -502,7 +508,7 @@ static int row_grid(int64_t rows) {
 static int copy_threads_per_row(int vec_per_row) { return vec_per_row <= 64 ? 32 : 64; }
 static int fold_threads_per_row(int vec_per_row) { return vec_per_row <= 32 ? 32 : (vec_per_row <= 64 ? 64 : 128); }
 
-template <typename Index>
+template <bool SKIP = false, typename Index>
 static void launch_copy_rows(const void* src, const Index* index, const int32_t* num_mtiles, void* dst, int64_t rows,
                              int vec_per_row, int div, cudaStream_t s) {
   const int tpr = copy_threads_per_row(vec_per_row);
@@ -511,8 +517,8 @@ static void launch_copy_rows(const void* src, const Index* index, const int32_t*
   const int grid = static_cast<int>(groups < (1 << 30) ? (groups > 0 ? groups : 1) : (1 << 30));
   const uint4* in = static_cast<const uint4*>(src);
   uint4* out = static_cast<uint4*>(dst);
-  if (tpr == 32) launch_kernel(copy_rows_kernel<Index, 32>, grid, kRowThreads, s, in, index, num_mtiles, out, rows, vec_per_row, div);
-  else launch_kernel(copy_rows_kernel<Index, 64>, grid, kRowThreads, s, in, index, num_mtiles, out, rows, vec_per_row, div);
+  if (tpr == 32) launch_kernel(copy_rows_kernel<Index, 32, SKIP>, grid, kRowThreads, s, in, index, num_mtiles, out, rows, vec_per_row, div);
+  else launch_kernel(copy_rows_kernel<Index, 64, SKIP>, grid, kRowThreads, s, in, index, num_mtiles, out, rows, vec_per_row, div);
 }
 
 // row_src == nullptr: the padding rows are left as they are.
@@ -610,15 +616,24 @@ extern "C" int moe_store_to_host(const void* src, void* dst_pinned_host, size_t 
   return MOE_OK;
 }
 
-extern "C" int moe_gather_rows(const void* src, int64_t src_rows, const int32_t* row_src, const int32_t* num_mtiles,
-                               void* dst, int64_t padded_rows, int cols, int div, int dtype, void* stream) {
+namespace moe {
+int gather_rows(const void* src, int64_t src_rows, const int32_t* row_src, const int32_t* num_mtiles, void* dst,
+                int64_t padded_rows, int cols, int div, int dtype, void* stream, bool skip_marked) {
   MOE_CHECK_ARG(src && row_src && num_mtiles && dst, "moe_gather_rows: null pointer argument");
   MOE_CHECK_ARG(aligned16(src) && aligned16(dst), "moe_gather_rows: pointers must be 16-byte aligned");
   MOE_CHECK_ARG(src_rows >= 0 && padded_rows > 0 && div > 0, "moe_gather_rows: bad sizes");
   MOE_ROW_COMMON_CHECKS("moe_gather_rows", cols, dtype);
-  launch_copy_rows(src, row_src, num_mtiles, dst, padded_rows, cols / 8, div, static_cast<cudaStream_t>(stream));
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (skip_marked) launch_copy_rows<true>(src, row_src, num_mtiles, dst, padded_rows, cols / 8, div, s);
+  else launch_copy_rows(src, row_src, num_mtiles, dst, padded_rows, cols / 8, div, s);
   MOE_CUDA(cudaGetLastError());
   return MOE_OK;
+}
+}  // namespace moe
+
+extern "C" int moe_gather_rows(const void* src, int64_t src_rows, const int32_t* row_src, const int32_t* num_mtiles,
+                               void* dst, int64_t padded_rows, int cols, int div, int dtype, void* stream) {
+  return gather_rows(src, src_rows, row_src, num_mtiles, dst, padded_rows, cols, div, dtype, stream, false);
 }
 
 namespace moe {

@@ -82,3 +82,55 @@ def test_permute_round_trip_with_and_without_a_score_gradient(T, k, cols, native
     ref = (x.float()[:, None, :] * x.float()[:, None, :].expand(T, k, cols)).sum(-1)
     # fp32 sum of `cols` products, rounded once to bf16
     assert bool(((leaf.grad.float() - ref).abs() <= ref.abs() * 2.0 ** -8 + cols * 2.0 ** -23 * ref.abs()).all())
+
+
+@pytest.mark.parametrize("cols", [8, 520, 2056])
+def test_every_negative_index_is_a_zero_row(cols, native):
+    """-1, -2 and any other negative index, in 32 and 64 bits (where the low half may be positive): a row of zeros."""
+    from moe_explore.expert_permute import row_gather
+
+    g = torch.Generator(device="cuda").manual_seed(cols)
+    x = torch.randn(40, cols, generator=g, device="cuda").bfloat16()
+    idx = torch.randint(0, 40, (300,), generator=g, device="cuda")
+    idx[::7] = torch.tensor([-1, -2, -3, -2 ** 31], device="cuda").repeat(11)[:43]
+    expect = lambda i, div: torch.where(i[:, None] >= 0, x[i.clamp_min(0) // div], torch.zeros((), dtype=x.dtype, device="cuda"))
+    assert torch.equal(row_gather(x, idx), expect(idx, 1))
+    rows = torch.full((384, cols), 7.0, device="cuda").bfloat16()
+    native.gather_rows(x, torch.cat([idx, idx[:84]]).int(), torch.tensor([3, 2, 3, 0], dtype=torch.int32, device="cuda"), rows, 3)
+    assert torch.equal(rows, expect(torch.cat([idx, idx[:84]]), 3))
+    idx[5:9] = torch.tensor([-2 ** 32 + 1, -2 ** 32, -2 ** 62, -2 ** 33 + 7], device="cuda")
+    for div in (1, 3):
+        out = torch.full((300, cols), 7.0, device="cuda").bfloat16()
+        native.index_rows(x, idx, out, div=div)
+        assert torch.equal(out, expect(idx, div))
+
+
+@pytest.mark.parametrize("act", [None, "swiglu"])
+@pytest.mark.parametrize("gather,scatter", [(True, False), (True, True), (False, True)])
+def test_functional_gemm_with_negative_positions(gather, scatter, act, native):
+    """Negative entries of permute_indices: a zero input row with gather, no output row with scatter."""
+    from moe_explore.triton_kernels.m_grouped_gemm import MGroupedGEMMParams, m_grouped_gemm
+
+    rows = (70, 0, 129, 1, 300)
+    R, K, N = sum(rows), 136, 208
+    g = torch.Generator(device="cuda").manual_seed(R)
+    groups = torch.tensor([0] + list(rows), dtype=torch.int32).cumsum(0).to(torch.int32).cuda()
+    w = (torch.randn(len(rows), K, N, generator=g, device="cuda") * 0.1).bfloat16()
+    x = torch.randn(R, K, generator=g, device="cuda").bfloat16()
+    perm = torch.randperm(R, generator=g, device="cuda")
+    bad = torch.arange(0, R, 9, device="cuda")
+    holes = perm.clone()
+    holes[bad] = torch.tensor([-1, -2, -7, -2 ** 32 + 3], device="cuda").repeat(R)[:bad.numel()]
+
+    def run(p):
+        del_me = [torch.full((n << 18,), float("nan"), device="cuda") for n in (1, 1, 2, 4)]
+        del del_me
+        return m_grouped_gemm(x, MGroupedGEMMParams(w, groups, p, gather, scatter, R, 1, activation=act))
+
+    full, out = run(perm), run(holes)
+    if scatter:
+        stored = perm[(holes >= 0).nonzero().flatten()]
+        assert torch.equal(out[stored], full[stored])
+    else:
+        full[bad] = 0
+        assert torch.equal(out, full)
