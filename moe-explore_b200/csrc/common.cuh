@@ -196,6 +196,11 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 }
 
 // See chained_launches(): waits for the kernels this one was chained to / lets the next chained kernel start its prologue.
+// A chained kernel begins before its predecessor has written the last of what it reads.  So in a kernel that can be launched
+// chained nothing may be promised to be constant for the kernel's whole life: its pointer parameters carry no __restrict__ and it
+// reads without __ldg (either lets the compiler use the non-coherent path, or move a load over the wait); what the
+// predecessor wrote is then read by ordinary loads after grid_wait(), which makes it visible.  Functions that run after the wait
+// may take __restrict__ pointers: their promise begins there.
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

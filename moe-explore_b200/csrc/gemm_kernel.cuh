@@ -142,7 +142,7 @@ struct TileCoord {
 // Rows of expert e that exist, in whole 64-row blocks, at most its padded range (whatever the prefix says).
 __device__ __forceinline__ int live_rows(const GemmArgs& args, int e, int padded) {
   if (args.group_indices == nullptr) return padded;
-  const int rows = (__ldg(args.group_indices + e + 1) - __ldg(args.group_indices + e) + 63) & ~63;
+  const int rows = (args.group_indices[e + 1] - args.group_indices[e] + 63) & ~63;
   return rows < padded ? (rows > 0 ? rows : 0) : padded;
 }
 
@@ -288,10 +288,10 @@ __device__ __forceinline__ TileCoord decode_tile(int t, int mt, int nt, const Wi
     int lo = win.e0, hi = win.e1;
     while (hi - lo > 1) {
       const int mid = (lo + hi) >> 1;
-      if ((__ldg(args.pair_prefix + mid) - base) * nt <= t) lo = mid; else hi = mid;
+      if ((args.pair_prefix[mid] - base) * nt <= t) lo = mid; else hi = mid;
     }
-    span_begin = __ldg(args.pair_prefix + lo);
-    int span_end = __ldg(args.pair_prefix + lo + 1);
+    span_begin = args.pair_prefix[lo];
+    int span_end = args.pair_prefix[lo + 1];
     // a window given as a pair range may begin or end inside this expert: walk only its part of the expert
     if (span_begin < base) span_begin = base;
     if (span_end > win.p_end) span_end = win.p_end;
@@ -313,31 +313,31 @@ __device__ __forceinline__ TileCoord decode_tile(int t, int mt, int nt, const Wi
   if (KG) {
     c.m0 = (m_idx * CTAS + rank) * BM;
     c.expert = expert;
-    c.k_row0 = __ldg(args.pad_offsets + expert);
-    c.kiters = live_rows(args, expert, __ldg(args.pad_offsets + expert + 1) - c.k_row0) / BK;  // multiples of 64
+    c.k_row0 = args.pad_offsets[expert];
+    c.kiters = live_rows(args, expert, args.pad_offsets[expert + 1] - c.k_row0) / BK;  // multiples of 64
     c.live = BM;
     c.a_row = 0;
   } else {
     int tile = m_idx;
     if (CTAS == 2) {
       // one load: first tile (bits 0-19), expert (bits 20-30), "has a second tile" (bit 31)
-      const uint32_t info = static_cast<uint32_t>(__ldg(args.tile_pairs + m_idx));
+      const uint32_t info = static_cast<uint32_t>(args.tile_pairs[m_idx]);
       const bool second = (info >> 31) != 0;
       tile = static_cast<int>(info & 0xFFFFFu);
       c.expert = static_cast<int>((info >> 20) & 0x7FFu);
       c.active = rank == 0 || second;
       if (rank == 1 && second) tile += 1;  // an inactive second CTA re-reads the first tile and stores nothing
     } else {
-      c.expert = __ldg(args.mtile_expert + tile);
+      c.expert = args.mtile_expert[tile];
     }
     c.m0 = tile * BM;
     c.a_row = c.m0;
     c.live = BM;
     if (args.group_indices != nullptr) {
-      const int base = __ldg(args.pad_offsets + c.expert);
+      const int base = args.pad_offsets[c.expert];
       const int left = live_rows(args, c.expert, 1 << 30) - (c.m0 - base);
       c.live = left < BM ? (left > 64 ? left : 64) : BM;
-      if (args.a_compact) c.a_row = c.m0 - base + __ldg(args.group_indices + c.expert);
+      if (args.a_compact) c.a_row = c.m0 - base + args.group_indices[c.expert];
     }
     c.k_row0 = 0;
     c.kiters = (args.k_dim + BK - 1) / BK;
@@ -458,7 +458,7 @@ __device__ __forceinline__ void dglu_row(const float (&da)[32], uint4 (&h)[8]) {
 // Source rows of four consecutive padded rows, as the gather4 copy wants them: row_src / div, or `oob` (a row
 // index outside the tensor, which the copy fills with zeros) for padding rows.
 __device__ __forceinline__ int4 gather_rows4(const int32_t* row_src, int first, int div, int oob) {
-  const int4 j = __ldg(reinterpret_cast<const int4*>(row_src + first));
+  const int4 j = *reinterpret_cast<const int4*>(row_src + first);
   int4 r;
   r.x = j.x < 0 ? oob : j.x / div;
   r.y = j.y < 0 ? oob : j.y / div;
@@ -825,19 +825,19 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
           int32_t r = -1;
           if (row_ok) {
             if (args.push_bases != nullptr) {
-              const int32_t rk = __ldg(args.push_rank + row);
+              const int32_t rk = args.push_rank[row];
               if (rk >= 0) {
                 row_out = reinterpret_cast<T*>(args.push_bases[rk]);
-                r = __ldg(args.push_row + row);
+                r = args.push_row[row];
               }
             } else {
-              r = __ldg(args.push_row + row);
+              r = args.push_row[row];
             }
           }
           row_ok = r >= 0;
           if (row_ok) out_row = r;
         } else if (EPI == EPI_ACT && args.combine_row_src != nullptr) {
-          const int32_t j = row_ok ? __ldg(args.combine_row_src + row) : -1;
+          const int32_t j = row_ok ? args.combine_row_src[row] : -1;
           row_ok = j >= 0;
           if (row_ok) {
             out_row = j / args.combine_topk;

@@ -182,9 +182,8 @@ namespace moe {
 constexpr int kTransposeTile = 32;
 template <typename T>
 __global__ void __launch_bounds__(256)
-router_backward_kernel(const T* __restrict__ logits, const int64_t* __restrict__ experts, const T* __restrict__ d_scores,
-                       const T* __restrict__ router_w, float* __restrict__ dl, T* __restrict__ dlogits, T* __restrict__ router_t,
-                       int64_t num_tokens, int E, int topk, int cols, int token_blocks) {
+router_backward_kernel(const T* logits, const int64_t* experts, const T* d_scores, const T* router_w, float* dl, T* dlogits,
+                       T* router_t, int64_t num_tokens, int E, int topk, int cols, int token_blocks) {
   const int ld = (E + 7) & ~7;  // of dlogits
   grid_release();
   grid_wait();

@@ -27,12 +27,10 @@ __device__ __forceinline__ int64_t source_row(int64_t j, int div) {
 // dst[r, :] = src[index[r] / div, :], zeros where index[r] < 0.  `num_mtiles` (nullable): only the first 128 * num_mtiles[0]
 // rows are in use.  SKIP (maps the library itself wrote, never a caller's indices): rows marked kSkipRow stay untouched.
 template <typename Index, int TPR, bool SKIP>
-__global__ void __launch_bounds__(kRowThreads)
-copy_rows_kernel(const uint4* __restrict__ src, const Index* __restrict__ index, const int32_t* __restrict__ num_mtiles,
-                 uint4* __restrict__ dst, int64_t rows, int vec_per_row, int div) {
+__device__ __forceinline__ void copy_rows(const uint4* __restrict__ src, const Index* __restrict__ index,
+                                          const int32_t* __restrict__ num_mtiles, uint4* __restrict__ dst, int64_t rows,
+                                          int vec_per_row, int div) {
   constexpr int kRows = kRowThreads / TPR;
-  grid_release();
-  grid_wait();
   if (num_mtiles != nullptr) {
     const int64_t in_use = static_cast<int64_t>(*num_mtiles) * MOE_TILE_M;
     rows = in_use < rows ? in_use : rows;
@@ -56,6 +54,14 @@ copy_rows_kernel(const uint4* __restrict__ src, const Index* __restrict__ index,
         if (v0 + i * TPR < vec_per_row) d[v0 + i * TPR] = u[i];
     }
   }
+}
+template <typename Index, int TPR, bool SKIP>
+__global__ void __launch_bounds__(kRowThreads)
+copy_rows_kernel(const uint4* src, const Index* index, const int32_t* num_mtiles, uint4* dst, int64_t rows, int vec_per_row,
+                 int div) {
+  grid_release();
+  grid_wait();
+  copy_rows<Index, TPR, SKIP>(src, index, num_mtiles, dst, rows, vec_per_row, div);
 }
 
 // Zeroes the padding rows (row_src < 0) among the rows in use: a warp looks at 64 rows at a time (two loads and ballots;
@@ -85,13 +91,10 @@ __device__ __forceinline__ void zero_padding(const int32_t* __restrict__ row_src
 // times, and the tokens of an expert are scattered over the whole input).  The second part of the grid
 // zeroes the padding rows.
 template <int TPR>
-__global__ void __launch_bounds__(kRowThreads)
-dispatch_rows_kernel(const uint4* __restrict__ src, const int32_t* __restrict__ dst_row,
-                     const int32_t* __restrict__ row_src, const int32_t* __restrict__ num_mtiles,
-                     uint4* __restrict__ dst, int64_t num_tokens, int topk, int vec_per_row, int token_blocks,
-                     bool live_blocks_only) {
-  grid_release();
-  grid_wait();
+__device__ __forceinline__ void dispatch_tokens(const uint4* __restrict__ src, const int32_t* __restrict__ dst_row,
+                                                const int32_t* __restrict__ row_src, const int32_t* __restrict__ num_mtiles,
+                                                uint4* __restrict__ dst, int64_t num_tokens, int topk, int vec_per_row,
+                                                int token_blocks, bool live_blocks_only) {
   constexpr int kRows = kRowThreads / TPR;
   if (static_cast<int>(blockIdx.x) >= token_blocks) {
     zero_padding(row_src, num_mtiles, dst, vec_per_row, (blockIdx.x - token_blocks) * (kRowThreads / 32) + (threadIdx.x >> 5),
@@ -118,6 +121,14 @@ dispatch_rows_kernel(const uint4* __restrict__ src, const int32_t* __restrict__ 
       }
     }
   }
+}
+template <int TPR>
+__global__ void __launch_bounds__(kRowThreads)
+dispatch_rows_kernel(const uint4* src, const int32_t* dst_row, const int32_t* row_src, const int32_t* num_mtiles, uint4* dst,
+                     int64_t num_tokens, int topk, int vec_per_row, int token_blocks, bool live_blocks_only) {
+  grid_release();
+  grid_wait();
+  dispatch_tokens<TPR>(src, dst_row, row_src, num_mtiles, dst, num_tokens, topk, vec_per_row, token_blocks, live_blocks_only);
 }
 
 // Row window of a pull: everything, or the rows of the experts of chunk `chunk_index` of `chunk_count` (the same
@@ -344,11 +355,9 @@ struct FoldExtra {
 };
 
 template <typename T, int TPR, int SLOTS, bool EXTRA>
-__global__ void __launch_bounds__(kRowThreads)
-combine_topk_kernel(const uint4* __restrict__ ys, const T* __restrict__ scores, const int32_t* __restrict__ dst_row,
-                    uint4* __restrict__ out, int64_t num_tokens, int topk, int vec_per_row, FoldExtra extra) {
-  grid_release();
-  grid_wait();
+__device__ __forceinline__ void fold_tokens(const uint4* __restrict__ ys, const T* __restrict__ scores,
+                                            const int32_t* __restrict__ dst_row, uint4* __restrict__ out, int64_t num_tokens,
+                                            int topk, int vec_per_row, const FoldExtra& extra) {
   constexpr int kRows = kRowThreads / TPR;
   const int lane = threadIdx.x % TPR;
   for (int64_t t = static_cast<int64_t>(blockIdx.x) * kRows + threadIdx.x / TPR; t < num_tokens;
@@ -390,6 +399,14 @@ combine_topk_kernel(const uint4* __restrict__ ys, const T* __restrict__ scores, 
     }
   }
 }
+template <typename T, int TPR, int SLOTS, bool EXTRA>
+__global__ void __launch_bounds__(kRowThreads)
+combine_topk_kernel(const uint4* ys, const T* scores, const int32_t* dst_row, uint4* out, int64_t num_tokens, int topk,
+                    int vec_per_row, FoldExtra extra) {
+  grid_release();
+  grid_wait();
+  fold_tokens<T, TPR, SLOTS, EXTRA>(ys, scores, dst_row, out, num_tokens, topk, vec_per_row, extra);
+}
 
 // One warp's share of the backward fold: gs row = scale * dout row (unless gs is null), and the dot product of the dout and
 // ys rows (complete in every lane).
@@ -426,10 +443,9 @@ __device__ __forceinline__ float combine_bwd_row(const uint4* __restrict__ d, co
 // 128 x 8 of 4 KB 16.4 -> 12.5.
 template <typename T>
 __global__ void __launch_bounds__(kRowThreads)
-combine_bwd_tokens_kernel(const uint4* __restrict__ dout, const T* __restrict__ scores, const uint4* __restrict__ ys,
-                          const int32_t* __restrict__ dst_row, const int32_t* __restrict__ row_src,
-                          const int32_t* __restrict__ num_mtiles, uint4* __restrict__ gs, T* __restrict__ dscores,
-                          int64_t num_slots, int topk, int vec_per_row, int slot_blocks, bool live_blocks_only) {
+combine_bwd_tokens_kernel(const uint4* dout, const T* scores, const uint4* ys, const int32_t* dst_row, const int32_t* row_src,
+                          const int32_t* num_mtiles, uint4* gs, T* dscores, int64_t num_slots, int topk, int vec_per_row,
+                          int slot_blocks, bool live_blocks_only) {
   grid_release();
   grid_wait();
   constexpr int kWarps = kRowThreads / 32;
