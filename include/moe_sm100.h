@@ -224,6 +224,11 @@ int moe_unpad_rows(const void* src, const int32_t* dst_row, void* out, int64_t n
 int moe_index_rows(const void* src, const int64_t* index, void* out, int64_t num_rows, int div,
                    int cols, int dtype, void* stream);
 
+/* inverse[index[r]] = r for the entries of `index` in [0, num_rows), -1 where none points: the row map that
+ * moe_combine_topk and moe_unpad_rows take, from the permutation moe_routing_metadata writes (whose tail is -1 when ids were
+ * dropped).  Entries >= num_rows are skipped and reported (status 5). */
+int moe_inverse_rows(const int64_t* index, int32_t* inverse, int64_t num_rows, int32_t* status, void* stream);
+
 /* out[t, :] = sum_s scale(t,s) * ys[dst_row[t*topk+s], :], fp32 accumulation, one rounding.
  * scores: [T, topk] in `dtype`, or NULL for scale 1 (used for dX). */
 int moe_combine_topk(const void* ys, const void* scores, const int32_t* dst_row, void* out,

@@ -64,6 +64,18 @@ copy_rows_kernel(const uint4* src, const Index* index, const int32_t* num_mtiles
   copy_rows<Index, TPR, SKIP>(src, index, num_mtiles, dst, rows, vec_per_row, div);
 }
 
+// inverse[index[r]] = r; `inverse` holds -1 everywhere before.  Negative entries (positions the routing metadata dropped) name
+// nothing; one past the end is reported and skipped.
+__global__ void __launch_bounds__(kRowThreads)
+inverse_rows_kernel(const int64_t* __restrict__ index, int32_t* __restrict__ inverse, int64_t rows, int32_t* status) {
+  for (int64_t r = static_cast<int64_t>(blockIdx.x) * kRowThreads + threadIdx.x; r < rows;
+       r += static_cast<int64_t>(gridDim.x) * kRowThreads) {
+    const int64_t j = index[r];
+    if (j >= rows && status != nullptr) atomicCAS(status, 0, DS_BAD_LAYOUT);
+    if (j >= 0 && j < rows) inverse[j] = static_cast<int32_t>(r);
+  }
+}
+
 // Zeroes the padding rows (row_src < 0) among the rows in use: a warp looks at 64 rows at a time (two loads and ballots;
 // a load per row made this the longest part of a dispatch) and clears the ones it finds.  `live_blocks_only`: 64-row blocks
 // without a routed row are left alone.
@@ -778,6 +790,19 @@ extern "C" int moe_index_rows(const void* src, const int64_t* index, void* out, 
   MOE_CHECK_ARG(aligned16(src) && aligned16(out), "moe_index_rows: pointers must be 16-byte aligned");
   MOE_ROW_COMMON_CHECKS("moe_index_rows", cols, dtype);
   launch_copy_rows(src, index, nullptr, out, num_rows, cols / 8, div, static_cast<cudaStream_t>(stream));
+  MOE_CUDA(cudaGetLastError());
+  return MOE_OK;
+}
+
+extern "C" int moe_inverse_rows(const int64_t* index, int32_t* inverse, int64_t num_rows, int32_t* status, void* stream) {
+  MOE_CHECK_ARG(num_rows >= 0 && num_rows < (1ll << 31), "moe_inverse_rows: num_rows=%lld is outside [0, 2^31)",
+                (long long)num_rows);
+  if (num_rows == 0) return MOE_OK;
+  MOE_CHECK_ARG(index && inverse, "moe_inverse_rows: null pointer argument");
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  MOE_CUDA(cudaMemsetAsync(inverse, 0xFF, static_cast<size_t>(num_rows) * sizeof(int32_t), s));
+  inverse_rows_kernel<<<row_grid((num_rows + kRowThreads - 1) / kRowThreads), kRowThreads, 0, s>>>(index, inverse, num_rows,
+                                                                                               status);
   MOE_CUDA(cudaGetLastError());
   return MOE_OK;
 }

@@ -79,6 +79,7 @@ SIGNATURES = {
                                      c_int, c_int, c_void_p, c_void_p]),
     "moe_unpad_rows": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int, c_void_p]),
     "moe_index_rows": (c_int, [c_void_p] * 3 + [c_int64, c_int, c_int, c_int, c_void_p]),
+    "moe_inverse_rows": (c_int, [c_void_p, c_void_p, c_int64, c_void_p, c_void_p]),
     "moe_combine_topk": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int, c_int, c_void_p]),
     "moe_scale_and_reduce": (c_int, [c_void_p] * 3 + [c_int64, c_int, c_int, c_int, c_void_p]),
     "moe_combine_bwd": (c_int, [c_void_p] * 7 + [c_int64, c_int, c_int64, c_int, c_int, c_void_p]),
@@ -430,6 +431,16 @@ def index_rows(src, index, out, div=1):
         rc = load().moe_index_rows(_ptr(src), _ptr(index), _ptr(out), out.size(0), div, out.size(1), dtype_code(src.dtype),
                                    _stream())
     _check("moe_index_rows", rc)
+    _count(1)
+
+
+def inverse_rows(index, inverse, status):
+    """inverse[index[r]] = r (int64 -> int32), -1 where no entry points; negative entries name nothing."""
+    require_cuda(index, inverse)
+    assert index.dtype is torch.int64 and index.numel() == inverse.numel()
+    with timed("routing"):
+        rc = load().moe_inverse_rows(_ptr(index), _ptr(inverse), index.numel(), _ptr(status), _stream())
+    _check("moe_inverse_rows", rc)
     _count(1)
 
 

@@ -14,7 +14,7 @@ import torch
 
 from moe_explore import _native
 from moe_explore.functional.scale_and_reduce import scale_and_reduce
-from moe_explore.routing_plan import build_routing_plan
+from moe_explore.routing_plan import build_routing_plan, device_status
 
 
 @dataclass
@@ -54,8 +54,9 @@ def row_gather(tokens: torch.Tensor, indices: torch.Tensor) -> torch.Tensor:
 
 
 def row_scatter(tokens: torch.Tensor, indices: torch.Tensor) -> torch.Tensor:
-    """``out[indices[r]] = tokens[r]``; ``indices`` must be a permutation
-    (triton_kernels/row_gather_scatter.py:91-116)."""
+    """``out[indices[r]] = tokens[r]``; ``indices`` must be a permutation (triton_kernels/row_gather_scatter.py:91-116), but for
+    entries of -1 (positions ``get_token_indices`` dropped): their rows go nowhere and the rows of ``out`` that nothing
+    reaches are zero.  An entry past the end is reported through the device's status word."""
     inverse = _inverse(tokens, indices)
     out = torch.empty_like(tokens)
     _native.unpad_rows(tokens.contiguous(), inverse, out)
@@ -66,7 +67,7 @@ def _inverse(tokens: torch.Tensor, indices: torch.Tensor) -> torch.Tensor:
     _native.require_cuda(tokens, indices)
     assert tokens.dim() == 2 and indices.dim() == 1 and indices.numel() == tokens.size(0)
     inverse = torch.empty(indices.numel(), dtype=torch.int32, device=tokens.device)
-    inverse[indices] = torch.arange(indices.numel(), dtype=torch.int32, device=tokens.device)
+    _native.inverse_rows(indices.to(torch.int64).contiguous(), inverse, device_status(tokens.get_device()))
     return inverse
 
 

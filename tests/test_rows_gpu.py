@@ -134,3 +134,52 @@ def test_functional_gemm_with_negative_positions(gather, scatter, act, native):
     else:
         full[bad] = 0
         assert torch.equal(out, full)
+
+
+@pytest.mark.parametrize("T,k,cols", [(2, 1, 8), (65, 3, 520), (700, 8, 2048)])
+def test_permute_round_trip_with_dropped_slots(T, k, cols, native):
+    """Ids outside [0, E) leave -1 at the tail of the permutation: such slots add nothing, all others are exact, with and
+    without a gradient of the scores."""
+    from moe_explore.expert_permute import row_scatter
+
+    E = 16
+    g = torch.Generator(device="cuda").manual_seed(T)
+    x = torch.randn(T, cols, generator=g, device="cuda").bfloat16()
+    idx = torch.stack([torch.randperm(E, generator=g, device="cuda")[:k] for _ in range(T)])
+    idx[0, 0], idx[T // 2, k - 1], idx[T - 1, k // 2] = E, -3, 10 ** 9
+    dropped = (idx < 0) | (idx >= E)
+    scores = torch.rand(T, k, generator=g, device="cuda").bfloat16()
+    poison = [torch.full((n << 10,), 0x7FFFFFFF, dtype=torch.int32, device="cuda") for n in (1, 1, 2, 4, 8, 16, 64)]
+    del poison
+    grouped = expert_input_permute(x, idx, E, k)
+    flat = scores.masked_fill(dropped, 0)
+    # fp32 sum of k exact products, rounded once
+    terms = x.float()[:, None, :] * flat.float()[..., None]
+    bound = terms.sum(1).abs() * 2.0 ** -8 + k * 2.0 ** -23 * terms.abs().sum(1)
+    leaf = scores.clone().requires_grad_()
+    out, out_grad = (expert_output_permute(grouped, s, k, x.shape) for s in (scores, leaf))
+    assert bool(((out.float() - terms.sum(1)).abs() <= bound).all()) and torch.equal(out, out_grad)
+    out_grad.backward(x)
+    assert not leaf.grad[dropped].any() and bool(leaf.grad[~dropped].any()) == bool((~dropped).any())
+    rows = row_scatter(grouped.tokens, grouped.indices)
+    assert torch.equal(rows, x.repeat_interleave(k, 0).masked_fill(dropped.reshape(-1, 1), 0))
+    assert native.read_status(build_routing_plan(idx, E, k).status, reset=True) == 100
+
+
+@pytest.mark.parametrize("rows", [1, 255, 256, 257, 70000])
+def test_inverse_rows(rows, native):
+    from moe_explore.routing_plan import device_status
+
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    index = torch.randperm(rows, generator=g, device="cuda")
+    index[::5] = -1 - index[::5]
+    out = torch.full((rows,), 7, dtype=torch.int32, device="cuda")
+    native.read_status(device_status(), reset=True)
+    native.inverse_rows(index, out, device_status())
+    expect = torch.full_like(out, -1)
+    live = index >= 0
+    expect[index[live]] = torch.arange(rows, dtype=torch.int32, device="cuda")[live]
+    assert torch.equal(out, expect) and native.read_status(device_status()) == 0
+    index[0] = rows   # (was negative) one past the end: named in the status word, written nowhere
+    native.inverse_rows(index, out, device_status())
+    assert torch.equal(out, expect) and native.read_status(device_status(), reset=True) == 5
