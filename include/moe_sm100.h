@@ -119,6 +119,9 @@ int moe_router_topk(const void* logits, void* scores, int64_t* indices, int32_t*
  * `status` is set to 100.  Workspace: moe_routing_workspace_bytes(R, E) bytes.
  * --------------------------------------------------------------------------------- */
 size_t moe_routing_workspace_bytes(int64_t num_rows, int num_experts);
+/* Up to this many rows the current device takes moe_routing_metadata in one launch (131072 on a whole B200, fewer where only
+ * smaller clusters fit); moe_expert_forward needs no workspace up to here. */
+int64_t moe_routing_one_launch_rows(int num_experts);
 int moe_routing_metadata(const int64_t* expert_idx, int64_t num_rows, int num_experts,
                          int32_t* group_indices, int64_t* perm, int32_t* pad_offsets,
                          int32_t* row_src, int32_t* dst_row, int32_t* mtile_expert,
@@ -417,7 +420,7 @@ int moe_kgrouped_gemm_gather(const void* src, int64_t src_rows, const int32_t* r
  *   identity       num_experts = topk = 1 and every score is 1: group_indices holds {0, num_tokens} (read, not written); x,
  *                  grad_out, out and dx stand in the place of xs, gs, ys and dxs, and MOE_FWD_DISPATCH / FOLD and MOE_BWD_FOLD /
  *                  FOLD_DX / ROUTER do not apply
- *   workspace      for MOE_FWD_ROUTE of more than 131072 rows, moe_routing_workspace_bytes(num_tokens * topk, num_experts)
+ *   workspace      for MOE_FWD_ROUTE of more than moe_routing_one_launch_rows(num_experts) rows, moe_routing_workspace_bytes(num_tokens * topk, num_experts)
  *                  bytes
  *   addend         NULL, or a [num_tokens, d] tensor that the fold adds (not with fused_combine)
  *   dl             NULL, or the router's backward is part of the pass: scores are the softmax of the selected `logits`

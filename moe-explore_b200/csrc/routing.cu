@@ -3,7 +3,8 @@
 //
 // Replaces get_token_indices (reference: src/moe_explore/expert_permute.py:19-41), which runs
 // torch.argsort + torch.histc + torch.cumsum as three or more launches.  Here it is a counting sort (the number of
-// distinct keys, E, is small): one launch of one cluster (route_cluster_kernel) up to kClusterRows rows, and for
+// distinct keys, E, is small): one launch of one cluster (route_cluster_kernel) up to kClusterRows rows (fewer where the device
+// takes only smaller clusters: max_route_cluster), and for
 // more rows the chip-wide form:
 //   1. chunk_histogram : each warp owns a contiguous chunk of kChunk flat positions and counts
 //                        its ids per expert in shared memory (warp-aggregated via match.any);
@@ -314,6 +315,7 @@ route_cluster_kernel(const int64_t* __restrict__ ids, int64_t R, int E, int held
     }
     cta_cnt[e] = run;
   }
+  __syncwarp();  // the cluster barriers below are .aligned: every warp reaches them as a whole
   cluster_sync_all();
   int32_t total = 0, before = 0;
   if (e < E) {
@@ -324,6 +326,7 @@ route_cluster_kernel(const int64_t* __restrict__ ids, int64_t R, int E, int held
     }
   }
   // no CTA may exit while another still reads its counts: arrive here, wait at the end
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
 
   // 3. prefix sums over the experts (every CTA for itself): rows, padded rows, row-tile pairs
@@ -422,25 +425,57 @@ route_cluster_kernel(const int64_t* __restrict__ ids, int64_t R, int E, int held
                                  ((m + 1) * MOE_TILE_M < sh_pad[lo + 1] ? 0x80000000u : 0u));
     }
   }
+  __syncwarp();
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-static int route_cluster(const int64_t* ids, int64_t R, int E, const RouteOut& out, int32_t* status, cudaStream_t s) {
-  // as many CTAs as there are 1024-row shares (the scattered stores of the placement are what one SM is slow at)
-  int ctas = 1;
-  while (ctas < kMaxCluster && static_cast<int64_t>(ctas) * kRouteThreads < R) ctas *= 2;
-  const int64_t share = static_cast<int64_t>(ctas) * kRouteThreads;
-  const int held = static_cast<int>((R + share - 1) / share);
-  const size_t smem = (static_cast<size_t>(kRouteWarps) * E + 6 * static_cast<size_t>(E) + 2) * sizeof(int32_t);
-  static std::atomic<bool> ready[64];
+static size_t route_smem_bytes(int E) {
+  return (static_cast<size_t>(kRouteWarps) * E + 6 * static_cast<size_t>(E) + 2) * sizeof(int32_t);
+}
+
+// The largest cluster (a power of two up to kMaxCluster) that can run on the current device.  A whole B200 takes all 16 CTAs in
+// a GPC; a device with fewer SMs to a GPC may not, and a launch of a cluster that fits nowhere fails.  Asked once per
+// device, for at most 256 experts and for more (39 and 155 KB of shared memory per CTA).
+static int max_route_cluster(int E, int* out) {
+  static std::atomic<int> known[64][2];
+  const int wide = E > 256 ? 1 : 0;
   int dev = 0;
   MOE_CUDA(cudaGetDevice(&dev));
-  if (dev < 0 || dev >= 64 || !ready[dev].load(std::memory_order_acquire)) {
+  const bool keep = dev >= 0 && dev < 64;
+  int ctas = keep ? known[dev][wide].load(std::memory_order_acquire) : 0;
+  if (ctas == 0) {
     MOE_CUDA(cudaFuncSetAttribute(route_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (kRouteWarps + 6) * kMaxExperts * 4 + 8));
+                                  static_cast<int>(route_smem_bytes(kMaxExperts))));
     MOE_CUDA(cudaFuncSetAttribute(route_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    if (dev >= 0 && dev < 64) ready[dev].store(true, std::memory_order_release);
+    for (ctas = kMaxCluster; ctas > 1; ctas /= 2) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(static_cast<unsigned>(ctas), 1, 1);
+      cfg.blockDim = dim3(kRouteThreads, 1, 1);
+      cfg.dynamicSmemBytes = route_smem_bytes(wide ? kMaxExperts : 256);
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = static_cast<unsigned>(ctas);
+      attr[0].val.clusterDim.y = 1;
+      attr[0].val.clusterDim.z = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      int clusters = 0;
+      if (cudaOccupancyMaxActiveClusters(&clusters, route_cluster_kernel, &cfg) == cudaSuccess && clusters > 0) break;
+      cudaGetLastError();  // a size the device refuses is an answer, not an error
+    }
+    if (keep) known[dev][wide].store(ctas, std::memory_order_release);
   }
+  *out = ctas;
+  return MOE_OK;
+}
+
+static int route_cluster(const int64_t* ids, int64_t R, int E, int max_ctas, const RouteOut& out, int32_t* status, cudaStream_t s) {
+  // as many CTAs as there are 1024-row shares (the scattered stores of the placement are what one SM is slow at)
+  int ctas = 1;
+  while (ctas < max_ctas && static_cast<int64_t>(ctas) * kRouteThreads < R) ctas *= 2;
+  const int64_t share = static_cast<int64_t>(ctas) * kRouteThreads;
+  const int held = static_cast<int>((R + share - 1) / share);
+  const size_t smem = route_smem_bytes(E);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(ctas), 1, 1);
   cfg.blockDim = dim3(kRouteThreads, 1, 1);
@@ -611,6 +646,12 @@ extern "C" size_t moe_routing_workspace_bytes(int64_t num_rows, int num_experts)
   return 2 * static_cast<size_t>(chunks) * num_experts * sizeof(int32_t);  // chunk histogram + chunk offsets
 }
 
+extern "C" int64_t moe_routing_one_launch_rows(int num_experts) {
+  int ctas = 1;
+  if (num_experts <= 0 || num_experts > kMaxExperts || max_route_cluster(num_experts, &ctas) != MOE_OK) ctas = 1;
+  return static_cast<int64_t>(ctas) * kRouteThreads * kHeld;
+}
+
 namespace moe {
 
 int routing_metadata(const int64_t* expert_idx, int64_t num_rows, int num_experts, int32_t* group_indices, int64_t* perm,
@@ -629,16 +670,23 @@ int routing_metadata(const int64_t* expert_idx, int64_t num_rows, int num_expert
   MOE_CHECK_ARG(num_rows == 0 || expert_idx != nullptr, "moe_routing_metadata: expert_idx is null");
   MOE_CHECK_ARG((mtile_expert == nullptr) == (num_mtiles == nullptr) && (tile_pairs == nullptr || mtile_expert != nullptr),
                 "moe_routing_metadata: mtile_expert, tile_pairs and num_mtiles go together");
-  MOE_CHECK_ARG((!workspace_always && num_rows <= kClusterRows) ||
-                    (workspace != nullptr && workspace_bytes >= moe_routing_workspace_bytes(num_rows, num_experts)),
+  const bool scratch = workspace != nullptr && workspace_bytes >= moe_routing_workspace_bytes(num_rows, num_experts);
+  int64_t cluster_rows = kClusterRows;
+  int max_ctas = kMaxCluster;
+  if (scratch || !workspace_always) {
+    const int rc = max_route_cluster(num_experts, &max_ctas);
+    if (rc != MOE_OK) return rc;
+    cluster_rows = static_cast<int64_t>(max_ctas) * kRouteThreads * kHeld;
+  }
+  MOE_CHECK_ARG(scratch || (!workspace_always && num_rows <= cluster_rows),
                 "moe_routing_metadata: workspace of %zu bytes is smaller than the %zu required", workspace_bytes,
                 moe_routing_workspace_bytes(num_rows, num_experts));
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (num_rows <= kClusterRows) {
+  if (num_rows <= cluster_rows) {
     const RouteOut out{group_indices, perm, pad_offsets, row_src, dst_row, mtile_expert, tile_pairs, num_mtiles,
                        static_cast<int32_t>(moe_mtiles_bound(num_rows, num_experts)),
                        static_cast<int32_t>(moe_padded_rows_bound(num_rows, num_experts))};
-    return route_cluster(expert_idx, num_rows, num_experts, out, status, s);
+    return route_cluster(expert_idx, num_rows, num_experts, max_ctas, out, status, s);
   }
   int32_t* chunk_hist = static_cast<int32_t*>(workspace);
   const int64_t chunks = num_chunks(num_rows);

@@ -7,6 +7,7 @@ library's own error text when a call returns a non-zero status.
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 from ctypes import c_int, c_int32, c_int64, c_size_t, c_void_p, c_char_p, POINTER
 
@@ -20,7 +21,8 @@ MOE_DTYPE_BF16 = 0
 MOE_DTYPE_F16 = 1
 ACT_CODES = {None: 0, "none": 0, "silu": 1, "gelu": 2, "swiglu": 3, "geglu": 4, "approx_gelu": 5}
 TILE_M = 128
-ROUTE_ONE_LAUNCH_ROWS = 131072   # csrc/routing.cu: up to here the routing metadata is one launch
+ROUTE_ONE_LAUNCH_ROWS = 131072   # csrc/routing.cu: up to here a whole B200 takes the routing metadata in one launch
+ROUTE_CHIP_WIDE_LAUNCHES = 4     # ... and beyond
 # codes a kernel may leave in a status word (include/moe_sm100.h, moe_check_status)
 STATUS_WAVE_FALLBACK = 4
 STATUS_BAD_LAYOUT = 5
@@ -66,6 +68,7 @@ SIGNATURES = {
     "moe_padded_rows_bound": (c_int64, [c_int64, c_int]),
     "moe_mtiles_bound": (c_int64, [c_int64, c_int]),
     "moe_routing_workspace_bytes": (c_size_t, [c_int64, c_int]),
+    "moe_routing_one_launch_rows": (c_int64, [c_int]),
     "moe_routing_metadata": (c_int, [c_void_p, c_int64, c_int] + [c_void_p] * 9 + [c_void_p, c_size_t, c_void_p]),
     "moe_routing_static_scratch_bytes": (c_size_t, []),
     "moe_routing_metadata_static": (c_int, [c_void_p, c_int64, c_int] + [c_void_p] * 9 + [c_void_p]),
@@ -276,7 +279,7 @@ def routing_metadata(expert_idx, num_experts, group_indices, perm, pad_offsets, 
                                      _ptr(workspace),
                                      workspace.numel() * workspace.element_size(), _stream())
     _check("moe_routing_metadata", rc)
-    _count(1 if expert_idx.numel() <= ROUTE_ONE_LAUNCH_ROWS else 3)
+    _count(routing_launches(expert_idx.numel(), num_experts))
 
 
 def routing_metadata_static(expert_idx, num_experts, group_indices, perm, pad_offsets, row_src, dst_row, mtile_expert,
@@ -289,7 +292,18 @@ def routing_metadata_static(expert_idx, num_experts, group_indices, perm, pad_of
                                             _ptr(mtile_expert), _ptr(tile_pairs), _ptr(num_mtiles), _ptr(status),
                                             _stream())
     _check("moe_routing_metadata_static", rc)
-    _count(1 if expert_idx.numel() <= ROUTE_ONE_LAUNCH_ROWS else 3)
+    _count(routing_launches(expert_idx.numel(), num_experts))
+
+
+@functools.lru_cache(maxsize=None)
+def _one_launch_rows(device: int, wide: bool) -> int:
+    return int(load().moe_routing_one_launch_rows(1024 if wide else 256))
+
+
+def routing_launches(num_rows: int, num_experts: int) -> int:
+    """Kernels that the routing metadata takes on the current device; a workspace is used when there is more than one."""
+    fits = num_rows <= _one_launch_rows(torch.cuda.current_device(), num_experts > 256)
+    return 1 if fits else ROUTE_CHIP_WIDE_LAUNCHES
 
 
 def routing_workspace_bytes(num_rows: int, num_experts: int) -> int:

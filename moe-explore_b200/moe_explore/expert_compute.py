@@ -76,9 +76,10 @@ def _forward(x, scores, weight1, weight2, routing, act, gather_in_gemm: bool, fu
         status = device_status(x.get_device())
         plan_ptrs = _packed_pointers(words, offsets, status)
         ids = flat.data_ptr()
-        if rows > _native.ROUTE_ONE_LAUNCH_ROWS:
+        launches = _native.routing_launches(rows, E)
+        if launches > 1:
             workspace = torch.empty(max(_native.routing_workspace_bytes(rows, E), 16), dtype=torch.uint8, device=x.device)
-        steps.append((_native.FWD_ROUTE, "routing", 1 if workspace is None else 3))
+        steps.append((_native.FWD_ROUTE, "routing", launches))
     xs = None if gather_in_gemm else new(rp, d)
     # the un-activated product, needed by the backward pass (not kept for inference or without an activation)
     pre_act = new(rp, n1) if (act is not None and needs_grad) else None
