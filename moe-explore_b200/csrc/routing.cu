@@ -513,7 +513,7 @@ __global__ void __launch_bounds__(kMaxExperts)
 layout_from_groups_kernel(const int32_t* __restrict__ group_indices, int64_t R, int E, const int64_t* __restrict__ perm,
                           int scatter, GroupsOut out, int32_t* status) {
   __shared__ int32_t sh_lo[kMaxExperts], sh_cnt[kMaxExperts], sh_pad[kMaxExperts + 1], sh_pair[kMaxExperts + 1];
-  __shared__ int32_t sums[2][32];
+  __shared__ int32_t sums[2][32], cut[2];
   const int e = threadIdx.x, lane = e & 31, warp = e >> 5;
   grid_release();
   int32_t cnt = 0, lo = 0;
@@ -526,29 +526,45 @@ layout_from_groups_kernel(const int32_t* __restrict__ group_indices, int64_t R, 
     if (bad && blockIdx.x == 0 && status != nullptr) atomicCAS(status, 0, DS_BAD_LAYOUT);
     cnt = bad ? 0 : hi - lo;
   }
-  const int32_t padded = (cnt + MOE_TILE_M - 1) / MOE_TILE_M * MOE_TILE_M;
-  const int32_t pairs = (padded / MOE_TILE_M + 1) / 2;
+  int32_t padded = (cnt + MOE_TILE_M - 1) / MOE_TILE_M * MOE_TILE_M;
+  int32_t pairs = (padded / MOE_TILE_M + 1) / 2;
+  // (capped: the sum over a prefix that is none can exceed 32 bits)
+  constexpr int32_t kCap = 1 << 29;
   int32_t in_p = padded, in_q = pairs;
 #pragma unroll
   for (int off = 1; off < 32; off <<= 1) {
     const int32_t a = __shfl_up_sync(0xFFFFFFFFu, in_p, off);
     const int32_t b = __shfl_up_sync(0xFFFFFFFFu, in_q, off);
-    if (lane >= off) { in_p += a; in_q += b; }
+    if (lane >= off) { in_p = min(in_p + a, kCap); in_q += b; }
   }
   if (lane == 31) { sums[0][warp] = in_p; sums[1][warp] = in_q; }
   __syncthreads();
   if (warp < 2) {
     int32_t v = sums[warp][lane];
-    const int32_t own = v;
 #pragma unroll
     for (int off = 1; off < 32; off <<= 1) {
       const int32_t a = __shfl_up_sync(0xFFFFFFFFu, v, off);
-      if (lane >= off) v += a;
+      if (lane >= off) v = min(v + a, kCap);
     }
-    sums[warp][lane] = v - own;
+    const int32_t before = __shfl_up_sync(0xFFFFFFFFu, v, 1);
+    sums[warp][lane] = lane > 0 ? before : 0;
   }
   __syncthreads();
-  const int32_t p1 = in_p + sums[0][warp], q1 = in_q + sums[1][warp];
+  int32_t p1 = in_p + sums[0][warp], q1 = in_q + sums[1][warp];
+  // A prefix that runs back and forth can give its experts more rows than there are, and the maps are sized for R: experts
+  // whose padded rows would end past them are refused as well (the status word has been set by the step back).
+  const bool over = e < E && p1 > out.mtiles_bound * MOE_TILE_M;
+  if (__syncthreads_or(over)) {
+    if (e == 0) { cut[0] = 0; cut[1] = 0; }
+    __syncthreads();
+    if (e < E && !over) { atomicMax(&cut[0], p1); atomicMax(&cut[1], q1); }
+    __syncthreads();
+    if (over) {
+      cnt = padded = pairs = 0;
+      p1 = cut[0];
+      q1 = cut[1];
+    }
+  }
   if (e < E) {
     sh_lo[e] = lo;
     sh_cnt[e] = cnt;

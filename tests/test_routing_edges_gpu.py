@@ -39,3 +39,30 @@ def test_one_launch_up_to_the_largest_cluster_the_device_takes(native):
     g = torch.Generator().manual_seed(1)
     for rows in (131072, 131071, 65535, 8193):
         _check_against_oracle(torch.randint(0, 1024, (rows, 1), generator=g), 1024)
+
+
+@pytest.mark.parametrize("rows,experts", [(1000, 3), (1000, 40), (40000, 1024)])
+def test_prefix_that_runs_back_and_forth_stays_inside_the_maps(rows, experts, native):
+    """0, R, 0, R, ...: every other group has all the rows, together many times what the maps hold.  Status 5, no map entry
+    past the bound, and the functional GEMM on such groups computes the groups that were kept."""
+    from moe_explore.routing_plan import device_status, plan_from_groups
+    from moe_explore.triton_kernels.m_grouped_gemm import MGroupedGEMMParams, m_grouped_gemm
+
+    groups = torch.tensor([0, rows] * ((experts + 1) // 2) + ([rows] if experts % 2 == 0 else []), dtype=torch.int32)[:experts + 1]
+    bound = native.mtiles_bound(rows, experts)
+    tiles = (rows + 127) // 128
+    kept = min(bound // tiles, (experts + 1) // 2)
+    assert (experts + 1) // 2 * tiles > bound   # what the maps would have to hold
+    native.read_status(device_status(), reset=True)
+    plan = plan_from_groups(groups.cuda(), rows)
+    assert native.read_status(plan.status, reset=True) == 5
+    assert plan.num_mtiles.tolist() == [kept * tiles, kept * ((tiles + 1) // 2), bound, 0]
+    assert int(plan.pad_offsets.max()) == int(plan.pad_offsets[-1]) == kept * tiles * 128
+    assert plan.mtile_expert[: kept * tiles].tolist() == [2 * (m // tiles) for m in range(kept * tiles)]
+    assert int(plan.row_src.max()) < rows and int(plan.dst_row.max()) < plan.padded_rows
+    assert int(plan.tile_pairs[bound + experts]) == kept * ((tiles + 1) // 2)
+    x = torch.randn(rows, 64, device="cuda").bfloat16()
+    w = torch.zeros(experts, 64, 72, device="cuda").bfloat16()
+    out = m_grouped_gemm(x, MGroupedGEMMParams(w, groups.cuda(), torch.arange(rows, device="cuda"), True, True, rows, 1))
+    torch.cuda.synchronize()
+    assert not out.any() and native.read_status(device_status(), reset=True) == 5
