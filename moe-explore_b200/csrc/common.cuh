@@ -511,14 +511,16 @@ template <> __device__ __forceinline__ void red_add_v8<__half>(void* ptr, const 
 }
 
 // Activation math (fp32).
-// 1 / y for y >= 1: the hardware's approximation and one Newton step, without the range checks and the slow-path branch of a
-// division.  The branch kept the compiler from interleaving the elements of an epilogue row, which with two warps per
-// scheduler is the whole speed of the gated epilogues.  y is capped below infinity (1 / inf would turn into inf * 0).
+// 1 / y for y >= 1 (infinity included): one step of the Newton-Raphson iteration r' = r + r (1 - y r), whose relative error is the
+// square of r's, from the hardware's approximation (relative error 2^-23: the step leaves the rounding of its last
+// operation).  Straight-line code, because the elements of an epilogue row have to be interleaved: with two warps per scheduler
+// that is the whole speed of the gated epilogues (dGLU at 16384 tokens x 4 slots, 60 experts, K 2048: 229 -> 204 us against the
+// division operator).  The cap makes the step from r = 0 at y = infinity a finite one; r itself is taken of y, so that results
+// below the normal range (gates under -87) and NaN come out as they are.
 __device__ __forceinline__ float reciprocal_ge1(float y) {
-  y = fminf(y, 3.0e38f);
   float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(y));
-  return fmaf(r, fmaf(-y, r, 1.0f), r);
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(y));
+  return fmaf(r, fmaf(-fminf(y, 3.0e38f), r, 1.0f), r);
 }
 __device__ __forceinline__ float sigmoidf_fast(float x) { return reciprocal_ge1(1.0f + __expf(-x)); }
 __device__ __forceinline__ float silu_f(float x) { return x * sigmoidf_fast(x); }
