@@ -12,7 +12,6 @@ namespace moe {
   MOE_INST(BN, true, false, EPI_GLU, false)     \
   MOE_INST(BN, true, false, EPI_ACT_AUX, false) \
   MOE_INST(BN, true, true, EPI_ACT, false)      \
-  MOE_INST(BN, true, true, EPI_ACT_AUX, false)  \
   MOE_INST(BN, false, false, EPI_ACT, true)
 MOE_INST_BN(128)
 MOE_INST_BN(256)

@@ -23,7 +23,6 @@ namespace moe {
   MOE_EXTERN(T, CTAS, BN, true, false, EPI_GLU, false, true)      \
   MOE_EXTERN(T, CTAS, BN, true, false, EPI_ACT_AUX, false, true)  \
   MOE_EXTERN(T, CTAS, BN, true, true, EPI_ACT, false, true)       \
-  MOE_EXTERN(T, CTAS, BN, true, true, EPI_ACT_AUX, false, true)   \
   MOE_EXTERN(T, CTAS, BN, false, false, EPI_ACT, true, true)
 #define MOE_EXTERN_ALL(T, CTAS) MOE_EXTERN_BN(T, CTAS, 128) MOE_EXTERN_BN(T, CTAS, 256)
 MOE_EXTERN_ALL(__nv_bfloat16, 2)
@@ -245,9 +244,7 @@ static int mgrouped_dispatch(const void* a, const void* w, int64_t a_rows, int64
     if (rc != MOE_OK) return rc;
     rc = make_tmap(&td, dtype, args.out, 2, dims, box);
     if (rc != MOE_OK) return rc;
-    if (gather)
-      return w_transposed ? launch<T, BN, true, true, EPI_ACT_AUX, false, CTAS, true>(ta, tb, tc, td, args, lp)
-                          : launch<T, BN, true, false, EPI_ACT_AUX, false, CTAS, true>(ta, tb, tc, td, args, lp);
+    if (gather) return launch<T, BN, true, false, EPI_ACT_AUX, false, CTAS, true>(ta, tb, tc, td, args, lp);  // forward only
     return w_transposed ? launch<T, BN, true, true, EPI_ACT_AUX, false, CTAS, false>(ta, tb, tc, td, args, lp)
                         : launch<T, BN, true, false, EPI_ACT_AUX, false, CTAS, false>(ta, tb, tc, td, args, lp);
   }

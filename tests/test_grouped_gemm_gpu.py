@@ -540,3 +540,48 @@ def test_metadata_built_for_another_row_bound_is_refused(native):
     assert bool((out == 3.0).all())
     with pytest.raises(native.MoeNativeError, match="does not describe"):
         plan.check()
+
+
+@pytest.mark.parametrize("w_transposed", [False, True])
+@pytest.mark.parametrize("gather", [False, True])
+@pytest.mark.parametrize("rows,N,act,dtype", [
+    ((5, 0, 130, 64, 1), 72, None, torch.bfloat16),          # one-CTA kernels, narrow column tiles
+    ((5, 0, 130, 64, 1), 264, "silu", torch.float16),        # ... and a ragged second wide one
+    ((700, 257, 300), 72, "gelu", torch.float16),            # CTA pairs
+    ((700, 257, 300), 264, None, torch.bfloat16),
+])
+def test_scatter_entry_point(rows, N, act, dtype, gather, w_transposed, native):
+    """moe_mgrouped_gemm_scatter (for callers of the C library; the Python functional GEMM has its own call): every row at its
+    mapped place and no other row touched, rows of A from the padded layout or gathered by the loads, both weight layouts."""
+    from moe_explore.routing_plan import plan_from_groups
+
+    K, E, R, topk = 136, len(rows), sum(rows), 2
+    g = torch.Generator(device="cuda").manual_seed(R + N)
+    plan = plan_from_groups(torch.tensor([0] + list(rows), dtype=torch.int32).cumsum(0).to(torch.int32).cuda(), R)
+    x = torch.randn(R, K, generator=g, device="cuda").to(dtype)
+    w = (torch.randn(E, N, K, generator=g, device="cuda") * 0.1).to(dtype)
+    pos = plan.row_src.long()
+    perm = torch.randperm(R, generator=g, device="cuda")
+    perm[::11] = -1                                         # not stored
+    out_rows = torch.where(pos >= 0, perm[pos.clamp_min(0)], -1).int()
+    if gather:                                              # row r of the groups is token source[r] // topk
+        source = torch.randint(0, R * topk, (R,), generator=g, device="cuda")
+        a, a_rows = x, torch.where(pos >= 0, source[pos.clamp_min(0)], -1).int()
+        rows_in = x[source // topk]
+    else:
+        a, a_rows = torch.empty(plan.padded_rows, K, dtype=dtype, device="cuda"), None
+        native.gather_rows(x, plan.row_src, plan.num_mtiles, a, 1)
+        rows_in = x
+    out = torch.full((R, N), 7.0, dtype=dtype, device="cuda")
+    native.mgrouped_gemm_scatter(a, w if w_transposed else w.transpose(1, 2).contiguous(), out, out_rows, plan.mtile_expert,
+                                 plan.tile_pairs, plan.num_mtiles, plan.padded_rows, w_transposed, act, a_row_src=a_rows,
+                                 a_div=topk, status=plan.status)
+    expert = torch.repeat_interleave(torch.arange(E), torch.tensor(rows)).cuda()
+    ref = torch.bmm(rows_in.float()[:, None], w.float()[expert].transpose(1, 2))[:, 0]
+    ref = {None: lambda v: v, "silu": torch.nn.functional.silu, "gelu": torch.nn.functional.gelu}[act](ref)
+    stored = perm >= 0
+    assert relerr(out[perm[stored]], ref[stored]) <= TOL
+    untouched = torch.ones(R, dtype=torch.bool, device="cuda")
+    untouched[perm[stored]] = False
+    assert int(untouched.sum()) == int((~stored).sum()) and bool((out[untouched] == 7).all())
+    assert native.read_status(plan.status) == 0
