@@ -12,10 +12,12 @@
 // Limits and rules
 //   * the array holds kStaticScratchBytes (1 MiB); a problem whose scratch requirement
 //     (moe_routing_workspace_bytes) is larger is rejected with MOE_ERR_UNSUPPORTED;
+//   * up to moe_routing_one_launch_rows(num_experts) rows the one-launch form does the work and the array is
+//     not touched; the limits and the rule below hold for all calls, so that callers need not know the line;
 //   * every call on a device shares the one array: two calls that overlap on the GPU (different
 //     streams, or different host threads) race on it -- serialise them;
 //   * the array keeps whatever the previous call left in it; nothing in it has to start at zero,
-//     because the histogram kernel overwrites every word the later kernels read;
+//     because the chip-wide form's histogram kernel overwrites every word its later kernels read;
 //   * the first call on each device looks up the array's device address (one
 //     cudaGetSymbolAddress, no allocation); make that first call outside any stream capture.
 #include "common.cuh"

@@ -1,7 +1,7 @@
 // Row movement around the grouped GEMMs: gather token rows into the padded expert-sorted
 // layout, fold the top-k slots back into token order with the router weights, and the
-// backward of that fold.  All kernels are HBM-bound: 16-byte vector accesses, one warp per
-// row segment, fp32 accumulation where values are summed.
+// backward of that fold.  All kernels are HBM-bound: 16-byte vector accesses, 32 to 128 threads
+// per row, fp32 accumulation where values are summed.
 //
 // Replace row_gather / row_scatter (reference: src/moe_explore/triton_kernels/row_gather_scatter.py:36-116)
 // and scale_and_reduce (src/moe_explore/functional/scale_and_reduce.py:3-5).
@@ -516,7 +516,7 @@ __global__ void store_words_to_host_kernel(const unsigned long long* __restrict_
   __threadfence_system();
 }
 
-// Zeroes the padding rows (row_src < 0) of a [rows, vec_per_row] buffer in the padded layout: one warp per row.
+// Zeroes the padding rows (row_src < 0) of a [rows, vec_per_row] buffer in the padded layout: a warp looks after 64 rows.
 __global__ void __launch_bounds__(kRowThreads)
 zero_padding_rows_kernel(const int32_t* __restrict__ row_src, const int32_t* __restrict__ num_mtiles, uint4* __restrict__ dst,
                          int vec_per_row) {

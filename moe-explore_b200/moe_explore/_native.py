@@ -270,6 +270,11 @@ def run_pass(name: str, p, steps, rows: int) -> None:
         _count(launches)
 
 
+# One binding per C entry point follows.  The layer itself launches through ``run_pass``; dispatch_rows, dispatch_rows_only,
+# combine_bwd_tokens, mgrouped_gemm_gather / _combine / _scatter and kgrouped_gemm_gather are the single steps behind it, bound for
+# callers that build a pass of their own and for the tests that hold the passes against them.
+
+
 def routing_metadata(expert_idx, num_experts, group_indices, perm, pad_offsets, row_src, dst_row, mtile_expert,
                      tile_pairs, num_mtiles, status, workspace):
     require_cuda(expert_idx)

@@ -136,7 +136,8 @@ def build_routing_plan(expert_indices: torch.Tensor, num_experts: int, topk: int
 
 def plan_from_groups(group_indices: torch.Tensor, num_rows: int) -> RoutingPlan:
     """Plan for rows that are already grouped: ``group_indices`` int32 [E+1] exclusive prefix of ``num_rows``.
-    A prefix that does not run monotonically from 0 to ``num_rows`` is reported through the status word."""
+    A prefix that does not run monotonically from 0 to ``num_rows`` is reported through the status word.  For callers that run
+    ``expert_compute`` on rows of their own grouping (``m_grouped_gemm`` lays its rows out by itself)."""
     _native.require_cuda(group_indices)
     assert group_indices.dtype is torch.int32 and group_indices.dim() == 1
     num_experts = group_indices.numel() - 1

@@ -73,3 +73,11 @@ def test_static_scratch_entry_rejects_oversized_problems(native):
         native.routing_metadata_static(idx, experts, out["group_indices"], out["perm"], out["pad_offsets"],
                                        out["row_src"], out["dst_row"], out["mtile_expert"], out["tile_pairs"],
                                        out["num_mtiles"], out["status"])
+
+
+def test_static_scratch_above_the_one_launch_rows(native):
+    """The row counts at which the scratch is in fact used (the smaller problems above are one launch without it)."""
+    g = torch.Generator().manual_seed(22)
+    for rows, experts in ((140001, 60), (262144, 200), (140001, 60), (131073, 3)):
+        assert native.routing_launches(rows, experts) > 1
+        _run_both(torch.randint(0, experts, (rows, 1), generator=g), experts, native)
