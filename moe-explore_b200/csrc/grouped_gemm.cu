@@ -361,10 +361,14 @@ static int mgrouped_common(const char* name, const void* a, const void* w, void*
   // a work item streams half as many weight columns per tensor-core cycle as two independent CTAs do (measured at
   // 64 rows per expert, DeepSeek-V3 shape: gate/up 4.10 -> 2.69 ms, down 2.01 -> 1.38; at 16 rows per expert,
   // OLMoE shape: -6..12 %; at 128 rows per expert 0..5 %).
-  // Epilogues that move only the result (plain stores, gated without the saved product) leave the one-CTA kernels ahead up
-  // to 192 rows per expert, where a pair's second CTA is idle for a third of the pairs (188 rows, 128 experts, K 2048:
-  // gate/up 232 -> 218 us, down 180 -> 166; at 256 rows 185 -> 188 and 121 -> 119; with side tiles 239 -> 248 at 188).
-  const bool light = epi == EPI_ACT || (epi == EPI_GLU && x.aux_out == nullptr);
+  // Inside a pass (the routed counts are known, so the one-CTA kernels leave out the halves of tiles without routed rows)
+  // epilogues that move only the result (plain stores, gated without the saved product) stay with one CTA up to 192 rows per
+  // expert.  What decides is how many pairs have an idle second CTA, and that the host does not know: it depends on how unevenly
+  // the rows fall.  Forward pass of 3001 tokens x 8 slots, 128 experts, K 2048 (188 rows per expert), one CTA / pairs: even
+  // routing 465 / 433 us, moderately uneven (0.5 N(0, 1) on the logits) 472 / 496, Zipf(1.1) 476 / 510.  Over 136-188 rows and
+  // 16 to 128 experts: even -5 to +14 % (training +8), moderate -6 to +7, Zipf -12 to 0.  Without the counts, even routing at
+  // 144-192 rows is 6-17 % slower on one CTA (64 experts, K 2048, 160 rows: 140 / 124 and 85 / 77), so there the line is 128.
+  const bool light = x.counts.group_indices != nullptr && (epi == EPI_ACT || (epi == EPI_GLU && x.aux_out == nullptr));
   const long long mean_rows_per_expert = (padded_rows - static_cast<long long>(E) * (BM - 1)) / E;
   const bool pairs = tile_pairs != nullptr &&
                      (o.single_cta == 0 ? mean_rows_per_expert > (light ? BM + BM / 2 : BM) : o.single_cta < 0);
