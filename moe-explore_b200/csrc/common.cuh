@@ -364,6 +364,8 @@ __device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, int c0, int
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 // Wait until the bulk stores committed by this thread have finished READING shared memory (the buffer may be reused).
 __device__ __forceinline__ void bulk_wait_read_all() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+// The same, all but the last committed group.
+__device__ __forceinline__ void bulk_wait_read_one() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
 // Wait until the bulk stores committed by this thread are complete.
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 // Orders this thread's generic-proxy shared-memory writes before later async-proxy (TMA) reads of them.

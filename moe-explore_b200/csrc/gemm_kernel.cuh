@@ -75,8 +75,7 @@ struct GemmArgs {
   const int32_t* num_mtiles;    // M-grouped: device int32[4] = {tiles in use, tile pairs in use, tile bound, 0}
   const int32_t* pad_offsets;   // K-grouped, and with group_indices: padded row offsets [E+1]
   // Optional prefix of the routed rows per expert [E+1].  With it, only the 64-row blocks of an expert's padded range that
-  // hold a routed row exist: M-grouped kernels store nothing into the others (and the one-CTA kernels do not load them),
-  // K-grouped kernels contract over the others' rows not at all.
+  // hold a routed row exist: M-grouped kernels store nothing into the others, K-grouped kernels contract over the others' rows not at all.
   const int32_t* group_indices;
   int32_t a_compact;            // M-grouped, with group_indices: A holds the routed rows without padding, expert by expert
   int32_t mtiles_bound;         // M-grouped: padded_rows / 128 as the caller sees it (checked against num_mtiles[2])
@@ -137,6 +136,7 @@ struct TileCoord {
   int a_row;    // M-grouped: row of A the tile begins at (m0, or its unpadded counterpart; the rows after the expert's last
                 // one are then the next expert's, and nothing is stored for them)
   int live;     // M-grouped: rows of the tile that exist (64 or 128, see GemmArgs::group_indices)
+  int unit_rows;  // M-grouped: rows of the whole row unit that exist, in 64-row blocks (the tile's, or the pair's)
 };
 
 // Rows of expert e that exist, in whole 64-row blocks, at most its padded range (whatever the prefix says).
@@ -316,9 +316,11 @@ __device__ __forceinline__ TileCoord decode_tile(int t, int mt, int nt, const Wi
     c.k_row0 = args.pad_offsets[expert];
     c.kiters = live_rows(args, expert, args.pad_offsets[expert + 1] - c.k_row0) / BK;  // multiples of 64
     c.live = BM;
+    c.unit_rows = BM;
     c.a_row = 0;
   } else {
     int tile = m_idx;
+    c.unit_rows = BM;
     if (CTAS == 2) {
       // one load: first tile (bits 0-19), expert (bits 20-30), "has a second tile" (bit 31)
       const uint32_t info = static_cast<uint32_t>(args.tile_pairs[m_idx]);
@@ -326,6 +328,7 @@ __device__ __forceinline__ TileCoord decode_tile(int t, int mt, int nt, const Wi
       tile = static_cast<int>(info & 0xFFFFFu);
       c.expert = static_cast<int>((info >> 20) & 0x7FFu);
       c.active = rank == 0 || second;
+      c.unit_rows = second ? 2 * BM : BM;
       if (rank == 1 && second) tile += 1;  // an inactive second CTA re-reads the first tile and stores nothing
     } else {
       c.expert = args.mtile_expert[tile];
@@ -337,6 +340,7 @@ __device__ __forceinline__ TileCoord decode_tile(int t, int mt, int nt, const Wi
       const int base = args.pad_offsets[c.expert];
       const int left = live_rows(args, c.expert, 1 << 30) - (c.m0 - base);
       c.live = left < BM ? (left > 64 ? left : 64) : BM;
+      if (left < c.unit_rows) c.unit_rows = left > 64 ? left : 64;
       if (args.a_compact) c.a_row = c.m0 - base + args.group_indices[c.expert];
     }
     c.k_row0 = 0;
@@ -344,6 +348,39 @@ __device__ __forceinline__ TileCoord decode_tile(int t, int mt, int nt, const Wi
   }
   return c;
 }
+
+// The work items of one worker, as a warp walks them: every lane decodes one of the next 32 items, and the warp takes them from
+// its lanes in turn.  Decoding is a chain of two dependent loads (the unit, then its expert's row counts), 1000 to 2000 cycles
+// under load in an in-order warp; item by item it left the copy engine and the tensor cores without instructions for that
+// long per item, whatever was still queued.
+template <bool KG, int CTAS>
+struct ItemWalk {
+  TileCoord mine;
+  int first, stride, count, mt, nt, BN, rank;  // of the worker's items, `count` items in the launch
+  __device__ __forceinline__ ItemWalk(int unit, int num_units, int ntiles, int mt_, int nt_, int BN_, int rank_)
+      : mine{}, first(unit), stride(num_units), count(ntiles), mt(mt_), nt(nt_), BN(BN_), rank(rank_) {}
+  // The i-th item; i = 0, 1, 2, ... in this order, by all lanes of the warp.
+  __device__ __forceinline__ TileCoord get(int i, const Window& win, const GemmArgs& args) {
+    if ((i & 31) == 0) {
+      const int t = first + (i + static_cast<int>(threadIdx.x & 31)) * stride;
+      // (an item that does not exist is not decoded: when no row tile is in use the maps hold nothing to decode)
+      if (t < count) mine = decode_tile<KG, CTAS>(t, mt, nt, win, args, BN, rank);
+      __syncwarp();
+    }
+    const int src = i & 31;
+    TileCoord c;
+    c.m0 = __shfl_sync(0xFFFFFFFFu, mine.m0, src);
+    c.n0 = __shfl_sync(0xFFFFFFFFu, mine.n0, src);
+    c.expert = __shfl_sync(0xFFFFFFFFu, mine.expert, src);
+    c.k_row0 = __shfl_sync(0xFFFFFFFFu, mine.k_row0, src);
+    c.kiters = KG ? __shfl_sync(0xFFFFFFFFu, mine.kiters, src) : (args.k_dim + BK - 1) / BK;
+    c.active = __shfl_sync(0xFFFFFFFFu, mine.active ? 1 : 0, src) != 0;
+    c.a_row = __shfl_sync(0xFFFFFFFFu, mine.a_row, src);
+    c.live = __shfl_sync(0xFFFFFFFFu, mine.live, src);
+    c.unit_rows = __shfl_sync(0xFFFFFFFFu, mine.unit_rows, src);
+    return c;
+  }
+};
 
 // Wave barrier of the persistent workers.  With a static stride every worker's i-th work item belongs to the same
 // "wave" of neighbouring tiles; workers that share operand tiles only hit in L2 while they stream through them
@@ -403,6 +440,18 @@ __device__ __forceinline__ void apply_act(float (&v)[32], int act) {
     for (int i = 0; i < 32; ++i) v[i] = gelu_tanh_f(v[i]);
   }
 }
+__device__ __forceinline__ void mul_dact(float (&v)[32], const float (&x)[32], int act) {
+  if (act == MOE_ACT_SILU) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] *= dsilu_f(x[i]);
+  } else if (act == MOE_ACT_GELU) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] *= dgelu_f(x[i]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] *= dgelu_tanh_f(x[i]);
+  }
+}
 template <typename T>
 __device__ __forceinline__ void mul_dact(float (&v)[32], const uint4 (&pre)[4], int act) {
   float x[32];
@@ -416,16 +465,7 @@ __device__ __forceinline__ void mul_dact(float (&v)[32], const uint4 (&pre)[4], 
       x[qq * 8 + 2 * i + 1] = f.y;
     }
   }
-  if (act == MOE_ACT_SILU) {
-#pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] *= dsilu_f(x[i]);
-  } else if (act == MOE_ACT_GELU) {
-#pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] *= dgelu_f(x[i]);
-  } else {
-#pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] *= dgelu_tanh_f(x[i]);
-  }
+  mul_dact(v, x, act);
 }
 
 // Gated backward of one register row: da = gradient of the activated value, h = the saved (gate, up) pairs, replaced by
@@ -559,9 +599,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       // Mixtral shape with the branches compiled out), because the loop then no longer is the short elected-lane
       // sequence the operand pipeline needs once per 512 tensor-core cycles.
       constexpr bool gather = GATHER;
-      // (a worker without an item decodes none: when no row tile is in use the maps hold nothing to decode)
-      TileCoord c_next{};
-      if (unit < ntiles) c_next = decode_tile<KG, CTAS>(unit, mt, nt, win, args, BN, rank);
+      ItemWalk<KG, CTAS> items(unit, num_units, ntiles, mt, nt, BN, rank);
+      TileCoord c_next = items.get(0, win, args);
       // M-grouped gather: lane l owns rows 4l..4l+3 of the tile for all of its stages
       int4 rows_next = make_int4(0, 0, 0, 0);
       if (gather && !KG && unit < ntiles) rows_next = gather_rows4(args.a_row_src, c_next.m0 + 4 * lane, args.a_div, args.a_rows);
@@ -570,9 +609,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       for (int t = unit; t < ntiles && ok; t += num_units, ++wave) {
         const TileCoord c = c_next;
         const int4 rows_m = rows_next;
-        // fetch the next work item's coordinates now; the loads complete while this tile streams
         if (t + num_units < ntiles) {
-          c_next = decode_tile<KG, CTAS>(t + num_units, mt, nt, win, args, BN, rank);
+          c_next = items.get(wave + 1, win, args);
           if (gather && !KG) rows_next = gather_rows4(args.a_row_src, c_next.m0 + 4 * lane, args.a_div, args.a_rows);
         }
         if (wave_sync && wave > 0 &&
@@ -609,12 +647,9 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
           const bool remote = kPair && rank != 0;
           const uint32_t fb = remote ? mapa_shared(full_bar + 8 * stage, 0) : full_bar + 8 * stage;
           const bool leader_lane = elect_one();
-          // one-CTA kernels (few rows per expert) fetch the A tile in halves and leave out a half without routed rows
-          constexpr bool kHalves = !KG && !kPair && !GATHER;
-          const bool both = !kHalves || c.live > 64;
           if (leader_lane) {
             if (remote) mbar_arrive_expect_tx_cluster(fb, Plan::kStageBytes);
-            else mbar_arrive_expect_tx(fb, both ? Plan::kStageBytes : Plan::kStageBytes - Plan::kABytes / 2);
+            else mbar_arrive_expect_tx(fb, Plan::kStageBytes);
           }
           if (gather) {
             // all 32 lanes: 4 rows x 128 bytes each = the whole 128 x 64 (or 64 x 128) A tile of the stage
@@ -679,7 +714,6 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
               }
             } else {
               if (!gather) tma_load_2d(sa, &tmap_a, kb * BK, c.a_row, fb, pol);
-              if (kHalves && both) tma_load_2d(sa + Plan::kABytes / 2, &tmap_a, kb * BK, c.a_row + 64, fb, pol);
               if (B_K) {
                 tma_load_3d(sb, &tmap_b, kb * BK, c.n0 + bcol, c.expert, fb, pol);
               } else if (args.b_blocked) {
@@ -722,11 +756,10 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       uint32_t acc_phase = 0;
       bool ok = true;
       bool ready = false;  // the stage about to be consumed was already seen full
-      TileCoord c_next{};
-      if (unit < ntiles) c_next = decode_tile<KG, CTAS>(unit, mt, nt, win, args, BN, rank);
+      ItemWalk<KG, CTAS> items(unit, num_units, ntiles, mt, nt, BN, rank);
+      int item = 0;
       for (int t = unit; t < ntiles && ok; t += num_units) {
-        const TileCoord c = c_next;
-        if (t + num_units < ntiles) c_next = decode_tile<KG, CTAS>(t + num_units, mt, nt, win, args, BN, rank);
+        const TileCoord c = items.get(item++, win, args);
         if (c.kiters == 0) continue;  // empty expert: the epilogue writes zeros on its own
         if (!__all_sync(0xFFFFFFFFu, mbar_wait(tempty_bar + 8 * acc, acc_phase ^ 1, wctx, DS_TIMEOUT_MMA))) {
           ok = false;
@@ -804,11 +837,10 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     const auto side_parity = [](uint32_t n) { return Plan::kTilesPerWarp == 2 ? (n >> 1) & 1 : n & 1; };
     const int co_row = lane >> 3;  // coalesced access: row within a group of four
     const int co_ck = lane & 7;    // and 16-byte piece of the row's 128 bytes
-    TileCoord c_next{};
-    if (unit < ntiles) c_next = decode_tile<KG, CTAS>(unit, mt, nt, win, args, BN, rank);
+    ItemWalk<KG, CTAS> items(unit, num_units, ntiles, mt, nt, BN, rank);
+    int item = 0;
     for (int t = unit; t < ntiles; t += num_units) {
-      const TileCoord c = c_next;
-      if (t + num_units < ntiles) c_next = decode_tile<KG, CTAS>(t + num_units, mt, nt, win, args, BN, rank);
+      const TileCoord c = items.get(item++, win, args);
       const bool have_acc = c.kiters != 0;
       const int row = c.m0 + row_in_tile;
       const bool quad_live = KG || (c.active && quad * 32 < c.live);  // this warp's 32 rows exist
@@ -1221,32 +1253,31 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, 
            const LaunchParams& lp);
 
 #ifdef MOE_GEMM_DEFINE_LAUNCH
-template <typename T, int BN, bool A_K, bool B_K, int EPI, bool KG, int CTAS, bool GATHER>
-int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const CUtensorMap& td, GemmArgs args,
-           const LaunchParams& lp) {
-  auto kernel = grouped_gemm_kernel<T, BN, A_K, B_K, EPI, KG, CTAS, GATHER>;
-  constexpr int smem = SmemPlan<BN, CTAS, EPI>::kTotal;
-  static_assert(SmemPlan<BN, CTAS, EPI>::kStages >= 3, "too few operand stages");
-  static std::atomic<int> grid_for_device[64];  // 0 = not configured yet (zero-initialised)
+// Launch configuration of a persistent kernel with as many workers as fit the current device (capped by lp.max_ctas), kept per
+// device in `grids` (0 = not configured yet; two threads racing at the first launch compute the same value twice).
+struct PersistentLaunch {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[2];
+};
+template <int CTAS, typename Kernel>
+int configure(PersistentLaunch& l, Kernel kernel, int smem, std::atomic<int> (&grids)[64], const LaunchParams& lp) {
   int dev = 0;
   MOE_CUDA(cudaGetDevice(&dev));
-  cudaLaunchConfig_t cfg = {};
+  cudaLaunchConfig_t& cfg = l.cfg;
   cfg.blockDim = dim3(kThreads, 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = lp.stream;
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = CTAS;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
+  l.attr[0].id = cudaLaunchAttributeClusterDimension;
+  l.attr[0].val.clusterDim.x = CTAS;
+  l.attr[0].val.clusterDim.y = 1;
+  l.attr[0].val.clusterDim.z = 1;
   constexpr int kClusterAttrs = CTAS > 1 ? 1 : 0;
-  attr[kClusterAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[kClusterAttrs].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
+  l.attr[kClusterAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  l.attr[kClusterAttrs].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = l.attr;
   cfg.numAttrs = kClusterAttrs;
-  int grid = (dev >= 0 && dev < 64) ? grid_for_device[dev].load(std::memory_order_acquire) : 0;
+  int grid = (dev >= 0 && dev < 64) ? grids[dev].load(std::memory_order_acquire) : 0;
   if (grid == 0) {
-    // First launch of this variant on this device (two threads racing here compute the same value twice).
     MOE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     grid = sm_count() / CTAS * CTAS;
     if (CTAS > 1) {
@@ -1261,16 +1292,27 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, 
       }
       if (clusters * CTAS < grid) grid = clusters * CTAS;
     }
-    if (dev >= 0 && dev < 64) grid_for_device[dev].store(grid, std::memory_order_release);
+    if (dev >= 0 && dev < 64) grids[dev].store(grid, std::memory_order_release);
   }
-  {
-    const int limit = lp.max_ctas / CTAS * CTAS;
-    if (limit >= CTAS && limit < grid) grid = limit;
-  }
-  if (args.wave_workers <= 0) args.wave_workers = grid / CTAS;
+  const int limit = lp.max_ctas / CTAS * CTAS;
+  if (limit >= CTAS && limit < grid) grid = limit;
   cfg.gridDim = dim3(static_cast<unsigned>(grid), 1, 1);
   cfg.numAttrs = kClusterAttrs + (lp.chained ? 1 : 0);
-  MOE_CUDA(cudaLaunchKernelEx(&cfg, kernel, ta, tb, tc, td, args));
+  return MOE_OK;
+}
+
+template <typename T, int BN, bool A_K, bool B_K, int EPI, bool KG, int CTAS, bool GATHER>
+int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const CUtensorMap& td, GemmArgs args,
+           const LaunchParams& lp) {
+  auto kernel = grouped_gemm_kernel<T, BN, A_K, B_K, EPI, KG, CTAS, GATHER>;
+  constexpr int smem = SmemPlan<BN, CTAS, EPI>::kTotal;
+  static_assert(SmemPlan<BN, CTAS, EPI>::kStages >= 3, "too few operand stages");
+  static std::atomic<int> grids[64];
+  PersistentLaunch l;
+  const int rc = configure<CTAS>(l, kernel, smem, grids, lp);
+  if (rc != MOE_OK) return rc;
+  if (args.wave_workers <= 0) args.wave_workers = static_cast<int>(l.cfg.gridDim.x) / CTAS;
+  MOE_CUDA(cudaLaunchKernelEx(&l.cfg, kernel, ta, tb, tc, td, args));
   return MOE_OK;
 }
 #endif  // MOE_GEMM_DEFINE_LAUNCH

@@ -1,6 +1,6 @@
 // Host side of the grouped GEMMs: argument checks, tensor maps (cached), scheduling choices and the
 // C entry points.  The kernel itself is in gemm_kernel.cuh; its variants are instantiated in gemm_inst_*.cu.
-#include "gemm_kernel.cuh"
+#include "gemm_t_kernel.cuh"
 
 #include <mutex>
 
@@ -30,6 +30,20 @@ MOE_EXTERN_ALL(__nv_bfloat16, 1)
 MOE_EXTERN_ALL(__half, 2)
 MOE_EXTERN_ALL(__half, 1)
 
+#define MOE_EXTERN_T(T, UNIT, W_K, EPI) \
+  extern template int launch_t<T, UNIT, W_K, EPI>(const TMaps&, const GemmArgs&, const LaunchParams&);
+#define MOE_EXTERN_T_ALL(T, UNIT)           \
+  MOE_EXTERN_T(T, UNIT, false, EPI_ACT)     \
+  MOE_EXTERN_T(T, UNIT, false, EPI_GLU)     \
+  MOE_EXTERN_T(T, UNIT, false, EPI_ACT_AUX) \
+  MOE_EXTERN_T(T, UNIT, true, EPI_ACT)      \
+  MOE_EXTERN_T(T, UNIT, true, EPI_ACT_AUX)  \
+  MOE_EXTERN_T(T, UNIT, true, EPI_DGLU)
+MOE_EXTERN_T_ALL(__nv_bfloat16, 128)
+MOE_EXTERN_T_ALL(__nv_bfloat16, 256)
+MOE_EXTERN_T_ALL(__half, 128)
+MOE_EXTERN_T_ALL(__half, 256)
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -56,11 +70,12 @@ struct TmapKey {
   const void* ptr;
   int dtype;
   int rank;
+  int swizzle;
   uint64_t dims[4];
   uint64_t strides[3];  // bytes, of dims 1..rank-1
   uint32_t box[4];
   bool operator==(const TmapKey& o) const {
-    if (ptr != o.ptr || dtype != o.dtype || rank != o.rank) return false;
+    if (ptr != o.ptr || dtype != o.dtype || rank != o.rank || swizzle != o.swizzle) return false;
     for (int i = 0; i < rank; ++i)
       if (dims[i] != o.dims[i] || box[i] != o.box[i]) return false;
     for (int i = 0; i + 1 < rank; ++i)
@@ -74,14 +89,15 @@ static TmapKey g_tmap_keys[kTmapCacheSize];
 static CUtensorMap g_tmap_vals[kTmapCacheSize];
 static int g_tmap_used = 0, g_tmap_next = 0;
 
-// Tensor map with the 128-byte swizzle; dims[0] is the contiguous dimension.  `strides` (bytes, for dims 1..rank-1)
+// Tensor map (by default with the 128-byte swizzle); dims[0] is the contiguous dimension.  `strides` (bytes, for dims 1..rank-1)
 // may be null for a dense row-major tensor.
 static int make_tmap(CUtensorMap* map, int dtype, const void* ptr, int rank, const uint64_t* dims,
-                     const uint32_t* box, const uint64_t* strides = nullptr) {
+                     const uint32_t* box, const uint64_t* strides = nullptr, bool swizzle = true) {
   TmapKey key{};
   key.ptr = ptr;
   key.dtype = dtype;
   key.rank = rank;
+  key.swizzle = swizzle;
   uint64_t dense = 2;
   for (int i = 0; i < rank; ++i) {
     key.dims[i] = dims[i];
@@ -113,7 +129,7 @@ static int make_tmap(CUtensorMap* map, int dtype, const void* ptr, int rank, con
   }
   CUresult r = fn(map, dtype == MOE_DTYPE_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
                   rank, const_cast<void*>(ptr), gdim, gstride, bdim, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                  swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
     set_error("cuTensorMapEncodeTiled failed with CUresult %d (rank %d, dims %llu x %llu x %llu)", (int)r, rank,
               (unsigned long long)dims[0], (unsigned long long)(rank > 1 ? dims[1] : 1),
@@ -200,7 +216,7 @@ static int mgrouped_dispatch(const void* a, const void* w, int64_t a_rows, int64
   const bool gather = args.a_row_src != nullptr;  // selects the kernel variant whose operand loads gather rows
   {
     const uint64_t dims[2] = {(uint64_t)K, (uint64_t)a_rows};
-    const uint32_t box[2] = {BK, args.a_row_src != nullptr ? 1u : (uint32_t)(CTAS == 1 ? BM / 2 : BM)};
+    const uint32_t box[2] = {BK, args.a_row_src != nullptr ? 1u : (uint32_t)BM};
     int rc = make_tmap(&ta, dtype, a, 2, dims, box);
     if (rc != MOE_OK) return rc;
   }
@@ -260,6 +276,56 @@ static int mgrouped_dispatch(const void* a, const void* w, int64_t a_rows, int64
     if (rc != MOE_OK) return rc;
   }
   return launch<T, BN, true, true, EPI_DGLU, false, CTAS, false>(ta, tb, tc, td, args, lp);
+}
+
+// The same with transposed tiles (gemm_t_kernel.cuh).
+template <typename T, int UNIT>
+static int mgrouped_dispatch_t(const void* a, const void* w, int64_t a_rows, int64_t out_rows, int K, int N, int E, int w_transposed,
+                               int epi, const GemmArgs& args, int dtype, const LaunchParams& lp) {
+  TMaps m;
+  int rc;
+  if (w_transposed) {
+    const uint64_t dims[3] = {(uint64_t)K, (uint64_t)N, (uint64_t)E};
+    const uint32_t box[3] = {BK, 128, 1};
+    rc = make_tmap(&m.w, dtype, w, 3, dims, box);
+  } else if (args.b_blocked) {
+    rc = make_tmap_blocked(&m.w, dtype, w, (uint64_t)K, (uint64_t)N, (uint64_t)E, BK, 2);
+  } else {
+    const uint64_t dims[3] = {(uint64_t)N, (uint64_t)K, (uint64_t)E};
+    const uint32_t box[3] = {64, BK, 1};
+    rc = make_tmap(&m.w, dtype, w, 3, dims, box);
+  }
+  if (rc != MOE_OK) return rc;
+  for (int i = 0; i < 4; ++i) {
+    if (i >= UNIT / 64) {
+      m.r[i] = m.r[0];
+      continue;
+    }
+    const uint64_t dims[2] = {(uint64_t)K, (uint64_t)a_rows};
+    const uint32_t box[2] = {BK, 32u * (i + 1)};
+    rc = make_tmap(&m.r[i], dtype, a, 2, dims, box);
+    if (rc != MOE_OK) return rc;
+  }
+  // results and saved products: 32 rows x a warp's 32 weight columns (16 results of gated ones, 32 saved pairs)
+  m.c = m.d = m.w;
+  const uint64_t cols_d = epi == EPI_GLU ? N / 2 : epi == EPI_DGLU ? 2 * N : N;
+  const uint32_t box_d[2] = {epi == EPI_GLU ? 16u : epi == EPI_DGLU ? 64u : 32u, 32};
+  if (args.out_tma) {
+    const uint64_t dims[2] = {cols_d, (uint64_t)out_rows};
+    rc = make_tmap(&m.d, dtype, args.out, 2, dims, box_d, nullptr, epi == EPI_DGLU);
+    if (rc != MOE_OK) return rc;
+  }
+  const void* side = args.aux_in != nullptr ? args.aux_in : args.aux_out;
+  if (side != nullptr) {
+    const uint64_t dims[2] = {epi == EPI_DGLU ? cols_d : (uint64_t)N, (uint64_t)args.mtiles_bound * BM};
+    const uint32_t box[2] = {epi == EPI_DGLU ? 64u : 32u, 32};
+    rc = make_tmap(&m.c, dtype, side, 2, dims, box, nullptr, epi == EPI_DGLU);
+    if (rc != MOE_OK) return rc;
+  }
+  if (epi == EPI_ACT) return w_transposed ? launch_t<T, UNIT, true, EPI_ACT>(m, args, lp) : launch_t<T, UNIT, false, EPI_ACT>(m, args, lp);
+  if (epi == EPI_GLU) return launch_t<T, UNIT, false, EPI_GLU>(m, args, lp);
+  if (epi == EPI_DGLU) return launch_t<T, UNIT, true, EPI_DGLU>(m, args, lp);
+  return w_transposed ? launch_t<T, UNIT, true, EPI_ACT_AUX>(m, args, lp) : launch_t<T, UNIT, false, EPI_ACT_AUX>(m, args, lp);
 }
 
 static int mgrouped_common(const char* name, const void* a, const void* w, void* out, const MExtras& x,
@@ -338,6 +404,27 @@ static int mgrouped_common(const char* name, const void* a, const void* w, void*
   lp.stream = static_cast<cudaStream_t>(stream);
   lp.max_ctas = o.max_ctas > 0 ? o.max_ctas : 0;
   lp.chained = chained_launches();
+  const long long mean_rows_per_expert = (padded_rows - static_cast<long long>(E) * (BM - 1)) / E;
+  const int64_t a_rows = x.gather_row_src != nullptr ? x.gather_rows : (x.counts.a_rows >= 0 ? x.counts.a_rows : padded_rows);
+  const int64_t out_rows = x.counts.out_rows >= 0 ? x.counts.out_rows : padded_rows;
+  // Inside a pass (the routed counts are known): transposed tiles while an expert has few enough rows for its last tile to
+  // matter; from six pairs of tiles on (2048 rows of the widest layer: equal within the power-bound spread of 4 %) the
+  // expert-aligned, wave-synchronised walk of the other kernel.  Row units of one tile up to 160 rows per expert, of two
+  // from there on: a unit of two tiles shares each weight step among up to 256 rows, one of a single tile keeps eight stages in
+  // flight instead of six and wastes less on rare experts (training sums of the four contractions, 32 experts, d 2048, I
+  // 1024, us, one / two tiles; even, moderately uneven, Zipf routing: 64 rows 210 / 216, 206 / 235, 226 / 233; 128 rows
+  // 229 / 231, 229 / 237, 247 / 269; 160 rows 245 / 235, 234 / 264, 261 / 254; 224 rows 260 / 265, 284 / 297, 322 / 298;
+  // 320 rows 343 / 326, 344 / 329, 350 / 320).
+  if (x.counts.group_indices != nullptr && tile_pairs != nullptr && x.gather_row_src == nullptr && x.push_bases == nullptr &&
+      options == nullptr && mean_rows_per_expert < 6 * 2 * BM) {
+    args.out_tma = x.push_row == nullptr && x.combine_row_src == nullptr;
+#define MOE_MG_T(TYPE)                                                                                                 \
+  (mean_rows_per_expert > 160                                                                                          \
+       ? mgrouped_dispatch_t<TYPE, 256>(a, w, a_rows, out_rows, K, N, E, w_transposed, epi, args, dtype, lp)           \
+       : mgrouped_dispatch_t<TYPE, 128>(a, w, a_rows, out_rows, K, N, E, w_transposed, epi, args, dtype, lp))
+    return dtype == MOE_DTYPE_BF16 ? MOE_MG_T(__nv_bfloat16) : MOE_MG_T(__half);
+#undef MOE_MG_T
+  }
   {
     // The wave barrier cuts the DRAM reads of every M-grouped GEMM to about the algorithmic bytes (gate/up at
     // the Mixtral shape: 6.4 -> 2.1 GB), but only long contractions get faster (K = 14336: -1.2 %, K = 28672:
@@ -361,19 +448,12 @@ static int mgrouped_common(const char* name, const void* a, const void* w, void*
   // a work item streams half as many weight columns per tensor-core cycle as two independent CTAs do (measured at
   // 64 rows per expert, DeepSeek-V3 shape: gate/up 4.10 -> 2.69 ms, down 2.01 -> 1.38; at 16 rows per expert,
   // OLMoE shape: -6..12 %; at 128 rows per expert 0..5 %).
-  // Inside a pass (the routed counts are known, so the one-CTA kernels leave out the halves of tiles without routed rows)
-  // epilogues that move only the result (plain stores, gated without the saved product) stay with one CTA up to 192 rows per
-  // expert.  What decides is how many pairs have an idle second CTA, and that the host does not know: it depends on how unevenly
-  // the rows fall.  Forward pass of 3001 tokens x 8 slots, 128 experts, K 2048 (188 rows per expert), one CTA / pairs: even
-  // routing 465 / 433 us, moderately uneven (0.5 N(0, 1) on the logits) 472 / 496, Zipf(1.1) 476 / 510.  Over 136-188 rows and
-  // 16 to 128 experts: even -5 to +14 % (training +8), moderate -6 to +7, Zipf -12 to 0.  Without the counts, even routing at
-  // 144-192 rows is 6-17 % slower on one CTA (64 experts, K 2048, 160 rows: 140 / 124 and 85 / 77), so there the line is 128.
-  const bool light = x.counts.group_indices != nullptr && (epi == EPI_ACT || (epi == EPI_GLU && x.aux_out == nullptr));
-  const long long mean_rows_per_expert = (padded_rows - static_cast<long long>(E) * (BM - 1)) / E;
+  // (Even routing at 144-192 rows is 6-17 % slower on one CTA: 64 experts, K 2048, 160 rows: 140 / 124 and 85 / 77 us.)  A pass
+  // that gathers its rows in the loads stays with one CTA up to 192 where the epilogue moves only the result.
+  const bool light = x.counts.group_indices != nullptr && x.gather_row_src != nullptr &&
+                     (epi == EPI_ACT || (epi == EPI_GLU && x.aux_out == nullptr));
   const bool pairs = tile_pairs != nullptr &&
                      (o.single_cta == 0 ? mean_rows_per_expert > (light ? BM + BM / 2 : BM) : o.single_cta < 0);
-  const int64_t a_rows = x.gather_row_src != nullptr ? x.gather_rows : (x.counts.a_rows >= 0 ? x.counts.a_rows : padded_rows);
-  const int64_t out_rows = x.counts.out_rows >= 0 ? x.counts.out_rows : padded_rows;
 #define MOE_MG(TYPE)                                                                                              \
   (pairs ? (bn == 256 ? mgrouped_dispatch<TYPE, 256, 2>(a, w, a_rows, out_rows, K, N, E, w_transposed, epi, args, dtype, lp) \
                       : mgrouped_dispatch<TYPE, 128, 2>(a, w, a_rows, out_rows, K, N, E, w_transposed, epi, args, dtype, lp)) \

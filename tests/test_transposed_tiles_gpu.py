@@ -1,0 +1,58 @@
+"""The contractions of a pass on transposed tiles against the same steps through the entry points that take 128-row tiles."""
+import pytest
+import torch
+
+from moe_explore.expert_compute import routed_expert_compute
+from moe_explore.routing_plan import build_routing_plan
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("act", [None, "silu", "gelu", "swiglu", "geglu"])
+@pytest.mark.parametrize("d,inter", [(264, 200), (128, 320), (72, 8)])    # columns past a tile, a CTA, a warp; K past a step
+@pytest.mark.parametrize("rows", [
+    (1, 31, 32, 33, 63, 64, 65, 127, 128, 129, 0, 300),       # row units of one tile
+    (193, 255, 256, 257, 320, 0, 449, 129),                   # of two, with one, with a rest
+])
+def test_a_pass_equals_its_steps(rows, d, inter, act, dtype, native):
+    """Every element is the same sum of the same products in the same order: bit for bit."""
+    E = len(rows)
+    ids = torch.repeat_interleave(torch.arange(E), torch.tensor(rows))
+    ids = ids[torch.randperm(len(ids), generator=torch.Generator().manual_seed(d))].view(-1, 1).cuda()
+    T = ids.size(0)
+    gen = torch.Generator(device="cuda").manual_seed(inter)
+    mk = lambda *s, std=1.0: (torch.randn(*s, generator=gen, device="cuda") * std).to(dtype)
+    n1 = 2 * inter if act in ("swiglu", "geglu") else inter
+    x, scores = mk(T, d), torch.rand(T, 1, generator=gen, device="cuda").to(dtype)
+    w1, w2, grad = mk(E, d, n1, std=0.1), mk(E, inter, d, std=0.1), mk(T, d)
+    leaves = [t.requires_grad_() for t in (x, scores, w1, w2)]
+    out = routed_expert_compute(*leaves, ids, E, 1, act)
+    got = [out.detach()] + list(torch.autograd.grad(out, leaves, grad))
+    with torch.no_grad():
+        assert torch.equal(routed_expert_compute(*leaves, ids, E, 1, act), got[0])
+        fused = routed_expert_compute(*leaves, ids, E, 1, act, fused_combine=True)
+        assert torch.equal(fused, got[0])     # one slot: one addition to zero
+
+        plan = build_routing_plan(ids, E, 1)
+        maps = (plan.mtile_expert, plan.tile_pairs, plan.num_mtiles)
+        new = lambda n: torch.empty(plan.padded_rows, n, dtype=dtype, device="cuda")
+        xs, pre, hidden, ys, gs, d_pre, dxs = new(d), new(n1) if act else None, new(inter), new(d), new(d), new(n1), new(d)
+        native.gather_rows(x, plan.row_src, plan.num_mtiles, xs, 1)
+        native.mgrouped_gemm(xs, w1, hidden, pre, *maps, False, act, plan.status)
+        native.mgrouped_gemm(hidden, w2, ys, None, *maps, False, None, plan.status)
+        d_scores = torch.empty_like(scores)
+        native.combine_bwd_tokens(grad, scores, ys, plan.dst_row, plan.row_src, plan.num_mtiles, gs, d_scores, 1)
+        if act is None:
+            native.mgrouped_gemm(gs, w2, d_pre, None, *maps, True, None, plan.status)
+        else:
+            native.mgrouped_gemm_dglu(gs, w2, pre, d_pre, *maps, act, plan.status)
+        native.mgrouped_gemm(d_pre, w1, dxs, None, *maps, True, None, plan.status)
+        ref, dx, dw1, dw2 = torch.empty_like(x), torch.empty_like(x), torch.empty_like(w1), torch.empty_like(w2)
+        native.combine_topk(ys, scores, plan.dst_row, ref, 1)
+        native.combine_topk(dxs, None, plan.dst_row, dx, 1)
+        native.kgrouped_gemm(xs, d_pre, dw1, plan.pad_offsets, plan.status)
+        native.kgrouped_gemm(hidden, gs, dw2, plan.pad_offsets, plan.status)
+    for a, b in zip(got, (ref, dx, d_scores, dw1, dw2)):
+        assert torch.equal(a, b)
+    assert native.read_status(plan.status) == 0
