@@ -6,7 +6,7 @@
 namespace moe {
 #define MOE_INST(BN, A_K, B_K, EPI, KG) \
   template int launch<__nv_bfloat16, BN, A_K, B_K, EPI, KG, 1, true>(const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, \
-                                                        const CUtensorMap&, GemmArgs, const LaunchParams&);
+                                                        const CUtensorMap&, GemmArgs, const LaunchParams&, const ShortStepsOf<KG>::type&);
 #define MOE_INST_BN(BN)                        \
   MOE_INST(BN, true, false, EPI_ACT, false)     \
   MOE_INST(BN, true, false, EPI_GLU, false)     \

@@ -9,7 +9,7 @@ namespace moe {
 #define MOE_EXTERN(T, CTAS, BN, A_K, B_K, EPI, KG, GATHER)                                                       \
   extern template int launch<T, BN, A_K, B_K, EPI, KG, CTAS, GATHER>(const CUtensorMap&, const CUtensorMap&,       \
                                                                      const CUtensorMap&, const CUtensorMap&, GemmArgs, \
-                                                                     const LaunchParams&);
+                                                                     const LaunchParams&, const ShortStepsOf<KG>::type&);
 // every variant without the row gather; with it, the variants the gathering entry points reach
 #define MOE_EXTERN_BN(T, CTAS, BN)                                \
   MOE_EXTERN(T, CTAS, BN, true, false, EPI_ACT, false, false)     \
@@ -467,34 +467,36 @@ static int mgrouped_common(const char* name, const void* a, const void* w, void*
 template <typename T, int BN, int CTAS>
 static int kgrouped_dispatch(const void* a, const void* b, int64_t a_rows, int64_t b_rows, int M, int N,
                              const GemmArgs& args, int dtype, const LaunchParams& lp) {
+  // operands in boxes of BK contracted rows, and of 16 and 32 for an expert's last step (without routed counts there is none)
   CUtensorMap ta, tb;
-  if (args.a_blocked) {
-    int rc = make_tmap_blocked(&ta, dtype, a, (uint64_t)a_rows, (uint64_t)M, 0, BK, BM / 64);
-    if (rc != MOE_OK) return rc;
-  } else {
-    const uint64_t dims[2] = {(uint64_t)M, (uint64_t)a_rows};
-    const uint32_t box[2] = {64, args.a_row_src != nullptr ? 1u : (uint32_t)BK};
-    int rc = make_tmap(&ta, dtype, a, 2, dims, box);
-    if (rc != MOE_OK) return rc;
+  ShortSteps small;
+  const auto operand = [&](CUtensorMap* map, const void* p, bool blocked, int64_t rows, int cols, int block_cols, uint32_t depth) {
+    if (blocked) return make_tmap_blocked(map, dtype, p, (uint64_t)rows, (uint64_t)cols, 0, depth, (uint32_t)(block_cols / 64));
+    const uint64_t dims[2] = {(uint64_t)cols, (uint64_t)rows};
+    const uint32_t box[2] = {64, depth};
+    return make_tmap(map, dtype, p, 2, dims, box);
+  };
+  const bool gather = args.a_row_src != nullptr;
+  const bool short_steps = args.short_steps != 0;
+  int rc = operand(&ta, a, args.a_blocked, a_rows, M, BM, gather ? 1 : BK);
+  if (rc == MOE_OK) rc = operand(&tb, b, args.b_blocked, b_rows, N, BN / CTAS, BK);
+  for (int i = 0; i < 2 && rc == MOE_OK; ++i) {
+    small.a[i] = ta;
+    small.b[i] = tb;
+    if (!short_steps) continue;
+    rc = operand(&small.a[i], a, args.a_blocked, a_rows, M, BM, 16 << i);
+    if (rc == MOE_OK) rc = operand(&small.b[i], b, args.b_blocked, b_rows, N, BN / CTAS, 16 << i);
   }
-  if (args.b_blocked) {
-    int rc = make_tmap_blocked(&tb, dtype, b, (uint64_t)b_rows, (uint64_t)N, 0, BK, (uint32_t)(BN / CTAS / 64));
-    if (rc != MOE_OK) return rc;
-  } else {
-    const uint64_t dims[2] = {(uint64_t)N, (uint64_t)b_rows};
-    const uint32_t box[2] = {64, BK};
-    int rc = make_tmap(&tb, dtype, b, 2, dims, box);
-    if (rc != MOE_OK) return rc;
-  }
+  if (rc != MOE_OK) return rc;
   CUtensorMap td = ta;
   if (args.out_tma) {
     const uint64_t dims[3] = {(uint64_t)N, (uint64_t)M, (uint64_t)args.num_experts};
     const uint32_t box[3] = {64, 32, 1};
-    int rc = make_tmap(&td, dtype, args.out, 3, dims, box);
+    rc = make_tmap(&td, dtype, args.out, 3, dims, box);
     if (rc != MOE_OK) return rc;
   }
-  return args.a_row_src != nullptr ? launch<T, BN, false, false, EPI_ACT, true, CTAS, true>(ta, tb, ta, td, args, lp)
-                                   : launch<T, BN, false, false, EPI_ACT, true, CTAS, false>(ta, tb, ta, td, args, lp);
+  return gather ? launch<T, BN, false, false, EPI_ACT, true, CTAS, true>(ta, tb, ta, td, args, lp, small)
+                                   : launch<T, BN, false, false, EPI_ACT, true, CTAS, false>(ta, tb, ta, td, args, lp, small);
 }
 
 static int kgrouped_common(const char* name, const void* a, int64_t gather_rows, const int32_t* gather_row_src,
@@ -540,6 +542,8 @@ static int kgrouped_common(const char* name, const void* a, int64_t gather_rows,
   // expert, DeepSeek-V3 shape: weight1 gradient 4.00 -> 3.48 ms; at 128 rows per expert pairs are 9 % faster)
   const long long mean_rows_per_expert = (padded_rows - static_cast<long long>(num_experts) * (BM - 1)) / num_experts;
   const bool pairs = o.single_cta == 0 ? mean_rows_per_expert > 64 : o.single_cta < 0;
+  // (above four steps an eighth of the loads at most is saved, for four more tensor maps per call)
+  args.short_steps = counts.group_indices != nullptr && gather_row_src == nullptr && mean_rows_per_expert <= 4 * BK ? 1 : 0;
   const int64_t a_rows = gather_row_src != nullptr ? gather_rows : (counts.a_rows >= 0 ? counts.a_rows : padded_rows);
   const int64_t b_rows = counts.b_rows >= 0 ? counts.b_rows : padded_rows;
 #define MOE_KG(TYPE)                                                                                      \
