@@ -46,7 +46,7 @@ extern "C" {
 
 #define MOE_DTYPE_BF16 0
 #define MOE_DTYPE_F16 1
-#define MOE_DTYPE_F32 2 /* accepted by moe_router_topk only */
+#define MOE_DTYPE_F32 2 /* accepted by moe_router_topk and moe_router_tail only */
 
 #define MOE_ACT_NONE 0
 #define MOE_ACT_SILU 1
@@ -95,6 +95,12 @@ int64_t moe_mtiles_bound(int64_t num_rows, int num_experts);
 int moe_router_topk(const void* logits, void* scores, int64_t* indices, int32_t* expert_counts,
                     int64_t num_tokens, int num_experts, int topk, int softmax_before_topk,
                     int normalize, int dtype, void* stream);
+
+/* The same with torch's choices instead of a tie rule of its own: what softmax(dtype=float32), torch.topk(sorted=False),
+ * softmax and division by the sum leave, bit for bit -- larger values in ascending expert index, then values equal to the
+ * k-th in ascending index, NaN above all.  E <= 1024, k <= min(32, E). */
+int moe_router_tail(const void* logits, void* scores, int64_t* indices, int64_t num_tokens, int num_experts, int topk,
+                    int softmax_before_topk, int normalize, int dtype, void* stream);
 
 /* ---------------------------------------------------------------------------------
  * (a) Routing metadata.  Replaces get_token_indices (src/moe_explore/expert_permute.py:19-41):

@@ -173,6 +173,156 @@ extern "C" int moe_router_topk(const void* logits, void* scores, int64_t* indice
 
 namespace moe {
 
+// The router tail with torch's choices: what softmax, torch.topk(sorted=False), softmax, division by the sum and the cast leave,
+// in one launch instead of four to seven (one of which, the radix selection, takes 18-44 us for 3000 to 16384 tokens).  A warp
+// per token.
+//   * Selection: keys order as the bits do (-0 below +0, NaN above all); the k-th largest key by rounds of redux.sync over what is
+//     below the last one; then, as torch writes them, the larger keys in ascending expert index, then keys equal to the k-th in
+//     ascending index until k are there.
+//   * Arithmetic: the fp32 operations of those launches in their order (a lane's elements 32 apart one by one, then a butterfly,
+//     far lanes first), so scores are the same bits.
+// 16384 tokens x 60 experts, four launches of 48 us -> 7.8; 3001 x 128, six of 36 -> 5.0; one token, four of 9.6 -> 2.1.
+__device__ __forceinline__ uint32_t order_key(float f) {
+  const uint32_t u = __float_as_uint(f);
+  return f != f ? 0xFFFFFFFFu : u ^ ((u >> 31) ? 0xFFFFFFFFu : 0x80000000u);
+}
+
+template <typename T, int PER_LANE>
+__global__ void __launch_bounds__(kRouterWarps * 32)
+router_tail_kernel(const T* __restrict__ logits, T* __restrict__ scores, int64_t* __restrict__ indices, int64_t num_tokens, int E,
+                   int topk, int softmax_before, int normalize) {
+  __shared__ float sh_val[kRouterWarps][32];
+  __shared__ int sh_idx[kRouterWarps][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t t = static_cast<int64_t>(blockIdx.x) * kRouterWarps + warp;
+  if (t >= num_tokens) return;
+  const T* row = logits + t * E;
+  float v[PER_LANE];  // expert i * 32 + lane
+#pragma unroll
+  for (int i = 0; i < PER_LANE; ++i) {
+    const int e = i * 32 + lane;
+    v[i] = e < E ? load_logit<T>(row + e) : -CUDART_INF_F;
+  }
+  if (softmax_before) {
+    float top = v[0];
+#pragma unroll
+    for (int i = 1; i < PER_LANE; ++i) top = top > v[i] ? top : v[i];
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+      const float o = __shfl_xor_sync(0xFFFFFFFFu, top, off);
+      top = top < o ? o : top;
+    }
+    float sum = 0.0f;
+#pragma unroll
+    for (int i = 0; i < PER_LANE; ++i) {
+      v[i] = expf(v[i] - top);
+      sum += v[i];
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, off);
+#pragma unroll
+    for (int i = 0; i < PER_LANE; ++i) v[i] = v[i] / sum;
+  }
+  uint32_t key[PER_LANE];  // 0: no expert (every expert's key is larger)
+#pragma unroll
+  for (int i = 0; i < PER_LANE; ++i) key[i] = i * 32 + lane < E ? order_key(v[i]) : 0u;
+  uint32_t kth = 0;
+  for (int left = topk, first = 1; left > 0; first = 0) {
+    uint32_t best = 0;
+#pragma unroll
+    for (int i = 0; i < PER_LANE; ++i)
+      if (first || key[i] < kth) best = key[i] > best ? key[i] : best;
+    kth = __reduce_max_sync(0xFFFFFFFFu, best);
+#pragma unroll
+    for (int i = 0; i < PER_LANE; ++i) left -= __popc(__ballot_sync(0xFFFFFFFFu, key[i] == kth));
+  }
+  int place = 0;
+#pragma unroll
+  for (int pass = 0; pass < 2; ++pass) {
+#pragma unroll
+    for (int i = 0; i < PER_LANE; ++i) {
+      const bool take = pass == 0 ? key[i] > kth : key[i] == kth;
+      const unsigned all = __ballot_sync(0xFFFFFFFFu, take);
+      const int at = place + __popc(all & ((1u << lane) - 1));
+      if (take && at < topk) {
+        sh_val[warp][at] = v[i];
+        sh_idx[warp][at] = i * 32 + lane;
+      }
+      place += __popc(all);
+    }
+  }
+  __syncwarp();
+  const bool mine = lane < topk;
+  float s = mine ? sh_val[warp][lane] : -CUDART_INF_F;
+  if (!softmax_before) {
+    float top = s;
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+      const float o = __shfl_xor_sync(0xFFFFFFFFu, top, off);
+      top = top < o ? o : top;
+    }
+    s = mine ? expf(s - top) : 0.0f;
+    float sum = s;
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, off);
+    s = s / sum;
+  }
+  if (normalize) {
+    float sum = mine ? s : 0.0f;
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, off);
+    s = s / sum;
+  }
+  if (mine) {
+    store_score<T>(scores + t * topk + lane, s);
+    indices[t * topk + lane] = sh_idx[warp][lane];
+  }
+}
+
+template <typename T>
+static int launch_router_tail(const void* logits, void* scores, int64_t* indices, int64_t num_tokens, int E, int topk,
+                              int softmax_before, int normalize, cudaStream_t s) {
+  const int blocks = static_cast<int>((num_tokens + kRouterWarps - 1) / kRouterWarps);
+  const T* l = static_cast<const T*>(logits);
+  T* sc = static_cast<T*>(scores);
+#define MOE_TAIL(PL) \
+  router_tail_kernel<T, PL><<<blocks, kRouterWarps * 32, 0, s>>>(l, sc, indices, num_tokens, E, topk, softmax_before, normalize)
+  if (E <= 32) MOE_TAIL(1);
+  else if (E <= 64) MOE_TAIL(2);
+  else if (E <= 128) MOE_TAIL(4);
+  else if (E <= 256) MOE_TAIL(8);
+  else if (E <= 512) MOE_TAIL(16);
+  else MOE_TAIL(32);
+#undef MOE_TAIL
+  MOE_CUDA(cudaGetLastError());
+  return MOE_OK;
+}
+
+}  // namespace moe
+
+extern "C" int moe_router_tail(const void* logits, void* scores, int64_t* indices, int64_t num_tokens, int num_experts, int topk,
+                               int softmax_before_topk, int normalize, int dtype, void* stream) {
+  MOE_CHECK_ARG(num_tokens >= 0 && num_experts > 0 && topk > 0, "moe_router_tail: bad sizes T=%lld E=%d k=%d",
+                (long long)num_tokens, num_experts, topk);
+  if (num_experts > 32 * kRouterMaxPerLane || topk > 32 || topk > num_experts || num_tokens > (1ll << 33)) {
+    set_error("moe_router_tail: supports E <= %d and k <= min(32, E); got E=%d k=%d", 32 * kRouterMaxPerLane, num_experts, topk);
+    return MOE_ERR_UNSUPPORTED;
+  }
+  if (num_tokens == 0) return MOE_OK;
+  MOE_CHECK_ARG(logits && scores && indices, "moe_router_tail: null pointer argument");
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (dtype == MOE_DTYPE_BF16)
+    return launch_router_tail<__nv_bfloat16>(logits, scores, indices, num_tokens, num_experts, topk, softmax_before_topk, normalize, s);
+  if (dtype == MOE_DTYPE_F16)
+    return launch_router_tail<__half>(logits, scores, indices, num_tokens, num_experts, topk, softmax_before_topk, normalize, s);
+  if (dtype == MOE_DTYPE_F32)
+    return launch_router_tail<float>(logits, scores, indices, num_tokens, num_experts, topk, softmax_before_topk, normalize, s);
+  set_error("moe_router_tail: unknown dtype %d", dtype);
+  return MOE_ERR_INVALID;
+}
+
+namespace moe {
+
 // Backward of the router tail "softmax over the topk selected logits (, renormalised: the same gradient, the softmax sums to
 // one)" in one launch: a warp per token recomputes the probabilities p from the logits and leaves
 //   dl[t, s] = p_s (d_s - sum_j p_j d_j)   in fp32, and the dense row of it in the 16-bit type (what the router-weight

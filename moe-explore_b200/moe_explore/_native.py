@@ -74,6 +74,7 @@ SIGNATURES = {
     "moe_routing_metadata_static": (c_int, [c_void_p, c_int64, c_int] + [c_void_p] * 9 + [c_void_p]),
     "moe_layout_from_groups": (c_int, [c_void_p, c_int64, c_int] + [c_void_p] * 7 + [c_void_p]),
     "moe_router_topk": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int, c_int, c_int, c_int, c_void_p]),
+    "moe_router_tail": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int, c_int, c_int, c_int, c_void_p]),
     "moe_store_to_host": (c_int, [c_void_p, c_void_p, c_size_t, c_void_p]),
     "moe_copy_blocks": (c_int, [POINTER(c_void_p), POINTER(c_void_p), POINTER(c_size_t), c_int, c_void_p]),
     "moe_zero_padding_rows": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int, c_void_p]),
@@ -342,6 +343,23 @@ def router_topk(logits, topk: int, softmax_before_topk: bool, normalize: bool, w
     _check("moe_router_topk", rc)
     _count(1)
     return scores, indices, counts
+
+
+ROUTER_TAIL_EXPERTS, ROUTER_TAIL_TOPK = 1024, 32
+
+
+def router_tail(logits, topk: int, softmax_before_topk: bool, normalize: bool):
+    """Scores [T, k] in the logits' type and indices int64 [T, k] as torch's launches leave them (see moe_router_tail)."""
+    T, E = logits.shape
+    scores = torch.empty(T, topk, dtype=logits.dtype, device=logits.device)
+    indices = torch.empty(T, topk, dtype=torch.int64, device=logits.device)
+    with timed("router:topk"):
+        rc = load().moe_router_tail(logits.data_ptr(), scores.data_ptr(), indices.data_ptr(), T, E, topk,
+                                    1 if softmax_before_topk else 0, 1 if normalize else 0,
+                                    2 if logits.dtype is torch.float32 else dtype_code(logits.dtype), _stream())
+    _check("moe_router_tail", rc)
+    _count(1)
+    return scores, indices
 
 
 _PINNED = {}

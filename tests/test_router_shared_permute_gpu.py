@@ -133,3 +133,53 @@ def test_expert_input_and_output_permute(native):
     # every token's k copies of its own row, weighted: x[t] * sum_s scores[t, s] (fp32 fold, one rounding)
     expect = (x.float() * scores.float().sum(-1, keepdim=True))
     assert back.shape == x.shape and relerr(back, expect) <= 1e-2
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("softmax_before,normalize", [(False, False), (False, True), (True, False), (True, True)])
+@pytest.mark.parametrize("T,E,k", [(1, 8, 1), (7, 8, 8), (3, 31, 5), (300, 33, 2), (513, 60, 4), (1000, 64, 8), (65, 100, 6),
+                                   (2048, 128, 7), (70, 257, 9), (33, 1024, 32), (5, 600, 31), (9, 20, 13)])
+def test_router_tail_leaves_the_bits_of_the_torch_ops(T, E, k, softmax_before, normalize, dtype, native):
+    """Scores and indices against the launches the kernel stands for, among ties (every third row is a few distinct values),
+    signed zeros, infinities and NaN."""
+    from moe_explore.params import TopkRouterParams
+    from moe_explore.router import topk_of_logits
+
+    g = torch.Generator(device="cuda").manual_seed(T + E)
+    logits = torch.randn(T, E, generator=g, device="cuda") * 2
+    logits[::3] = (logits[::3] * 0.7).round()
+    if T > 6:
+        logits[1, ::2], logits[1, 1::2] = 0.0, -0.0
+        logits[2, E // 2] = float("nan")
+        logits[3, :2] = float("inf")
+        logits[4, 1:] = float("-inf")
+        logits[5] = float("-inf")
+    logits = logits.to(dtype)
+    p = TopkRouterParams(None, k, softmax_before, normalize)
+    seen = []
+    real, native.router_tail = native.router_tail, lambda *a: seen.append(1) or real(*a)
+    try:
+        scores, idx = topk_of_logits(logits, p, dtype)
+    finally:
+        native.router_tail = real
+    ref_s, ref_i = topk_of_logits(logits.clone().requires_grad_(), p, dtype)     # a gradient wanted: the single ops
+    assert len(seen) == 1 and ref_s.requires_grad
+    assert torch.equal(idx, ref_i) and scores.dtype is dtype
+    assert torch.equal(scores.nan_to_num(nan=-7.0), ref_s.detach().nan_to_num(nan=-7.0))
+
+
+def test_router_tail_leaves_transforms_to_the_single_ops(native):
+    from moe_explore.params import TopkRouterParams
+    from moe_explore.router import topk_of_logits
+    import torch.autograd.forward_ad as fwd
+
+    p = TopkRouterParams(None, 2, True, True)
+    logits = torch.randn(4, 6, 8, device="cuda")
+    ref = torch.stack([topk_of_logits(row, p, torch.float32)[0] for row in logits])
+    assert torch.equal(torch.func.vmap(lambda row: topk_of_logits(row, p, torch.float32)[0])(logits), ref)
+    with fwd.dual_level():
+        out, _ = topk_of_logits(fwd.make_dual(logits[0], torch.ones_like(logits[0])), p, torch.float32)
+        assert fwd.unpack_dual(out).tangent is not None
+    with torch.no_grad():
+        out, _ = topk_of_logits(logits[0].t().contiguous().t(), p, torch.float32)      # other strides: the single ops
+        assert torch.equal(out, ref[0])
