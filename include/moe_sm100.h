@@ -454,6 +454,7 @@ typedef struct moe_expert_pass {
   const void *logits, *router_w;
   float* dl;
   void *dlogits, *router_t;
+  int32_t softmax_before_topk, normalize; /* MOE_FWD_TAIL */
 } moe_expert_pass;
 
 /* sizeof(moe_expert_pass), for bindings that declare the struct themselves. */
@@ -465,6 +466,7 @@ size_t moe_expert_pass_size(void);
 #define MOE_FWD_DOWN 8
 #define MOE_FWD_FOLD 16
 #define MOE_FWD_ALL 31
+#define MOE_FWD_TAIL 32 /* first: moe_router_tail of `logits` into `scores` and `expert_idx` */
 int moe_expert_forward(const moe_expert_pass* pass, int steps, void* stream);
 
 #define MOE_BWD_FOLD 1    /* gs, d_scores */

@@ -45,7 +45,8 @@ class ExpertPass(ctypes.Structure):
                                         "dst_row", "mtile_expert", "tile_pairs", "num_mtiles", "status", "workspace")] + \
                [("workspace_bytes", c_size_t)] + \
                [(f, c_void_p) for f in ("xs", "pre_act", "hidden", "ys", "out", "grad_out", "gs", "d_scores", "d_pre", "dxs", "dx",
-                                        "d_w1", "d_w2", "addend", "logits", "router_w", "dl", "dlogits", "router_t")]
+                                        "d_w1", "d_w2", "addend", "logits", "router_w", "dl", "dlogits", "router_t")] + \
+               [(f, c_int32) for f in ("softmax_before_topk", "normalize")]
 
 
 class RowsPass(ctypes.Structure):
@@ -250,7 +251,7 @@ def _opt(options):
 
 
 ROWS_LAYOUT, ROWS_GATHER, ROWS_GEMM = 1, 2, 4
-FWD_ROUTE, FWD_DISPATCH, FWD_UP, FWD_DOWN, FWD_FOLD = 1, 2, 4, 8, 16
+FWD_ROUTE, FWD_DISPATCH, FWD_UP, FWD_DOWN, FWD_FOLD, FWD_TAIL = 1, 2, 4, 8, 16, 32
 BWD_FOLD, BWD_DOWN, BWD_UP, BWD_FOLD_DX, BWD_DW1, BWD_DW2, BWD_ROUTER = 1, 2, 4, 8, 16, 32, 64
 
 

@@ -13,12 +13,14 @@ it has no backward.  The gradients follow from out[t] = sum_s score[t,s] * (act(
 """
 from __future__ import annotations
 
+import functools
+
 import torch
 
 from moe_explore import _native
 from moe_explore.functional.activation import is_glu
 from moe_explore.params import TopkRouterParams
-from moe_explore.router import topk_of_logits
+from moe_explore.router import nothing_watches, tail_in_one_kernel, topk_of_logits
 from moe_explore.routing_plan import RoutingPlan, device_status, packed_layout
 
 
@@ -27,19 +29,56 @@ def _plan_pointers(plan: RoutingPlan):
                                         plan.tile_pairs, plan.num_mtiles, plan.status))
 
 
-def _packed_pointers(words: torch.Tensor, offsets, status: torch.Tensor):
-    base = words.data_ptr()
+def _packed_pointers(base: int, offsets, status: torch.Tensor):
     return tuple(base + o for o in offsets) + (status.data_ptr(),)
 
 
 class _Pass:
     """What the backward pass needs to know about its forward pass besides the saved tensors."""
-    __slots__ = ("sizes", "routing", "act", "gathered")
+    __slots__ = ("sizes", "routing", "act", "gathered", "scratch", "tail")
 
 
-def _forward(x, scores, weight1, weight2, routing, act, gather_in_gemm: bool, fused_combine: bool, needs_grad: bool, addend=None):
-    """-> (out, _Pass, tensors to save)."""
-    _native.require_cuda(x, scores, weight1, weight2)
+# Up to here the buffers of a pass are cut from one allocation, above each is one of its own.  An allocation costs the host 1.7 us
+# and a pass had seven to twelve: with the router's tail in the same library call, one token takes 88 -> 58 us (the host is what
+# it waits for), and the host issues a training pass of 64 MB (1777 tokens x 3 slots, 12 experts of 776 x 1544) in 250 us instead of
+# 300.  Larger passes wait for the GPU, and one large block is harder to place than several.
+SCRATCH_IN_ONE = 256 << 20
+
+
+@functools.lru_cache(maxsize=256)
+def _cuts(sizes):
+    offsets, total = [], 0
+    for n in sizes:
+        offsets.append(total)
+        total += (n + 255) // 256 * 256
+    return tuple(offsets), total
+
+
+def _buffers(sizes, device):
+    """(tensors, addresses) of buffers of these many bytes (0: none, address None)."""
+    offsets, total = _cuts(sizes)
+    if total <= SCRATCH_IN_ONE:
+        block = torch.empty(total, dtype=torch.uint8, device=device)
+        tensors = (block,)
+    else:
+        tensors = tuple(torch.empty(n, dtype=torch.uint8, device=device) for n in sizes if n)
+    return tensors, _addresses(sizes, tensors)
+
+
+def _addresses(sizes, tensors):
+    offsets, total = _cuts(sizes)
+    if total <= SCRATCH_IN_ONE:
+        base = tensors[0].data_ptr()
+        return [base + o if n else None for o, n in zip(offsets, sizes)]
+    rest = iter(tensors)
+    return [next(rest).data_ptr() if n else None for n in sizes]
+
+
+def _forward(x, scores, weight1, weight2, routing, act, gather_in_gemm: bool, fused_combine: bool, needs_grad: bool, addend=None,
+             tail=None):
+    """-> (out, _Pass, tensors to save).  ``tail`` = (logits, softmax before top-k, normalize): scores and expert indices are the
+    router's tail of these logits, taken as part of the pass (``scores`` and the indices of ``routing`` are then None)."""
+    _native.require_cuda(x, weight1, weight2)
     assert x.dim() == 2 and weight1.dim() == 3 and weight2.dim() == 3
     T, d = x.shape
     E, d1, n1 = weight1.shape
@@ -47,45 +86,51 @@ def _forward(x, scores, weight1, weight2, routing, act, gather_in_gemm: bool, fu
     assert d1 == d and weight2.size(0) == E and weight2.size(2) == d, "weight shapes do not match the input"
     assert n1 == (2 * inter if is_glu(act) else inter), "weight1 width does not match weight2 and the activation"
     planned = isinstance(routing, RoutingPlan)
+    flat = None
     if planned:
         topk = routing.topk
         assert routing.num_rows == T * topk and routing.num_experts == E
     else:
         indices, num_experts, topk = routing
-        flat = indices.reshape(-1).contiguous()
-        assert flat.numel() == T * topk and num_experts == E
+        assert num_experts == E
+        if tail is None:
+            flat = indices.reshape(-1).contiguous()
+            assert flat.numel() == T * topk
+        else:
+            assert tail[0].shape == (T, E) and tail[0].dtype is x.dtype and tail[0].is_contiguous()
     x = x.contiguous()
-    scores = scores.to(x.dtype).contiguous()
+    if tail is None:
+        _native.require_cuda(scores)
+        scores = scores.to(x.dtype).contiguous()
     weight1 = weight1.contiguous()
     weight2 = weight2.contiguous()
     code = _native.dtype_code(x.dtype)
     act_code = _native.ACT_CODES[act]
     rows = T * topk
-    new = lambda *shape: torch.empty(shape, dtype=x.dtype, device=x.device)
     fold = not fused_combine or needs_grad   # the backward pass needs the per-slot rows for the router-weight gradient
 
     steps = []
-    words = workspace = None
+    workspace = None
     if planned:
-        rp = routing.padded_rows
-        ids = None
-        plan_ptrs = _plan_pointers(routing)
+        rp, num_words = routing.padded_rows, 0
     else:
         rp, offsets, num_words = packed_layout(rows, E)
-        words = torch.empty(num_words, dtype=torch.int32, device=x.device)
-        status = device_status(x.get_device())
-        plan_ptrs = _packed_pointers(words, offsets, status)
-        ids = flat.data_ptr()
         launches = _native.routing_launches(rows, E)
         if launches > 1:
             workspace = torch.empty(max(_native.routing_workspace_bytes(rows, E), 16), dtype=torch.uint8, device=x.device)
+        if tail is not None:
+            steps.append((_native.FWD_TAIL, "router:topk", 1))
         steps.append((_native.FWD_ROUTE, "routing", launches))
-    xs = None if gather_in_gemm else new(rp, d)
-    # the un-activated product, needed by the backward pass (not kept for inference or without an activation)
-    pre_act = new(rp, n1) if (act is not None and needs_grad) else None
-    hidden = new(rp, inter)
-    ys = new(rp, d) if fold else None
-    out = new(T, d)
+    # index arrays, scores and indices of the tail, expert-sorted input, un-activated product (needed by the backward pass; not
+    # kept for inference or without an activation), activated product, per-slot rows
+    scratch = (4 * num_words, 2 * rows if tail else 0, 8 * rows if tail else 0, 0 if gather_in_gemm else 2 * rp * d,
+               2 * rp * n1 if act is not None and needs_grad else 0, 2 * rp * inter, 2 * rp * d if fold else 0)
+    buffers, (words, tail_scores, tail_ids, xs, pre_act, hidden, ys) = _buffers(scratch, x.device)
+    if planned:
+        plan_ptrs = _plan_pointers(routing)
+    else:
+        plan_ptrs = _packed_pointers(words, offsets, device_status(x.get_device()))
+    out = torch.empty(T, d, dtype=x.dtype, device=x.device)
     kind = "glu" if is_glu(act) else "plain"
     if not gather_in_gemm:
         steps.append((_native.FWD_DISPATCH, "rows:gather", 1))
@@ -99,11 +144,14 @@ def _forward(x, scores, weight1, weight2, routing, act, gather_in_gemm: bool, fu
         assert fold and addend.shape == out.shape and addend.dtype is out.dtype and addend.is_cuda
         addend = addend.contiguous()
     ptr = _native._ptr
+    ids = tail_ids if tail is not None else ptr(flat)
     p = _native.ExpertPass(
-        T, rp, d, inter, E, topk, act_code, code, gather_in_gemm, not fold, needs_grad, 0, ids, x.data_ptr(), scores.data_ptr(),
-        weight1.data_ptr(), weight2.data_ptr(), *plan_ptrs, ptr(workspace),
-        0 if workspace is None else workspace.numel(), ptr(xs), ptr(pre_act), hidden.data_ptr(), ptr(ys), out.data_ptr())
+        T, rp, d, inter, E, topk, act_code, code, gather_in_gemm, not fold, needs_grad, 0, ids, x.data_ptr(),
+        tail_scores if tail is not None else scores.data_ptr(), weight1.data_ptr(), weight2.data_ptr(), *plan_ptrs, ptr(workspace),
+        0 if workspace is None else workspace.numel(), xs, pre_act, hidden, ys, out.data_ptr())
     p.addend = ptr(addend)
+    if tail is not None:
+        p.logits, p.softmax_before_topk, p.normalize = tail[0].data_ptr(), bool(tail[1]), bool(tail[2])
     _native.run_pass("moe_expert_forward", p, steps, rows)
     if not needs_grad:
         return out, None, ()
@@ -112,31 +160,38 @@ def _forward(x, scores, weight1, weight2, routing, act, gather_in_gemm: bool, fu
     info.routing = routing if planned else None
     info.act = act
     info.gathered = bool(gather_in_gemm)
-    return out, info, (x if gather_in_gemm else xs, pre_act, hidden, ys, scores, weight1, weight2, words)
+    info.scratch = scratch
+    info.tail = tail is not None
+    return out, info, (x if gather_in_gemm else None, scores, weight1, weight2, *buffers)
 
 
 def _backward(info: _Pass, saved, grad_out, router=None):
-    """-> (dx, d_scores, d_w1, d_w2[, dlogits]); ``router`` = (logits, router weight, expert indices) makes the router's tail and
-    its share of dx part of the pass."""
-    xs, pre_act, hidden, ys, scores, weight1, weight2, words = saved
+    """-> (dx, d_scores, d_w1, d_w2[, dlogits]); ``router`` = (logits, router weight, expert indices or None where the pass took
+    the router's tail) makes the router's tail and its share of dx part of the pass."""
+    x, scores, weight1, weight2, *buffers = saved
     T, d, inter, E, topk, rp, n1 = info.sizes
     act = info.act
     rows = T * topk
     grad_out = grad_out.contiguous()
+    words, tail_scores, tail_ids, xs, pre_act, hidden, ys = _addresses(info.scratch, buffers)
     new = lambda *shape: torch.empty(shape, dtype=grad_out.dtype, device=grad_out.device)
 
-    gs, d_scores, d_pre, dxs, dx = new(rp, d), new(T, topk), new(rp, n1), new(rp, d), new(T, d)
+    # score-scaled dOut rows, gradient of the un-activated product, per-slot rows of dX; with a router the gradient of the selected
+    # logits in fp32 and the transposed router weight
+    scratch = (2 * rp * d, 2 * rp * n1, 2 * rp * d) + ((4 * rows, 2 * E * d) if router is not None else (0, 0))
+    held, (gs, d_pre, dxs, dl, router_t) = _buffers(scratch, grad_out.device)
+    d_scores, dx = new(T, topk), new(T, d)
     d_w1, d_w2 = torch.empty_like(weight1), torch.empty_like(weight2)
     if info.routing is not None:
         plan_ptrs = _plan_pointers(info.routing)
     else:
-        plan_ptrs = _packed_pointers(words, packed_layout(rows, E)[1], device_status(words.get_device()))
-    ptr = _native._ptr
+        plan_ptrs = _packed_pointers(words, packed_layout(rows, E)[1], device_status(grad_out.get_device()))
+    rows_in = x.data_ptr() if info.gathered else xs
     p = _native.ExpertPass(
         T, rp, d, inter, E, topk, _native.ACT_CODES[act], _native.dtype_code(grad_out.dtype), info.gathered, False, True, 0, None,
-        xs.data_ptr(), scores.data_ptr(), weight1.data_ptr(), weight2.data_ptr(), *plan_ptrs, None, 0, xs.data_ptr(),
-        ptr(pre_act), hidden.data_ptr(), ys.data_ptr(), None, grad_out.data_ptr(), gs.data_ptr(), d_scores.data_ptr(),
-        d_pre.data_ptr(), dxs.data_ptr(), dx.data_ptr(), d_w1.data_ptr(), d_w2.data_ptr())
+        rows_in, tail_scores if info.tail else scores.data_ptr(), weight1.data_ptr(), weight2.data_ptr(), *plan_ptrs, None, 0,
+        rows_in, pre_act, hidden, ys, None, grad_out.data_ptr(), gs, d_scores.data_ptr(), d_pre, dxs, dx.data_ptr(),
+        d_w1.data_ptr(), d_w2.data_ptr())
     steps = [(_native.BWD_FOLD, "rows:combine_bwd", 1),
              (_native.BWD_DOWN, "mgrouped_gemm:wt" if act is None else "mgrouped_gemm:dglu", 1),
              (_native.BWD_UP, "mgrouped_gemm:wt", 1), (_native.BWD_FOLD_DX, "rows:combine", 1),
@@ -145,10 +200,10 @@ def _backward(info: _Pass, saved, grad_out, router=None):
     dlogits = None
     if router is not None:
         logits, router_weight, indices = router
-        dl = torch.empty(T, topk, dtype=torch.float32, device=grad_out.device)
-        dlogits, router_t = new(T, (E + 7) // 8 * 8), new(E, d)
-        p.logits, p.router_w, p.expert_idx = logits.data_ptr(), router_weight.data_ptr(), indices.data_ptr()
-        p.dl, p.dlogits, p.router_t = dl.data_ptr(), dlogits.data_ptr(), router_t.data_ptr()
+        dlogits = new(T, (E + 7) // 8 * 8)
+        p.logits, p.router_w = logits.data_ptr(), router_weight.data_ptr()
+        p.expert_idx = tail_ids if indices is None else indices.data_ptr()
+        p.dl, p.dlogits, p.router_t = dl, dlogits.data_ptr(), router_t
         steps.insert(1, (_native.BWD_ROUTER, "router:bwd", 1))
     _native.run_pass("moe_expert_backward", p, steps, rows)
     return dx, d_scores, d_w1, d_w2, dlogits
@@ -182,10 +237,14 @@ class RoutedLayer(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, router_weight, weight1, weight2, router_params, num_experts: int, act: str, gather_in_gemm: bool, addend):
         logits = x @ router_weight
-        scores, indices = topk_of_logits(logits, router_params, x.dtype)
-        indices = indices.contiguous()
+        if tail_in_one_kernel(logits, router_params, x.dtype):
+            scores = indices = None
+            tail = (logits, router_params.softmax_before_topk, router_params.normalize_routing)
+        else:
+            scores, indices = topk_of_logits(logits, router_params, x.dtype)
+            indices, tail = indices.contiguous(), None
         out, ctx.info, saved = _forward(x, scores, weight1, weight2, (indices, num_experts, router_params.topk), act,
-                                        gather_in_gemm, False, True, addend)
+                                        gather_in_gemm, False, True, addend, tail)
         ctx.save_for_backward(x, logits, router_weight, indices, *saved)
         return out
 
@@ -233,7 +292,7 @@ class DenseExpert(torch.autograd.Function):
 
     @staticmethod
     def _pass(x, weight1, weight2, act, words, groups, offsets, rp, keep):
-        group_ptr, *plan_ptrs = _packed_pointers(words, offsets, device_status(x.get_device()))
+        group_ptr, *plan_ptrs = _packed_pointers(words.data_ptr(), offsets, device_status(x.get_device()))
         return _native.ExpertPass(
             x.size(0), rp, x.size(1), weight2.size(1), 1, 1, _native.ACT_CODES[act], _native.dtype_code(x.dtype), 0, 0, keep, 1,
             None, x.data_ptr(), None, weight1.data_ptr(), weight2.data_ptr(), groups.data_ptr(), *plan_ptrs)
@@ -325,3 +384,35 @@ def routed_layer(x, router_params, weight1, weight2, num_experts: int, act, gath
         gather_in_gemm = GATHER_IN_GEMM_DEFAULT
     return RoutedLayer.apply(x, router_params.router_weight, weight1, weight2, router_params, num_experts,
                              None if act is None else str(act), bool(gather_in_gemm), addend)
+
+
+def router_and_experts_at_once(x, router_params, weight1, weight2, num_experts: int, topk: int, addend=None) -> bool:
+    """Whether ``inference_pass`` stands for router and experts: plain 16-bit CUDA tensors and nothing that has to see the single
+    steps (no gradient, no transform, no tracing, no mode)."""
+    if type(router_params) is not TopkRouterParams:
+        return False
+    tensors = (x, router_params.router_weight, weight1, weight2) + (() if addend is None else (addend,))
+    if not all(type(t) in _PLAIN and t.is_cuda for t in tensors):
+        return False
+    if torch.is_grad_enabled() and any(t.requires_grad for t in tensors):
+        return False
+    return (x.dtype in (torch.bfloat16, torch.float16) and x.dim() == 2 and x.size(0) > 0
+            and router_params.router_weight.dim() == 2 and router_params.router_weight.size(1) == num_experts
+            and router_params.topk == topk and nothing_watches(x))
+
+
+def inference_pass(x, router_params, weight1, weight2, num_experts: int, act, gather_in_gemm=None, fused_combine: bool = False,
+                   addend=None) -> torch.Tensor:
+    """Router and experts without gradients: one allocation besides the result and the logits, and one library call after the
+    logits' GEMM."""
+    if gather_in_gemm is None:
+        gather_in_gemm = GATHER_IN_GEMM_DEFAULT
+    logits = x @ router_params.router_weight
+    if tail_in_one_kernel(logits, router_params, x.dtype):
+        scores = indices = None
+        tail = (logits, router_params.softmax_before_topk, router_params.normalize_routing)
+    else:
+        scores, indices = topk_of_logits(logits, router_params, x.dtype)
+        tail = None
+    return _forward(x, scores, weight1, weight2, (indices, num_experts, router_params.topk), None if act is None else str(act),
+                    bool(gather_in_gemm), bool(fused_combine), False, addend, tail)[0]

@@ -10,7 +10,8 @@ from __future__ import annotations
 
 import torch
 
-from moe_explore.expert_compute import dense_expert, routed_expert_compute, routed_layer, router_joins_the_pass
+from moe_explore.expert_compute import (dense_expert, inference_pass, routed_expert_compute, routed_layer,
+                                        router_and_experts_at_once, router_joins_the_pass)
 from moe_explore.functional.activation import activation
 from moe_explore.params import MLPParams, MOEParams, TopkRouterParams
 from moe_explore.router import fused_topk_router, router
@@ -52,6 +53,10 @@ def topk_moe_forward(input: torch.Tensor, params: MOEParams, autotune_mode=None,
     if not fused_router and router_joins_the_pass(input, params.router_params, params.num_experts, params.topk):
         out = routed_layer(input, params.router_params, ep.weight1, ep.weight2, params.num_experts, ep.activation,
                            gather_in_gemm=gather_in_gemm, addend=addend)
+    elif not fused_router and router_and_experts_at_once(input, params.router_params, ep.weight1, ep.weight2, params.num_experts,
+                                                         params.topk, addend):
+        out = inference_pass(input, params.router_params, ep.weight1, ep.weight2, params.num_experts, ep.activation,
+                             gather_in_gemm=gather_in_gemm, fused_combine=fused_combine, addend=addend)
     else:
         if fused_router and isinstance(params.router_params, TopkRouterParams):
             scores, indices = fused_topk_router(input, params.router_params)

@@ -36,7 +36,7 @@ def topk_router(input: torch.Tensor, router_params: TopkRouterParams):
 
 def topk_of_logits(logits: torch.Tensor, router_params: TopkRouterParams, dtype: torch.dtype):
     """Everything of ``topk_router`` after the linear layer."""
-    if _tail_in_one_kernel(logits, router_params, dtype):
+    if tail_in_one_kernel(logits, router_params, dtype):
         return _native.router_tail(logits, router_params.topk, bool(router_params.softmax_before_topk),
                                    bool(router_params.normalize_routing))
     if router_params.softmax_before_topk:
@@ -49,19 +49,22 @@ def topk_of_logits(logits: torch.Tensor, router_params: TopkRouterParams, dtype:
     return scores.to(dtype), indices
 
 
-def _tail_in_one_kernel(logits: torch.Tensor, p: TopkRouterParams, dtype: torch.dtype) -> bool:
-    """Plain logits in the result's type on the current device, with nothing that has to see the single ops: no gradient, no
-    transform, no tracing, no mode.  (One token to 16384 x 60 experts: 2 to 8 us for what takes 10 to 48 in four to six
-    launches.)"""
+def nothing_watches(t: torch.Tensor) -> bool:
+    """No transform, tracer or mode has to see the single ops on ``t``, and it lies on the current device."""
+    return (forward_ad._current_level < 0 and not torch._C._functorch.is_functorch_wrapped_tensor(t)
+            and torch._C._len_torch_dispatch_stack() == 0 and torch._C._len_torch_function_stack() == 0
+            and not torch.compiler.is_compiling() and not torch.jit.is_tracing()
+            and t.get_device() == torch.cuda.current_device())
+
+
+def tail_in_one_kernel(logits: torch.Tensor, p: TopkRouterParams, dtype: torch.dtype) -> bool:
+    """Plain logits in the result's type, without a gradient, that nothing watches.  (One token to 16384 x 60 experts: 2 to 8 us
+    for what takes 10 to 48 in four to six launches.)"""
     return (type(logits) is torch.Tensor and logits.is_cuda and logits.dtype is dtype
             and dtype in (torch.bfloat16, torch.float16, torch.float32) and logits.dim() == 2 and logits.size(0) > 0
             and type(p.topk) is int and 0 < p.topk <= min(logits.size(1), _native.ROUTER_TAIL_TOPK)
             and logits.size(1) <= _native.ROUTER_TAIL_EXPERTS and logits.is_contiguous()
-            and not (logits.requires_grad and torch.is_grad_enabled()) and forward_ad._current_level < 0
-            and not torch._C._functorch.is_functorch_wrapped_tensor(logits)
-            and torch._C._len_torch_dispatch_stack() == 0 and torch._C._len_torch_function_stack() == 0
-            and not torch.compiler.is_compiling() and not torch.jit.is_tracing()
-            and logits.get_device() == torch.cuda.current_device())
+            and not (logits.requires_grad and torch.is_grad_enabled()) and nothing_watches(logits))
 
 
 class _FusedTopk(torch.autograd.Function):

@@ -220,3 +220,40 @@ def test_refused_group_with_all_the_rows(gather, scatter, native):
                                                    torch.arange(R, device="cuda"), gather, scatter, R, 1))
         torch.cuda.synchronize()
         assert out.shape == (R, N) and native.read_status(device_status(), reset=True) == 5
+
+
+@pytest.mark.parametrize("one_block", [True, False])
+def test_scratch_in_one_block_or_several(one_block, monkeypatch, native):
+    """The same bits however the buffers of a pass are allocated and wherever the saved ones come back to."""
+    from moe_explore import expert_compute as ec
+    from moe_explore.functional.topk_moe import topk_moe_forward
+    from moe_explore.params import MLPParams, MOEParams, TopkRouterParams
+
+    T, d, inter, E, k = 77, 136, 200, 6, 2
+    g = torch.Generator(device="cuda").manual_seed(3)
+    mk = lambda *s, std=1.0: (torch.randn(*s, generator=g, device="cuda") * std).bfloat16()
+    leaves = [mk(T, d), mk(d, E, std=0.1), mk(E, d, 2 * inter, std=0.1), mk(E, inter, d, std=0.1)]
+    grad = mk(T, d)
+
+    def run(softmax_before):
+        x, wr, w1, w2 = p = [t.clone().requires_grad_() for t in leaves]
+        params = MOEParams(TopkRouterParams(wr, k, softmax_before, True), MLPParams(w1, w2, "swiglu"), E, k)
+        moved = torch.autograd.graph.saved_tensors_hooks(lambda t: t.clone(), lambda t: t.clone())
+        with moved:
+            _poison()
+            out = topk_moe_forward(x, params)
+            _poison()
+            grads = torch.autograd.grad(out, p, grad)
+        with torch.no_grad():
+            again = topk_moe_forward(x, params)                  # router and experts without a gradient: one call
+            _poison()
+            assert torch.equal(again, out)
+            composed = topk_moe_forward(x, params, fused_combine=False, gather_in_gemm=True)
+            assert torch.equal(composed, out)
+        return [out.detach(), *grads]
+
+    ref = [run(b) for b in (False, True)]
+    if not one_block:
+        monkeypatch.setattr(ec, "SCRATCH_IN_ONE", 0)
+        for b in (False, True):
+            assert all(torch.equal(x, y) for x, y in zip(run(b), ref[b]))
