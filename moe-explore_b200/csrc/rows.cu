@@ -78,22 +78,27 @@ inverse_rows_kernel(const int64_t* __restrict__ index, int32_t* __restrict__ inv
 
 // Zeroes the padding rows (row_src < 0) among the rows in use: a warp looks at 64 rows at a time (two loads and ballots;
 // a load per row made this the longest part of a dispatch) and clears the ones it finds.  `live_blocks_only`: 64-row blocks
-// without a routed row are left alone.
+// without a routed row are left alone.  Where there are fewer blocks than warps a warp clears 512 bytes of each row: with whole
+// rows 64 experts with 16 rows of 4 KB each were 12.6 MB for 64 warps (dispatch 20.9 -> 12.3 us, backward fold 16.9 -> 7.7; 1001
+// tokens x 8, Zipf routing 25.4 -> 20.9 and 28.0 -> 21.8; 69000 rows gain nothing from it, 66 -> 70).
 __device__ __forceinline__ void zero_padding(const int32_t* __restrict__ row_src, const int32_t* __restrict__ num_mtiles,
                                              uint4* __restrict__ dst, int vec_per_row, int warp, int warps,
                                              bool live_blocks_only) {
   const int64_t rows_in_use = static_cast<int64_t>(*num_mtiles) * MOE_TILE_M;  // a multiple of 64
   const int lane = threadIdx.x & 31;
-  for (int64_t p0 = static_cast<int64_t>(warp) * 64; p0 < rows_in_use; p0 += static_cast<int64_t>(warps) * 64) {
+  const int parts = rows_in_use / 64 < warps ? (vec_per_row + 31) / 32 : 1;
+  const int64_t units = rows_in_use / 64 * parts;
+  for (int64_t unit = warp; unit < units; unit += warps) {
+    const int64_t p0 = unit / parts * 64;
+    const int v0 = static_cast<int>(unit % parts) * 32 + lane;
+    const int v_end = parts > 1 && v0 + 32 - lane < vec_per_row ? v0 + 32 - lane : vec_per_row;
     const unsigned lo = __ballot_sync(0xFFFFFFFFu, row_src[p0 + lane] < 0);
     const unsigned hi = __ballot_sync(0xFFFFFFFFu, row_src[p0 + 32 + lane] < 0);
     unsigned long long pads = (static_cast<unsigned long long>(hi) << 32) | lo;
     if (live_blocks_only && pads == ~0ull) continue;
-    while (pads != 0) {
+    for (; pads != 0; pads &= pads - 1) {
       const int b = __ffsll(static_cast<long long>(pads)) - 1;
-      pads &= pads - 1;
-      uint4* d = dst + (p0 + b) * vec_per_row;
-      for (int v = lane; v < vec_per_row; v += 32) d[v] = make_uint4(0, 0, 0, 0);
+      for (int v = v0; v < v_end; v += 32) dst[(p0 + b) * vec_per_row + v] = make_uint4(0, 0, 0, 0);
     }
   }
 }

@@ -183,3 +183,17 @@ def test_inverse_rows(rows, native):
     index[0] = rows   # (was negative) one past the end: named in the status word, written nowhere
     native.inverse_rows(index, out, device_status())
     assert torch.equal(out, expect) and native.read_status(device_status(), reset=True) == 5
+
+
+@pytest.mark.parametrize("cols", [8, 256, 264, 1000, 2048])
+@pytest.mark.parametrize("rows", [(1, 63, 64, 65, 0, 127), (700, 1000) * 80])     # fewer 64-row blocks than warps, and more
+def test_padding_rows_and_only_they_are_zeroed(rows, cols, native):
+    from moe_explore.routing_plan import plan_from_groups
+
+    groups = torch.tensor((0,) + rows, dtype=torch.int32).cumsum(0).int().cuda()
+    plan = plan_from_groups(groups, sum(rows))
+    used = int(plan.num_mtiles[0]) * 128
+    buf = torch.ones(used + 128, cols, dtype=torch.bfloat16, device="cuda")
+    native.zero_padding_rows(plan.row_src, plan.num_mtiles, buf)
+    expect = (plan.row_src[:used] >= 0).to(buf.dtype)[:, None].expand(used, cols)
+    assert torch.equal(buf[:used], expect) and bool((buf[used:] == 1).all())
