@@ -227,6 +227,18 @@ struct Window {
   int p_end;    // CTA pairs: one past the last pair of the window (a window may begin and end inside an expert)
 };
 
+// Before the wait for the kernels before: the translations of the index arrays, which the first loads after the wait would miss
+// (a prefetch into L2 is no read: what the arrays hold may still be about to change).
+__device__ __forceinline__ void prefetch_maps(const GemmArgs& args) {
+  const void* p = nullptr;
+  if (threadIdx.x == 32) p = args.num_mtiles;
+  else if (threadIdx.x == 33) p = args.tile_pairs;
+  else if (threadIdx.x == 34) p = args.mtile_expert;
+  else if (threadIdx.x == 35) p = args.group_indices;
+  else if (threadIdx.x == 36) p = args.pad_offsets;
+  if (p != nullptr) asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+}
+
 // Number of (row unit, column tile) work items and the row-unit / column-tile counts.  A row unit is
 // one 128-row tile (one CTA) or a pair of them (CTA pair).
 template <bool KG, int CTAS>
@@ -240,25 +252,29 @@ __device__ __forceinline__ int total_tiles(const GemmArgs& args, int& mt, int& n
     mt = (args.m_dim + BM * CTAS - 1) / (BM * CTAS);
     return args.num_experts * mt * nt;
   }
-  mt = args.num_mtiles[CTAS - 1];
+  // (the three words are asked for together: a load that follows another's result waits 0.5 to 1 us more for the first tile)
+  const int tiles = args.num_mtiles[0], pairs = args.num_mtiles[1], bound = args.num_mtiles[2];
+  mt = CTAS == 2 ? pairs : tiles;
   if (args.pair_prefix != nullptr) {
-    if (args.num_mtiles[2] != args.mtiles_bound) {
+    if (bound != args.mtiles_bound) {
       // the pair prefix sits at tile_pairs[bound]: metadata built for another bound cannot be walked
       if (threadIdx.x == 0 && args.status != nullptr) atomicCAS(args.status, 0, DS_BAD_LAYOUT);
       mt = 0;
       return 0;
     }
-    const int pairs = args.num_mtiles[1];
     int p0, p1;
     if (args.pair_end > args.pair_begin) {
       // an explicit range of the pair list; the experts it touches are found by the search in decode_tile
       p0 = args.pair_begin < pairs ? args.pair_begin : pairs;
       p1 = args.pair_end < pairs ? args.pair_end : pairs;
+    } else if (args.expert_end <= args.expert_begin && args.chunk_count <= 1) {
+      p0 = 0;
+      p1 = pairs;
     } else {
       if (args.expert_end > args.expert_begin) {
         win.e0 = args.expert_begin;
         win.e1 = args.expert_end < args.num_experts ? args.expert_end : args.num_experts;
-      } else if (args.chunk_count > 1) {
+      } else {
         win.e0 = static_cast<int>(static_cast<long long>(args.num_experts) * args.chunk_index / args.chunk_count);
         win.e1 = static_cast<int>(static_cast<long long>(args.num_experts) * (args.chunk_index + 1) / args.chunk_count);
       }
@@ -270,8 +286,7 @@ __device__ __forceinline__ int total_tiles(const GemmArgs& args, int& mt, int& n
       win.m_begin = p0;
       mt = p1 - p0;
     } else {  // one-CTA kernels: the same window expressed in tiles
-      const int tiles = args.num_mtiles[0];
-      win.m_begin = p0 < pairs ? (args.tile_pairs[p0] & 0xFFFFF) : tiles;
+      win.m_begin = p0 == 0 ? 0 : p0 < pairs ? (args.tile_pairs[p0] & 0xFFFFF) : tiles;
       mt = (p1 < pairs ? (args.tile_pairs[p1] & 0xFFFFF) : tiles) - win.m_begin;
     }
   }
@@ -598,6 +613,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       tmem_relinquish();
     }
   }
+  prefetch_maps(args);
   grid_wait();  // nothing above reads or writes global memory
   tc_fence_before();
   __syncthreads();

@@ -168,6 +168,7 @@ grouped_gemm_kernel(const __grid_constant__ TMaps maps, const GemmArgs args) {
     tmem_alloc_pair(smem_u32(tmem_slot), kTmemCols);
     tmem_relinquish_pair();
   }
+  prefetch_maps(args);
   grid_wait();  // nothing above reads or writes global memory
   tc_fence_before();
   __syncthreads();
