@@ -513,18 +513,27 @@ template <> __device__ __forceinline__ void red_add_v8<__half>(void* ptr, const 
 }
 
 // Activation math (fp32).
-// 1 / y for y >= 1 (infinity included): one step of the Newton-Raphson iteration r' = r + r (1 - y r), whose relative error is the
+// e^x, 0 below the normal range (the flushing form of the hardware's 2^x: the other one scales its argument by a compare and two
+// predicated products around it).
+__device__ __forceinline__ float exp_flush(float x) {
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x * 1.4426950408889634f));
+  return r;
+}
+// 1 / (1 + e^-x).  The reciprocal is one step of the Newton-Raphson iteration r' = r + r (1 - y r), whose relative error is the
 // square of r's, from the hardware's approximation (relative error 2^-23: the step leaves the rounding of its last
 // operation).  Straight-line code, because the elements of an epilogue row have to be interleaved: with two warps per scheduler
 // that is the whole speed of the gated epilogues (dGLU at 16384 tokens x 4 slots, 60 experts, K 2048: 229 -> 204 us against the
-// division operator).  The cap makes the step from r = 0 at y = infinity a finite one; r itself is taken of y, so that results
-// below the normal range (gates under -87) and NaN come out as they are.
-__device__ __forceinline__ float reciprocal_ge1(float y) {
+// division operator).  y is a quarter of 1 + e^-x, so that the flushing forms serve: e^-x below the normal range adds nothing to 1,
+// and 4 / (1 + e^-x) stays above it; the last product may then leave a result below (gates under -87).  The cap makes the step
+// from r = 0 at y = infinity a finite one; r itself is taken of y, so that NaN comes out as it is.  Same bits as with the general
+// forms, 9 operations for 16: a 32 x 32 block of the gated backward 2093 -> 1743 cycles, of a forward SiLU 2450 -> 2330.
+__device__ __forceinline__ float sigmoidf_fast(float x) {
+  const float y = fmaf(0.25f, exp_flush(-x), 0.25f);
   float r;
-  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(y));
-  return fmaf(r, fmaf(-fminf(y, 3.0e38f), r, 1.0f), r);
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(y));
+  return 0.25f * fmaf(r, fmaf(-fminf(y, 1.0e38f), r, 1.0f), r);
 }
-__device__ __forceinline__ float sigmoidf_fast(float x) { return reciprocal_ge1(1.0f + __expf(-x)); }
 __device__ __forceinline__ float silu_f(float x) { return x * sigmoidf_fast(x); }
 __device__ __forceinline__ float gelu_f(float x) { return 0.5f * x * (1.0f + erff(x * 0.70710678118654752f)); }
 // tanh form: 0.5 x (1 + tanh(sqrt(2/pi) (x + 0.044715 x^3)))

@@ -43,25 +43,27 @@ struct TPlan {
   static constexpr int kTotal = kStages * kStageBytes + kStagingBytes + kBarrierBytes + 1024;
 };
 
-// One 32 x 32 block, lane = column, v[j] = row j, as 16-bit elements into a dense tile of 32 rows x 64 bytes.
+// One 32 x 32 block, lane = column, v[j] = row j, as the 16-bit words of a dense tile of 32 rows x 64 bytes.  Turning and storing
+// are apart, so that the shuffles of a block overlap, and the wait for the store that last read the tile comes after the math.
 template <typename T>
-__device__ __forceinline__ void turn_block(const float (&v)[32], uint32_t tile, int lane) {
+__device__ __forceinline__ void turn_block(const float (&v)[32], uint32_t (&w)[16], int lane) {
   const uint32_t sel = (lane & 1) ? 0x3276u : 0x5410u;
-  const uint32_t addr = tile + (lane & 1) * 64 + (lane >> 1) * 4;
-  uint32_t w[16];
 #pragma unroll
   for (int i = 0; i < 16; ++i) {
     const uint32_t own = Elem<T>::pack2(v[2 * i], v[2 * i + 1]);
     w[i] = __byte_perm(own, __shfl_xor_sync(0xFFFFFFFFu, own, 1), sel);
   }
+}
+__device__ __forceinline__ void store_block(const uint32_t (&w)[16], uint32_t tile, int lane) {
+  const uint32_t addr = tile + (lane & 1) * 64 + (lane >> 1) * 4;
 #pragma unroll
   for (int i = 0; i < 16; ++i) asm volatile("st.shared.b32 [%0], %1;" ::"r"(addr + i * 128), "r"(w[i]) : "memory");
 }
 
-// The gated activation of such a block (even lanes gate, odd lanes up) into a dense tile of 32 rows x 32 bytes: even lanes
-// compute even rows, odd lanes odd rows.
+// The gated activation of such a block (even lanes gate, odd lanes up), 32 rows x 32 bytes: even lanes compute even rows, odd
+// lanes odd rows.
 template <typename T, bool GEGLU>
-__device__ __forceinline__ void turn_glu(const float (&v)[32], uint32_t tile, int lane) {
+__device__ __forceinline__ void turn_glu(const float (&v)[32], uint32_t (&w)[8], int lane) {
   const bool odd = lane & 1;
   float g[16];
 #pragma unroll
@@ -72,13 +74,14 @@ __device__ __forceinline__ void turn_glu(const float (&v)[32], uint32_t tile, in
     g[i] = (GEGLU ? gelu_f(gate) : silu_f(gate)) * up;
   }
   const uint32_t sel = (lane & 2) ? 0x3276u : 0x5410u;
-  const uint32_t addr = tile + (lane & 3) * 32 + (lane >> 2) * 4;
-  uint32_t w[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const uint32_t own = Elem<T>::pack2(g[2 * i], g[2 * i + 1]);
     w[i] = __byte_perm(own, __shfl_xor_sync(0xFFFFFFFFu, own, 2), sel);
   }
+}
+__device__ __forceinline__ void store_glu(const uint32_t (&w)[8], uint32_t tile, int lane) {
+  const uint32_t addr = tile + (lane & 3) * 32 + (lane >> 2) * 4;
 #pragma unroll
   for (int i = 0; i < 8; ++i) asm volatile("st.shared.b32 [%0], %1;" ::"r"(addr + i * 128), "r"(w[i]) : "memory");
 }
@@ -352,10 +355,12 @@ grouped_gemm_kernel(const __grid_constant__ TMaps maps, const GemmArgs args) {
           apply_act(v, args.act);
           const uint32_t tile = stage_base + (turn & 1) * 2048;
           ++turn;
+          uint32_t w[16];
           if (args.out_tma) {
+            turn_block<T>(v, w, lane);
             if (lane == 0) bulk_wait_read_one();  // the store before the last has read this tile
             __syncwarp();
-            turn_block<T>(v, tile, lane);
+            store_block(w, tile, lane);
             fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) {
@@ -378,7 +383,8 @@ grouped_gemm_kernel(const __grid_constant__ TMaps maps, const GemmArgs args) {
             } else {
               dst = args.push_row[row0 + lane];
             }
-            turn_block<T>(v, tile, lane);
+            turn_block<T>(v, w, lane);
+            store_block(w, tile, lane);
             __syncwarp();
             const int piece = lane & 3;
             const bool in = col0 + piece * 8 < N;
@@ -403,6 +409,10 @@ grouped_gemm_kernel(const __grid_constant__ TMaps maps, const GemmArgs args) {
           const bool aux = args.aux_out != nullptr;
           const uint32_t tile = stage_base + (aux ? 2048 : (turn & 1) * 1024);
           ++turn;
+          uint32_t w[16], g[8];
+          if (aux) turn_block<T>(v, w, lane);
+          if (args.act == MOE_ACT_GEGLU) turn_glu<T, true>(v, g, lane);
+          else turn_glu<T, false>(v, g, lane);
           if (args.out_tma) {
             if (lane == 0) {
               if (aux) bulk_wait_read_all();
@@ -410,9 +420,8 @@ grouped_gemm_kernel(const __grid_constant__ TMaps maps, const GemmArgs args) {
             }
             __syncwarp();
           }
-          if (aux) turn_block<T>(v, stage_base, lane);
-          if (args.act == MOE_ACT_GEGLU) turn_glu<T, true>(v, tile, lane);
-          else turn_glu<T, false>(v, tile, lane);
+          if (aux) store_block(w, stage_base, lane);
+          store_glu(g, tile, lane);
           if (args.out_tma) {
             fence_proxy_async_smem();
             __syncwarp();
@@ -458,8 +467,10 @@ grouped_gemm_kernel(const __grid_constant__ TMaps maps, const GemmArgs args) {
             x[r] = Elem<T>::unpack2(u).x;
           }
           mul_dact(v, x, args.act);
+          uint32_t w[16];
+          turn_block<T>(v, w, lane);
           __syncwarp();
-          turn_block<T>(v, side, lane);
+          store_block(w, side, lane);
           fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) {
@@ -468,11 +479,14 @@ grouped_gemm_kernel(const __grid_constant__ TMaps maps, const GemmArgs args) {
           }
           ++q;
         } else {  // EPI_ACT_AUX, forward: un-activated and activated product from one tile each
+          uint32_t w[16], g[16];
+          turn_block<T>(v, w, lane);
+          apply_act(v, args.act);
+          turn_block<T>(v, g, lane);
           if (lane == 0) bulk_wait_read_all();
           __syncwarp();
-          turn_block<T>(v, stage_base, lane);
-          apply_act(v, args.act);
-          turn_block<T>(v, stage_base + 2048, lane);
+          store_block(w, stage_base, lane);
+          store_block(g, stage_base + 2048, lane);
           fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) {
