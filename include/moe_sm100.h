@@ -455,6 +455,8 @@ typedef struct moe_expert_pass {
   float* dl;
   void *dlogits, *router_t;
   int32_t softmax_before_topk, normalize; /* MOE_FWD_TAIL */
+  int32_t* counters; /* four words of this pass's own (not `gather`'s forward, not `identity`), or NULL: the contractions claim their
+                      * work items from them instead of dealing them out.  Written by MOE_FWD_DISPATCH / MOE_BWD_FOLD */
 } moe_expert_pass;
 
 /* sizeof(moe_expert_pass), for bindings that declare the struct themselves. */
@@ -495,6 +497,7 @@ typedef struct moe_rows_pass {
   const int64_t* perm;
   int32_t *pad_offsets, *in_rows, *out_rows, *mtile_expert, *tile_pairs, *num_mtiles, *status;
   void* padded;
+  int32_t* counters; /* four words of this call's own, or NULL; written by MOE_ROWS_LAYOUT */
 } moe_rows_pass;
 
 size_t moe_rows_pass_size(void);

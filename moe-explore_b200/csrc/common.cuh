@@ -93,7 +93,12 @@ struct RowCounts {
   int64_t a_rows = -1;
   int64_t b_rows = -1;    // K-grouped
   int64_t out_rows = -1;  // M-grouped plain stores, one expert
+  // A word that work items are claimed from (GemmArgs::work_counter), zero; null: they are dealt out.
+  uint32_t* work_counter = nullptr;
+  int64_t routed_rows = -1;  // with work_counter: about how many rows there are (for the choice whether to use it)
 };
+// Words that the first row kernel of a pass, or its layout kernel, sets to zero for the contractions after it.
+constexpr int kWorkCounters = 4;
 
 // The entry points of the same names, told which rows exist.
 int mgrouped_gemm(const void* a, const void* w, void* out, void* pre_act, const int32_t* mtile_expert, const int32_t*
@@ -129,7 +134,10 @@ int mgrouped_gemm_rows(const void* a, int64_t compact_rows, const void* w, void*
 int gather_rows(const void* src, int64_t src_rows, const int32_t* row_src, const int32_t* num_mtiles, void* dst,
                 int64_t padded_rows, int cols, int div, int dtype, void* stream, bool skip_marked);
 int dispatch_rows(const void* src, const int32_t* dst_row, const int32_t* row_src, const int32_t* num_mtiles, void* dst,
-                  int64_t num_tokens, int topk, int64_t padded_rows, int cols, int dtype, void* stream, bool live_blocks_only);
+                  int64_t num_tokens, int topk, int64_t padded_rows, int cols, int dtype, void* stream, bool live_blocks_only,
+                  uint32_t* work_counters);
+int dispatch_rows_only(const void* src, const int32_t* dst_row, void* dst, int64_t num_tokens, int topk, int cols, int dtype,
+                       void* stream, uint32_t* work_counters);
 // moe_combine_topk with further summands, all nullable (FoldExtra in csrc/rows.cu).
 int combine_topk(const void* ys, const void* scores, const int32_t* dst_row, void* out, int64_t num_tokens, int topk, int cols,
                  int dtype, const void* addend, const float* dlogits, const int64_t* experts, const void* router_t,
@@ -140,7 +148,7 @@ int router_backward(const void* logits, const int64_t* experts, const void* d_sc
                     void* stream);
 int combine_bwd_tokens(const void* dout, const void* scores, const void* ys, const int32_t* dst_row, const int32_t* row_src,
                        const int32_t* num_mtiles, void* gs, void* dscores, int64_t num_tokens, int topk, int cols, int dtype,
-                       void* stream, bool live_blocks_only);
+                       void* stream, bool live_blocks_only, uint32_t* work_counters);
 
 // Status codes written by kernels into the caller's device status word.
 enum DeviceStatus : int {
@@ -417,6 +425,13 @@ __device__ __forceinline__ void cluster_sync_all() {
 }
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+// Four words into either CTA's shared memory, their 16 bytes credited to that CTA's barrier when they are there (visible to whoever
+// waits for it, as a copy's bytes are).
+__device__ __forceinline__ void st_async_v4(uint32_t cluster_addr, int a, int b, int c, int d, uint32_t cluster_bar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];"
+               ::"r"(cluster_addr), "r"(a), "r"(b), "r"(c), "r"(d), "r"(cluster_bar)
+               : "memory");
 }
 __device__ __forceinline__ void mbar_arrive_expect_tx_cluster(uint32_t cluster_addr, uint32_t bytes) {
   // default (CTA-scope) ordering: the operand bytes are published by the copies' own complete_tx, not by this

@@ -123,6 +123,9 @@ struct GemmArgs {
   uint32_t* wave_counter;  // non-null: workers start every work item together (grid-wide arrival counter, zeroed
                            // by the host before the launch)
   int32_t wave_workers;    // arrivals per wave the barrier waits for (the number of workers of the launch)
+  // Non-null: work items after a worker's first are claimed from this word (0 before the launch and again after it), see
+  // ItemQueue.  CTA pairs of the K-grouped and of the transposed kernels.
+  uint32_t* work_counter;
   int32_t group_m;  // row units per scheduling group
   long long wait_limit;  // cycles after which a device-side wait gives up
   int32_t* status;
@@ -140,6 +143,7 @@ struct TileCoord {
                 // one are then the next expert's, and nothing is stored for them)
   int live;     // M-grouped: rows of the tile that exist (64 or 128, see GemmArgs::group_indices)
   int unit_rows;  // M-grouped: rows of the whole row unit that exist, in 64-row blocks (the tile's, or the pair's)
+  bool valid;     // false: there is no further item
 };
 
 // K-grouped: rows of expert e to contract over, in steps of 16 (what follows an expert's last row up to the end of its 64-row
@@ -214,7 +218,7 @@ struct SmemPlan {
   static constexpr int kStagingTile = 32 * 128;
   static constexpr int kTilesPerWarp = ((EPI == EPI_DGLU && CTAS == 2) || EPI == EPI_ACT_AUX) ? 2 : 1;
   static constexpr int kStagingBytes = kEpilogueWarps * kTilesPerWarp * kStagingTile;
-  static constexpr int kBarrierBytes = 512;
+  static constexpr int kBarrierBytes = 1024;
   static constexpr int kBudget = 232448 - 1024 - kBarrierBytes - kStagingBytes;  // 227 KB minus alignment slack
   static constexpr int kStages = (kBudget / kStageBytes) > 8 ? 8 : (kBudget / kStageBytes);
   static constexpr int kTotal = kStages * kStageBytes + kStagingBytes + kBarrierBytes + 1024;
@@ -399,6 +403,7 @@ struct ItemWalk {
     }
     const int src = i & 31;
     TileCoord c;
+    c.valid = first + i * stride < count;
     c.m0 = __shfl_sync(0xFFFFFFFFu, mine.m0, src);
     c.n0 = __shfl_sync(0xFFFFFFFFu, mine.n0, src);
     c.expert = __shfl_sync(0xFFFFFFFFu, mine.expert, src);
@@ -412,6 +417,102 @@ struct ItemWalk {
     return c;
   }
 };
+
+// Work items claimed one by one instead of dealt out: with a fixed stride the slowest worker is 5 to 11 % behind the mean where
+// rows fall unevenly (simulated with the stage costs measured; claimed 1 to 5 %), and where the items are equal the SMs are not --
+// storing weight gradients, some were done after 68 us and others after 100.  The second CTA's idle MMA warp is the scheduler: it
+// claims an item with one atomic addition, decodes it and writes it into a ring of four slots in both CTAs' shared memory; the other
+// nineteen roles read it there.  A worker's first item is its index; M-grouped workers claim the next one when the leader's producer
+// has begun the last one claimed, so that at most one unbegun item is held.  Every worker's claims end with one that
+// finds nothing left; the claim that is the last of all puts the word back to zero.
+constexpr int kQueueSlots = 4;
+struct ItemQueue {
+  uint32_t full, empty, taken;  // barriers: [slots] in each CTA; [slots] and one in the second CTA
+  uint32_t slots;               // [slots][8] words in each CTA
+
+  __device__ __forceinline__ explicit ItemQueue(uint32_t area) : full(area), empty(area + 32), taken(area + 64), slots(area + 128) {}
+  __device__ __forceinline__ void init() const {  // by one thread of each CTA
+    for (int s = 0; s < kQueueSlots; ++s) {
+      mbar_init(full + 8 * s, 1);
+      mbar_init(empty + 8 * s, 2 * (1 + kEpilogueWarps) + 1);
+    }
+    mbar_init(taken, 1);
+  }
+  // The i-th item, by all lanes of a warp of either CTA; an item that is not valid where the wait gave up (then the abort flag is set).
+  template <bool KG>
+  __device__ __forceinline__ TileCoord get(int i, const GemmArgs& args, bool mark_taken, const WaitCtx& w, int code) const {
+    const int s = i & (kQueueSlots - 1);
+    TileCoord c{};
+    if (!__all_sync(0xFFFFFFFFu, mbar_wait(full + 8 * s, (i / kQueueSlots) & 1, w, code))) return c;
+    // Each lane reads a word and the warp exchanges them.  The exchange uses what was loaded, so no load is outstanding when the
+    // arrival on the other CTA's barrier is issued.  (An arrival alone overtook the loads now and then, the slot was rewritten
+    // under them, and one item in a million was another one.  Ordering it by a release at cluster scope instead waits for all of the
+    // warp's memory traffic: weight gradients of 128 tokens 95 -> 155 us.)
+    uint32_t mine;
+    asm volatile("ld.shared.b32 %0, [%1];" : "=r"(mine) : "r"(slots + 32 * s + 4 * (threadIdx.x & 7)) : "memory");
+    int word[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) word[j] = static_cast<int>(__shfl_sync(0xFFFFFFFFu, mine, j));
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) {
+      mbar_arrive_cluster(mapa_shared(empty + 8 * s, 1));
+      if (!KG && mark_taken) mbar_arrive_cluster(mapa_shared(taken, 1));
+    }
+    c.m0 = word[0];
+    c.n0 = word[1];
+    c.expert = word[2];
+    c.k_row0 = KG ? word[3] : 0;
+    c.a_row = KG ? 0 : word[3];
+    c.kiters = KG ? word[4] : (args.k_dim + BK - 1) / BK;
+    c.unit_rows = KG ? BM : word[4];
+    c.live = BM;
+    c.k_last = KG ? word[5] : BK;
+    c.active = true;
+    c.valid = word[7] != 0;
+    return c;
+  }
+  // The scheduler, by all lanes of a warp of the second CTA.
+  template <bool KG, int CTAS>
+  __device__ __forceinline__ void serve(int unit, int num_units, int ntiles, int mt, int nt, int BN, const Window& win, const GemmArgs& args,
+                                        const WaitCtx& w) const {
+    const int lane = threadIdx.x & 31;
+    uint32_t claimed = 0;
+    const auto claim = [&]() {
+      if (lane == 0) {
+        claimed = atomicAdd(args.work_counter, 1u);
+        if (claimed == static_cast<uint32_t>(ntiles) - 1) *args.work_counter = 0;
+      }
+    };
+    int t = unit;
+    for (int i = 0;; ++i) {
+      const int s = i & (kQueueSlots - 1);
+      if (i > 0) {
+        if (!KG) {
+          if (!__all_sync(0xFFFFFFFFu, mbar_wait(taken, (i - 1) & 1, w, DS_TIMEOUT_PRODUCER))) return;
+          claim();
+        }
+        const uint32_t n = __shfl_sync(0xFFFFFFFFu, claimed, 0);
+        t = n < static_cast<uint32_t>(ntiles) ? num_units + static_cast<int>(n) : ntiles;
+      }
+      const bool valid = t < ntiles;
+      if (KG && valid) claim();  // items are short: the next claim is under way while this one waits for its slot
+      TileCoord c{};
+      if (valid) c = decode_tile<KG, CTAS>(t, mt, nt, win, args, BN, KG ? lane & 1 : 0);
+      if (i >= kQueueSlots &&
+          !__all_sync(0xFFFFFFFFu, mbar_wait(empty + 8 * s, (i / kQueueSlots - 1) & 1, w, DS_TIMEOUT_PRODUCER))) return;
+      if (lane < 2) {
+        const uint32_t to = mapa_shared(slots + 32 * s, static_cast<uint32_t>(lane));
+        const uint32_t bar = mapa_shared(full + 8 * s, static_cast<uint32_t>(lane));
+        mbar_arrive_expect_tx_cluster(bar, 32);
+        st_async_v4(to, c.m0, c.n0, c.expert, KG ? c.k_row0 : c.a_row, bar);
+        st_async_v4(to + 16, KG ? c.kiters : c.unit_rows, KG ? c.k_last : 0, 0, valid ? 1 : 0, bar);
+      }
+      __syncwarp();
+      if (!valid) return;
+    }
+  }
+};
+constexpr int kQueueOffset = 512;  // of the queue in the barrier area
 
 // Wave barrier of the persistent workers.  With a static stride every worker's i-th work item belongs to the same
 // "wave" of neighbouring tiles; workers that share operand tiles only hit in L2 while they stream through them
@@ -573,7 +674,12 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   const uint32_t epi_bar = smem_u32(bars + 2 * kStages + 4);    // [kEpilogueWarps][2]  (dGLU side-input tiles)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kStages + 4 + 2 * kEpilogueWarps);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  static_assert((2 * 8 + 4 + 2 * kEpilogueWarps) * 8 + 8 <= Plan::kBarrierBytes, "barrier area too small");
+  static_assert((2 * 8 + 4 + 2 * kEpilogueWarps) * 8 + 8 <= kQueueOffset && kQueueOffset + 128 + kQueueSlots * 32 <= Plan::kBarrierBytes,
+                "barrier area too small");
+  // items claimed at run time (K-grouped pairs): a compile-time possibility, the other kernels' loops carry none of it
+  constexpr bool kQueue = KG && kPair && !GATHER;
+  const ItemQueue queue(smem_u32(bars) + kQueueOffset);
+  const bool queued = kQueue && args.work_counter != nullptr;
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -597,6 +703,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       mbar_init(tempty_bar + 8 * a, kEpilogueWarps * CTAS);
     }
     for (int i = 0; i < 2 * kEpilogueWarps; ++i) mbar_init(epi_bar + 8 * i, 1);
+    if (kQueue) queue.init();
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tmap_a);
@@ -624,6 +731,11 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   int mt, nt;
   Window win;
   const int ntiles = total_tiles<KG, CTAS>(args, mt, nt, win, BN);
+  ItemWalk<KG, CTAS> walk(unit, num_units, ntiles, mt, nt, BN, rank);
+  const auto item = [&](int i, bool mark_taken, int code) {
+    if (kQueue && queued) return queue.template get<KG>(i, args, mark_taken, wctx, code);
+    return walk.get(i, win, args);
+  };
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
@@ -641,19 +753,19 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       // Mixtral shape with the branches compiled out), because the loop then no longer is the short elected-lane
       // sequence the operand pipeline needs once per 512 tensor-core cycles.
       constexpr bool gather = GATHER;
-      ItemWalk<KG, CTAS> items(unit, num_units, ntiles, mt, nt, BN, rank);
-      TileCoord c_next = items.get(0, win, args);
+      TileCoord c_next = item(0, rank == 0, DS_TIMEOUT_PRODUCER);
       // M-grouped gather: lane l owns rows 4l..4l+3 of the tile for all of its stages
       int4 rows_next = make_int4(0, 0, 0, 0);
       if (gather && !KG && unit < ntiles) rows_next = gather_rows4(args.a_row_src, c_next.m0 + 4 * lane, args.a_div, args.a_rows);
       bool wave_sync = !KG && args.wave_counter != nullptr && rank == 0;
       int wave = 0;
-      for (int t = unit; t < ntiles && ok; t += num_units, ++wave) {
+      for (; c_next.valid && ok; ++wave) {
         const TileCoord c = c_next;
         const int4 rows_m = rows_next;
-        if (t + num_units < ntiles) {
-          c_next = items.get(wave + 1, win, args);
-          if (gather && !KG) rows_next = gather_rows4(args.a_row_src, c_next.m0 + 4 * lane, args.a_div, args.a_rows);
+        if (gather) {
+          // the next work item's rows: their indices are loaded while this tile streams
+          c_next = item(wave + 1, false, DS_TIMEOUT_PRODUCER);
+          if (!KG && c_next.valid) rows_next = gather_rows4(args.a_row_src, c_next.m0 + 4 * lane, args.a_div, args.a_rows);
         }
         if (wave_sync && wave > 0 &&
             !__all_sync(0xFFFFFFFFu, wave_wait(args.wave_counter, static_cast<uint32_t>(args.wave_workers) * wave, wctx))) {
@@ -783,6 +895,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
           rows_k = rows_k_next;
           if (++stage == kStages) { stage = 0; phase ^= 1; }
         }
+        if (!gather) c_next = item(wave + 1, rank == 0, DS_TIMEOUT_PRODUCER);
       }
       // all operand loads are issued: the next chained kernel may come up beside the last tile's contraction and epilogue (from
       // the start of this kernel on, its waiting CTAs cost more than they hid)
@@ -793,7 +906,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         const int waves = (ntiles + num_units - 1) / num_units;
         for (int w = wave + 1; w < waves; ++w) atomicAdd(args.wave_counter, 1u);
       }
-      if (!ok) {
+      if (!ok || *abort_flag) {
         // Let copies that were already issued land before the CTA releases its shared memory.
         for (int i = 0; i < 2000; ++i) __nanosleep(1000);
       }
@@ -810,10 +923,9 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       uint32_t acc_phase = 0;
       bool ok = true;
       bool ready = false;  // the stage about to be consumed was already seen full
-      ItemWalk<KG, CTAS> items(unit, num_units, ntiles, mt, nt, BN, rank);
-      int item = 0;
-      for (int t = unit; t < ntiles && ok; t += num_units) {
-        const TileCoord c = items.get(item++, win, args);
+      for (int i = 0; ok; ++i) {
+        const TileCoord c = item(i, false, DS_TIMEOUT_MMA);
+        if (!c.valid) break;
         if (c.kiters == 0) continue;  // empty expert: the epilogue writes zeros on its own
         if (!__all_sync(0xFFFFFFFFu, mbar_wait(tempty_bar + 8 * acc, acc_phase ^ 1, wctx, DS_TIMEOUT_MMA))) {
           ok = false;
@@ -869,6 +981,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       if (!ok || *abort_flag) {
         for (int i = 0; i < 2000; ++i) __nanosleep(1000);
       }
+    } else if (kQueue && queued) {
+      queue.template serve<KG, CTAS>(unit, num_units, ntiles, mt, nt, BN, win, args, wctx);
     }
   } else {
     // ------------------------------ epilogue ----------------------------------
@@ -894,10 +1008,9 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     const auto side_parity = [](uint32_t n) { return Plan::kTilesPerWarp == 2 ? (n >> 1) & 1 : n & 1; };
     const int co_row = lane >> 3;  // coalesced access: row within a group of four
     const int co_ck = lane & 7;    // and 16-byte piece of the row's 128 bytes
-    ItemWalk<KG, CTAS> items(unit, num_units, ntiles, mt, nt, BN, rank);
-    int item = 0;
-    for (int t = unit; t < ntiles; t += num_units) {
-      const TileCoord c = items.get(item++, win, args);
+    for (int i = 0;; ++i) {
+      const TileCoord c = item(i, false, DS_TIMEOUT_EPILOGUE);
+      if (!c.valid) break;
       const bool have_acc = c.kiters != 0;
       const int row = c.m0 + row_in_tile;
       const bool quad_live = KG || (c.active && quad * 32 < c.live);  // this warp's 32 rows exist

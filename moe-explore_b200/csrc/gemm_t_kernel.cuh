@@ -37,7 +37,7 @@ struct TPlan {
   // per epilogue warp: two 32-row x 128-byte tiles of the saved product (gated backward); otherwise 4 KB, cut by the epilogue
   static constexpr int kWarpStaging = EPI == EPI_DGLU ? 8192 : 4096;
   static constexpr int kStagingBytes = kEpilogueWarps * kWarpStaging;
-  static constexpr int kBarrierBytes = 512;
+  static constexpr int kBarrierBytes = 1024;
   static constexpr int kBudget = 232448 - 1024 - kBarrierBytes - kStagingBytes;
   static constexpr int kStages = (kBudget / kStageBytes) > 8 ? 8 : (kBudget / kStageBytes);
   static constexpr int kTotal = kStages * kStageBytes + kStagingBytes + kBarrierBytes + 1024;
@@ -136,7 +136,10 @@ grouped_gemm_kernel(const __grid_constant__ TMaps maps, const GemmArgs args) {
   const uint32_t epi_bar = smem_u32(bars + 2 * kStages + 4);     // [kEpilogueWarps][2]  (saved product tiles)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kStages + 4 + 2 * kEpilogueWarps);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  static_assert((2 * 8 + 4 + 2 * kEpilogueWarps) * 8 + 8 <= Plan::kBarrierBytes, "barrier area too small");
+  static_assert((2 * 8 + 4 + 2 * kEpilogueWarps) * 8 + 8 <= kQueueOffset && kQueueOffset + 128 + kQueueSlots * 32 <= Plan::kBarrierBytes,
+                "barrier area too small");
+  const ItemQueue queue(smem_u32(bars) + kQueueOffset);
+  const bool queued = args.work_counter != nullptr;
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -160,6 +163,7 @@ grouped_gemm_kernel(const __grid_constant__ TMaps maps, const GemmArgs args) {
       mbar_init(tempty_bar + 8 * a, kEpilogueWarps * 2);
     }
     for (int i = 0; i < 2 * kEpilogueWarps; ++i) mbar_init(epi_bar + 8 * i, 1);
+    queue.init();
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&maps.w);
@@ -182,6 +186,10 @@ grouped_gemm_kernel(const __grid_constant__ TMaps maps, const GemmArgs args) {
   int mt, nt;
   Window win;
   const int ntiles = total_tiles<false, kTilesPerUnit>(args, mt, nt, win, BN);
+  ItemWalk<false, kTilesPerUnit> walk(unit, num_units, ntiles, mt, nt, BN, 0);
+  const auto item = [&](int i, bool mark_taken, int code) {
+    return queued ? queue.template get<false>(i, args, mark_taken, wctx, code) : walk.get(i, win, args);
+  };
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
@@ -192,10 +200,9 @@ grouped_gemm_kernel(const __grid_constant__ TMaps maps, const GemmArgs args) {
     const uint64_t pol = l2_policy_evict_normal();
     // operand arrival is credited to the leader's barriers, in its own and in the cluster window alike
     const uint32_t full_leader = mapa_shared(full_bar, 0);
-    ItemWalk<false, kTilesPerUnit> items(unit, num_units, ntiles, mt, nt, BN, 0);
-    int item = 0;
-    for (int t = unit; t < ntiles && ok; t += num_units) {
-      const TileCoord c = items.get(item++, win, args);
+    for (int i = 0; ok; ++i) {
+      const TileCoord c = item(i, rank == 0, DS_TIMEOUT_PRODUCER);
+      if (!c.valid) break;
       const int steps = (c.unit_rows + 63) >> 6;  // of 64 rows, 32 in each CTA
       const CUtensorMap* rows_map = &maps.r[steps - 1];
       const int row0 = c.a_row + rank * steps * 32;
@@ -230,7 +237,7 @@ grouped_gemm_kernel(const __grid_constant__ TMaps maps, const GemmArgs args) {
       }
     }
     grid_release();  // all operand loads are issued: the next chained kernel may come up beside the last tile
-    if (!ok) {
+    if (!ok || *abort_flag) {
       // Let copies that were already issued land before the CTA releases its shared memory.
       for (int i = 0; i < 2000; ++i) __nanosleep(1000);
     }
@@ -245,10 +252,9 @@ grouped_gemm_kernel(const __grid_constant__ TMaps maps, const GemmArgs args) {
       uint32_t acc_phase = 0;
       bool ok = true;
       bool ready = false;  // the stage about to be consumed was already seen full
-      ItemWalk<false, kTilesPerUnit> items(unit, num_units, ntiles, mt, nt, BN, 0);
-      int item = 0;
-      for (int t = unit; t < ntiles && ok; t += num_units) {
-        const TileCoord c = items.get(item++, win, args);
+      for (int i = 0; ok; ++i) {
+        const TileCoord c = item(i, false, DS_TIMEOUT_MMA);
+        if (!c.valid) break;
         const uint32_t idesc = idesc0 | (static_cast<uint32_t>((c.unit_rows + 63) >> 6) * 8u) << 17;
         if (!__all_sync(0xFFFFFFFFu, mbar_wait(tempty_bar + 8 * acc, acc_phase ^ 1, wctx, DS_TIMEOUT_MMA))) {
           ok = false;
@@ -289,6 +295,8 @@ grouped_gemm_kernel(const __grid_constant__ TMaps maps, const GemmArgs args) {
       if (!ok || *abort_flag) {
         for (int i = 0; i < 2000; ++i) __nanosleep(1000);
       }
+    } else if (queued) {
+      queue.template serve<false, kTilesPerUnit>(unit, num_units, ntiles, mt, nt, BN, win, args, wctx);
     }
   } else {
     // ------------------------------ epilogue ----------------------------------
@@ -306,10 +314,9 @@ grouped_gemm_kernel(const __grid_constant__ TMaps maps, const GemmArgs args) {
     uint32_t turn = 0;   // staging tile of plain and gated results, two in turn
     const bool side_input = EPI == EPI_DGLU || (EPI == EPI_ACT_AUX && args.aux_in != nullptr);
     constexpr uint32_t kSideTile = EPI == EPI_DGLU ? 4096 : 2048;
-    ItemWalk<false, kTilesPerUnit> items(unit, num_units, ntiles, mt, nt, BN, 0);
-    int item = 0;
-    for (int t = unit; t < ntiles; t += num_units) {
-      const TileCoord c = items.get(item++, win, args);
+    for (int i = 0;; ++i) {
+      const TileCoord c = item(i, false, DS_TIMEOUT_EPILOGUE);
+      if (!c.valid) break;
       const int col0 = c.n0 + rank * 128 + quad * 32;  // this warp's first weight column
       const int chunks = col0 < N ? ((c.unit_rows + 63) >> 6) * 2 : 0;
       if (side_input && half < chunks) {

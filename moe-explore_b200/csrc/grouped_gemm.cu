@@ -191,6 +191,12 @@ static moe_gemm_options resolve(const moe_gemm_options* o) {
 // half-empty last 256-column tile is far cheaper than narrow tiles throughout.
 static int pick_bn(int N) { return N <= 128 ? 128 : 256; }
 
+// Whether CTA pairs claim their work items (ItemQueue) or have them dealt out: the ring costs 1 to 2 us per launch, so from ten
+// items per pair on.  Launches with 4 items per pair 30 -> 32 us and 7 items 86 -> 87, but with 14 items and uneven rows 183 -> 179,
+// with 55 equal ones (weight gradients, 128 tokens) 107 -> 95 and 55 -> 51, and the whole 8192-token pass of 64 experts of
+// 7168 x 2048 under Zipf routing 19.9 -> 18.9 ms.
+static bool worth_claiming(int64_t items) { return items >= 10ll * (sm_count() / 2); }
+
 // What an M-grouped call may add to the plain contraction.
 struct MExtras {
   void* aux_out = nullptr;
@@ -418,6 +424,11 @@ static int mgrouped_common(const char* name, const void* a, const void* w, void*
   if (x.counts.group_indices != nullptr && tile_pairs != nullptr && x.gather_row_src == nullptr && x.push_bases == nullptr &&
       options == nullptr && mean_rows_per_expert < 6 * 2 * BM) {
     args.out_tma = x.push_row == nullptr && x.combine_row_src == nullptr;
+    // about a unit per expert that has rows, and for every further UNIT rows one
+    const int64_t unit = mean_rows_per_expert > 160 ? 256 : 128;
+    const int64_t hit = x.counts.routed_rows < E ? x.counts.routed_rows : E;
+    const int64_t units = x.counts.routed_rows / unit + hit / 2 > hit ? x.counts.routed_rows / unit + hit / 2 : hit;
+    if (worth_claiming(units * ((N + 255) / 256))) args.work_counter = x.counts.work_counter;
 #define MOE_MG_T(TYPE)                                                                                                 \
   (mean_rows_per_expert > 160                                                                                          \
        ? mgrouped_dispatch_t<TYPE, 256>(a, w, a_rows, out_rows, K, N, E, w_transposed, epi, args, dtype, lp)           \
@@ -541,7 +552,10 @@ static int kgrouped_common(const char* name, const void* a, int64_t gather_rows,
   // CTA pairs unless the contraction is at most one 64-row step per expert on average (measured at 64 rows per
   // expert, DeepSeek-V3 shape: weight1 gradient 4.00 -> 3.48 ms; at 128 rows per expert pairs are 9 % faster)
   const long long mean_rows_per_expert = (padded_rows - static_cast<long long>(num_experts) * (BM - 1)) / num_experts;
-  const bool pairs = o.single_cta == 0 ? mean_rows_per_expert > 64 : o.single_cta < 0;
+  // ... unless the pairs claim their work items (at most one step: 106.0 / 105.5 us dealt out, 64 experts x 2048 x 2048)
+  const int64_t items = static_cast<int64_t>(num_experts) * ((M + 2 * BM - 1) / (2 * BM)) * ((N + bn - 1) / bn);
+  args.work_counter = gather_row_src == nullptr && worth_claiming(items) ? counts.work_counter : nullptr;
+  const bool pairs = o.single_cta == 0 ? mean_rows_per_expert > 64 || args.work_counter != nullptr : o.single_cta < 0;
   // (above four steps an eighth of the loads at most is saved, for four more tensor maps per call)
   args.short_steps = counts.group_indices != nullptr && gather_row_src == nullptr && mean_rows_per_expert <= 4 * BK ? 1 : 0;
   const int64_t a_rows = gather_row_src != nullptr ? gather_rows : (counts.a_rows >= 0 ? counts.a_rows : padded_rows);

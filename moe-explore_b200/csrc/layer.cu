@@ -5,6 +5,13 @@
 
 namespace moe {
 
+// `counts` for a contraction that claims its work items from word `i`.
+static RowCounts claiming(const RowCounts& counts, uint32_t* counters, int i) {
+  RowCounts c = counts;
+  c.work_counter = counters != nullptr ? counters + i : nullptr;
+  return c;
+}
+
 static bool glu(int act) { return act == MOE_ACT_SWIGLU || act == MOE_ACT_GEGLU; }
 
 }  // namespace moe
@@ -33,7 +40,9 @@ extern "C" int moe_expert_forward(const moe_expert_pass* p, int steps, void* str
                              p->inter, p->d, 1, 0, MOE_ACT_NONE, p->dtype, 0, 1, nullptr, p->status, stream, out));
     return MOE_OK;
   }
-  const RowCounts counts{p->pad_offsets, p->group_indices};
+  RowCounts counts{p->pad_offsets, p->group_indices};
+  counts.routed_rows = rows;
+  uint32_t* const counters = p->gather ? nullptr : reinterpret_cast<uint32_t*>(p->counters);
   if (steps & MOE_FWD_TAIL)
     MOE_STEP(moe_router_tail(p->logits, const_cast<void*>(p->scores), const_cast<int64_t*>(p->expert_idx), p->num_tokens,
                              p->num_experts, p->topk, p->softmax_before_topk, p->normalize, p->dtype, stream));
@@ -45,9 +54,9 @@ extern "C" int moe_expert_forward(const moe_expert_pass* p, int steps, void* str
     // rows do not mix in a forward pass, and only a weight gradient contracts over the padding rows
     if (p->keep)
       MOE_STEP(dispatch_rows(p->x, p->dst_row, p->row_src, p->num_mtiles, p->xs, p->num_tokens, p->topk, p->padded_rows, p->d,
-                                 p->dtype, stream, true));
+                                 p->dtype, stream, true, counters));
     else
-      MOE_STEP(moe_dispatch_rows_only(p->x, p->dst_row, p->xs, p->num_tokens, p->topk, p->d, p->dtype, stream));
+      MOE_STEP(dispatch_rows_only(p->x, p->dst_row, p->xs, p->num_tokens, p->topk, p->d, p->dtype, stream, counters));
   }
   if (steps & MOE_FWD_UP) {
     if (p->gather)
@@ -57,7 +66,7 @@ extern "C" int moe_expert_forward(const moe_expert_pass* p, int steps, void* str
     else
       MOE_STEP(mgrouped_gemm(p->xs, p->w1, p->hidden, p->pre_act, p->mtile_expert, p->tile_pairs, p->num_mtiles,
                                  p->padded_rows, p->d, up_cols, p->num_experts, 0, p->act, p->dtype, 0, 1, nullptr, p->status,
-                                 stream, counts));
+                                 stream, claiming(counts, counters, 0)));
   }
   if (steps & MOE_FWD_DOWN) {
     if (p->fused_combine) {
@@ -65,10 +74,10 @@ extern "C" int moe_expert_forward(const moe_expert_pass* p, int steps, void* str
       chained_launches() = false;  // the memset stands between
       MOE_STEP(mgrouped_gemm_combine(p->hidden, p->w2, p->out, p->row_src, p->scores, p->topk, p->mtile_expert, p->tile_pairs,
                                          p->num_mtiles, p->padded_rows, p->inter, p->d, p->num_experts, 0, p->dtype, nullptr,
-                                         p->status, stream, counts));
+                                         p->status, stream, claiming(counts, counters, 1)));
     } else {
       MOE_STEP(mgrouped_gemm(p->hidden, p->w2, p->ys, nullptr, p->mtile_expert, p->tile_pairs, p->num_mtiles, p->padded_rows,
-                                 p->inter, p->d, p->num_experts, 0, MOE_ACT_NONE, p->dtype, 0, 1, nullptr, p->status, stream, counts));
+                                 p->inter, p->d, p->num_experts, 0, MOE_ACT_NONE, p->dtype, 0, 1, nullptr, p->status, stream, claiming(counts, counters, 1)));
     }
   }
   if ((steps & MOE_FWD_FOLD) && !p->fused_combine)
@@ -103,38 +112,40 @@ extern "C" int moe_expert_backward(const moe_expert_pass* p, int steps, void* st
                              nullptr, p->status, stream, right));
     return MOE_OK;
   }
-  const RowCounts counts{p->pad_offsets, p->group_indices};
+  RowCounts counts{p->pad_offsets, p->group_indices};
+  counts.routed_rows = p->num_tokens * p->topk;
+  uint32_t* const counters = reinterpret_cast<uint32_t*>(p->counters);
   if (steps & MOE_BWD_FOLD)
     MOE_STEP(combine_bwd_tokens(p->grad_out, p->scores, p->ys, p->dst_row, p->row_src, p->num_mtiles, p->gs, p->d_scores,
-                                    p->num_tokens, p->topk, p->d, p->dtype, stream, true));
+                                    p->num_tokens, p->topk, p->d, p->dtype, stream, true, counters));
   if ((steps & MOE_BWD_ROUTER) && p->dl != nullptr)
     MOE_STEP(router_backward(p->logits, p->expert_idx, p->d_scores, p->router_w, p->dl, p->dlogits, p->router_t, p->num_tokens,
                              p->num_experts, p->topk, p->d, p->dtype, stream));
   if (steps & MOE_BWD_DOWN) {
     if (p->act == MOE_ACT_NONE)  // linear "activation": d_pre = gs @ W2^T
       MOE_STEP(mgrouped_gemm(p->gs, p->w2, p->d_pre, nullptr, p->mtile_expert, p->tile_pairs, p->num_mtiles, p->padded_rows,
-                                 p->d, p->inter, p->num_experts, 1, MOE_ACT_NONE, p->dtype, 0, 1, nullptr, p->status, stream, counts));
+                                 p->d, p->inter, p->num_experts, 1, MOE_ACT_NONE, p->dtype, 0, 1, nullptr, p->status, stream, claiming(counts, counters, 0)));
     else
       MOE_STEP(mgrouped_gemm_dglu(p->gs, p->w2, p->pre_act, p->d_pre, p->mtile_expert, p->tile_pairs, p->num_mtiles,
                                       p->padded_rows, p->d, p->inter, p->num_experts, p->act, p->dtype, 0, 1, nullptr, p->status,
-                                      stream, counts));
+                                      stream, claiming(counts, counters, 0)));
   }
   if (steps & MOE_BWD_UP)
     MOE_STEP(mgrouped_gemm(p->d_pre, p->w1, p->dxs, nullptr, p->mtile_expert, p->tile_pairs, p->num_mtiles, p->padded_rows,
-                               up_cols, p->d, p->num_experts, 1, MOE_ACT_NONE, p->dtype, 0, 1, nullptr, p->status, stream, counts));
+                               up_cols, p->d, p->num_experts, 1, MOE_ACT_NONE, p->dtype, 0, 1, nullptr, p->status, stream, claiming(counts, counters, 1)));
   if (steps & MOE_BWD_FOLD_DX)
     MOE_STEP(combine_topk(p->dxs, nullptr, p->dst_row, p->dx, p->num_tokens, p->topk, p->d, p->dtype, nullptr, p->dl,
                           p->expert_idx, p->router_t, stream));
   if (steps & MOE_BWD_DW1) {
     if (p->gather)  // x is the layer input in token order: its rows are gathered by the loads again
       MOE_STEP(kgrouped_gemm_gather(p->x, p->num_tokens, p->row_src, p->topk, p->d_pre, p->d_w1, p->pad_offsets,
-                                        p->padded_rows, p->d, up_cols, p->num_experts, p->dtype, nullptr, p->status, stream, counts));
+                                        p->padded_rows, p->d, up_cols, p->num_experts, p->dtype, nullptr, p->status, stream, claiming(counts, counters, 2)));
     else
       MOE_STEP(kgrouped_gemm(p->xs, p->d_pre, p->d_w1, p->pad_offsets, p->padded_rows, p->d, up_cols, p->num_experts, p->dtype,
-                                 nullptr, p->status, stream, counts));
+                                 nullptr, p->status, stream, claiming(counts, counters, 2)));
   }
   if (steps & MOE_BWD_DW2)
     MOE_STEP(kgrouped_gemm(p->hidden, p->gs, p->d_w2, p->pad_offsets, p->padded_rows, p->inter, p->d, p->num_experts, p->dtype,
-                               nullptr, p->status, stream, counts));
+                               nullptr, p->status, stream, claiming(counts, counters, 3)));
   return MOE_OK;
 }

@@ -507,6 +507,7 @@ struct GroupsOut {
   int32_t* in_rows;
   int32_t* out_rows;
   int32_t mtiles_bound;
+  uint32_t* work_counters;
 };
 
 __global__ void __launch_bounds__(kMaxExperts)
@@ -516,6 +517,7 @@ layout_from_groups_kernel(const int32_t* __restrict__ group_indices, int64_t R, 
   __shared__ int32_t sums[2][32], cut[2];
   const int e = threadIdx.x, lane = e & 31, warp = e >> 5;
   grid_release();
+  if (out.work_counters != nullptr && blockIdx.x == 0 && e < kWorkCounters) out.work_counters[e] = 0;
   int32_t cnt = 0, lo = 0;
   if (e < E) {
     // a prefix that is not monotone, does not start at 0 or does not end at R describes no layout: such experts
@@ -764,7 +766,7 @@ extern "C" int moe_layout_from_groups(const int32_t* group_indices, int64_t num_
                 "moe_layout_from_groups: mtile_expert, tile_pairs and num_mtiles go together");
   return layout_from_groups(group_indices, num_rows, num_experts, nullptr, 0,
                             GroupsOut{pad_offsets, row_src, dst_row, mtile_expert, tile_pairs, num_mtiles, nullptr, nullptr,
-                                      static_cast<int32_t>(moe_mtiles_bound(num_rows, num_experts))},
+                                      static_cast<int32_t>(moe_mtiles_bound(num_rows, num_experts)), nullptr},
                             status, static_cast<cudaStream_t>(stream));
 }
 
@@ -789,13 +791,16 @@ extern "C" int moe_rows_gemm(const moe_rows_pass* p, int steps, void* stream) {
     MOE_STEP(layout_from_groups(p->group_indices, p->num_rows, p->num_experts, p->gather || p->scatter ? p->perm : nullptr,
                                 p->scatter,
                                 GroupsOut{p->pad_offsets, nullptr, nullptr, p->mtile_expert, p->tile_pairs, p->num_mtiles,
-                                          p->gather ? p->in_rows : nullptr, p->out_rows, static_cast<int32_t>(mtiles)},
+                                          p->gather ? p->in_rows : nullptr, p->out_rows, static_cast<int32_t>(mtiles),
+                                          reinterpret_cast<uint32_t*>(p->counters)},
                                 p->status, static_cast<cudaStream_t>(stream)));
   if ((steps & MOE_ROWS_GATHER) && p->gather)
     MOE_STEP(gather_rows(p->a, p->a_rows, p->in_rows, p->num_mtiles, p->padded, padded_rows, p->k_dim, p->topk, p->dtype, stream,
                          true));
   if (steps & MOE_ROWS_GEMM) {
-    const RowCounts counts{p->pad_offsets, p->group_indices};
+    RowCounts counts{p->pad_offsets, p->group_indices};
+    counts.work_counter = reinterpret_cast<uint32_t*>(p->counters);
+    counts.routed_rows = p->num_rows;
     // rows that are in expert order already are read where they are; gathered ones from their padded copy
     MOE_STEP(mgrouped_gemm_rows(p->gather ? p->padded : p->a, p->gather ? -1 : p->a_rows, p->w, p->out, p->out_rows,
                                 p->mtile_expert, p->tile_pairs, p->num_mtiles, padded_rows, p->k_dim, p->n_dim, p->num_experts,

@@ -103,6 +103,11 @@ __device__ __forceinline__ void zero_padding(const int32_t* __restrict__ row_src
   }
 }
 
+// See kWorkCounters.
+__device__ __forceinline__ void zero_counters(uint32_t* work_counters) {
+  if (work_counters != nullptr && blockIdx.x == 0 && threadIdx.x < kWorkCounters) work_counters[threadIdx.x] = 0;
+}
+
 // Token-major form of the same movement for the layer's own dispatch: dst[dst_row[t*topk + s], :] = src[t, :].
 // Every token row is read from HBM once and written topk times (the row-major gather re-reads it topk
 // times, and the tokens of an expert are scattered over the whole input).  The second part of the grid
@@ -142,9 +147,10 @@ __device__ __forceinline__ void dispatch_tokens(const uint4* __restrict__ src, c
 template <int TPR>
 __global__ void __launch_bounds__(kRowThreads)
 dispatch_rows_kernel(const uint4* src, const int32_t* dst_row, const int32_t* row_src, const int32_t* num_mtiles, uint4* dst,
-                     int64_t num_tokens, int topk, int vec_per_row, int token_blocks, bool live_blocks_only) {
+                     int64_t num_tokens, int topk, int vec_per_row, int token_blocks, bool live_blocks_only, uint32_t* work_counters) {
   grid_release();
   grid_wait();
+  zero_counters(work_counters);
   dispatch_tokens<TPR>(src, dst_row, row_src, num_mtiles, dst, num_tokens, topk, vec_per_row, token_blocks, live_blocks_only);
 }
 
@@ -462,9 +468,10 @@ template <typename T>
 __global__ void __launch_bounds__(kRowThreads)
 combine_bwd_tokens_kernel(const uint4* dout, const T* scores, const uint4* ys, const int32_t* dst_row, const int32_t* row_src,
                           const int32_t* num_mtiles, uint4* gs, T* dscores, int64_t num_slots, int topk, int vec_per_row,
-                          int slot_blocks, bool live_blocks_only) {
+                          int slot_blocks, bool live_blocks_only, uint32_t* work_counters) {
   grid_release();
   grid_wait();
+  zero_counters(work_counters);
   constexpr int kWarps = kRowThreads / 32;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (static_cast<int>(blockIdx.x) >= slot_blocks) {
@@ -556,15 +563,16 @@ static void launch_copy_rows(const void* src, const Index* index, const int32_t*
 
 // row_src == nullptr: the padding rows are left as they are.
 static void launch_dispatch(const void* src, const int32_t* dst_row, const int32_t* row_src, const int32_t* num_mtiles, void* dst,
-                            int64_t num_tokens, int topk, int vec_per_row, cudaStream_t s, bool live_blocks_only = false) {
+                            int64_t num_tokens, int topk, int vec_per_row, cudaStream_t s, bool live_blocks_only = false,
+                            uint32_t* work_counters = nullptr) {
   const int tpr = copy_threads_per_row(vec_per_row);
   const int64_t groups = (num_tokens + kRowThreads / tpr - 1) / (kRowThreads / tpr);
   const int token_blocks = static_cast<int>(groups < (1 << 30) ? groups : (1 << 30));
   const int blocks = token_blocks + (row_src != nullptr ? sm_count() : 0);
   const uint4* in = static_cast<const uint4*>(src);
   uint4* out = static_cast<uint4*>(dst);
-  if (tpr == 32) launch_kernel(dispatch_rows_kernel<32>, blocks, kRowThreads, s, in, dst_row, row_src, num_mtiles, out, num_tokens, topk, vec_per_row, token_blocks, live_blocks_only);
-  else launch_kernel(dispatch_rows_kernel<64>, blocks, kRowThreads, s, in, dst_row, row_src, num_mtiles, out, num_tokens, topk, vec_per_row, token_blocks, live_blocks_only);
+  if (tpr == 32) launch_kernel(dispatch_rows_kernel<32>, blocks, kRowThreads, s, in, dst_row, row_src, num_mtiles, out, num_tokens, topk, vec_per_row, token_blocks, live_blocks_only, work_counters);
+  else launch_kernel(dispatch_rows_kernel<64>, blocks, kRowThreads, s, in, dst_row, row_src, num_mtiles, out, num_tokens, topk, vec_per_row, token_blocks, live_blocks_only, work_counters);
 }
 
 // The slots whose loads are issued together: the smallest power of two that covers topk, at most 8 (a wider one wastes
@@ -672,12 +680,13 @@ extern "C" int moe_gather_rows(const void* src, int64_t src_rows, const int32_t*
 namespace moe {
 int dispatch_rows(const void* src, const int32_t* dst_row, const int32_t* row_src, const int32_t* num_mtiles, void* dst,
                   int64_t num_tokens, int topk, int64_t padded_rows, int cols, int dtype, void* stream, bool
-                  live_blocks_only) {
+                  live_blocks_only, uint32_t* work_counters) {
   MOE_CHECK_ARG(num_tokens >= 0 && topk > 0 && padded_rows > 0, "moe_dispatch_rows: bad sizes");
   MOE_CHECK_ARG(src && dst_row && row_src && num_mtiles && dst, "moe_dispatch_rows: null pointer argument");
   MOE_CHECK_ARG(aligned16(src) && aligned16(dst), "moe_dispatch_rows: pointers must be 16-byte aligned");
   MOE_ROW_COMMON_CHECKS("moe_dispatch_rows", cols, dtype);
-  launch_dispatch(src, dst_row, row_src, num_mtiles, dst, num_tokens, topk, cols / 8, static_cast<cudaStream_t>(stream), live_blocks_only);
+  launch_dispatch(src, dst_row, row_src, num_mtiles, dst, num_tokens, topk, cols / 8, static_cast<cudaStream_t>(stream), live_blocks_only,
+                  work_counters);
   MOE_CUDA(cudaGetLastError());
   return MOE_OK;
 }
@@ -686,17 +695,23 @@ int dispatch_rows(const void* src, const int32_t* dst_row, const int32_t* row_sr
 extern "C" int moe_dispatch_rows(const void* src, const int32_t* dst_row, const int32_t* row_src, const int32_t*
                                  num_mtiles, void* dst, int64_t num_tokens, int topk, int64_t padded_rows, int cols, int
                                  dtype, void* stream) {
-  return dispatch_rows(src, dst_row, row_src, num_mtiles, dst, num_tokens, topk, padded_rows, cols, dtype, stream, false);
+  return dispatch_rows(src, dst_row, row_src, num_mtiles, dst, num_tokens, topk, padded_rows, cols, dtype, stream, false, nullptr);
 }
 
 extern "C" int moe_dispatch_rows_only(const void* src, const int32_t* dst_row, void* dst, int64_t num_tokens, int topk,
                                       int cols, int dtype, void* stream) {
+  return dispatch_rows_only(src, dst_row, dst, num_tokens, topk, cols, dtype, stream, nullptr);
+}
+
+int moe::dispatch_rows_only(const void* src, const int32_t* dst_row, void* dst, int64_t num_tokens, int topk, int cols, int dtype,
+                            void* stream, uint32_t* work_counters) {
   MOE_CHECK_ARG(num_tokens >= 0 && topk > 0, "moe_dispatch_rows_only: bad sizes");
   MOE_CHECK_ARG(src && dst_row && dst, "moe_dispatch_rows_only: null pointer argument");
   MOE_CHECK_ARG(aligned16(src) && aligned16(dst), "moe_dispatch_rows_only: pointers must be 16-byte aligned");
   MOE_ROW_COMMON_CHECKS("moe_dispatch_rows_only", cols, dtype);
   if (num_tokens == 0) return MOE_OK;
-  launch_dispatch(src, dst_row, nullptr, nullptr, dst, num_tokens, topk, cols / 8, static_cast<cudaStream_t>(stream));
+  launch_dispatch(src, dst_row, nullptr, nullptr, dst, num_tokens, topk, cols / 8, static_cast<cudaStream_t>(stream), false,
+                  work_counters);
   MOE_CUDA(cudaGetLastError());
   return MOE_OK;
 }
@@ -851,7 +866,7 @@ extern "C" int moe_combine_topk(const void* ys, const void* scores, const int32_
 namespace moe {
 int combine_bwd_tokens(const void* dout, const void* scores, const void* ys, const int32_t* dst_row, const int32_t*
                        row_src, const int32_t* num_mtiles, void* gs, void* dscores, int64_t num_tokens, int topk, int
-                       cols, int dtype, void* stream, bool live_blocks_only) {
+                       cols, int dtype, void* stream, bool live_blocks_only, uint32_t* work_counters) {
   MOE_CHECK_ARG(dout && scores && ys && dst_row && row_src && num_mtiles && gs && dscores,
                 "moe_combine_bwd_tokens: null pointer argument");
   MOE_CHECK_ARG(aligned16(dout) && aligned16(ys) && aligned16(gs), "moe_combine_bwd_tokens: pointers must be 16-byte aligned");
@@ -864,11 +879,11 @@ int combine_bwd_tokens(const void* dout, const void* scores, const void* ys, con
   if (dtype == MOE_DTYPE_BF16) {
     launch_kernel(
         combine_bwd_tokens_kernel<__nv_bfloat16>, blocks, kRowThreads, s, static_cast<const uint4*>(dout), static_cast<const __nv_bfloat16*>(scores), static_cast<const uint4*>(ys), dst_row,
-        row_src, num_mtiles, static_cast<uint4*>(gs), static_cast<__nv_bfloat16*>(dscores), slots, topk, cols / 8, slot_blocks, live_blocks_only);
+        row_src, num_mtiles, static_cast<uint4*>(gs), static_cast<__nv_bfloat16*>(dscores), slots, topk, cols / 8, slot_blocks, live_blocks_only, work_counters);
   } else {
     launch_kernel(
         combine_bwd_tokens_kernel<__half>, blocks, kRowThreads, s, static_cast<const uint4*>(dout), static_cast<const __half*>(scores), static_cast<const uint4*>(ys), dst_row, row_src,
-        num_mtiles, static_cast<uint4*>(gs), static_cast<__half*>(dscores), slots, topk, cols / 8, slot_blocks, live_blocks_only);
+        num_mtiles, static_cast<uint4*>(gs), static_cast<__half*>(dscores), slots, topk, cols / 8, slot_blocks, live_blocks_only, work_counters);
   }
   MOE_CUDA(cudaGetLastError());
   return MOE_OK;
@@ -879,7 +894,7 @@ extern "C" int moe_combine_bwd_tokens(const void* dout, const void* scores, cons
                                       int32_t* row_src, const int32_t* num_mtiles, void* gs, void* dscores, int64_t
                                       num_tokens, int topk, int cols, int dtype, void* stream) {
   return combine_bwd_tokens(dout, scores, ys, dst_row, row_src, num_mtiles, gs, dscores, num_tokens, topk, cols, dtype,
-                            stream, false);
+                            stream, false, nullptr);
 }
 
 extern "C" int moe_combine_bwd(const void* dout, const void* scores, const void* ys, const int32_t* row_src,

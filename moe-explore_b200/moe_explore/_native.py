@@ -24,6 +24,7 @@ TILE_M = 128
 ROUTE_ONE_LAUNCH_ROWS = 131072   # csrc/routing.cu: up to here a whole B200 takes the routing metadata in one launch
 ROUTE_CHIP_WIDE_LAUNCHES = 4     # ... and beyond
 # codes a kernel may leave in a status word (include/moe_sm100.h, moe_check_status)
+WORK_COUNTERS = 4   # words a pass claims its work items from
 STATUS_WAVE_FALLBACK = 4
 STATUS_BAD_LAYOUT = 5
 STATUS_BAD_EXPERT_ID = 100
@@ -46,7 +47,7 @@ class ExpertPass(ctypes.Structure):
                [("workspace_bytes", c_size_t)] + \
                [(f, c_void_p) for f in ("xs", "pre_act", "hidden", "ys", "out", "grad_out", "gs", "d_scores", "d_pre", "dxs", "dx",
                                         "d_w1", "d_w2", "addend", "logits", "router_w", "dl", "dlogits", "router_t")] + \
-               [(f, c_int32) for f in ("softmax_before_topk", "normalize")]
+               [(f, c_int32) for f in ("softmax_before_topk", "normalize")] + [("counters", c_void_p)]
 
 
 class RowsPass(ctypes.Structure):
@@ -54,7 +55,7 @@ class RowsPass(ctypes.Structure):
     _fields_ = [(f, c_int64) for f in ("num_rows", "a_rows")] + \
                [(f, c_int32) for f in ("num_experts", "k_dim", "n_dim", "topk", "act", "dtype", "gather", "scatter")] + \
                [(f, c_void_p) for f in ("a", "w", "out", "group_indices", "perm", "pad_offsets", "in_rows", "out_rows",
-                                        "mtile_expert", "tile_pairs", "num_mtiles", "status", "padded")]
+                                        "mtile_expert", "tile_pairs", "num_mtiles", "status", "padded", "counters")]
 
 
 # name -> (restype, argtypes); the single source for both binding and the symbol-export test

@@ -122,10 +122,11 @@ def _forward(x, scores, weight1, weight2, routing, act, gather_in_gemm: bool, fu
             steps.append((_native.FWD_TAIL, "router:topk", 1))
         steps.append((_native.FWD_ROUTE, "routing", launches))
     # index arrays, scores and indices of the tail, expert-sorted input, un-activated product (needed by the backward pass; not
-    # kept for inference or without an activation), activated product, per-slot rows
+    # kept for inference or without an activation), activated product, per-slot rows, words the contractions claim work items from
     scratch = (4 * num_words, 2 * rows if tail else 0, 8 * rows if tail else 0, 0 if gather_in_gemm else 2 * rp * d,
-               2 * rp * n1 if act is not None and needs_grad else 0, 2 * rp * inter, 2 * rp * d if fold else 0)
-    buffers, (words, tail_scores, tail_ids, xs, pre_act, hidden, ys) = _buffers(scratch, x.device)
+               2 * rp * n1 if act is not None and needs_grad else 0, 2 * rp * inter, 2 * rp * d if fold else 0,
+               4 * _native.WORK_COUNTERS)
+    buffers, (words, tail_scores, tail_ids, xs, pre_act, hidden, ys, counters) = _buffers(scratch, x.device)
     if planned:
         plan_ptrs = _plan_pointers(routing)
     else:
@@ -149,7 +150,7 @@ def _forward(x, scores, weight1, weight2, routing, act, gather_in_gemm: bool, fu
         T, rp, d, inter, E, topk, act_code, code, gather_in_gemm, not fold, needs_grad, 0, ids, x.data_ptr(),
         tail_scores if tail is not None else scores.data_ptr(), weight1.data_ptr(), weight2.data_ptr(), *plan_ptrs, ptr(workspace),
         0 if workspace is None else workspace.numel(), xs, pre_act, hidden, ys, out.data_ptr())
-    p.addend = ptr(addend)
+    p.addend, p.counters = ptr(addend), counters
     if tail is not None:
         p.logits, p.softmax_before_topk, p.normalize = tail[0].data_ptr(), bool(tail[1]), bool(tail[2])
     _native.run_pass("moe_expert_forward", p, steps, rows)
@@ -173,13 +174,14 @@ def _backward(info: _Pass, saved, grad_out, router=None):
     act = info.act
     rows = T * topk
     grad_out = grad_out.contiguous()
-    words, tail_scores, tail_ids, xs, pre_act, hidden, ys = _addresses(info.scratch, buffers)
+    words, tail_scores, tail_ids, xs, pre_act, hidden, ys, _ = _addresses(info.scratch, buffers)
     new = lambda *shape: torch.empty(shape, dtype=grad_out.dtype, device=grad_out.device)
 
     # score-scaled dOut rows, gradient of the un-activated product, per-slot rows of dX; with a router the gradient of the selected
     # logits in fp32 and the transposed router weight
-    scratch = (2 * rp * d, 2 * rp * n1, 2 * rp * d) + ((4 * rows, 2 * E * d) if router is not None else (0, 0))
-    held, (gs, d_pre, dxs, dl, router_t) = _buffers(scratch, grad_out.device)
+    scratch = (2 * rp * d, 2 * rp * n1, 2 * rp * d, 4 * _native.WORK_COUNTERS) + \
+        ((4 * rows, 2 * E * d) if router is not None else (0, 0))
+    held, (gs, d_pre, dxs, counters, dl, router_t) = _buffers(scratch, grad_out.device)
     d_scores, dx = new(T, topk), new(T, d)
     d_w1, d_w2 = torch.empty_like(weight1), torch.empty_like(weight2)
     if info.routing is not None:
@@ -192,6 +194,7 @@ def _backward(info: _Pass, saved, grad_out, router=None):
         rows_in, tail_scores if info.tail else scores.data_ptr(), weight1.data_ptr(), weight2.data_ptr(), *plan_ptrs, None, 0,
         rows_in, pre_act, hidden, ys, None, grad_out.data_ptr(), gs, d_scores.data_ptr(), d_pre, dxs, dx.data_ptr(),
         d_w1.data_ptr(), d_w2.data_ptr())
+    p.counters = counters
     steps = [(_native.BWD_FOLD, "rows:combine_bwd", 1),
              (_native.BWD_DOWN, "mgrouped_gemm:wt" if act is None else "mgrouped_gemm:dglu", 1),
              (_native.BWD_UP, "mgrouped_gemm:wt", 1), (_native.BWD_FOLD_DX, "rows:combine", 1),

@@ -80,18 +80,19 @@ def m_grouped_gemm(token: torch.Tensor, params: MGroupedGEMMParams, autotune_mod
     _native.run_pass("moe_rows_gemm", _native.RowsPass(
         rows, token.size(0), num_experts, k_dim, n_dim, params.topk if params.gather else 1, _native.ACT_CODES[act],
         _native.dtype_code(token.dtype), bool(params.gather), bool(params.scatter), token.data_ptr(), weight.data_ptr(),
-        out.data_ptr(), groups.data_ptr(), ptr(perm), *[base + o for o in offsets],
-        device_status(token.get_device()).data_ptr(), ptr(padded)), steps, rows)
+        out.data_ptr(), groups.data_ptr(), ptr(perm), *[base + o for o in offsets[:-1]],
+        device_status(token.get_device()).data_ptr(), ptr(padded), base + offsets[-1]), steps, rows)
     return out
 
 
 @functools.lru_cache(maxsize=256)
 def _maps_layout(rows: int, num_experts: int):
-    """(padded rows, byte offsets of pad_offsets, in_rows, out_rows, mtile_expert, tile_pairs, num_mtiles, int32 words)."""
+    """(padded rows, byte offsets of pad_offsets, in_rows, out_rows, mtile_expert, tile_pairs, num_mtiles, work counters, int32
+    words)."""
     rp = _native.padded_rows_bound(rows, num_experts)
     tiles = rp // _native.TILE_M
     offsets, words = [], 0
-    for n in (num_experts + 1, rp, rp, tiles, tiles + num_experts + 1, 4):
+    for n in (num_experts + 1, rp, rp, tiles, tiles + num_experts + 1, 4, _native.WORK_COUNTERS):
         offsets.append(4 * words)
         words += (n + 3) // 4 * 4
     return rp, tuple(offsets), words
