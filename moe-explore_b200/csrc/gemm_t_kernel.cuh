@@ -176,11 +176,11 @@ grouped_gemm_kernel(const __grid_constant__ TMaps maps, const GemmArgs args) {
     tmem_relinquish_pair();
   }
   prefetch_maps(args);
-  grid_wait();  // nothing above reads or writes global memory
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();  // the peer's barriers must be initialised before anything arrives on them
   tc_fence_after();
+  grid_wait();  // nothing above reads or writes global memory
   const uint32_t tmem_base = *tmem_slot;
 
   int mt, nt;
