@@ -137,7 +137,7 @@ int dispatch_rows(const void* src, const int32_t* dst_row, const int32_t* row_sr
                   int64_t num_tokens, int topk, int64_t padded_rows, int cols, int dtype, void* stream, bool live_blocks_only,
                   uint32_t* work_counters);
 int dispatch_rows_only(const void* src, const int32_t* dst_row, void* dst, int64_t num_tokens, int topk, int cols, int dtype,
-                       void* stream, uint32_t* work_counters);
+                       void* stream, uint32_t* work_counters, void* clear);
 // moe_combine_topk with further summands, all nullable (FoldExtra in csrc/rows.cu).
 int combine_topk(const void* ys, const void* scores, const int32_t* dst_row, void* out, int64_t num_tokens, int topk, int cols,
                  int dtype, const void* addend, const float* dlogits, const int64_t* experts, const void* router_t,

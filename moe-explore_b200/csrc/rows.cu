@@ -111,12 +111,12 @@ __device__ __forceinline__ void zero_counters(uint32_t* work_counters) {
 // Token-major form of the same movement for the layer's own dispatch: dst[dst_row[t*topk + s], :] = src[t, :].
 // Every token row is read from HBM once and written topk times (the row-major gather re-reads it topk
 // times, and the tokens of an expert are scattered over the whole input).  The second part of the grid
-// zeroes the padding rows.
+// zeroes the padding rows.  `clear`: a buffer like src that is set to zero on the way.
 template <int TPR>
 __device__ __forceinline__ void dispatch_tokens(const uint4* __restrict__ src, const int32_t* __restrict__ dst_row,
                                                 const int32_t* __restrict__ row_src, const int32_t* __restrict__ num_mtiles,
                                                 uint4* __restrict__ dst, int64_t num_tokens, int topk, int vec_per_row,
-                                                int token_blocks, bool live_blocks_only) {
+                                                int token_blocks, bool live_blocks_only, uint4* __restrict__ clear) {
   constexpr int kRows = kRowThreads / TPR;
   if (static_cast<int>(blockIdx.x) >= token_blocks) {
     zero_padding(row_src, num_mtiles, dst, vec_per_row, (blockIdx.x - token_blocks) * (kRowThreads / 32) + (threadIdx.x >> 5),
@@ -133,6 +133,11 @@ __device__ __forceinline__ void dispatch_tokens(const uint4* __restrict__ src, c
 #pragma unroll
       for (int i = 0; i < kRowLoads; ++i)
         u[i] = v0 + i * TPR < vec_per_row ? s[v0 + i * TPR] : make_uint4(0, 0, 0, 0);
+      if (clear != nullptr) {
+#pragma unroll
+        for (int i = 0; i < kRowLoads; ++i)
+          if (v0 + i * TPR < vec_per_row) clear[t * vec_per_row + v0 + i * TPR] = make_uint4(0, 0, 0, 0);
+      }
       for (int k = 0; k < topk; ++k) {
         const int32_t p = rows[k];  // negative: the routing metadata dropped this (token, slot)
         if (p < 0) continue;
@@ -147,11 +152,12 @@ __device__ __forceinline__ void dispatch_tokens(const uint4* __restrict__ src, c
 template <int TPR>
 __global__ void __launch_bounds__(kRowThreads)
 dispatch_rows_kernel(const uint4* src, const int32_t* dst_row, const int32_t* row_src, const int32_t* num_mtiles, uint4* dst,
-                     int64_t num_tokens, int topk, int vec_per_row, int token_blocks, bool live_blocks_only, uint32_t* work_counters) {
+                     int64_t num_tokens, int topk, int vec_per_row, int token_blocks, bool live_blocks_only, uint32_t* work_counters,
+                     uint4* clear) {
   grid_release();
   grid_wait();
   zero_counters(work_counters);
-  dispatch_tokens<TPR>(src, dst_row, row_src, num_mtiles, dst, num_tokens, topk, vec_per_row, token_blocks, live_blocks_only);
+  dispatch_tokens<TPR>(src, dst_row, row_src, num_mtiles, dst, num_tokens, topk, vec_per_row, token_blocks, live_blocks_only, clear);
 }
 
 // Row window of a pull: everything, or the rows of the experts of chunk `chunk_index` of `chunk_count` (the same
@@ -564,15 +570,15 @@ static void launch_copy_rows(const void* src, const Index* index, const int32_t*
 // row_src == nullptr: the padding rows are left as they are.
 static void launch_dispatch(const void* src, const int32_t* dst_row, const int32_t* row_src, const int32_t* num_mtiles, void* dst,
                             int64_t num_tokens, int topk, int vec_per_row, cudaStream_t s, bool live_blocks_only = false,
-                            uint32_t* work_counters = nullptr) {
+                            uint32_t* work_counters = nullptr, void* clear = nullptr) {
   const int tpr = copy_threads_per_row(vec_per_row);
   const int64_t groups = (num_tokens + kRowThreads / tpr - 1) / (kRowThreads / tpr);
   const int token_blocks = static_cast<int>(groups < (1 << 30) ? groups : (1 << 30));
   const int blocks = token_blocks + (row_src != nullptr ? sm_count() : 0);
   const uint4* in = static_cast<const uint4*>(src);
   uint4* out = static_cast<uint4*>(dst);
-  if (tpr == 32) launch_kernel(dispatch_rows_kernel<32>, blocks, kRowThreads, s, in, dst_row, row_src, num_mtiles, out, num_tokens, topk, vec_per_row, token_blocks, live_blocks_only, work_counters);
-  else launch_kernel(dispatch_rows_kernel<64>, blocks, kRowThreads, s, in, dst_row, row_src, num_mtiles, out, num_tokens, topk, vec_per_row, token_blocks, live_blocks_only, work_counters);
+  if (tpr == 32) launch_kernel(dispatch_rows_kernel<32>, blocks, kRowThreads, s, in, dst_row, row_src, num_mtiles, out, num_tokens, topk, vec_per_row, token_blocks, live_blocks_only, work_counters, static_cast<uint4*>(clear));
+  else launch_kernel(dispatch_rows_kernel<64>, blocks, kRowThreads, s, in, dst_row, row_src, num_mtiles, out, num_tokens, topk, vec_per_row, token_blocks, live_blocks_only, work_counters, static_cast<uint4*>(clear));
 }
 
 // The slots whose loads are issued together: the smallest power of two that covers topk, at most 8 (a wider one wastes
@@ -700,18 +706,18 @@ extern "C" int moe_dispatch_rows(const void* src, const int32_t* dst_row, const 
 
 extern "C" int moe_dispatch_rows_only(const void* src, const int32_t* dst_row, void* dst, int64_t num_tokens, int topk,
                                       int cols, int dtype, void* stream) {
-  return dispatch_rows_only(src, dst_row, dst, num_tokens, topk, cols, dtype, stream, nullptr);
+  return dispatch_rows_only(src, dst_row, dst, num_tokens, topk, cols, dtype, stream, nullptr, nullptr);
 }
 
 int moe::dispatch_rows_only(const void* src, const int32_t* dst_row, void* dst, int64_t num_tokens, int topk, int cols, int dtype,
-                            void* stream, uint32_t* work_counters) {
+                            void* stream, uint32_t* work_counters, void* clear) {
   MOE_CHECK_ARG(num_tokens >= 0 && topk > 0, "moe_dispatch_rows_only: bad sizes");
   MOE_CHECK_ARG(src && dst_row && dst, "moe_dispatch_rows_only: null pointer argument");
   MOE_CHECK_ARG(aligned16(src) && aligned16(dst), "moe_dispatch_rows_only: pointers must be 16-byte aligned");
   MOE_ROW_COMMON_CHECKS("moe_dispatch_rows_only", cols, dtype);
   if (num_tokens == 0) return MOE_OK;
   launch_dispatch(src, dst_row, nullptr, nullptr, dst, num_tokens, topk, cols / 8, static_cast<cudaStream_t>(stream), false,
-                  work_counters);
+                  work_counters, clear);
   MOE_CUDA(cudaGetLastError());
   return MOE_OK;
 }
