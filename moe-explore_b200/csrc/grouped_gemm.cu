@@ -415,22 +415,23 @@ static int mgrouped_common(const char* name, const void* a, const void* w, void*
   const int64_t out_rows = x.counts.out_rows >= 0 ? x.counts.out_rows : padded_rows;
   // Inside a pass (the routed counts are known): transposed tiles while an expert has few enough rows for its last tile to
   // matter; from six pairs of tiles on (2048 rows of the widest layer: equal within the power-bound spread of 4 %) the
-  // expert-aligned, wave-synchronised walk of the other kernel.  Row units of one tile up to 160 rows per expert, of two
-  // from there on: a unit of two tiles shares each weight step among up to 256 rows, one of a single tile keeps eight stages in
-  // flight instead of six and wastes less on rare experts (training sums of the four contractions, 32 experts, d 2048, I
-  // 1024, us, one / two tiles; even, moderately uneven, Zipf routing: 64 rows 210 / 216, 206 / 235, 226 / 233; 128 rows
-  // 229 / 231, 229 / 237, 247 / 269; 160 rows 245 / 235, 234 / 264, 261 / 254; 224 rows 260 / 265, 284 / 297, 322 / 298;
-  // 320 rows 343 / 326, 344 / 329, 350 / 320).
+  // expert-aligned, wave-synchronised walk of the other kernel.  Row units of one tile up to 112 rows per expert (160 in the gated
+  // backward, whose second staging tile costs the large units a stage), of two from there on: a unit of two tiles shares each
+  // weight step among up to 256 rows, one of a single tile keeps eight stages in flight instead of six and wastes less on rare
+  // experts.  64 experts, d 2048, I 1024, us, one / two tiles; even, moderately uneven, Zipf routing: forward pass's two
+  // contractions, 96 rows 159 / 162, 162 / 173, 177 / 182; 128 rows 178 / 170, 180 / 180, 195 / 189; 192 rows 213 / 188, 213 / 196,
+  // 229 / 218; 320 rows 301 / 277, 309 / 268, 320 / 276.  Gated backward, 128 rows 93 / 90, 90 / 85, 89 / 101; 160 rows 90 / 86,
+  // 92 / 93, 90 / 91; 224 rows 97 / 94, 102 / 98, 106 / 103.
   if (x.counts.group_indices != nullptr && tile_pairs != nullptr && x.gather_row_src == nullptr && x.push_bases == nullptr &&
       options == nullptr && mean_rows_per_expert < 6 * 2 * BM) {
     args.out_tma = x.push_row == nullptr && x.combine_row_src == nullptr;
     // about a unit per expert that has rows, and for every further UNIT rows one
-    const int64_t unit = mean_rows_per_expert > 160 ? 256 : 128;
+    const int64_t unit = mean_rows_per_expert > (epi == EPI_DGLU ? 160 : 112) ? 256 : 128;
     const int64_t hit = x.counts.routed_rows < E ? x.counts.routed_rows : E;
     const int64_t units = x.counts.routed_rows / unit + hit / 2 > hit ? x.counts.routed_rows / unit + hit / 2 : hit;
     if (worth_claiming(units * ((N + 255) / 256))) args.work_counter = x.counts.work_counter;
 #define MOE_MG_T(TYPE)                                                                                                 \
-  (mean_rows_per_expert > 160                                                                                          \
+  (unit == 256                                                                                                         \
        ? mgrouped_dispatch_t<TYPE, 256>(a, w, a_rows, out_rows, K, N, E, w_transposed, epi, args, dtype, lp)           \
        : mgrouped_dispatch_t<TYPE, 128>(a, w, a_rows, out_rows, K, N, E, w_transposed, epi, args, dtype, lp))
     return dtype == MOE_DTYPE_BF16 ? MOE_MG_T(__nv_bfloat16) : MOE_MG_T(__half);
