@@ -98,9 +98,11 @@ int moe_router_topk(const void* logits, void* scores, int64_t* indices, int32_t*
 
 /* The same with torch's choices instead of a tie rule of its own: what softmax(dtype=float32), torch.topk(sorted=False),
  * softmax and division by the sum leave, bit for bit -- larger values in ascending expert index, then values equal to the
- * k-th in ascending index, NaN above all.  E <= 1024, k <= min(32, E). */
-int moe_router_tail(const void* logits, void* scores, int64_t* indices, int64_t num_tokens, int num_experts, int topk,
-                    int softmax_before_topk, int normalize, int dtype, void* stream);
+ * k-th in ascending index, NaN above all.  With `bias` (fp32 [E], may be NULL) the selection is by value + bias and the scores are
+ * the values without it.  normalize: 0 no, 1 by the sum, 2 by the sum but not less than 1e-12.  scores_dtype: dtype, or any with
+ * fp32 logits.  E <= 1024, k <= min(32, E). */
+int moe_router_tail(const void* logits, const float* bias, void* scores, int64_t* indices, int64_t num_tokens, int num_experts,
+                    int topk, int softmax_before_topk, int normalize, int dtype, int scores_dtype, void* stream);
 
 /* ---------------------------------------------------------------------------------
  * (a) Routing metadata.  Replaces get_token_indices (src/moe_explore/expert_permute.py:19-41):
@@ -457,6 +459,9 @@ typedef struct moe_expert_pass {
   int32_t softmax_before_topk, normalize; /* MOE_FWD_TAIL */
   int32_t* counters; /* four words of this pass's own (not `gather`'s forward, not `identity`), or NULL: the contractions claim their
                       * work items from them instead of dealing them out.  Written by MOE_FWD_DISPATCH / MOE_BWD_FOLD */
+  const float* router_bias; /* MOE_FWD_TAIL: see moe_router_tail */
+  int32_t logits_dtype;
+  int32_t own_tie_rule; /* MOE_FWD_TAIL by moe_router_topk instead */
 } moe_expert_pass;
 
 /* sizeof(moe_expert_pass), for bindings that declare the struct themselves. */
@@ -468,7 +473,7 @@ size_t moe_expert_pass_size(void);
 #define MOE_FWD_DOWN 8
 #define MOE_FWD_FOLD 16
 #define MOE_FWD_ALL 31
-#define MOE_FWD_TAIL 32 /* first: moe_router_tail of `logits` into `scores` and `expert_idx` */
+#define MOE_FWD_TAIL 32 /* first: moe_router_tail (moe_router_topk) of `logits` into `scores` and `expert_idx` */
 int moe_expert_forward(const moe_expert_pass* pass, int steps, void* stream);
 
 #define MOE_BWD_FOLD 1    /* gs, d_scores */

@@ -43,9 +43,16 @@ extern "C" int moe_expert_forward(const moe_expert_pass* p, int steps, void* str
   RowCounts counts{p->pad_offsets, p->group_indices};
   counts.routed_rows = rows;
   uint32_t* const counters = p->gather ? nullptr : reinterpret_cast<uint32_t*>(p->counters);
-  if (steps & MOE_FWD_TAIL)
-    MOE_STEP(moe_router_tail(p->logits, const_cast<void*>(p->scores), const_cast<int64_t*>(p->expert_idx), p->num_tokens,
-                             p->num_experts, p->topk, p->softmax_before_topk, p->normalize, p->dtype, stream));
+  if (steps & MOE_FWD_TAIL) {
+    void* const scores = const_cast<void*>(p->scores);
+    int64_t* const experts = const_cast<int64_t*>(p->expert_idx);
+    if (p->own_tie_rule)
+      MOE_STEP(moe_router_topk(p->logits, scores, experts, nullptr, p->num_tokens, p->num_experts, p->topk,
+                               p->softmax_before_topk, p->normalize, p->dtype, stream));
+    else
+      MOE_STEP(moe_router_tail(p->logits, p->router_bias, scores, experts, p->num_tokens, p->num_experts, p->topk,
+                               p->softmax_before_topk, p->normalize, p->logits_dtype, p->dtype, stream));
+  }
   if (steps & MOE_FWD_ROUTE)
     MOE_STEP(routing_metadata(p->expert_idx, rows, p->num_experts, p->group_indices, nullptr, p->pad_offsets, p->row_src,
                               p->dst_row, p->mtile_expert, p->tile_pairs, p->num_mtiles, p->status, p->workspace,

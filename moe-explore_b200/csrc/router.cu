@@ -187,10 +187,12 @@ __device__ __forceinline__ uint32_t order_key(float f) {
   return f != f ? 0xFFFFFFFFu : u ^ ((u >> 31) ? 0xFFFFFFFFu : 0x80000000u);
 }
 
-template <typename T, int PER_LANE>
+//   * With `bias` the selection is by probability + bias and the scores are the probabilities (the ERNIE router); its sum is
+//     held at 1e-12 or above (normalize 2).
+template <typename T, typename S, int PER_LANE>
 __global__ void __launch_bounds__(kRouterWarps * 32)
-router_tail_kernel(const T* __restrict__ logits, T* __restrict__ scores, int64_t* __restrict__ indices, int64_t num_tokens, int E,
-                   int topk, int softmax_before, int normalize) {
+router_tail_kernel(const T* __restrict__ logits, const float* __restrict__ bias, S* __restrict__ scores, int64_t* __restrict__ indices,
+                   int64_t num_tokens, int E, int topk, int softmax_before, int normalize) {
   __shared__ float sh_val[kRouterWarps][32];
   __shared__ int sh_idx[kRouterWarps][32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -225,7 +227,10 @@ router_tail_kernel(const T* __restrict__ logits, T* __restrict__ scores, int64_t
   }
   uint32_t key[PER_LANE];  // 0: no expert (every expert's key is larger)
 #pragma unroll
-  for (int i = 0; i < PER_LANE; ++i) key[i] = i * 32 + lane < E ? order_key(v[i]) : 0u;
+  for (int i = 0; i < PER_LANE; ++i) {
+    const int e = i * 32 + lane;
+    key[i] = e < E ? order_key(bias != nullptr ? v[i] + bias[e] : v[i]) : 0u;
+  }
   uint32_t kth = 0;
   for (int left = topk, first = 1; left > 0; first = 0) {
     uint32_t best = 0;
@@ -271,22 +276,23 @@ router_tail_kernel(const T* __restrict__ logits, T* __restrict__ scores, int64_t
     float sum = mine ? s : 0.0f;
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, off);
+    if (normalize == 2) sum = sum < 1e-12f ? 1e-12f : sum;
     s = s / sum;
   }
   if (mine) {
-    store_score<T>(scores + t * topk + lane, s);
+    store_score<S>(scores + t * topk + lane, s);
     indices[t * topk + lane] = sh_idx[warp][lane];
   }
 }
 
-template <typename T>
-static int launch_router_tail(const void* logits, void* scores, int64_t* indices, int64_t num_tokens, int E, int topk,
-                              int softmax_before, int normalize, cudaStream_t s) {
+template <typename T, typename S>
+static int launch_router_tail(const void* logits, const float* bias, void* scores, int64_t* indices, int64_t num_tokens, int E,
+                              int topk, int softmax_before, int normalize, cudaStream_t s) {
   const int blocks = static_cast<int>((num_tokens + kRouterWarps - 1) / kRouterWarps);
   const T* l = static_cast<const T*>(logits);
-  T* sc = static_cast<T*>(scores);
+  S* sc = static_cast<S*>(scores);
 #define MOE_TAIL(PL) \
-  router_tail_kernel<T, PL><<<blocks, kRouterWarps * 32, 0, s>>>(l, sc, indices, num_tokens, E, topk, softmax_before, normalize)
+  router_tail_kernel<T, S, PL><<<blocks, kRouterWarps * 32, 0, s>>>(l, bias, sc, indices, num_tokens, E, topk, softmax_before, normalize)
   if (E <= 32) MOE_TAIL(1);
   else if (E <= 64) MOE_TAIL(2);
   else if (E <= 128) MOE_TAIL(4);
@@ -300,8 +306,9 @@ static int launch_router_tail(const void* logits, void* scores, int64_t* indices
 
 }  // namespace moe
 
-extern "C" int moe_router_tail(const void* logits, void* scores, int64_t* indices, int64_t num_tokens, int num_experts, int topk,
-                               int softmax_before_topk, int normalize, int dtype, void* stream) {
+extern "C" int moe_router_tail(const void* logits, const float* bias, void* scores, int64_t* indices, int64_t num_tokens,
+                               int num_experts, int topk, int softmax_before_topk, int normalize, int dtype, int scores_dtype,
+                               void* stream) {
   MOE_CHECK_ARG(num_tokens >= 0 && num_experts > 0 && topk > 0, "moe_router_tail: bad sizes T=%lld E=%d k=%d",
                 (long long)num_tokens, num_experts, topk);
   if (num_experts > 32 * kRouterMaxPerLane || topk > 32 || topk > num_experts || num_tokens > (1ll << 33)) {
@@ -311,13 +318,17 @@ extern "C" int moe_router_tail(const void* logits, void* scores, int64_t* indice
   if (num_tokens == 0) return MOE_OK;
   MOE_CHECK_ARG(logits && scores && indices, "moe_router_tail: null pointer argument");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (dtype == MOE_DTYPE_BF16)
-    return launch_router_tail<__nv_bfloat16>(logits, scores, indices, num_tokens, num_experts, topk, softmax_before_topk, normalize, s);
-  if (dtype == MOE_DTYPE_F16)
-    return launch_router_tail<__half>(logits, scores, indices, num_tokens, num_experts, topk, softmax_before_topk, normalize, s);
-  if (dtype == MOE_DTYPE_F32)
-    return launch_router_tail<float>(logits, scores, indices, num_tokens, num_experts, topk, softmax_before_topk, normalize, s);
-  set_error("moe_router_tail: unknown dtype %d", dtype);
+#define MOE_TAIL_TYPES(CODE, T, SCODE, S)                                                                              \
+  if (dtype == CODE && scores_dtype == SCODE)                                                                          \
+    return launch_router_tail<T, S>(logits, bias, scores, indices, num_tokens, num_experts, topk, softmax_before_topk, \
+                                    normalize, s);
+  MOE_TAIL_TYPES(MOE_DTYPE_BF16, __nv_bfloat16, MOE_DTYPE_BF16, __nv_bfloat16)
+  MOE_TAIL_TYPES(MOE_DTYPE_F16, __half, MOE_DTYPE_F16, __half)
+  MOE_TAIL_TYPES(MOE_DTYPE_F32, float, MOE_DTYPE_F32, float)
+  MOE_TAIL_TYPES(MOE_DTYPE_F32, float, MOE_DTYPE_BF16, __nv_bfloat16)
+  MOE_TAIL_TYPES(MOE_DTYPE_F32, float, MOE_DTYPE_F16, __half)
+#undef MOE_TAIL_TYPES
+  set_error("moe_router_tail: dtypes %d, %d", dtype, scores_dtype);
   return MOE_ERR_INVALID;
 }
 

@@ -47,7 +47,8 @@ class ExpertPass(ctypes.Structure):
                [("workspace_bytes", c_size_t)] + \
                [(f, c_void_p) for f in ("xs", "pre_act", "hidden", "ys", "out", "grad_out", "gs", "d_scores", "d_pre", "dxs", "dx",
                                         "d_w1", "d_w2", "addend", "logits", "router_w", "dl", "dlogits", "router_t")] + \
-               [(f, c_int32) for f in ("softmax_before_topk", "normalize")] + [("counters", c_void_p)]
+               [(f, c_int32) for f in ("softmax_before_topk", "normalize")] + [("counters", c_void_p)] + \
+               [("router_bias", c_void_p), ("logits_dtype", c_int32), ("own_tie_rule", c_int32)]
 
 
 class RowsPass(ctypes.Structure):
@@ -76,7 +77,7 @@ SIGNATURES = {
     "moe_routing_metadata_static": (c_int, [c_void_p, c_int64, c_int] + [c_void_p] * 9 + [c_void_p]),
     "moe_layout_from_groups": (c_int, [c_void_p, c_int64, c_int] + [c_void_p] * 7 + [c_void_p]),
     "moe_router_topk": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int, c_int, c_int, c_int, c_void_p]),
-    "moe_router_tail": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int, c_int, c_int, c_int, c_void_p]),
+    "moe_router_tail": (c_int, [c_void_p] * 4 + [c_int64, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p]),
     "moe_store_to_host": (c_int, [c_void_p, c_void_p, c_size_t, c_void_p]),
     "moe_copy_blocks": (c_int, [POINTER(c_void_p), POINTER(c_void_p), POINTER(c_size_t), c_int, c_void_p]),
     "moe_zero_padding_rows": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int, c_void_p]),
@@ -350,15 +351,21 @@ def router_topk(logits, topk: int, softmax_before_topk: bool, normalize: bool, w
 ROUTER_TAIL_EXPERTS, ROUTER_TAIL_TOPK = 1024, 32
 
 
-def router_tail(logits, topk: int, softmax_before_topk: bool, normalize: bool):
-    """Scores [T, k] in the logits' type and indices int64 [T, k] as torch's launches leave them (see moe_router_tail)."""
+def float_code(dtype: torch.dtype) -> int:
+    """``dtype_code``, fp32 included (the router's kernels)."""
+    return 2 if dtype is torch.float32 else dtype_code(dtype)
+
+
+def router_tail(logits, topk: int, softmax_before_topk: bool, normalize: int, bias=None, dtype=None):
+    """Scores [T, k] in ``dtype`` (the logits') and indices int64 [T, k] as torch's launches leave them (see moe_router_tail)."""
     T, E = logits.shape
-    scores = torch.empty(T, topk, dtype=logits.dtype, device=logits.device)
+    dtype = logits.dtype if dtype is None else dtype
+    scores = torch.empty(T, topk, dtype=dtype, device=logits.device)
     indices = torch.empty(T, topk, dtype=torch.int64, device=logits.device)
     with timed("router:topk"):
-        rc = load().moe_router_tail(logits.data_ptr(), scores.data_ptr(), indices.data_ptr(), T, E, topk,
-                                    1 if softmax_before_topk else 0, 1 if normalize else 0,
-                                    2 if logits.dtype is torch.float32 else dtype_code(logits.dtype), _stream())
+        rc = load().moe_router_tail(logits.data_ptr(), _ptr(bias), scores.data_ptr(), indices.data_ptr(), T, E, topk,
+                                    1 if softmax_before_topk else 0, int(normalize), float_code(logits.dtype), float_code(dtype),
+                                    _stream())
     _check("moe_router_tail", rc)
     _count(1)
     return scores, indices

@@ -19,8 +19,8 @@ import torch
 
 from moe_explore import _native
 from moe_explore.functional.activation import is_glu
-from moe_explore.params import TopkRouterParams
-from moe_explore.router import nothing_watches, tail_in_one_kernel, topk_of_logits
+from moe_explore.params import ErnieRouterParams, TopkRouterParams
+from moe_explore.router import ernie_router, fused_topk_of_logits, nothing_watches, tail_in_one_kernel, topk_of_logits
 from moe_explore.routing_plan import RoutingPlan, device_status, packed_layout
 
 
@@ -76,8 +76,9 @@ def _addresses(sizes, tensors):
 
 def _forward(x, scores, weight1, weight2, routing, act, gather_in_gemm: bool, fused_combine: bool, needs_grad: bool, addend=None,
              tail=None):
-    """-> (out, _Pass, tensors to save).  ``tail`` = (logits, softmax before top-k, normalize): scores and expert indices are the
-    router's tail of these logits, taken as part of the pass (``scores`` and the indices of ``routing`` are then None)."""
+    """-> (out, _Pass, tensors to save).  ``tail`` = (logits, softmax before top-k, normalize, bias or None, fused router's tie rule):
+    scores and expert indices are the router's tail of these logits, taken as part of the pass (``scores`` and the indices of
+    ``routing`` are then None)."""
     _native.require_cuda(x, weight1, weight2)
     assert x.dim() == 2 and weight1.dim() == 3 and weight2.dim() == 3
     T, d = x.shape
@@ -97,7 +98,7 @@ def _forward(x, scores, weight1, weight2, routing, act, gather_in_gemm: bool, fu
             flat = indices.reshape(-1).contiguous()
             assert flat.numel() == T * topk
         else:
-            assert tail[0].shape == (T, E) and tail[0].dtype is x.dtype and tail[0].is_contiguous()
+            assert tail[0].shape == (T, E) and tail[0].is_contiguous()
     x = x.contiguous()
     if tail is None:
         _native.require_cuda(scores)
@@ -152,7 +153,8 @@ def _forward(x, scores, weight1, weight2, routing, act, gather_in_gemm: bool, fu
         0 if workspace is None else workspace.numel(), xs, pre_act, hidden, ys, out.data_ptr())
     p.addend, p.counters = ptr(addend), counters
     if tail is not None:
-        p.logits, p.softmax_before_topk, p.normalize = tail[0].data_ptr(), bool(tail[1]), bool(tail[2])
+        p.logits, p.softmax_before_topk, p.normalize, p.router_bias = tail[0].data_ptr(), bool(tail[1]), int(tail[2]), ptr(tail[3])
+        p.logits_dtype, p.own_tie_rule = _native.float_code(tail[0].dtype), tail[4]
     _native.run_pass("moe_expert_forward", p, steps, rows)
     if not needs_grad:
         return out, None, ()
@@ -240,9 +242,9 @@ class RoutedLayer(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, router_weight, weight1, weight2, router_params, num_experts: int, act: str, gather_in_gemm: bool, addend):
         logits = x @ router_weight
-        if tail_in_one_kernel(logits, router_params, x.dtype):
+        if tail_in_one_kernel(logits, router_params.topk, x.dtype):
             scores = indices = None
-            tail = (logits, router_params.softmax_before_topk, router_params.normalize_routing)
+            tail = (logits, router_params.softmax_before_topk, bool(router_params.normalize_routing), None, False)
         else:
             scores, indices = topk_of_logits(logits, router_params, x.dtype)
             indices, tail = indices.contiguous(), None
@@ -392,7 +394,7 @@ def routed_layer(x, router_params, weight1, weight2, num_experts: int, act, gath
 def router_and_experts_at_once(x, router_params, weight1, weight2, num_experts: int, topk: int, addend=None) -> bool:
     """Whether ``inference_pass`` stands for router and experts: plain 16-bit CUDA tensors and nothing that has to see the single
     steps (no gradient, no transform, no tracing, no mode)."""
-    if type(router_params) is not TopkRouterParams:
+    if type(router_params) not in (TopkRouterParams, ErnieRouterParams):
         return False
     tensors = (x, router_params.router_weight, weight1, weight2) + (() if addend is None else (addend,))
     if not all(type(t) in _PLAIN and t.is_cuda for t in tensors):
@@ -405,17 +407,27 @@ def router_and_experts_at_once(x, router_params, weight1, weight2, num_experts: 
 
 
 def inference_pass(x, router_params, weight1, weight2, num_experts: int, act, gather_in_gemm=None, fused_combine: bool = False,
-                   addend=None) -> torch.Tensor:
+                   addend=None, fused_router: bool = False) -> torch.Tensor:
     """Router and experts without gradients: one allocation besides the result and the logits, and one library call after the
     logits' GEMM."""
     if gather_in_gemm is None:
         gather_in_gemm = GATHER_IN_GEMM_DEFAULT
-    logits = x @ router_params.router_weight
-    if tail_in_one_kernel(logits, router_params, x.dtype):
-        scores = indices = None
-        tail = (logits, router_params.softmax_before_topk, router_params.normalize_routing)
+    scores = indices = tail = None
+    if type(router_params) is ErnieRouterParams:
+        assert router_params.router_weight.dtype is torch.float32
+        with torch.autocast(device_type="cuda", enabled=False):
+            logits = x.float() @ router_params.router_weight
+        if tail_in_one_kernel(logits, router_params.topk, x.dtype, router_params.bias):
+            tail = (logits, True, 2, router_params.bias, False)
+        else:
+            scores, indices = ernie_router(x, router_params)
     else:
-        scores, indices = topk_of_logits(logits, router_params, x.dtype)
-        tail = None
+        logits = x @ router_params.router_weight
+        if tail_in_one_kernel(logits, router_params.topk, x.dtype):
+            tail = (logits, router_params.softmax_before_topk, bool(router_params.normalize_routing), None, fused_router)
+        elif fused_router:
+            scores, indices = fused_topk_of_logits(logits, router_params)
+        else:
+            scores, indices = topk_of_logits(logits, router_params, x.dtype)
     return _forward(x, scores, weight1, weight2, (indices, num_experts, router_params.topk), None if act is None else str(act),
                     bool(gather_in_gemm), bool(fused_combine), False, addend, tail)[0]

@@ -53,10 +53,9 @@ def topk_moe_forward(input: torch.Tensor, params: MOEParams, autotune_mode=None,
     if not fused_router and router_joins_the_pass(input, params.router_params, params.num_experts, params.topk):
         out = routed_layer(input, params.router_params, ep.weight1, ep.weight2, params.num_experts, ep.activation,
                            gather_in_gemm=gather_in_gemm, addend=addend)
-    elif not fused_router and router_and_experts_at_once(input, params.router_params, ep.weight1, ep.weight2, params.num_experts,
-                                                         params.topk, addend):
+    elif router_and_experts_at_once(input, params.router_params, ep.weight1, ep.weight2, params.num_experts, params.topk, addend):
         out = inference_pass(input, params.router_params, ep.weight1, ep.weight2, params.num_experts, ep.activation,
-                             gather_in_gemm=gather_in_gemm, fused_combine=fused_combine, addend=addend)
+                             gather_in_gemm=gather_in_gemm, fused_combine=fused_combine, addend=addend, fused_router=fused_router)
     else:
         if fused_router and isinstance(params.router_params, TopkRouterParams):
             scores, indices = fused_topk_router(input, params.router_params)

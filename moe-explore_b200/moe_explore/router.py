@@ -36,7 +36,7 @@ def topk_router(input: torch.Tensor, router_params: TopkRouterParams):
 
 def topk_of_logits(logits: torch.Tensor, router_params: TopkRouterParams, dtype: torch.dtype):
     """Everything of ``topk_router`` after the linear layer."""
-    if tail_in_one_kernel(logits, router_params, dtype):
+    if tail_in_one_kernel(logits, router_params.topk, dtype):
         return _native.router_tail(logits, router_params.topk, bool(router_params.softmax_before_topk),
                                    bool(router_params.normalize_routing))
     if router_params.softmax_before_topk:
@@ -57,12 +57,15 @@ def nothing_watches(t: torch.Tensor) -> bool:
             and t.get_device() == torch.cuda.current_device())
 
 
-def tail_in_one_kernel(logits: torch.Tensor, p: TopkRouterParams, dtype: torch.dtype) -> bool:
-    """Plain logits in the result's type, without a gradient, that nothing watches.  (One token to 16384 x 60 experts: 2 to 8 us
-    for what takes 10 to 48 in four to six launches.)"""
-    return (type(logits) is torch.Tensor and logits.is_cuda and logits.dtype is dtype
+def tail_in_one_kernel(logits: torch.Tensor, topk, dtype: torch.dtype, bias=None) -> bool:
+    """Plain logits in the result's type (with a bias: in fp32), without a gradient, that nothing watches.  (One token to 16384 x 60
+    experts: 2 to 8 us for what takes 10 to 48 in four to six launches.)"""
+    if bias is not None and not (type(bias) in (torch.Tensor, torch.nn.Parameter) and bias.is_cuda and bias.dtype is torch.float32
+                                 and bias.dim() == 1 and bias.size(0) == logits.size(-1) and bias.is_contiguous()):
+        return False
+    return (type(logits) is torch.Tensor and logits.is_cuda and logits.dtype is (dtype if bias is None else torch.float32)
             and dtype in (torch.bfloat16, torch.float16, torch.float32) and logits.dim() == 2 and logits.size(0) > 0
-            and type(p.topk) is int and 0 < p.topk <= min(logits.size(1), _native.ROUTER_TAIL_TOPK)
+            and type(topk) is int and 0 < topk <= min(logits.size(1), _native.ROUTER_TAIL_TOPK)
             and logits.size(1) <= _native.ROUTER_TAIL_EXPERTS and logits.is_contiguous()
             and not (logits.requires_grad and torch.is_grad_enabled()) and nothing_watches(logits))
 
@@ -104,7 +107,11 @@ def fused_topk_router(input: torch.Tensor, router_params: TopkRouterParams):
     on inputs with tied logits among the selected values the indices can differ from ``topk_router``'s; without
     such ties the set of experts per token is the same and the scores agree to one rounding of the 16-bit type.
     (router.py:17-35)"""
-    logits = input @ router_params.router_weight
+    return fused_topk_of_logits(input @ router_params.router_weight, router_params)
+
+
+def fused_topk_of_logits(logits: torch.Tensor, router_params: TopkRouterParams):
+    """Everything of ``fused_topk_router`` after the linear layer."""
     return _FusedTopk.apply(logits, router_params.topk, bool(router_params.softmax_before_topk),
                             bool(router_params.normalize_routing))
 
@@ -113,7 +120,10 @@ def ernie_router(input: torch.Tensor, router_params: ErnieRouterParams):
     """All-fp32 router with a selection-only bias and clamp-normalised weights (router.py:37-54)."""
     assert router_params.router_weight.dtype is torch.float32
     with torch.autocast(device_type=input.device.type, enabled=False):
-        probs = softmax(input.float() @ router_params.router_weight)
+        logits = input.float() @ router_params.router_weight
+        if tail_in_one_kernel(logits, router_params.topk, input.dtype, router_params.bias):
+            return _native.router_tail(logits, router_params.topk, True, 2, router_params.bias, input.dtype)
+        probs = softmax(logits)
         _, indices = torch.topk(probs + router_params.bias, k=router_params.topk, dim=-1, sorted=False)
         picked = torch.gather(probs, dim=-1, index=indices)
         picked = picked / torch.clamp(picked.sum(dim=-1, keepdim=True), min=1e-12)

@@ -183,3 +183,44 @@ def test_router_tail_leaves_transforms_to_the_single_ops(native):
     with torch.no_grad():
         out, _ = topk_of_logits(logits[0].t().contiguous().t(), p, torch.float32)      # other strides: the single ops
         assert torch.equal(out, ref[0])
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("T,E,k", [(1, 8, 1), (7, 8, 8), (300, 33, 2), (1000, 64, 8), (65, 257, 9), (3, 1024, 32)])
+def test_ernie_tail_leaves_the_bits_of_the_torch_ops(T, E, k, dtype, native):
+    from moe_explore.params import ErnieRouterParams
+    from moe_explore.router import ernie_router
+
+    g = torch.Generator(device="cuda").manual_seed(T + E)
+    x = torch.randn(T, 64, generator=g, device="cuda").to(dtype)
+    if T > 6:
+        x[1] = 0          # equal probabilities everywhere
+        x[2] = float("nan")
+    w = torch.randn(64, E, generator=g, device="cuda") * 0.2
+    for bias in (0.01 * torch.randn(E, generator=g, device="cuda"), torch.zeros(E, device="cuda")):
+        p = ErnieRouterParams(w, bias, k)
+        scores, idx = ernie_router(x, p)
+        ref_s, ref_i = ernie_router(x.clone().requires_grad_(), p)     # a gradient wanted: the single ops
+        assert ref_s.requires_grad and not scores.requires_grad and scores.dtype is dtype
+        assert torch.equal(idx, ref_i)
+        assert torch.equal(scores.nan_to_num(nan=-7.0), ref_s.detach().nan_to_num(nan=-7.0))
+
+
+@pytest.mark.parametrize("kind", ["topk", "fused", "ernie"])
+def test_routers_inside_a_forward_pass(kind, native):
+    """The layer without gradients against its router and its experts one after the other."""
+    from moe_explore.expert_compute import routed_expert_compute
+    from moe_explore.functional.topk_moe import topk_moe_forward
+    from moe_explore.params import ErnieRouterParams, MLPParams, MOEParams, TopkRouterParams
+    from moe_explore.router import fused_topk_router, router
+
+    T, d, inter, E, k = 45, 136, 72, 9, 3
+    g = torch.Generator(device="cuda").manual_seed(5)
+    mk = lambda *s, std=1.0: torch.randn(*s, generator=g, device="cuda") * std
+    x, w1, w2 = mk(T, d).bfloat16(), mk(E, d, 2 * inter, std=0.1).bfloat16(), mk(E, inter, d, std=0.1).bfloat16()
+    wr = mk(d, E, std=0.1)
+    rp = ErnieRouterParams(wr, mk(E, std=0.01), k) if kind == "ernie" else TopkRouterParams(wr.bfloat16(), k, True, True)
+    with torch.no_grad():
+        out = topk_moe_forward(x, MOEParams(rp, MLPParams(w1, w2, "swiglu"), E, k), fused_router=kind == "fused")
+        scores, idx = fused_topk_router(x, rp) if kind == "fused" else router(x, rp)
+        assert torch.equal(out, routed_expert_compute(x, scores, w1, w2, idx, E, k, "swiglu"))
