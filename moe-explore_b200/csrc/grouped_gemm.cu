@@ -422,14 +422,20 @@ static int mgrouped_common(const char* name, const void* a, const void* w, void*
   // contractions, 96 rows 159 / 162, 162 / 173, 177 / 182; 128 rows 178 / 170, 180 / 180, 195 / 189; 192 rows 213 / 188, 213 / 196,
   // 229 / 218; 320 rows 301 / 277, 309 / 268, 320 / 276.  Gated backward, 128 rows 93 / 90, 90 / 85, 89 / 101; 160 rows 90 / 86,
   // 92 / 93, 90 / 91; 224 rows 97 / 94, 102 / 98, 106 / 103.
+  // Where units of two tiles would occupy less than half of the pairs, units of one tile again: 8 experts, d 256, I 512, per
+  // contraction, 300 rows 16-21 / 18-25, 600 rows 12-20 / 16-26; at three quarters of the pairs either may be ahead (28 / 26 even,
+  // 23 / 27 Zipf).
   if (x.counts.group_indices != nullptr && tile_pairs != nullptr && x.gather_row_src == nullptr && x.push_bases == nullptr &&
       options == nullptr && mean_rows_per_expert < 6 * 2 * BM) {
     args.out_tma = x.push_row == nullptr && x.combine_row_src == nullptr;
-    // about a unit per expert that has rows, and for every further UNIT rows one
-    const int64_t unit = mean_rows_per_expert > (epi == EPI_DGLU ? 160 : 112) ? 256 : 128;
+    // about a unit per expert that has rows, and for every further `unit` rows one
     const int64_t hit = x.counts.routed_rows < E ? x.counts.routed_rows : E;
-    const int64_t units = x.counts.routed_rows / unit + hit / 2 > hit ? x.counts.routed_rows / unit + hit / 2 : hit;
-    if (worth_claiming(units * ((N + 255) / 256))) args.work_counter = x.counts.work_counter;
+    const auto items = [&](int64_t unit) {
+      const int64_t units = x.counts.routed_rows / unit + hit / 2;
+      return (units > hit ? units : hit) * ((N + 255) / 256);
+    };
+    const int64_t unit = mean_rows_per_expert > (epi == EPI_DGLU ? 160 : 112) && items(256) * 4 >= sm_count() ? 256 : 128;
+    if (worth_claiming(items(unit))) args.work_counter = x.counts.work_counter;
 #define MOE_MG_T(TYPE)                                                                                                 \
   (unit == 256                                                                                                         \
        ? mgrouped_dispatch_t<TYPE, 256>(a, w, a_rows, out_rows, K, N, E, w_transposed, epi, args, dtype, lp)           \

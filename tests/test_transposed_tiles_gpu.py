@@ -13,7 +13,8 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("d,inter", [(264, 200), (128, 320), (72, 8)])    # columns past a tile, a CTA, a warp; K past a step
 @pytest.mark.parametrize("rows", [
     (1, 31, 32, 33, 63, 64, 65, 127, 128, 129, 0, 300),       # row units of one tile
-    (193, 255, 256, 257, 320, 0, 449, 129),                   # of two, with one, with a rest
+    (193, 255, 256, 257, 320, 0, 449, 129),                   # the same, too few of them for larger ones
+    (193, 255, 256, 257, 320, 0, 449, 129) * 5,               # of two, with one, with a rest
 ])
 def test_a_pass_equals_its_steps(rows, d, inter, act, dtype, native):
     """Every element is the same sum of the same products in the same order: bit for bit."""
