@@ -43,8 +43,8 @@ int sm_count();  // SM count of the current device (cached per device)
 // Chained launches.  Inside one library call that launches several kernels in a row on one stream, the kernels after the
 // first are launched with programmatic stream serialization: their launch and prologue (barriers, TMEM, descriptors)
 // overlap the tail of the kernel before, and grid_wait() holds them back until that kernel has completed and its writes are
-// visible.  Every kernel that can be launched so calls grid_wait() before its first access to global memory, so the
-// order of the stream holds for all earlier kernels too.  Thread-local and set only for the duration of such a call.
+// visible.  Every kernel that can be launched so calls grid_wait() before its first access to global memory (but
+// for what RowCounts::settled names) and before it ends, so the order of the stream holds for all earlier kernels too.  Thread-local and set only for the duration of such a call.
 bool& chained_launches();
 
 class Chain {
@@ -96,6 +96,9 @@ struct RowCounts {
   // A word that work items are claimed from (GemmArgs::work_counter), zero; null: they are dealt out.
   uint32_t* work_counter = nullptr;
   int64_t routed_rows = -1;  // with work_counter: about how many rows there are (for the choice whether to use it)
+  // The kernel that wrote the maps and counts is complete, and so is whatever wrote the weights, before a contraction that is
+  // chained to the kernel before it can begin: that kernel (or one since) lets its successor up only after its own grid_wait().
+  bool settled = false;
 };
 // Words that the first row kernel of a pass, or its layout kernel, sets to zero for the contractions after it.
 constexpr int kWorkCounters = 4;

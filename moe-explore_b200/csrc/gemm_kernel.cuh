@@ -78,6 +78,7 @@ struct GemmArgs {
   // hold a routed row exist: M-grouped kernels store nothing into the others, K-grouped kernels contract over the others' rows not
   // at all.
   const int32_t* group_indices;
+  int32_t settled;              // transposed tiles: RowCounts::settled
   int32_t short_steps;          // K-grouped: the last step may be 16 or 32 deep (ShortSteps)
   int32_t a_compact;            // M-grouped, with group_indices: A holds the routed rows without padding, expert by expert
   int32_t mtiles_bound;         // M-grouped: padded_rows / 128 as the caller sees it (checked against num_mtiles[2])
@@ -488,6 +489,7 @@ struct ItemQueue {
       const int s = i & (kQueueSlots - 1);
       if (i > 0) {
         if (!KG) {
+          if (i == 1) grid_wait();  // the counter was set to zero by a kernel before this one
           if (!__all_sync(0xFFFFFFFFu, mbar_wait(taken, (i - 1) & 1, w, DS_TIMEOUT_PRODUCER))) return;
           claim();
         }

@@ -428,6 +428,7 @@ static int mgrouped_common(const char* name, const void* a, const void* w, void*
   if (x.counts.group_indices != nullptr && tile_pairs != nullptr && x.gather_row_src == nullptr && x.push_bases == nullptr &&
       options == nullptr && mean_rows_per_expert < 6 * 2 * BM) {
     args.out_tma = x.push_row == nullptr && x.combine_row_src == nullptr;
+    args.settled = x.counts.settled ? 1 : 0;
     // about a unit per expert that has rows, and for every further `unit` rows one
     const int64_t hit = x.counts.routed_rows < E ? x.counts.routed_rows : E;
     const auto items = [&](int64_t unit) {

@@ -29,6 +29,8 @@ extern "C" int moe_expert_forward(const moe_expert_pass* p, int steps, void* str
     // One expert, weight one: no row moves and nothing is folded.  The GEMMs read x and write out where they are.
     RowCounts in{p->pad_offsets, p->group_indices}, out = in;
     in.a_rows = out.out_rows = p->num_tokens;
+    in.settled = (steps & MOE_FWD_ROUTE) == 0;
+    out.settled = in.settled || (steps & MOE_FWD_UP) != 0;  // the contraction before waited for the layout
     if (steps & MOE_FWD_ROUTE)
       MOE_STEP(moe_layout_from_groups(p->group_indices, p->num_tokens, 1, p->pad_offsets, nullptr, nullptr, p->mtile_expert,
                                       p->tile_pairs, p->num_mtiles, p->status, stream));
@@ -43,6 +45,8 @@ extern "C" int moe_expert_forward(const moe_expert_pass* p, int steps, void* str
   RowCounts counts{p->pad_offsets, p->group_indices};
   counts.routed_rows = rows;
   uint32_t* const counters = p->gather ? nullptr : reinterpret_cast<uint32_t*>(p->counters);
+  // (the dispatch waits for the routing before it lets the contraction up, and so does a contraction)
+  counts.settled = (steps & MOE_FWD_ROUTE) == 0 || ((steps & MOE_FWD_DISPATCH) != 0 && !p->gather);
   if (steps & MOE_FWD_TAIL) {
     void* const scores = const_cast<void*>(p->scores);
     int64_t* const experts = const_cast<int64_t*>(p->expert_idx);
@@ -106,6 +110,7 @@ extern "C" int moe_expert_backward(const moe_expert_pass* p, int steps, void* st
   if (p->identity) {
     RowCounts in{p->pad_offsets, p->group_indices}, out = in, right = in;
     in.a_rows = out.out_rows = right.b_rows = p->num_tokens;
+    in.settled = out.settled = true;
     if (steps & MOE_BWD_DOWN) {
       if (p->act == MOE_ACT_NONE)
         MOE_STEP(mgrouped_gemm(p->grad_out, p->w2, p->d_pre, nullptr, p->mtile_expert, p->tile_pairs, p->num_mtiles,
@@ -127,6 +132,7 @@ extern "C" int moe_expert_backward(const moe_expert_pass* p, int steps, void* st
   }
   RowCounts counts{p->pad_offsets, p->group_indices};
   counts.routed_rows = p->num_tokens * p->topk;
+  counts.settled = true;  // nothing of a backward pass writes the metadata or the weights
   uint32_t* const counters = reinterpret_cast<uint32_t*>(p->counters);
   if (steps & MOE_BWD_FOLD)
     MOE_STEP(combine_bwd_tokens(p->grad_out, p->scores, p->ys, p->dst_row, p->row_src, p->num_mtiles, p->gs, p->d_scores,

@@ -154,8 +154,8 @@ __global__ void __launch_bounds__(kRowThreads)
 dispatch_rows_kernel(const uint4* src, const int32_t* dst_row, const int32_t* row_src, const int32_t* num_mtiles, uint4* dst,
                      int64_t num_tokens, int topk, int vec_per_row, int token_blocks, bool live_blocks_only, uint32_t* work_counters,
                      uint4* clear) {
+  grid_wait();  // before the release: what comes up next reads the routing metadata at once (RowCounts::settled)
   grid_release();
-  grid_wait();
   zero_counters(work_counters);
   dispatch_tokens<TPR>(src, dst_row, row_src, num_mtiles, dst, num_tokens, topk, vec_per_row, token_blocks, live_blocks_only, clear);
 }

@@ -57,3 +57,26 @@ def test_a_pass_equals_its_steps(rows, d, inter, act, dtype, native):
     for a, b in zip(got, (ref, dx, d_scores, dw1, dw2)):
         assert torch.equal(a, b)
     assert native.read_status(plan.status) == 0
+
+
+@pytest.mark.parametrize("tokens", [5, 700])     # one row unit per expert; more units than CTA pairs
+def test_operands_written_right_before_a_pass_are_the_ones_it_reads(tokens):
+    """The contractions ask for weights and row maps before the kernel before them has ended, but not before the pass begins."""
+    E, k, d, inter = 32, 4, 768, 512
+    gen = torch.Generator(device="cuda").manual_seed(tokens)
+    mk = lambda *s: torch.randn(*s, generator=gen, device="cuda").to(torch.bfloat16)
+    sets = [(mk(tokens, d), torch.rand(tokens, k, generator=gen, device="cuda").bfloat16(), mk(E, d, 2 * inter), mk(E, inter, d),
+             torch.rand(tokens, E, generator=gen, device="cuda").topk(k).indices, mk(tokens, d)) for _ in range(2)]
+
+    def run(x, scores, w1, w2, ids, grad):
+        leaves = [t.detach().requires_grad_() for t in (x, scores, w1, w2)]
+        out = routed_expert_compute(*leaves, ids, E, k, "swiglu")
+        return [out.detach()] + list(torch.autograd.grad(out, leaves, grad))
+
+    expected = [run(*s) for s in sets]
+    now = [t.clone() for t in sets[0]]
+    for i in range(20):
+        for t, new in zip(now, sets[i % 2]):
+            t.copy_(new)
+        for a, b in zip(run(*now), expected[i % 2]):
+            assert torch.equal(a, b)
