@@ -60,8 +60,9 @@ def nothing_watches(t: torch.Tensor) -> bool:
 def tail_in_one_kernel(logits: torch.Tensor, topk, dtype: torch.dtype, bias=None) -> bool:
     """Plain logits in the result's type (with a bias: in fp32), without a gradient, that nothing watches.  (One token to 16384 x 60
     experts: 2 to 8 us for what takes 10 to 48 in four to six launches.)"""
-    if bias is not None and not (type(bias) in (torch.Tensor, torch.nn.Parameter) and bias.is_cuda and bias.dtype is torch.float32
-                                 and bias.dim() == 1 and bias.size(0) == logits.size(-1) and bias.is_contiguous()):
+    if bias is not None and not (type(bias) in (torch.Tensor, torch.nn.Parameter) and bias.dtype is torch.float32
+                                 and bias.get_device() == logits.get_device() and bias.dim() == 1
+                                 and bias.size(0) == logits.size(-1) and bias.is_contiguous()):
         return False
     return (type(logits) is torch.Tensor and logits.is_cuda and logits.dtype is (dtype if bias is None else torch.float32)
             and dtype in (torch.bfloat16, torch.float16, torch.float32) and logits.dim() == 2 and logits.size(0) > 0

@@ -247,3 +247,37 @@ def test_harness_routings_and_tolerance_rule():
     H.assert_close(a, a)
     with pytest.raises(AssertionError):
         H.assert_close(a, a * 1.5)
+
+
+def test_a_bias_on_another_device_is_left_to_the_torch_ops(monkeypatch):
+    """``tail_in_one_kernel`` passes the bias on as an address: it has to lie where the logits do.  (Stand-ins: this needs two GPUs.)"""
+    import types
+
+    from moe_explore import router as R
+
+    class OnDevice:
+        is_cuda, dtype, requires_grad = True, torch.float32, False
+
+        def __init__(self, device, *shape):
+            self.device_index, self.shape = device, shape
+
+        def get_device(self):
+            return self.device_index
+
+        def dim(self):
+            return len(self.shape)
+
+        def size(self, i):
+            return self.shape[i]
+
+        def is_contiguous(self):
+            return True
+
+    shim = types.SimpleNamespace(**{n: getattr(torch, n) for n in ("float32", "float16", "bfloat16", "is_grad_enabled")},
+                                 Tensor=OnDevice, nn=types.SimpleNamespace(Parameter=OnDevice))
+    monkeypatch.setattr(R, "torch", shim)
+    monkeypatch.setattr(R, "nothing_watches", lambda *tensors: True)
+    logits = OnDevice(0, 4, 8)
+    assert R.tail_in_one_kernel(logits, 2, torch.bfloat16, OnDevice(0, 8))
+    assert not R.tail_in_one_kernel(logits, 2, torch.bfloat16, OnDevice(1, 8))
+    assert not R.tail_in_one_kernel(logits, 2, torch.bfloat16, OnDevice(-1, 8))     # on the host
