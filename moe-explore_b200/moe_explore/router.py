@@ -49,12 +49,12 @@ def topk_of_logits(logits: torch.Tensor, router_params: TopkRouterParams, dtype:
     return scores.to(dtype), indices
 
 
-def nothing_watches(t: torch.Tensor) -> bool:
-    """No transform, tracer or mode has to see the single ops on ``t``, and it lies on the current device."""
-    return (forward_ad._current_level < 0 and not torch._C._functorch.is_functorch_wrapped_tensor(t)
+def nothing_watches(*tensors: torch.Tensor) -> bool:
+    """No transform, tracer or mode has to see the single ops on these tensors, and they lie on the current device."""
+    return (forward_ad._current_level < 0 and not any(map(torch._C._functorch.is_functorch_wrapped_tensor, tensors))
             and torch._C._len_torch_dispatch_stack() == 0 and torch._C._len_torch_function_stack() == 0
             and not torch.compiler.is_compiling() and not torch.jit.is_tracing()
-            and t.get_device() == torch.cuda.current_device())
+            and all(t.get_device() == torch.cuda.current_device() for t in tensors))
 
 
 def tail_in_one_kernel(logits: torch.Tensor, topk, dtype: torch.dtype, bias=None) -> bool:
@@ -68,7 +68,8 @@ def tail_in_one_kernel(logits: torch.Tensor, topk, dtype: torch.dtype, bias=None
             and dtype in (torch.bfloat16, torch.float16, torch.float32) and logits.dim() == 2 and logits.size(0) > 0
             and type(topk) is int and 0 < topk <= min(logits.size(1), _native.ROUTER_TAIL_TOPK)
             and logits.size(1) <= _native.ROUTER_TAIL_EXPERTS and logits.is_contiguous()
-            and not (logits.requires_grad and torch.is_grad_enabled()) and nothing_watches(logits))
+            and not (logits.requires_grad and torch.is_grad_enabled())
+            and (nothing_watches(logits) if bias is None else nothing_watches(logits, bias)))
 
 
 class _FusedTopk(torch.autograd.Function):

@@ -185,6 +185,19 @@ def test_router_tail_leaves_transforms_to_the_single_ops(native):
         assert torch.equal(out, ref[0])
 
 
+def test_transforms_over_the_bias_see_the_single_ops(native):
+    from moe_explore.params import ErnieRouterParams
+    from moe_explore.router import ernie_router
+
+    x, w, biases = (torch.randn(*s, device="cuda") for s in ((5, 16), (16, 8), (3, 8)))
+    each = [ernie_router(x, ErnieRouterParams(w, b, 2)) for b in biases]
+    scores, indices = torch.func.vmap(lambda b: ernie_router(x, ErnieRouterParams(w, b, 2)))(biases)
+    assert torch.equal(scores, torch.stack([s for s, _ in each])) and torch.equal(indices, torch.stack([i for _, i in each]))
+    # the bias only selects: its gradient is zero
+    zero = torch.func.grad(lambda b: ernie_router(x, ErnieRouterParams(w, b, 2))[0].sum())(biases[0])
+    assert torch.equal(zero, torch.zeros_like(zero))
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
 @pytest.mark.parametrize("T,E,k", [(1, 8, 1), (7, 8, 8), (300, 33, 2), (1000, 64, 8), (65, 257, 9), (3, 1024, 32)])
 def test_ernie_tail_leaves_the_bits_of_the_torch_ops(T, E, k, dtype, native):
