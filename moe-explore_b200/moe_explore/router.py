@@ -50,11 +50,15 @@ def topk_of_logits(logits: torch.Tensor, router_params: TopkRouterParams, dtype:
 
 
 def nothing_watches(*tensors: torch.Tensor) -> bool:
-    """No transform, tracer or mode has to see the single ops on these tensors, and they lie on the current device."""
-    return (forward_ad._current_level < 0 and not any(map(torch._C._functorch.is_functorch_wrapped_tensor, tensors))
-            and torch._C._len_torch_dispatch_stack() == 0 and torch._C._len_torch_function_stack() == 0
-            and not torch.compiler.is_compiling() and not torch.jit.is_tracing()
-            and all(t.get_device() == torch.cuda.current_device() for t in tensors))
+    """No transform, tracer or mode has to see the single ops on these tensors, and they lie on the current device.  (Some of the
+    names are private to torch: one that is missing means that something may watch.)"""
+    try:
+        return (forward_ad._current_level < 0 and not any(map(torch._C._functorch.is_functorch_wrapped_tensor, tensors))
+                and torch._C._len_torch_dispatch_stack() == 0 and torch._C._len_torch_function_stack() == 0
+                and not torch.compiler.is_compiling() and not torch.jit.is_tracing()
+                and all(t.get_device() == torch.cuda.current_device() for t in tensors))
+    except AttributeError:
+        return False
 
 
 def tail_in_one_kernel(logits: torch.Tensor, topk, dtype: torch.dtype, bias=None) -> bool:

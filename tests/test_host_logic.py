@@ -281,3 +281,17 @@ def test_a_bias_on_another_device_is_left_to_the_torch_ops(monkeypatch):
     assert R.tail_in_one_kernel(logits, 2, torch.bfloat16, OnDevice(0, 8))
     assert not R.tail_in_one_kernel(logits, 2, torch.bfloat16, OnDevice(1, 8))
     assert not R.tail_in_one_kernel(logits, 2, torch.bfloat16, OnDevice(-1, 8))     # on the host
+
+
+@pytest.mark.parametrize("holder,name", [("torch.autograd.forward_ad", "_current_level"), ("torch._C", "_functorch"),
+                                         ("torch._C", "_len_torch_dispatch_stack"), ("torch._C", "_len_torch_function_stack")])
+def test_without_a_private_name_of_torch_something_may_watch(holder, name, monkeypatch):
+    import sys
+
+    from moe_explore import router as R
+
+    t = torch.zeros(2)
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: t.get_device())
+    assert R.nothing_watches(t)
+    monkeypatch.delattr(sys.modules[holder], name)
+    assert not R.nothing_watches(t)
