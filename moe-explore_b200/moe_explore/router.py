@@ -49,12 +49,19 @@ def topk_of_logits(logits: torch.Tensor, router_params: TopkRouterParams, dtype:
     return scores.to(dtype), indices
 
 
+def _only_default_devices() -> bool:
+    """The torch function modes in force are at most those of ``torch.set_default_device`` and ``with torch.device(...)``: they
+    choose where factory calls without a device allocate, and the calls here name theirs."""
+    return (torch._C._len_torch_function_stack() == 0
+            or all(type(m) is torch.utils._device.DeviceContext for m in torch.overrides._get_current_function_mode_stack()))
+
+
 def nothing_watches(*tensors: torch.Tensor) -> bool:
     """No transform, tracer or mode has to see the single ops on these tensors, and they lie on the current device.  (Some of the
     names are private to torch: one that is missing means that something may watch.)"""
     try:
         return (forward_ad._current_level < 0 and not any(map(torch._C._functorch.is_functorch_wrapped_tensor, tensors))
-                and torch._C._len_torch_dispatch_stack() == 0 and torch._C._len_torch_function_stack() == 0
+                and torch._C._len_torch_dispatch_stack() == 0 and _only_default_devices()
                 and not torch.compiler.is_compiling() and not torch.jit.is_tracing()
                 and all(t.get_device() == torch.cuda.current_device() for t in tensors))
     except AttributeError:

@@ -295,3 +295,26 @@ def test_without_a_private_name_of_torch_something_may_watch(holder, name, monke
     assert R.nothing_watches(t)
     monkeypatch.delattr(sys.modules[holder], name)
     assert not R.nothing_watches(t)
+
+
+def test_a_default_device_does_not_watch(monkeypatch):
+    from torch.overrides import TorchFunctionMode
+
+    from moe_explore import router as R
+
+    t = torch.zeros(2)
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: t.get_device())
+    with torch.device("cpu"):
+        assert R.nothing_watches(t)
+        with TorchFunctionMode():
+            assert not R.nothing_watches(t)
+    torch.set_default_device("meta")
+    try:
+        assert R.nothing_watches(t)
+    finally:
+        torch.set_default_device(None)
+
+    class Watching(torch.utils._device.DeviceContext):     # a mode of its own that happens to set the device too
+        pass
+    with Watching(torch.device("cpu")):
+        assert not R.nothing_watches(t)

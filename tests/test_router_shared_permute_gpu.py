@@ -237,3 +237,23 @@ def test_routers_inside_a_forward_pass(kind, native):
         out = topk_moe_forward(x, MOEParams(rp, MLPParams(w1, w2, "swiglu"), E, k), fused_router=kind == "fused")
         scores, idx = fused_topk_router(x, rp) if kind == "fused" else router(x, rp)
         assert torch.equal(out, routed_expert_compute(x, scores, w1, w2, idx, E, k, "swiglu"))
+
+
+@pytest.mark.parametrize("device", ["cuda", "cpu"])
+def test_a_default_device_leaves_a_forward_pass_as_it_is(device, native):
+    from moe_explore.functional.topk_moe import topk_moe_forward
+    from moe_explore.params import MLPParams, MOEParams, TopkRouterParams
+
+    E, d = 4, 64
+    x, wr, w1, w2 = ((torch.randn(*s, device="cuda") * 0.3).bfloat16() for s in ((9, d), (d, E), (E, d, 2 * d), (E, d, d)))
+    params = MOEParams(TopkRouterParams(wr, 2, True, True), MLPParams(w1, w2, "swiglu"), E, 2)
+    seen = []
+    real, native.run_pass = native.run_pass, lambda name, p, steps, rows: (seen.append([s[0] for s in steps]), real(name, p, steps, rows))
+    try:
+        with torch.no_grad():
+            out = topk_moe_forward(x, params)
+            with torch.device(device):
+                assert torch.equal(topk_moe_forward(x, params), out)
+    finally:
+        native.run_pass = real
+    assert seen[0] == seen[1] and native.FWD_TAIL in seen[1]
