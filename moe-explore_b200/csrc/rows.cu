@@ -713,7 +713,7 @@ int moe::dispatch_rows_only(const void* src, const int32_t* dst_row, void* dst, 
                             void* stream, uint32_t* work_counters, void* clear) {
   MOE_CHECK_ARG(num_tokens >= 0 && topk > 0, "moe_dispatch_rows_only: bad sizes");
   MOE_CHECK_ARG(src && dst_row && dst, "moe_dispatch_rows_only: null pointer argument");
-  MOE_CHECK_ARG(aligned16(src) && aligned16(dst), "moe_dispatch_rows_only: pointers must be 16-byte aligned");
+  MOE_CHECK_ARG(aligned16(src) && aligned16(dst) && aligned16(clear), "moe_dispatch_rows_only: pointers must be 16-byte aligned");
   MOE_ROW_COMMON_CHECKS("moe_dispatch_rows_only", cols, dtype);
   if (num_tokens == 0) return MOE_OK;
   launch_dispatch(src, dst_row, nullptr, nullptr, dst, num_tokens, topk, cols / 8, static_cast<cudaStream_t>(stream), false,

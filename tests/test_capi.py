@@ -101,3 +101,13 @@ def test_missing_library_fails_loudly(native, monkeypatch):
     monkeypatch.setattr(native, "LIB_PATH", "/nonexistent/libmoe_sm100.so")
     with pytest.raises(ImportError, match="no fallback"):
         native.load()
+
+
+def test_fused_fold_refuses_a_misaligned_output_before_the_dispatch_clears_it(native):
+    """The dispatch of such a pass sets the output to zero in 16-byte pieces."""
+    buf = (ctypes.c_char * 4096)()
+    base = ctypes.addressof(buf) + (-ctypes.addressof(buf)) % 16
+    p = native.ExpertPass(num_tokens=2, padded_rows=128, d=64, inter=64, num_experts=1, topk=1, fused_combine=1, x=base,
+                          dst_row=base, xs=base, out=base + 8)
+    rc = native.load().moe_expert_forward(ctypes.byref(p), native.FWD_DISPATCH, None)
+    assert rc == -1 and b"16-byte aligned" in native.load().moe_last_error()
