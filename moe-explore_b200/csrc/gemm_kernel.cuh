@@ -422,16 +422,24 @@ struct ItemWalk {
 // Work items claimed one by one instead of dealt out: with a fixed stride the slowest worker is 5 to 11 % behind the mean where
 // rows fall unevenly (simulated with the stage costs measured; claimed 1 to 5 %), and where the items are equal the SMs are not --
 // storing weight gradients, some were done after 68 us and others after 100.  The second CTA's idle MMA warp is the scheduler: it
-// claims an item with one atomic addition, decodes it and writes it into a ring of four slots in both CTAs' shared memory; the other
+// claims an item with one atomic addition, decodes it and writes it into a ring of five slots in both CTAs' shared memory; the other
 // nineteen roles read it there.  A worker's first item is its index; M-grouped workers claim the next one when the leader's producer
 // has begun the last one claimed, so that at most one unbegun item is held.  Every worker's claims end with one that
 // finds nothing left; the claim that is the last of all puts the word back to zero.
-constexpr int kQueueSlots = 4;
+// A role hands a slot back when it asks for the item after it.  Handing back goes to the other CTA, by an arrival that orders nothing
+// beyond this CTA, so what keeps the scheduler from rewriting a slot under a load is that the load's value is there: everything the
+// role did with the item (its copies, instructions and branches depend on the words it read) was issued before, and a word that
+// it does not use may be any.  Handed back right after the load, the arrival overtook it now and then: one item in a million was
+// another one.  A release at cluster scope waits for all of the warp's memory traffic instead (weight gradients of 128 tokens
+// 95 -> 155 us).
+constexpr int kQueueSlots = 5;
+constexpr int kQueueBarrierBytes = (16 * kQueueSlots + 8 + 15) / 16 * 16;
 struct ItemQueue {
   uint32_t full, empty, taken;  // barriers: [slots] in each CTA; [slots] and one in the second CTA
   uint32_t slots;               // [slots][8] words in each CTA
 
-  __device__ __forceinline__ explicit ItemQueue(uint32_t area) : full(area), empty(area + 32), taken(area + 64), slots(area + 128) {}
+  __device__ __forceinline__ explicit ItemQueue(uint32_t area)
+      : full(area), empty(area + 8 * kQueueSlots), taken(area + 16 * kQueueSlots), slots(area + kQueueBarrierBytes) {}
   __device__ __forceinline__ void init() const {  // by one thread of each CTA
     for (int s = 0; s < kQueueSlots; ++s) {
       mbar_init(full + 8 * s, 1);
@@ -439,26 +447,21 @@ struct ItemQueue {
     }
     mbar_init(taken, 1);
   }
-  // The i-th item, by all lanes of a warp of either CTA; an item that is not valid where the wait gave up (then the abort flag is set).
+  // The i-th item, by all lanes of a warp of either CTA that is done with the one before; an item that is not valid where the wait
+  // gave up (then the abort flag is set).
   template <bool KG>
   __device__ __forceinline__ TileCoord get(int i, const GemmArgs& args, bool mark_taken, const WaitCtx& w, int code) const {
-    const int s = i & (kQueueSlots - 1);
+    const int s = i % kQueueSlots;
+    if (i > 0 && (threadIdx.x & 31) == 0) mbar_arrive_cluster(mapa_shared(empty + 8 * ((i - 1) % kQueueSlots), 1));
     TileCoord c{};
     if (!__all_sync(0xFFFFFFFFu, mbar_wait(full + 8 * s, (i / kQueueSlots) & 1, w, code))) return c;
-    // Each lane reads a word and the warp exchanges them.  The exchange uses what was loaded, so no load is outstanding when the
-    // arrival on the other CTA's barrier is issued.  (An arrival alone overtook the loads now and then, the slot was rewritten
-    // under them, and one item in a million was another one.  Ordering it by a release at cluster scope instead waits for all of the
-    // warp's memory traffic: weight gradients of 128 tokens 95 -> 155 us.)
     uint32_t mine;
     asm volatile("ld.shared.b32 %0, [%1];" : "=r"(mine) : "r"(slots + 32 * s + 4 * (threadIdx.x & 7)) : "memory");
     int word[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) word[j] = static_cast<int>(__shfl_sync(0xFFFFFFFFu, mine, j));
     __syncwarp();
-    if ((threadIdx.x & 31) == 0) {
-      mbar_arrive_cluster(mapa_shared(empty + 8 * s, 1));
-      if (!KG && mark_taken) mbar_arrive_cluster(mapa_shared(taken, 1));
-    }
+    if (!KG && mark_taken && (threadIdx.x & 31) == 0) mbar_arrive_cluster(mapa_shared(taken, 1));
     c.m0 = word[0];
     c.n0 = word[1];
     c.expert = word[2];
@@ -486,7 +489,7 @@ struct ItemQueue {
     };
     int t = unit;
     for (int i = 0;; ++i) {
-      const int s = i & (kQueueSlots - 1);
+      const int s = i % kQueueSlots;
       if (i > 0) {
         if (!KG) {
           if (i == 1) grid_wait();  // the counter was set to zero by a kernel before this one
@@ -676,7 +679,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   const uint32_t epi_bar = smem_u32(bars + 2 * kStages + 4);    // [kEpilogueWarps][2]  (dGLU side-input tiles)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kStages + 4 + 2 * kEpilogueWarps);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  static_assert((2 * 8 + 4 + 2 * kEpilogueWarps) * 8 + 8 <= kQueueOffset && kQueueOffset + 128 + kQueueSlots * 32 <= Plan::kBarrierBytes,
+  static_assert((2 * 8 + 4 + 2 * kEpilogueWarps) * 8 + 8 <= kQueueOffset && kQueueOffset + kQueueBarrierBytes + kQueueSlots * 32 <= Plan::kBarrierBytes,
                 "barrier area too small");
   // items claimed at run time (K-grouped pairs): a compile-time possibility, the other kernels' loops carry none of it
   constexpr bool kQueue = KG && kPair && !GATHER;

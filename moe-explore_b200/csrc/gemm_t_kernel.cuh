@@ -136,7 +136,7 @@ grouped_gemm_kernel(const __grid_constant__ TMaps maps, const GemmArgs args) {
   const uint32_t epi_bar = smem_u32(bars + 2 * kStages + 4);     // [kEpilogueWarps][2]  (saved product tiles)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kStages + 4 + 2 * kEpilogueWarps);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  static_assert((2 * 8 + 4 + 2 * kEpilogueWarps) * 8 + 8 <= kQueueOffset && kQueueOffset + 128 + kQueueSlots * 32 <= Plan::kBarrierBytes,
+  static_assert((2 * 8 + 4 + 2 * kEpilogueWarps) * 8 + 8 <= kQueueOffset && kQueueOffset + kQueueBarrierBytes + kQueueSlots * 32 <= Plan::kBarrierBytes,
                 "barrier area too small");
   const ItemQueue queue(smem_u32(bars) + kQueueOffset);
   const bool queued = args.work_counter != nullptr;
