@@ -98,6 +98,8 @@ struct RowCounts {
   int64_t routed_rows = -1;  // with work_counter: about how many rows there are (for the choice whether to use it)
   // The kernel that wrote the maps and counts is complete, and so is whatever wrote the weights, before a contraction that is
   // chained to the kernel before it can begin: that kernel (or one since) lets its successor up only after its own grid_wait().
+  // Complete is not yet visible to every load before the contraction's own grid_wait(): it reads the maps and counts past L1
+  // (map_word in gemm_kernel.cuh), and the weights as copies, which do not go through L1.
   bool settled = false;
 };
 // Words that the first row kernel of a pass, or its layout kernel, sets to zero for the contractions after it.

@@ -147,18 +147,27 @@ struct TileCoord {
   bool valid;     // false: there is no further item
 };
 
+// A word of the row maps and counts (mtile_expert, tile_pairs, num_mtiles, pad_offsets, group_indices).  From the device's point
+// of coherence and not from L1: with RowCounts::settled they are read before this kernel's wait for the one before, which is what
+// would make an earlier kernel's writes visible to loads that may hit a line of L1.
+__device__ __forceinline__ int32_t map_word(const int32_t* p) {
+  int32_t v;
+  asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
 // K-grouped: rows of expert e to contract over, in steps of 16 (what follows an expert's last row up to the end of its 64-row
 // block is zero), at most its padded range.
 __device__ __forceinline__ int contracted_rows(const GemmArgs& args, int e, int padded) {
   if (args.group_indices == nullptr) return padded;
-  const int rows = (args.group_indices[e + 1] - args.group_indices[e] + 15) & ~15;
+  const int rows = (map_word(args.group_indices + e + 1) - map_word(args.group_indices + e) + 15) & ~15;
   return rows < padded ? (rows > 0 ? rows : 0) : padded;
 }
 
 // Rows of expert e that exist, in whole 64-row blocks, at most its padded range (whatever the prefix says).
 __device__ __forceinline__ int live_rows(const GemmArgs& args, int e, int padded) {
   if (args.group_indices == nullptr) return padded;
-  const int rows = (args.group_indices[e + 1] - args.group_indices[e] + 63) & ~63;
+  const int rows = (map_word(args.group_indices + e + 1) - map_word(args.group_indices + e) + 63) & ~63;
   return rows < padded ? (rows > 0 ? rows : 0) : padded;
 }
 
@@ -258,7 +267,7 @@ __device__ __forceinline__ int total_tiles(const GemmArgs& args, int& mt, int& n
     return args.num_experts * mt * nt;
   }
   // (the three words are asked for together: a load that follows another's result waits 0.5 to 1 us more for the first tile)
-  const int tiles = args.num_mtiles[0], pairs = args.num_mtiles[1], bound = args.num_mtiles[2];
+  const int tiles = map_word(args.num_mtiles), pairs = map_word(args.num_mtiles + 1), bound = map_word(args.num_mtiles + 2);
   mt = CTAS == 2 ? pairs : tiles;
   if (args.pair_prefix != nullptr) {
     if (bound != args.mtiles_bound) {
@@ -283,16 +292,16 @@ __device__ __forceinline__ int total_tiles(const GemmArgs& args, int& mt, int& n
         win.e0 = static_cast<int>(static_cast<long long>(args.num_experts) * args.chunk_index / args.chunk_count);
         win.e1 = static_cast<int>(static_cast<long long>(args.num_experts) * (args.chunk_index + 1) / args.chunk_count);
       }
-      p0 = args.pair_prefix[win.e0];
-      p1 = args.pair_prefix[win.e1];
+      p0 = map_word(args.pair_prefix + win.e0);
+      p1 = map_word(args.pair_prefix + win.e1);
     }
     win.p_end = p1;
     if (CTAS == 2) {
       win.m_begin = p0;
       mt = p1 - p0;
     } else {  // one-CTA kernels: the same window expressed in tiles
-      win.m_begin = p0 == 0 ? 0 : p0 < pairs ? (args.tile_pairs[p0] & 0xFFFFF) : tiles;
-      mt = (p1 < pairs ? (args.tile_pairs[p1] & 0xFFFFF) : tiles) - win.m_begin;
+      win.m_begin = p0 == 0 ? 0 : p0 < pairs ? (map_word(args.tile_pairs + p0) & 0xFFFFF) : tiles;
+      mt = (p1 < pairs ? (map_word(args.tile_pairs + p1) & 0xFFFFF) : tiles) - win.m_begin;
     }
   }
   return mt * nt;
@@ -319,10 +328,10 @@ __device__ __forceinline__ TileCoord decode_tile(int t, int mt, int nt, const Wi
     int lo = win.e0, hi = win.e1;
     while (hi - lo > 1) {
       const int mid = (lo + hi) >> 1;
-      if ((args.pair_prefix[mid] - base) * nt <= t) lo = mid; else hi = mid;
+      if ((map_word(args.pair_prefix + mid) - base) * nt <= t) lo = mid; else hi = mid;
     }
-    span_begin = args.pair_prefix[lo];
-    int span_end = args.pair_prefix[lo + 1];
+    span_begin = map_word(args.pair_prefix + lo);
+    int span_end = map_word(args.pair_prefix + lo + 1);
     // a window given as a pair range may begin or end inside this expert: walk only its part of the expert
     if (span_begin < base) span_begin = base;
     if (span_end > win.p_end) span_end = win.p_end;
@@ -344,8 +353,8 @@ __device__ __forceinline__ TileCoord decode_tile(int t, int mt, int nt, const Wi
   if (KG) {
     c.m0 = (m_idx * CTAS + rank) * BM;
     c.expert = expert;
-    c.k_row0 = args.pad_offsets[expert];
-    const int rows = contracted_rows(args, expert, args.pad_offsets[expert + 1] - c.k_row0);
+    c.k_row0 = map_word(args.pad_offsets + expert);
+    const int rows = contracted_rows(args, expert, map_word(args.pad_offsets + expert + 1) - c.k_row0);
     c.kiters = (rows + BK - 1) / BK;
     const int rest = rows & (BK - 1);
     c.k_last = rest == 0 || rest > 32 || args.short_steps == 0 ? BK : rest > 16 ? 32 : 16;
@@ -357,7 +366,7 @@ __device__ __forceinline__ TileCoord decode_tile(int t, int mt, int nt, const Wi
     c.unit_rows = BM;
     if (CTAS == 2) {
       // one load: first tile (bits 0-19), expert (bits 20-30), "has a second tile" (bit 31)
-      const uint32_t info = static_cast<uint32_t>(args.tile_pairs[m_idx]);
+      const uint32_t info = static_cast<uint32_t>(map_word(args.tile_pairs + m_idx));
       const bool second = (info >> 31) != 0;
       tile = static_cast<int>(info & 0xFFFFFu);
       c.expert = static_cast<int>((info >> 20) & 0x7FFu);
@@ -365,17 +374,17 @@ __device__ __forceinline__ TileCoord decode_tile(int t, int mt, int nt, const Wi
       c.unit_rows = second ? 2 * BM : BM;
       if (rank == 1 && second) tile += 1;  // an inactive second CTA re-reads the first tile and stores nothing
     } else {
-      c.expert = args.mtile_expert[tile];
+      c.expert = map_word(args.mtile_expert + tile);
     }
     c.m0 = tile * BM;
     c.a_row = c.m0;
     c.live = BM;
     if (args.group_indices != nullptr) {
-      const int base = args.pad_offsets[c.expert];
+      const int base = map_word(args.pad_offsets + c.expert);
       const int left = live_rows(args, c.expert, 1 << 30) - (c.m0 - base);
       c.live = left < BM ? (left > 64 ? left : 64) : BM;
       if (left < c.unit_rows) c.unit_rows = left > 64 ? left : 64;
-      if (args.a_compact) c.a_row = c.m0 - base + args.group_indices[c.expert];
+      if (args.a_compact) c.a_row = c.m0 - base + map_word(args.group_indices + c.expert);
     }
     c.k_row0 = 0;
     c.kiters = (args.k_dim + BK - 1) / BK;

@@ -80,3 +80,24 @@ def test_operands_written_right_before_a_pass_are_the_ones_it_reads(tokens):
             t.copy_(new)
         for a, b in zip(run(*now), expected[i % 2]):
             assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("tokens", [5, 700])
+def test_maps_are_the_ones_of_this_pass_and_not_of_the_one_before(tokens):
+    """Two routings in turn, out of a graph: each pass writes its row maps where the pass before had its own, and its contractions read
+    them before they wait for the kernel in front."""
+    E, k, d, inter = 32, 4, 256, 128
+    gen = torch.Generator(device="cuda").manual_seed(tokens)
+    mk = lambda *s: torch.randn(*s, generator=gen, device="cuda").to(torch.bfloat16)
+    x, scores, w1, w2 = mk(tokens, d), torch.rand(tokens, k, generator=gen, device="cuda").bfloat16(), mk(E, d, 2 * inter), mk(E, inter, d)
+    routings = [torch.rand(tokens, E, generator=gen, device="cuda").topk(k).indices for _ in range(2)]
+    with torch.no_grad():
+        expected = [routed_expert_compute(x, scores, w1, w2, ids, E, k, "swiglu") for ids in routings]
+        wrong = torch.zeros((), dtype=torch.int64, device="cuda")
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            for i in range(20):
+                wrong += torch.ne(routed_expert_compute(x, scores, w1, w2, routings[i % 2], E, k, "swiglu"), expected[i % 2]).any()
+        for _ in range(1000):
+            graph.replay()
+    assert not torch.equal(*expected) and int(wrong) == 0
