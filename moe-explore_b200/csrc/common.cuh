@@ -95,7 +95,7 @@ struct RowCounts {
   int64_t out_rows = -1;  // M-grouped plain stores, one expert
   // A word that work items are claimed from (GemmArgs::work_counter), zero; null: they are dealt out.
   uint32_t* work_counter = nullptr;
-  int64_t routed_rows = -1;  // with work_counter: about how many rows there are (for the choice whether to use it)
+  int64_t routed_rows = -1;  // M-grouped: about how many rows there are (what sizes row units and decides on claiming; required)
   // The kernel that wrote the maps and counts is complete, and so is whatever wrote the weights, before a contraction that is
   // chained to the kernel before it can begin: that kernel (or one since) lets its successor up only after its own grid_wait().
   // Complete is not yet visible to every load before the contraction's own grid_wait(): it reads the maps and counts past L1

@@ -425,17 +425,24 @@ static int mgrouped_common(const char* name, const void* a, const void* w, void*
   // Where units of two tiles would occupy less than half of the pairs, units of one tile again: 8 experts, d 256, I 512, per
   // contraction, 300 rows 16-21 / 18-25, 600 rows 12-20 / 16-26; at three quarters of the pairs either may be ahead (28 / 26 even,
   // 23 / 27 Zipf).
+  // One expert has no rare ones and its rows are known exactly: units of two tiles from 129 rows on.  d 7168, I 2048, whole passes out
+  // of a graph, one / two where the rule says so, forward and training: 300 rows 53 / 53, 158 / 154; 520 rows 77 / 69, 197 / 198; 768
+  // rows 84 / 72, 225 / 213; 1024 rows 92 / 79, 262 / 242; 1500 rows 120 / 118, 345 / 342.  d 4096, I 14336: 200 rows 122 / 106, 359 /
+  // 345; 300 rows 134 / 141, 402 / 406; 768 rows 302 / 234, 818 / 668.  d 2048, I 1408: one tile up to 768 rows, 1024 rows 35.6 / 34.4.
   if (x.counts.group_indices != nullptr && tile_pairs != nullptr && x.gather_row_src == nullptr && x.push_bases == nullptr &&
       options == nullptr && mean_rows_per_expert < 6 * 2 * BM) {
+    MOE_CHECK_ARG(x.counts.routed_rows >= 0, "%s: the number of routed rows is not set", name);
     args.out_tma = x.push_row == nullptr && x.combine_row_src == nullptr;
     args.settled = x.counts.settled ? 1 : 0;
-    // about a unit per expert that has rows, and for every further `unit` rows one
+    // about a unit per expert that has rows, and for every further `unit` rows one; with one expert the rows are known
     const int64_t hit = x.counts.routed_rows < E ? x.counts.routed_rows : E;
     const auto items = [&](int64_t unit) {
-      const int64_t units = x.counts.routed_rows / unit + hit / 2;
+      const int64_t units = E == 1 ? (x.counts.routed_rows + unit - 1) / unit : x.counts.routed_rows / unit + hit / 2;
       return (units > hit ? units : hit) * ((N + 255) / 256);
     };
-    const int64_t unit = mean_rows_per_expert > (epi == EPI_DGLU ? 160 : 112) && items(256) * 4 >= sm_count() ? 256 : 128;
+    const int64_t one_tile_rows = epi == EPI_DGLU ? 160 : E == 1 ? BM : 112;
+    const int64_t unit =
+        (E == 1 ? x.counts.routed_rows : mean_rows_per_expert) > one_tile_rows && items(256) * 4 >= sm_count() ? 256 : 128;
     if (worth_claiming(items(unit))) args.work_counter = x.counts.work_counter;
 #define MOE_MG_T(TYPE)                                                                                                 \
   (unit == 256                                                                                                         \

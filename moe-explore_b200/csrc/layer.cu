@@ -27,7 +27,9 @@ extern "C" int moe_expert_forward(const moe_expert_pass* p, int steps, void* str
   const Chain chain;
   if (p->identity) {
     // One expert, weight one: no row moves and nothing is folded.  The GEMMs read x and write out where they are.
-    RowCounts in{p->pad_offsets, p->group_indices}, out = in;
+    RowCounts in{p->pad_offsets, p->group_indices};
+    in.routed_rows = p->num_tokens;
+    RowCounts out = in;
     in.a_rows = out.out_rows = p->num_tokens;
     in.settled = (steps & MOE_FWD_ROUTE) == 0;
     out.settled = in.settled || (steps & MOE_FWD_UP) != 0;  // the contraction before waited for the layout
@@ -108,7 +110,9 @@ extern "C" int moe_expert_backward(const moe_expert_pass* p, int steps, void* st
   const int up_cols = glu(p->act) ? 2 * p->inter : p->inter;
   const Chain chain;
   if (p->identity) {
-    RowCounts in{p->pad_offsets, p->group_indices}, out = in, right = in;
+    RowCounts in{p->pad_offsets, p->group_indices};
+    in.routed_rows = p->num_tokens;
+    RowCounts out = in, right = in;
     in.a_rows = out.out_rows = right.b_rows = p->num_tokens;
     in.settled = out.settled = true;
     if (steps & MOE_BWD_DOWN) {

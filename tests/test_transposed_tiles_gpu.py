@@ -2,7 +2,7 @@
 import pytest
 import torch
 
-from moe_explore.expert_compute import routed_expert_compute
+from moe_explore.expert_compute import dense_expert, routed_expert_compute
 from moe_explore.routing_plan import build_routing_plan
 
 pytestmark = pytest.mark.gpu
@@ -101,3 +101,37 @@ def test_maps_are_the_ones_of_this_pass_and_not_of_the_one_before(tokens):
         for _ in range(1000):
             graph.replay()
     assert not torch.equal(*expected) and int(wrong) == 0
+
+
+@pytest.mark.parametrize("act", [None, "silu", "swiglu"])
+@pytest.mark.parametrize("T,d,inter", [(2, 1800, 1800), (128, 9480, 264), (129, 9480, 264), (520, 4616, 520),
+                                       (1400, 1800, 1800)])     # one-tile and two-tile row units, with one and with several units
+def test_one_dense_expert_equals_its_steps(T, d, inter, act, native):
+    gen = torch.Generator(device="cuda").manual_seed(T)
+    mk = lambda *s, std=1.0: (torch.randn(*s, generator=gen, device="cuda") * std).bfloat16()
+    n1 = 2 * inter if act == "swiglu" else inter
+    x, w1, w2 = leaves = [t.requires_grad_() for t in (mk(T, d), mk(1, d, n1, std=0.05), mk(1, inter, d, std=0.05))]
+    grad = mk(T, d)
+    out = dense_expert(*leaves, act)
+    got = [out.detach()] + list(torch.autograd.grad(out, leaves, grad))
+    with torch.no_grad():
+        assert torch.equal(dense_expert(*leaves, act), got[0])
+        plan = build_routing_plan(torch.zeros(T, 1, dtype=torch.int64, device="cuda"), 1, 1)
+        maps = (plan.mtile_expert, plan.tile_pairs, plan.num_mtiles)
+        new = lambda n: torch.empty(plan.padded_rows, n, dtype=x.dtype, device="cuda")
+        xs, pre, hidden, ys, gs, d_pre, dxs = new(d), new(n1) if act else None, new(inter), new(d), new(d), new(n1), new(d)
+        native.gather_rows(x, plan.row_src, plan.num_mtiles, xs, 1)
+        native.gather_rows(grad, plan.row_src, plan.num_mtiles, gs, 1)
+        native.mgrouped_gemm(xs, w1, hidden, pre, *maps, False, act, plan.status)
+        native.mgrouped_gemm(hidden, w2, ys, None, *maps, False, None, plan.status)
+        if act is None:
+            native.mgrouped_gemm(gs, w2, d_pre, None, *maps, True, None, plan.status)
+        else:
+            native.mgrouped_gemm_dglu(gs, w2, pre, d_pre, *maps, act, plan.status)
+        native.mgrouped_gemm(d_pre, w1, dxs, None, *maps, True, None, plan.status)
+        dw1, dw2 = torch.empty_like(w1), torch.empty_like(w2)
+        native.kgrouped_gemm(xs, d_pre, dw1, plan.pad_offsets, plan.status)
+        native.kgrouped_gemm(hidden, gs, dw2, plan.pad_offsets, plan.status)
+    for a, b in zip(got, (ys[:T], dxs[:T], dw1, dw2)):
+        assert torch.equal(a, b)
+    assert native.read_status(plan.status) == 0
