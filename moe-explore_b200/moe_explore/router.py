@@ -59,10 +59,11 @@ def _only_default_devices() -> bool:
 def nothing_watches(*tensors: torch.Tensor) -> bool:
     """No transform, tracer or mode has to see the single ops on these tensors, and they lie on the current device.  (Some of the
     names are private to torch: one that is missing means that something may watch.)"""
+    if torch.compiler.is_compiling():   # first: the names below are not traceable, and a graph without breaks may be wanted
+        return False
     try:
         return (forward_ad._current_level < 0 and not any(map(torch._C._functorch.is_functorch_wrapped_tensor, tensors))
-                and torch._C._len_torch_dispatch_stack() == 0 and _only_default_devices()
-                and not torch.compiler.is_compiling() and not torch.jit.is_tracing()
+                and torch._C._len_torch_dispatch_stack() == 0 and _only_default_devices() and not torch.jit.is_tracing()
                 and all(t.get_device() == torch.cuda.current_device() for t in tensors))
     except AttributeError:
         return False

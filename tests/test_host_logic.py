@@ -297,6 +297,13 @@ def test_without_a_private_name_of_torch_something_may_watch(holder, name, monke
     assert not R.nothing_watches(t)
 
 
+def test_a_compiled_graph_without_breaks_sees_the_single_ops():
+    from moe_explore import router as R
+
+    graph = torch.compile(lambda t: t + 1 if R.nothing_watches(t) else t - 1, backend="eager", fullgraph=True)
+    assert torch.equal(graph(torch.zeros(2)), -torch.ones(2))
+
+
 def test_a_default_device_does_not_watch(monkeypatch):
     from torch.overrides import TorchFunctionMode
 

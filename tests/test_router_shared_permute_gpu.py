@@ -198,6 +198,16 @@ def test_transforms_over_the_bias_see_the_single_ops(native):
     assert torch.equal(zero, torch.zeros_like(zero))
 
 
+def test_the_router_compiles_into_one_graph(native):
+    from moe_explore.params import ErnieRouterParams, TopkRouterParams
+    from moe_explore.router import router
+
+    x, w, bias = (torch.randn(*s, device="cuda") for s in ((5, 16), (16, 8), (8,)))
+    for p in (TopkRouterParams(w, 2, True, True), TopkRouterParams(w, 2, False, False), ErnieRouterParams(w, bias, 2)):
+        for got, want in zip(torch.compile(lambda x: router(x, p), backend="eager", fullgraph=True)(x), router(x, p)):
+            assert torch.equal(got, want)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
 @pytest.mark.parametrize("T,E,k", [(1, 8, 1), (7, 8, 8), (300, 33, 2), (1000, 64, 8), (65, 257, 9), (3, 1024, 32)])
 def test_ernie_tail_leaves_the_bits_of_the_torch_ops(T, E, k, dtype, native):
