@@ -3,7 +3,7 @@
 // gemm_kernel.cuh puts 128 rows on the tensor core's lanes, so a tile costs 128 rows whatever the expert has, and a pair's
 // second CTA idles where an expert ends in its first tile.  Here a CTA pair covers 256 weight columns and up to 256 rows of ONE
 // expert (a row unit: a pair of row tiles, or one tile), and the extent of the instruction along the rows is chosen per work
-// item in steps of 64: per 64-deep step a CTA loads its 16 KB of weights and 2 KB per 32 of its rows.  Nothing is computed
+// item in steps of 64: per 64-deep step a CTA loads its 16 KB of weights and 4 KB per 32 of its rows.  Nothing is computed
 // for rows beyond an expert's last 64-row block, a pair never has an idle half, and the weights in flight do not shrink with
 // the rows.  Bit-identical to the other kernels (the same products in the same order).
 // Sums of a training pass's four such contractions (32 experts, d 2048, I 1024, K 1024-2048; us, gemm_kernel.cuh -> here, rows

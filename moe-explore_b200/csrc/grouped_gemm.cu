@@ -64,8 +64,9 @@ static EncodeTiledFn encode_fn() {
 }
 
 // Tensor maps depend only on (address, element type, extents, box), never on the data, so they are kept: a training
-// step encodes the same dozen maps again and again (a few microseconds each, which is what small token counts
-// are bound by).  A small table with round-robin replacement, shared by all threads.
+// step of one layer uses the same 20 to 40 maps again and again, and the host is what small token counts are bound by.  A small
+// table with round-robin replacement, shared by all threads.  (Layers that replace each other's maps in it, 16 or 32 of them in
+// turn, cost the host no more each than two do.)
 struct TmapKey {
   const void* ptr;
   int dtype;

@@ -23,8 +23,8 @@ ACT_CODES = {None: 0, "none": 0, "silu": 1, "gelu": 2, "swiglu": 3, "geglu": 4, 
 TILE_M = 128
 ROUTE_ONE_LAUNCH_ROWS = 131072   # csrc/routing.cu: up to here a whole B200 takes the routing metadata in one launch
 ROUTE_CHIP_WIDE_LAUNCHES = 4     # ... and beyond
-# codes a kernel may leave in a status word (include/moe_sm100.h, moe_check_status)
 WORK_COUNTERS = 4   # words a pass claims its work items from
+# codes a kernel may leave in a status word (include/moe_sm100.h, moe_check_status)
 STATUS_WAVE_FALLBACK = 4
 STATUS_BAD_LAYOUT = 5
 STATUS_BAD_EXPERT_ID = 100

@@ -234,9 +234,9 @@ class ExpertCompute(torch.autograd.Function):
 
 
 class RoutedLayer(torch.autograd.Function):
-    """The layer with a router whose softmax runs over the selected logits: scores and indices by the same torch ops as
-    ``topk_router`` (bit-identical selection), their backward as part of the experts' backward pass.  The gradient of such logits
-    is zero outside the selection, so the router's share of the input gradient is topk scaled rows of the transposed
+    """The layer with a router whose softmax runs over the selected logits: scores and indices with the bits of ``topk_router`` (the
+    router's tail as part of the pass, or its torch ops), their backward as part of the experts' backward pass.  The gradient of such
+    logits is zero outside the selection, so the router's share of the input gradient is topk scaled rows of the transposed
     router weight, added by the fold in fp32, instead of a dense GEMM and an addition over [T, d]."""
 
     @staticmethod
