@@ -406,8 +406,8 @@ def router_and_experts_at_once(x, router_params, weight1, weight2, num_experts: 
             and router_params.topk == topk and nothing_watches(x))
 
 
-def inference_pass(x, router_params, weight1, weight2, num_experts: int, act, gather_in_gemm=None, fused_combine: bool = False,
-                   addend=None, fused_router: bool = False) -> torch.Tensor:
+def inference_pass(x, router_params, weight1, weight2, num_experts: int, topk: int, act, gather_in_gemm=None,
+                   fused_combine: bool = False, addend=None, fused_router: bool = False) -> torch.Tensor:
     """Router and experts without gradients: one allocation besides the result and the logits, and one library call after the
     logits' GEMM."""
     if gather_in_gemm is None:
@@ -429,5 +429,6 @@ def inference_pass(x, router_params, weight1, weight2, num_experts: int, act, ga
             scores, indices = fused_topk_of_logits(logits, router_params)
         else:
             scores, indices = topk_of_logits(logits, router_params, x.dtype)
-    return _forward(x, scores, weight1, weight2, (indices, num_experts, router_params.topk), None if act is None else str(act),
+    # (topk is the layer's: the router's may be anything that torch.topk takes and that equals it)
+    return _forward(x, scores, weight1, weight2, (indices, num_experts, topk), None if act is None else str(act),
                     bool(gather_in_gemm), bool(fused_combine), False, addend, tail)[0]

@@ -54,7 +54,7 @@ def topk_moe_forward(input: torch.Tensor, params: MOEParams, autotune_mode=None,
         out = routed_layer(input, params.router_params, ep.weight1, ep.weight2, params.num_experts, ep.activation,
                            gather_in_gemm=gather_in_gemm, addend=addend)
     elif router_and_experts_at_once(input, params.router_params, ep.weight1, ep.weight2, params.num_experts, params.topk, addend):
-        out = inference_pass(input, params.router_params, ep.weight1, ep.weight2, params.num_experts, ep.activation,
+        out = inference_pass(input, params.router_params, ep.weight1, ep.weight2, params.num_experts, params.topk, ep.activation,
                              gather_in_gemm=gather_in_gemm, fused_combine=fused_combine, addend=addend, fused_router=fused_router)
     else:
         if fused_router and isinstance(params.router_params, TopkRouterParams):

@@ -1,5 +1,6 @@
 """The steps either side of the expert GEMMs: the opt-in fused router kernel, the shared-expert branch and the
 stand-alone permute API, each against torch / the oracle on the GPU."""
+import numpy as np
 import pytest
 import torch
 
@@ -196,6 +197,17 @@ def test_transforms_over_the_bias_see_the_single_ops(native):
     # the bias only selects: its gradient is zero
     zero = torch.func.grad(lambda b: ernie_router(x, ErnieRouterParams(w, b, 2))[0].sum())(biases[0])
     assert torch.equal(zero, torch.zeros_like(zero))
+
+
+@pytest.mark.parametrize("router_topk", [torch.tensor(2), np.int64(2)], ids=["tensor", "numpy"])
+def test_a_router_may_count_its_slots_in_another_type(router_topk, native):
+    from moe_explore.functional.topk_moe import topk_moe_forward
+    from moe_explore.params import MLPParams, MOEParams, TopkRouterParams
+
+    E, d = 4, 64
+    x, wr, w1, w2 = ((torch.randn(*s, device="cuda") * 0.3).bfloat16() for s in ((9, d), (d, E), (E, d, 2 * d), (E, d, d)))
+    out = [topk_moe_forward(x, MOEParams(TopkRouterParams(wr, k, True, False), MLPParams(w1, w2, "swiglu"), E, 2)) for k in (2, router_topk)]
+    assert torch.equal(*out)
 
 
 def test_the_router_compiles_into_one_graph(native):
